@@ -100,6 +100,27 @@ def test_softmax_fully_masked_row_is_zero(et):
     assert (host(S) == 0).all()
 
 
+@pytest.mark.parametrize("L", [1, 7, 241, 242, 243, 499, 1017, 1019, 2034, 2035])
+@pytest.mark.parametrize("offset", [0, 3])
+def test_softmax_mask_rows_of_any_alignment(et, orc, L, offset):
+    """Lengths that are no multiple of 8 (both sides of each granule count per lane, and of the three-pass kernel), in a
+    buffer that starts anywhere: rows share 16-byte granules with their neighbours, which must stay untouched."""
+    nmat = 3
+    S = (util.rng(L).standard_normal((nmat, L, L)) * 3).astype(np.float16)
+    mask = util.rng(L + 1).standard_normal((L, L)).astype(np.float16)
+    valid = max(1, L - L // 5)
+    buf = torch.full((nmat * L * L + 16,), 7.0, dtype=torch.float16, device="cuda")
+    buf[offset:offset + nmat * L * L] = dev(S).reshape(-1)
+    mbuf = torch.zeros(L * L + 8, dtype=torch.float16, device="cuda")
+    mbuf[offset:offset + L * L] = dev(mask).reshape(-1)
+    view = buf[offset:offset + nmat * L * L].view(nmat, L, L)
+    et.softmax_mask(view, mbuf[offset:offset + L * L].view(L, L), valid)
+    torch.cuda.synchronize()
+    util.assert_close(host(view), orc.softmax_mask(S, mask, valid), what=f"softmax L={L} offset={offset}")
+    assert (host(view)[:, :, valid:] == 0).all()
+    assert (buf[:offset] == 7).all() and (buf[offset + nmat * L * L:] == 7).all()
+
+
 # ------------------------------------------------------------------ tile-pruned linear
 def _run_tile(et, orc, T, K, N, sparsity, seed, gelu=False, bernoulli=True, bias_std=0.05, size=None):
     rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, seed, bernoulli, bias_std)

@@ -8,16 +8,18 @@ namespace et {
 // General form. Q/K share q_pitch; scores != null replaces Q K^T by precomputed, already scaled
 // scores [batch][nhead][L][L] (equal-length sequences only). cu_seqlens (device, batch+1 ints) or, when
 // null, `batch` sequences of uniform_len tokens each. valid_lens (device) limits the keys per sequence.
-// max_len: the longest sequence of the batch when the caller knows it (0 = unknown); it only selects the kernel.
+// max_len: the longest sequence of the batch when the caller knows it (0 = unknown), v_cols: the columns of a compact V
+// when its row pitch is known to lie inside the allocation (0 = unknown); both only select the kernel.
 int attention_launch(half* Z, const half* Q, const half* K, const half* V, const half* scores,
                      int q_pitch, int v_pitch, const int* qk_head_ptr, const int* v_col_id,
                      const int* v_head_ptr, const half* mask, int mask_ld, const int* cu_seqlens,
                      const int* valid_lens, int batch, int uniform_len, int total_tokens, int d_model,
-                     int nhead, cudaStream_t st, int max_len = 0);
-// tcgen05 fast path (dense, head_dim 64, longest sequence known); ET_ERR_UNSUPPORTED outside its range.
-int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch,
-                        const half* mask, int mask_ld, const int* cu_seqlens, const int* valid_lens, int batch,
-                        int uniform_len, int total_tokens, int max_len, int d_model, int nhead, cudaStream_t st);
+                     int nhead, cudaStream_t st, int max_len = 0, int v_cols = 0);
+// tcgen05 path (head_dim 64, dense or column-pruned V, longest sequence known); ET_ERR_UNSUPPORTED outside its range.
+int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch, int v_cols,
+                        const int* v_head_ptr, const int* v_col_id, const half* mask, int mask_ld, const int* cu_seqlens,
+                        const int* valid_lens, int batch, int uniform_len, int total_tokens, int max_len, int d_model,
+                        int nhead, cudaStream_t st);
 // Reads and clears the current device's error word of the tcgen05 kernel's bounded waits (synchronises).
 int attention_tc_error(int* code);
 // One-time per-device set-up of that error word (no allocation); safe to call repeatedly.

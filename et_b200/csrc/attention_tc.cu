@@ -1,27 +1,35 @@
-// On-the-fly attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA) for the dense case with
-// head_dim 64: the fast path behind et_attention_otf /
-// et_attention_batch (the mma.sync kernel in attention.cu covers every other variant).
-// Replaces kernels/attention.cu:51-134 of the reference for that case.
+// On-the-fly attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA) for heads of 64, dense or with a compact,
+// column-pruned V: the path behind et_attention_otf / et_attention_batch / et_attention_prune and the encoder layers (the
+// mma.sync kernel in attention.cu covers the remaining variants).
+// Replaces kernels/attention.cu:51-134 and :149-271 of the reference for those cases.
 //
-// A CTA owns 128 queries of one head of one sequence, one TMEM lane and one thread per query:
-//   S_j = Q K_j^T      SS UMMA 128x64x16 (x4), Q and the 64-key block K_j in shared memory (TMA, 128-byte
-//                      swizzle), S_j accumulated in fp16 (as the reference's kernels accumulate their scores) in 64
-//                      TMEM columns
-//   softmax            four warps, one thread per query row, one pass per block: the row's 64 scores come out of
-//                      tensor memory two to a register (tcgen05.ld.pack::16b); row maximum, scale and reference point
-//                      (log2 domain) and the exponentials in packed fp16 arithmetic, no conversion; additive mask
-//                      and key validity in fp32 where a block needs them; if the maximum has grown by more than 2^8
-//                      the reference point moves and O is rescaled in place; P_j = 2^(s - reference) as packed fp16
-//                      over the first 32 score columns (tcgen05.st), row sum in fp32. No exchange between threads,
-//                      no second pass
-//   O += P_j V_j       TS UMMA 128x64x16 (x4): A = P_j read from tensor memory, B = V_j in shared memory as loaded
-//                      (rows = keys), used as an MN-major operand; Q K_{j+1}^T is issued right behind it into the
-//                      columns that hold P_j (tcgen05 operations execute in issue order)
-//   epilogue           O / row sum -> fp16 -> global, rows beyond the sequence are not written
-// The S x S matrix never leaves the SM. K_j / V_j stream through a two-stage ring. A CTA needs 48 KB of shared
-// memory, 128 TMEM columns and 160 threads, so four CTAs share an SM: while one CTA's softmax runs, the UMMAs,
-// loads and hand-overs of the other three are in flight. Every mbarrier wait is bounded; a wait that gives up
-// sets the error word and the CTA leaves through the common exit, freeing its tensor memory.
+// A work item is 128 queries of one head of one sequence; a block is 128 keys of it:
+//   S = Q K^T        SS UMMAs 128x128x16 (x4), Q and K_j in shared memory (TMA, 128-byte swizzle), fp32 in 128 TMEM columns
+//   softmax          eight warps, two threads per query row: a thread takes its 64 scores into registers in one go, which
+//                    frees the score columns at once: Q K^T of the NEXT block (of the next item, at the end of one) runs
+//                    while this block's exponentials are taken. Reference point and sum in fp32 (log2 domain); if the
+//                    maximum has grown by more than 2^8 the reference point moves and O is rescaled in place.
+//                    P = 2^(s - reference) as packed fp16 in 64 TMEM columns of its own.
+//   O += P V         TS UMMAs 128x64x16 (x8): A = P from tensor memory, B = V_j as loaded (rows = keys, MN-major)
+//   epilogue         O / row sum -> fp16 -> global, rows beyond the sequence are not written
+// Blocks that hold at most 64 keys take half of everything.
+//
+// What bounds it: the softmax warps, at two per scheduler. The special-function unit delivers 16 results per clock and SM
+// whatever the format (measured: ex2.f32 16.0, ex2.f16x2 8.0 pairs), so a 128 x 128 block costs it 1024 clocks, against 512
+// clocks of UMMAs and ~450 issue slots per warp; kPolyPairs of every 16 pairs of exponentials are evaluated on the FMA pipe
+// (Cody-Waite reduction and a cubic; 0, 2, 4, 6 of 16 measured: 84.7, 82.7, 83.6, 85.7 us at 64 x 512 tokens, 12 heads). The rest
+// of a warp's block is latency: tensor-memory load 160 clocks, maximum 340, hand-overs 600, of 2650.
+// Two CTAs share an SM (256 TMEM columns and ~100 KB of shared memory each), so that one's loads, maxima and hand-overs run
+// under the other's exponentials. The softmax warps get the registers of the other warpgroup (setmaxnreg): with 168 registers
+// and no hand-over a few values spilled, and a reload that missed the small L1 (shared memory takes the rest) cost ~300
+// clocks in the middle of a block (94 us); two threads per row and sixteen softmax warps at 96 registers: 102 us.
+// CTAs are persistent: the grid has one CTA per item, and a running CTA takes over the next one that has not started (cluster
+// launch control), so that ragged batches balance themselves and an item's loads and first Q K^T are under way while the
+// previous one is finished; its rows are written inside the next item's first block.
+// Measured against the form with 64-key blocks, fp16 scores and four CTAs per SM that it replaces (12 heads): 64 ragged
+// sequences of 32..512 tokens 71 -> 57 us, 256 x 128 tokens 47 -> 37, 32 x 256 19.8 -> 16.1, 64 x 512 87 -> 83; with an additive
+// mask (read twice there, one row per thread) 64 x 384 169 -> 117, 64 x 383 730 -> 121; scores are fp32 here.
+// Every mbarrier wait is bounded; a wait that gives up sets the error word and the CTA leaves through the common exit.
 #include <mutex>
 #include "attention.h"
 #include "common.h"
@@ -32,49 +40,63 @@ namespace et {
 
 namespace {
 
-// 64 keys per block and one thread per query row, four CTAs per SM. Measured at 256 x 512 tokens, 16 heads, with fp32
-// scores: 731 us; 128 keys and two CTAs per SM 812 us; two threads per row and three CTAs per SM 801 us; the earlier
-// two-pass form with 128 keys, two threads per row and two CTAs per SM 767 us. Sixteen resident softmax warps with
-// the shortest hand-overs between them win. With fp16 scores (below) 597 us.
-constexpr int kBQ = 128, kBK = 64, kHD = 64;
-constexpr int kNCh = kBK / 32;            // 32-column chunks of a score row
-// The kernel is a template on how Q K^T is accumulated. fp16, as the reference's kernels do (kernels/attention.cu:82:
-// c_t<half>), is the default: the scores come out of tensor memory already packed two to a register, the common pass
-// needs no fp32 -> fp16 conversion and half the registers. Its error grows with the size of the scores (one fp16
-// rounding of each 16-term partial sum): against exact arithmetic 2e-3 in the worst element for |q.k| up to 50, 1.4e-2
-// up to 165, 3e-2 up to 390. fp32 (attention_tc_set_scores_fp32) keeps 2e-3 throughout and takes ~1.5 times as long.
-constexpr int kTile = kBQ * kHD * 2;      // 16 KB: the 128 x 64 fp16 Q tile
-constexpr int kKVTile = kBK * kHD * 2;    // one key block of K or V
+constexpr int kBQ = 128, kBK = 128, kHD = 64;
+constexpr int kTile = kBQ * kHD * 2;      // 16 KB: a Q tile, a key block of K or of V
 constexpr int kSoftmaxWarps = 4;          // one thread per query row
-constexpr int kThreads = 32 * (kSoftmaxWarps + 1);   // + 1 warp whose lane 0 issues TMA and UMMA
-constexpr int kCtasPerSm = 4;
-constexpr int kTmemCols = 128;            // S 64 (P overlays its first 32 columns) | O 64: four CTAs share an SM's tensor memory
-constexpr uint32_t kPCol = 0, kOCol = kBK;
+constexpr int kThreads = 256;             // + a warp that requests the loads and hands out items, one that issues UMMAs, two idle
+// A thread of the softmax warps holds 128 scores. Registers are handed over between the two warpgroups: 256 threads start
+// with 128 each, 8 x 128 = 4 x 216 + 4 x 40.
+constexpr int kSoftmaxRegs = 216, kOtherRegs = 40;
+constexpr int kCtasPerSm = 2;
+constexpr int kTmemCols = 256;            // S 128 | P 64 | O 64
+constexpr uint32_t kSCol = 0, kPCol = 128, kOCol = 192;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleStep = 8.f;       // log2 units by which a row maximum must grow before O is rescaled
+constexpr int kItemRing = 4;
+constexpr int kMaskPitch = 272;           // bytes: seventeen 16-byte granules hold 128 mask values at any alignment; conflict-free
+constexpr int kMaskBytes = kSoftmaxWarps * 32 * kMaskPitch;
+constexpr int kScatterPitch = 136;        // bytes per staged output row (64 halfs + 8 bytes against bank conflicts)
+constexpr int kScatterBytes = kBQ * kScatterPitch;
+constexpr int kPolyPairs = 2;             // of 16 pairs of exponentials, how many go to the FMA pipe
 
 struct TcParams {
     half* Z;
     const half* mask;
     const int* cu_seqlens;
     const int* valid_lens;
+    const int* v_head_ptr;
+    const int* v_col_id;
     int z_pitch, mask_ld, batch, uniform_len;
     float scale_log2;
     int* err;
-    long long* prof;   // ET_ATTN_PROFILE builds: clock64 stamps of CTA (0,0)
 };
 
-#ifdef ET_ATTN_PROFILE
-#define AT_STAMP(slot) do { if (p.prof && blockIdx.x == 0 && blockIdx.y == 0) p.prof[(slot)] = clock64(); } while (0)
-#else
-#define AT_STAMP(slot) do { } while (0)
-#endif
+// A work item as the loading warp hands it to the others.
+struct Item {
+    int tok0, q0, len, valid, head;
+    int nkb;               // key blocks; < 0: no more items
+    int v_x, v_off, v_n, v_base;   // pruned V: first column of the copied box, of the head's window in it, width, index of its first column id
+    int v_add;             // second part of a wide window: only its own columns are written
+};
+
+template <bool kMask, bool kPruneV>
+struct Cfg {
+    static constexpr int kQS = (kMask || kPruneV) ? 1 : 2;
+    static constexpr int kKS = 2;
+    static constexpr int kVS = (kMask || kPruneV) ? 1 : 2;
+    static constexpr int kMaskAt = (kQS + kKS + kVS) * kTile;
+    static constexpr int kScatterAt = kMaskAt + (kMask ? kMaskBytes : 0);
+    static constexpr int kBytes = kScatterAt + (kPruneV ? kScatterBytes : 0);
+};
 
 struct TcShared {
-    uint64_t q_full, k_full[2], v_full[2];   // K/V blocks stream through a two-stage ring
-    uint64_t s_ready, p_ready, pv_done, o_done;
+    uint4 clc;                            // answer of the cluster launch control
+    uint64_t clc_full;
+    uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2];
+    uint64_t s_full, s_free, p_full, pv_done;
+    uint64_t item_full[kItemRing], item_empty[kItemRing];
+    Item item[kItemRing];
     uint32_t tmem_base;
-    int seq[3];
     volatile int abort;
 };
 
@@ -90,437 +112,647 @@ __device__ __forceinline__ float ex2_fast(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 2^x for two fp16 values at once (one special-function op); P is stored in fp16 anyway.
-__device__ __forceinline__ uint32_t ex2_h2(uint32_t x) {
-    uint32_t y;
-    asm("ex2.approx.f16x2 %0, %1;" : "=r"(y) : "r"(x));
-    return y;
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
 }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
 }
-
-// Sum of 32 packed fp16 values (each <= 1): two levels of packed adds (partial sums <= 4), then fp32. The row sum
-// is thereby the sum of exactly the fp16 P values that are multiplied with V.
-__device__ __forceinline__ float sum_packed(const uint32_t (&pk)[16]) {
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const half2* h2 = reinterpret_cast<const half2*>(pk) + 4 * i;
-        const float2 f = __half22float2(__hadd2(__hadd2(h2[0], h2[1]), __hadd2(h2[2], h2[3])));
-        s += f.x + f.y;
-    }
-    return s;
+// Two fp32 operations per instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n.reg .b64 x, y, z, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmov.b64 z, {%6, %7};\n"
+        "fma.rn.f32x2 w, x, y, z;\nmov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n.reg .b64 x, y, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 w, x, y;\nmov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+// 2^x for two values on the FMA and ALU pipes, x <= 127: x = n + f with n the nearest whole number (adding 1.5 * 2^23 leaves
+// n in the low bits of the sum) and |f| <= 1/2; 2^f by the cubic that interpolates it at the Chebyshev nodes of [-1/2, 1/2]
+// (largest relative error 1.0e-4, below half a unit of the fp16 that the result is rounded to); n goes into the exponent.
+__device__ __forceinline__ float2 ex2_poly2(float2 x) {
+    x.x = fmaxf(x.x, -126.f);
+    x.y = fmaxf(x.y, -126.f);
+    const float2 big = make_float2(12582912.f, 12582912.f), nbig = make_float2(-12582912.f, -12582912.f);
+    const float2 t = add2(x, big);
+    const float2 n = add2(t, nbig);
+    const float2 f = add2(x, make_float2(-n.x, -n.y));
+    float2 r = fma2(f, make_float2(0.0558382832f, 0.0558382832f), make_float2(0.242639482f, 0.242639482f));
+    r = fma2(r, f, make_float2(0.693136752f, 0.693136752f));
+    r = fma2(r, f, make_float2(0.999924541f, 0.999924541f));
+    float2 y;
+    y.x = __int_as_float(__float_as_int(r.x) + (__float_as_int(t.x) << 23));
+    y.y = __int_as_float(__float_as_int(r.y) + (__float_as_int(t.y) << 23));
+    return y;
 }
 
-// 32 additive mask values of one query row (keys k0..k0+31), times log2(e); zero where there is no mask row.
-__device__ __forceinline__ void load_mask32(float (&mk)[32], const half* mrow, int k0, int limit, bool vec) {
-    if (!mrow) {
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {   // bytes < 16: the rest is zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// Asks for a CTA of the grid that has not started; the answer (16 bytes) completes `bar`. Documented as undefined after an
+// answer that there is none: the caller stops there.
+__device__ __forceinline__ void clc_try_cancel(uint4* answer, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                     smem_u32(answer)),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ bool clc_query(const uint4* answer, int& x, int& y) {
+    uint32_t ok, cx, cy;
+    asm volatile(
+        "{\n.reg .b128 h;\n.reg .pred p;\nld.shared.b128 h, [%3];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\nselp.u32 %0, 1, 0, p;\nmov.u32 %1, 0;\nmov.u32 %2, 0;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, h;\n}"
+        : "=r"(ok), "=r"(cx), "=r"(cy)
+        : "r"(smem_u32(answer))
+        : "memory");
+    x = (int)cx;
+    y = (int)cy;
+    return ok != 0;
+}
+
+// Which queries block `blk` of head `h` is (whole warp): 32 sequences per round, each lane takes one, a prefix sum of their
+// query-block counts locates the block. nkb = -1: the block lies beyond the batch (the grid of a ragged batch has slack).
+__device__ __forceinline__ Item find_item(const TcParams& p, int blk, int h, int lane) {
+    Item it;
+    it.tok0 = it.q0 = it.len = it.valid = 0;
+    it.head = h;
+    it.v_x = h * kHD; it.v_off = 0; it.v_n = kHD; it.v_base = 0; it.v_add = 0;
+    int b = -1;
+    if (p.cu_seqlens) {
+        for (int base = 0; base < p.batch && b < 0; base += 32) {
+            const int i = base + lane;
+            const int t0 = i < p.batch ? p.cu_seqlens[i] : 0;
+            const int Li = i < p.batch ? p.cu_seqlens[i + 1] - t0 : 0;
+            const int nbi = (Li + kBQ - 1) / kBQ;
+            int incl = nbi;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) mk[i] = 0.f;
-        return;
-    }
-    if (vec && k0 + 32 <= limit) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(mrow + k0) + c);
-            const half2* h2 = reinterpret_cast<const half2*>(&v);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float2 f = __half22float2(h2[i]);
-                mk[c * 8 + 2 * i] = f.x * kLog2e;
-                mk[c * 8 + 2 * i + 1] = f.y * kLog2e;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, blk < incl);
+            if (hit) {
+                const int src = __ffs(hit) - 1;
+                const int excl = __shfl_sync(0xffffffffu, incl - nbi, src);
+                b = base + src;
+                it.tok0 = __shfl_sync(0xffffffffu, t0, src);
+                it.len = __shfl_sync(0xffffffffu, Li, src);
+                it.q0 = (blk - excl) * kBQ;
+            } else {
+                blk -= __shfl_sync(0xffffffffu, incl, 31);
             }
         }
     } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) mk[i] = (k0 + i < limit) ? __half2float(__ldg(mrow + k0 + i)) * kLog2e : 0.f;
+        const int nb = (p.uniform_len + kBQ - 1) / kBQ;
+        if (blk < nb * p.batch) { b = blk / nb; it.tok0 = b * p.uniform_len; it.q0 = (blk % nb) * kBQ; it.len = p.uniform_len; }
     }
+    it.nkb = -1;
+    if (b >= 0) {
+        it.valid = p.valid_lens ? min(p.valid_lens[b], it.len) : it.len;
+        it.nkb = it.valid > 0 ? (it.valid + kBK - 1) / kBK : 0;
+    }
+    return it;
 }
 
-template <bool kScoresF16>
+template <bool kMask, bool kPruneV>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
-                                                                  const __grid_constant__ CUtensorMap tmK,
-                                                                  const __grid_constant__ CUtensorMap tmV,
-                                                                  const __grid_constant__ TcParams p) {
+                                                                            const __grid_constant__ CUtensorMap tmK,
+                                                                            const __grid_constant__ CUtensorMap tmV,
+                                                                            const __grid_constant__ TcParams p) {
+    using C = Cfg<kMask, kPruneV>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* sQ = smem;
-    uint8_t* sK = smem + kTile;          // 2 stages
-    uint8_t* sV = sK + 2 * kKVTile;      // 2 stages
-    TcShared* sh = reinterpret_cast<TcShared*>(sV + 2 * kKVTile);
+    uint8_t* const sQ = smem;
+    uint8_t* const sK = sQ + C::kQS * kTile;
+    uint8_t* const sV = sK + C::kKS * kTile;
+    TcShared* const sh = reinterpret_cast<TcShared*>(smem + C::kBytes);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.y;
-    if (tid == 0) AT_STAMP(0);
     pdl_launch_dependents();
 
-    // The warp that issues the copies sets up the barriers, finds the CTA's work item and starts the first loads
-    // (Q, K_0, V_0, K_1, V_1) before anything CTA-wide happens: they are in flight during the tensor-memory
-    // allocation and the rendezvous. Q/K/V come from DRAM, and a wave's CTAs all start together.
     if (warp == kSoftmaxWarps) {
         if (lane == 0) {
-            mbar_init(&sh->q_full, 1);
-            for (int j = 0; j < 2; ++j) { mbar_init(&sh->k_full[j], 1); mbar_init(&sh->v_full[j], 1); }
-            mbar_init(&sh->s_ready, 1);
-            mbar_init(&sh->p_ready, kSoftmaxWarps);   // one arrive per softmax warp
+            mbar_init(&sh->clc_full, 1);
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(&sh->q_full[i], 1); mbar_init(&sh->q_empty[i], 1);
+                mbar_init(&sh->k_full[i], 1); mbar_init(&sh->k_empty[i], 1);
+                mbar_init(&sh->v_full[i], 1); mbar_init(&sh->v_empty[i], 1);
+            }
+            mbar_init(&sh->s_full, 1);
+            mbar_init(&sh->s_free, kSoftmaxWarps);
+            mbar_init(&sh->p_full, kSoftmaxWarps);
             mbar_init(&sh->pv_done, 1);
-            mbar_init(&sh->o_done, 1);
+            for (int i = 0; i < kItemRing; ++i) {
+                mbar_init(&sh->item_full[i], 1);
+                mbar_init(&sh->item_empty[i], kSoftmaxWarps + 1);
+            }
             sh->abort = 0;
             fence_mbar_init();
             prefetch_tmap(&tmQ);
             prefetch_tmap(&tmK);
             prefetch_tmap(&tmV);
         }
-        pdl_wait();   // lengths and activations come from the preceding kernels
-        int b = -1, tok0 = 0, q0 = 0, len = 0;
-        if (p.cu_seqlens) {
-            // 32 sequences per round: each lane takes one, a prefix sum of their query-block counts locates the block
-            int blk = blockIdx.x;
-            for (int base = 0; base < p.batch && b < 0; base += 32) {
-                const int i = base + lane;
-                const int t0 = i < p.batch ? p.cu_seqlens[i] : 0;
-                const int Li = i < p.batch ? p.cu_seqlens[i + 1] - t0 : 0;
-                const int nbi = (Li + kBQ - 1) / kBQ;
-                int incl = nbi;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const unsigned hit = __ballot_sync(0xffffffffu, blk < incl);
-                if (hit) {
-                    const int src = __ffs(hit) - 1;
-                    const int excl = __shfl_sync(0xffffffffu, incl - nbi, src);
-                    b = base + src;
-                    tok0 = __shfl_sync(0xffffffffu, t0, src);
-                    len = __shfl_sync(0xffffffffu, Li, src);
-                    q0 = (blk - excl) * kBQ;
-                } else {
-                    blk -= __shfl_sync(0xffffffffu, incl, 31);
-                }
-            }
-        } else {
-            const int nb = (p.uniform_len + kBQ - 1) / kBQ;
-            const int blk = blockIdx.x;
-            if (blk < nb * p.batch) { b = blk / nb; tok0 = b * p.uniform_len; q0 = (blk % nb) * kBQ; len = p.uniform_len; }
-        }
-        int nvalid = 0;
-        if (b >= 0) nvalid = p.valid_lens ? min(p.valid_lens[b], len) : len;
-        if (lane == 0) {
-            sh->seq[0] = b; sh->seq[1] = tok0; sh->seq[2] = q0;
-            if (b >= 0 && nvalid > 0) {
-                mbar_expect_tx(&sh->q_full, kTile);
-                tma_load_2d(sQ, &tmQ, h * kHD, tok0 + q0, &sh->q_full);
-                mbar_expect_tx(&sh->k_full[0], kKVTile);
-                tma_load_2d(sK, &tmK, h * kHD, tok0, &sh->k_full[0]);
-                mbar_expect_tx(&sh->v_full[0], kKVTile);
-                tma_load_2d(sV, &tmV, h * kHD, tok0, &sh->v_full[0]);
-                if (nvalid > kBK) {
-                    mbar_expect_tx(&sh->k_full[1], kKVTile);
-                    tma_load_2d(sK + kKVTile, &tmK, h * kHD, tok0 + kBK, &sh->k_full[1]);
-                    mbar_expect_tx(&sh->v_full[1], kKVTile);
-                    tma_load_2d(sV + kKVTile, &tmV, h * kHD, tok0 + kBK, &sh->v_full[1]);
-                }
-            }
-        }
-        __syncwarp();
+    } else if (warp == kSoftmaxWarps + 1) {
         tmem_alloc(&sh->tmem_base, kTmemCols);
         tmem_relinquish();
-    } else {
-        pdl_wait();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
-    if (tid == 0) AT_STAMP(1);
-    const int b = sh->seq[0], tok0 = sh->seq[1], q0 = sh->seq[2];
-    int nkb = 0, L = 0, valid = 0;
-    if (b >= 0) {
-        L = p.cu_seqlens ? p.cu_seqlens[b + 1] - p.cu_seqlens[b] : p.uniform_len;
-        valid = p.valid_lens ? min(p.valid_lens[b], L) : L;
-        nkb = (valid + kBK - 1) / kBK;
-    }
-
-    if (b >= 0 && nkb > 0) {
-        if (warp == kSoftmaxWarps) {
-            // ---- the issuing warp stays converged: every lane waits on the barriers, one elected lane issues the copies
-            // and the UMMAs (tcgen05 instructions issued from a divergent branch are slower)
-            auto load_k = [&](int j) {
-                const int st = j & 1;
-                mbar_expect_tx(&sh->k_full[st], kKVTile);
-                tma_load_2d(sK + (size_t)st * kKVTile, &tmK, h * kHD, tok0 + j * kBK, &sh->k_full[st]);
-            };
-            auto load_v = [&](int j) {
-                const int st = j & 1;
-                mbar_expect_tx(&sh->v_full[st], kKVTile);
-                tma_load_2d(sV + (size_t)st * kKVTile, &tmV, h * kHD, tok0 + j * kBK, &sh->v_full[st]);
-            };
-            // (Q and the first two K/V blocks were requested before the CTA-wide set-up)
-            const uint32_t idesc_qk = make_idesc_f16(128, kBK, false, false, kScoresF16);
-            const uint32_t idesc_pv = make_idesc_f16(128, 64, false, true);   // V is an MN-major B operand
-            const uint32_t qa = smem_u32(sQ);
-            auto issue_qk = [&](int j) {   // S = Q K_j^T into the S columns
-                const uint32_t ka = smem_u32(sK + (size_t)(j & 1) * kKVTile);
+    if (warp >= kSoftmaxWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    if (warp == kSoftmaxWarps) {
+        // ---- items and loads (all lanes stay together; lane 0 issues)
+        pdl_wait();   // lengths and activations come from the preceding kernels
+        int bx = blockIdx.x, by = blockIdx.y;
+        int ni = 0, nq = 0, nk = 0, nv = 0;   // items handed out, tiles requested
+        uint32_t clc_phase = 0;
+        bool ok = true;
+        for (;;) {
+            if (lane == 0) {
+                mbar_expect_tx(&sh->clc_full, 16);
+                clc_try_cancel(&sh->clc, &sh->clc_full);
+            }
+            Item it = find_item(p, bx, by, lane);
+            int vx0 = 0, vw = 0;
+            if constexpr (kPruneV) {
+                vx0 = p.v_head_ptr[by];
+                vw = p.v_head_ptr[by + 1] - vx0;
+            }
+            for (int part = 0; part < (kPruneV ? 2 : 1) && it.nkb >= 0 && ok; ++part) {
+                if constexpr (kPruneV) {
+                    // the head's compact columns start anywhere; the copied box of 64 starts at a multiple of 8. A window
+                    // that does not fit one box is done in two passes (the second starts at a multiple of 8 and holds at most 7 columns).
+                    const int c0 = part == 0 ? 0 : kHD - (vx0 & 7);   // columns of the window done by the first pass
+                    if (part > 0 && c0 >= vw) break;
+                    it.v_x = (vx0 + c0) & ~7;
+                    it.v_off = (vx0 + c0) & 7;
+                    it.v_n = min(vw - c0, kHD - it.v_off);
+                    it.v_base = vx0 + c0;
+                    it.v_add = part;
+                }
+                const int slot = ni % kItemRing;
+                if (!(ok = mbar_wait(&sh->item_empty[slot], ((uint32_t)(ni / kItemRing) & 1u) ^ 1u))) break;
+                if (lane == 0) {
+                    sh->item[slot] = it;
+                    mbar_arrive(&sh->item_full[slot]);
+                }
+                __syncwarp();
+                ++ni;
+                if (it.nkb == 0) continue;
+                const int qs = nq % C::kQS;
+                if (!(ok = mbar_wait(&sh->q_empty[qs], ((uint32_t)(nq / C::kQS) & 1u) ^ 1u))) break;
+                if (lane == 0) {
+                    mbar_expect_tx(&sh->q_full[qs], kTile);
+                    tma_load_2d(sQ + qs * kTile, &tmQ, it.head * kHD, it.tok0 + it.q0, &sh->q_full[qs]);
+                }
+                ++nq;
+                // K_0, then K_{j+1} ahead of V_j: the next Q K^T needs its block before this one's P V does
+                for (int j = -1; j < it.nkb && ok; ++j) {
+                    if (j + 1 < it.nkb) {
+                        const int ks = nk & 1;
+                        if (!(ok = mbar_wait(&sh->k_empty[ks], ((uint32_t)(nk >> 1) & 1u) ^ 1u))) break;
+                        if (lane == 0) {
+                            mbar_expect_tx(&sh->k_full[ks], kTile);
+                            tma_load_2d(sK + ks * kTile, &tmK, it.head * kHD, it.tok0 + (j + 1) * kBK, &sh->k_full[ks]);
+                        }
+                        ++nk;
+                    }
+                    if (j >= 0) {
+                        const int vs = nv % C::kVS;
+                        if (!(ok = mbar_wait(&sh->v_empty[vs], ((uint32_t)(nv / C::kVS) & 1u) ^ 1u))) break;
+                        if (lane == 0) {
+                            mbar_expect_tx(&sh->v_full[vs], kTile);
+                            tma_load_2d(sV + vs * kTile, &tmV, it.v_x, it.tok0 + j * kBK, &sh->v_full[vs]);
+                        }
+                        ++nv;
+                    }
+                }
+            }
+            // the answer is awaited even on the way out: nothing may be in flight towards shared memory when the CTA leaves
+            const bool answered = mbar_wait(&sh->clc_full, clc_phase);
+            clc_phase ^= 1u;
+            ok = ok && answered;
+            if (!ok) break;
+            const bool more = clc_query(&sh->clc, bx, by);
+            fence_proxy_async_smem();   // the answer has been read before the next one may be written
+            __syncwarp();
+            if (!more) break;
+        }
+        if (ok) {
+            const int slot = ni % kItemRing;
+            ok = mbar_wait(&sh->item_empty[slot], ((uint32_t)(ni / kItemRing) & 1u) ^ 1u);
+            if (ok && lane == 0) {
+                sh->item[slot].nkb = -1;
+                mbar_arrive(&sh->item_full[slot]);
+            }
+        }
+        if (!ok) {
+            if (lane == 0) {
+                atomicExch(p.err, 21);
+                sh->abort = 1;
+            }
+            // copies still in flight land before the CTA leaves (bounded)
+            for (int i = max(nq - C::kQS, 0); i < nq; ++i) mbar_wait(&sh->q_full[i % C::kQS], (uint32_t)(i / C::kQS) & 1u);
+            for (int i = max(nk - 2, 0); i < nk; ++i) mbar_wait(&sh->k_full[i & 1], (uint32_t)(i >> 1) & 1u);
+            for (int i = max(nv - C::kVS, 0); i < nv; ++i) mbar_wait(&sh->v_full[i % C::kVS], (uint32_t)(i / C::kVS) & 1u);
+        }
+        __syncwarp();
+    } else if (warp == kSoftmaxWarps + 1) {
+        // ---- UMMAs: the warp stays converged (every lane waits), one elected lane issues. Blocks are numbered through
+        // across items: Q K^T of block g + 1 is issued as soon as the scores of block g are in registers, ahead of P V of g.
+        const uint32_t idesc_qk = make_idesc_f16(128, kBK), idesc_qk_half = make_idesc_f16(128, kBK / 2);
+        const uint32_t idesc_pv = make_idesc_f16(128, kHD, false, true);   // V is an MN-major B operand
+        int ni = 0, nq = 0;
+        uint32_t g = 0;
+        bool ok = true, end = false;
+        int nkb = 0, valid = 0;      // current item
+        // takes the next item that has blocks (or the end); the items' slots go back at once: everything needed is kept here
+        auto next_item = [&]() -> bool {
+            for (;;) {
+                const int slot = ni % kItemRing;
+                if (!mbar_wait(&sh->item_full[slot], (uint32_t)(ni / kItemRing) & 1u)) return false;
+                nkb = sh->item[slot].nkb;
+                valid = sh->item[slot].valid;
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&sh->item_empty[slot]);
+                __syncwarp();
+                ++ni;
+                if (nkb < 0) { end = true; return true; }
+                if (nkb > 0) return true;
+            }
+        };
+        // S = Q K_j^T, block number gg; `last`: Q is not needed afterwards
+        auto issue_qk = [&](uint32_t gg, int qs, bool half, bool last) {
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t qa = smem_u32(sQ + qs * kTile), ka = smem_u32(sK + (gg & 1) * kTile);
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    umma_f16(tmem, make_smem_desc(qa + ks * 32, 16, 1024, 2), make_smem_desc(ka + ks * 32, 16, 1024, 2),
-                             idesc_qk, ks > 0);
-                umma_commit(&sh->s_ready);
-            };
-            if (lane == 0) AT_STAMP(10);
-            bool ok = mbar_wait(&sh->q_full, 0) && mbar_wait(&sh->k_full[0], 0);
-            if (lane == 0) AT_STAMP(11);
-            if (ok) {
-                tc_fence_after();
-                if (elect_one()) issue_qk(0);
-                if (lane == 0) AT_STAMP(13);
-            }
-            for (int j = 0; j < nkb && ok; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = (uint32_t)(j >> 1) & 1u;
-                if (sh->abort) { ok = false; break; }
-                // O += P_j V_j once the softmax warps have written P_j (and rescaled O)
-                ok = mbar_wait(&sh->p_ready, (uint32_t)j & 1u) && mbar_wait(&sh->v_full[st], ph);
-                if (!ok) break;
-                if (lane == 0) AT_STAMP(14 + 2 * j);
-                tc_fence_after();
-                if (elect_one()) {
-                    const uint32_t va = smem_u32(sV + (size_t)st * kKVTile);
-#pragma unroll
-                    for (int ks = 0; ks < kBK / 16; ++ks)   // P of keys 16ks..16ks+15: 8 packed columns
-                        umma_f16_ts(tmem + kOCol, tmem + kPCol + (uint32_t)(ks * 8), make_smem_desc(va + ks * 2048, 0, 1024, 2),
-                                    idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-                    umma_commit(&sh->pv_done);
-                }
-                if (lane == 0) AT_STAMP(15 + 2 * j);
-                if (j + 1 < nkb) {
-                    // S_{j+1} right behind it, into the columns that hold P_j: tcgen05 operations execute in issue
-                    // order, so Q K_{j+1}^T cannot overwrite P_j before P_j V_j has read it
-                    ok = mbar_wait(&sh->k_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-                        issue_qk(j + 1);
-                        if (j + 2 < nkb) load_k(j + 2);   // K_j's stage: Q K_j^T completed before the softmax of block j began
-                    }
-                    if (j + 2 < nkb) {
-                        // V_j's stage is free once P_j V_j has completed
-                        ok = mbar_wait(&sh->pv_done, (uint32_t)j & 1u);
-                        if (!ok) break;
-                        if (elect_one()) load_v(j + 2);
-                    }
-                }
-            }
-            if (elect_one()) {
-                umma_commit(&sh->o_done);
-                if (!ok) {
-                    atomicExch(p.err, 21);
-                    sh->abort = 1;
-                }
+                    umma_f16(tmem + kSCol, make_smem_desc(qa + ks * 32, 16, 1024, 2), make_smem_desc(ka + ks * 32, 16, 1024, 2),
+                             half ? idesc_qk_half : idesc_qk, ks > 0);
+                umma_commit(&sh->s_full);
+                umma_commit(&sh->k_empty[gg & 1]);
+                if (last) umma_commit(&sh->q_empty[qs]);
             }
             __syncwarp();
-        } else {
-            // ---- softmax warps: one thread per query row (TMEM lane) and key block
-            const int quarter = warp & 3;
-            const int row = quarter * 32 + lane;
-            const int qr = q0 + row;                       // query index inside the sequence
-            const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-            const bool has_mask = p.mask != nullptr;   // uniform: the masked code path is separate from the plain one
-            const half* mrow = (has_mask && qr < L) ? p.mask + (size_t)qr * p.mask_ld : nullptr;
-            const bool mask_vec = has_mask && (p.mask_ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.mask) & 15) == 0;
-            const uint32_t s_addr = tmem + lane_base;           // this row's scores of a block
-            const uint32_t p_addr = tmem + lane_base + kPCol;   // its P values as packed fp16 (over the first half of the score columns)
-            const uint32_t o_addr = tmem + lane_base + kOCol;   // its 64 output columns
-            float m_run = -INFINITY, l_run = 0.f;   // running maximum and running sum of the row
-            bool ok = true;
-            for (int j = 0; j < nkb; ++j) {
-                const bool got = !sh->abort && mbar_wait(&sh->s_ready, (uint32_t)j & 1u);   // every lane waits: no exchange
-                if (!got) {
-                    ok = false;
-                    sh->abort = 1;
-                    break;
-                }
-                if (tid == 0) AT_STAMP(30 + 4 * (j & 3));
-                tc_fence_after();
-                const int k0 = j * kBK;
-                const bool plain = !has_mask && k0 + kBK <= valid;   // uniform: no per-key validity selects needed
+        };
+        auto is_half = [&](int j) { return valid - j * kBK <= kBK / 2; };
 
-                // The row's 64 scores of this block. S_j could only be computed after P_{j-1} V_{j-1} (issue order), so
-                // O and the P columns are free to be written from here on.
-                uint32_t rp[32];        // fp16 scores: the row's 64 scores, two to a register
-                uint32_t rf[kNCh][32];  // fp32 scores
-                if constexpr (kScoresF16) {
-                    tmem_ld32_pack16(s_addr, rp);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < kNCh; ++c) tmem_ld32(s_addr + c * 32, rf[c]);
+        ok = next_item();
+        if (ok && !end) {
+            const int qs = nq % C::kQS;
+            ok = mbar_wait(&sh->q_full[qs], (uint32_t)(nq / C::kQS) & 1u) && mbar_wait(&sh->k_full[0], 0);
+            if (ok) issue_qk(0, qs, is_half(0), nkb == 1);
+            ++nq;
+        }
+        int j = 0;
+        while (ok && !end) {
+            const bool half = is_half(j);
+            const bool first = j == 0;
+            bool issued = false;
+            const uint32_t kb1 = (g + 1) & 1, kp1 = ((g + 1) >> 1) & 1;
+            if (j + 1 < nkb) {
+                ok = mbar_wait(&sh->s_free, g & 1) && mbar_wait(&sh->k_full[kb1], kp1);
+                if (!ok) break;
+                issue_qk(g + 1, (nq - 1) % C::kQS, is_half(j + 1), j + 2 == nkb);
+                issued = true;
+            } else if (mbar_try_wait(&sh->item_full[ni % kItemRing], (uint32_t)(ni / kItemRing) & 1u) &&
+                       sh->item[ni % kItemRing].nkb > 0) {
+                // the next item's first block, if its operands are there already: P V of this block does not wait for them
+                const int qs = nq % C::kQS;
+                if (C::kQS > 1 && mbar_try_wait(&sh->q_full[qs], (uint32_t)(nq / C::kQS) & 1u) && mbar_try_wait(&sh->k_full[kb1], kp1)) {
+                    ok = mbar_wait(&sh->s_free, g & 1) && next_item();
+                    if (!ok) break;
+                    issue_qk(g + 1, qs, is_half(0), nkb == 1);
+                    ++nq;
+                    j = -1;
+                    issued = true;
                 }
-                tmem_ld_wait();
-                // scores 2i and 2i+1 of chunk c as fp32
-                auto score2 = [&](int c, int i) -> float2 {
-                    if constexpr (kScoresF16) return __half22float2(*reinterpret_cast<const half2*>(&rp[c * 16 + i]));
-                    else return make_float2(__uint_as_float(rf[c][2 * i]), __uint_as_float(rf[c][2 * i + 1]));
-                };
-                // The general pass (additive mask, keys beyond the valid length): the scaled, masked scores (log2 domain)
-                // of one 32-column chunk in fp32. It is evaluated twice per block, for the maximum and for P, so that
-                // only the packed scores stay in registers in between.
-                auto general_chunk = [&](int c, float (&v)[32]) {
-                    const int kc = k0 + c * 32;
-                    if (has_mask) {
-                        float mk[32];
-                        load_mask32(mk, mrow, kc, valid, mask_vec);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float2 f = score2(c, i);
-                            v[2 * i] = (kc + 2 * i < valid) ? fmaf(f.x, p.scale_log2, mk[2 * i]) : -INFINITY;
-                            v[2 * i + 1] = (kc + 2 * i + 1 < valid) ? fmaf(f.y, p.scale_log2, mk[2 * i + 1]) : -INFINITY;
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float2 f = score2(c, i);
-                            v[2 * i] = (kc + 2 * i < valid) ? f.x * p.scale_log2 : -INFINITY;
-                            v[2 * i + 1] = (kc + 2 * i + 1 < valid) ? f.y * p.scale_log2 : -INFINITY;
-                        }
-                    }
-                };
-                float bmax = -INFINITY;
-                if (plain && kScoresF16) {
-                    half2 mx0 = *reinterpret_cast<const half2*>(&rp[0]), mx1 = *reinterpret_cast<const half2*>(&rp[1]);
-#pragma unroll
-                    for (int i = 2; i < 32; i += 2) {
-                        mx0 = __hmax2(mx0, *reinterpret_cast<const half2*>(&rp[i]));
-                        mx1 = __hmax2(mx1, *reinterpret_cast<const half2*>(&rp[i + 1]));
-                    }
-                    const float2 f = __half22float2(__hmax2(mx0, mx1));
-                    bmax = fmaxf(f.x, f.y) * p.scale_log2;   // the scale is positive: scale the maximum once
-                } else if (plain) {
-                    float raw[kNCh];
-#pragma unroll
-                    for (int c = 0; c < kNCh; ++c) raw[c] = -INFINITY;
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-#pragma unroll
-                        for (int c = 0; c < kNCh; ++c) raw[c] = fmaxf(raw[c], __uint_as_float(rf[c][i]));
-                    }
-#pragma unroll
-                    for (int c = 0; c < kNCh; ++c) bmax = fmaxf(bmax, raw[c]);
-                    bmax *= p.scale_log2;
-                } else {
-#pragma unroll
-                    for (int c = 0; c < kNCh; ++c) {
-                        float v[32];
-                        general_chunk(c, v);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) bmax = fmaxf(bmax, v[i]);
-                    }
-                }
-                // The reference point is kept representable in fp16 (the packed pass subtracts it in fp16), within range.
-                if (bmax > -INFINITY) bmax = __half2float(__float2half_rn(fminf(fmaxf(bmax, -60000.f), 60000.f)));
-                // The reference point of the exponentials moves only when the row maximum has grown by more than 2^8
-                // (P could leave the fp16 range); the final division by the row sum makes the result independent of it.
-                const bool grow = bmax > m_run + kRescaleStep;   // also true for the first finite score of a row
-                if (j > 0) {
-                    // P_{j-1} V_{j-1} has completed: it was issued before this block's Q K^T by the same thread, and the
-                    // commit that signalled S_j covers every earlier operation of that thread.
-                    if (__any_sync(0xffffffffu, grow)) {
-                        // O and the running sum move to the new reference point (0 when the row had nothing before)
-                        const float alpha = grow ? ((m_run == -INFINITY) ? 0.f : ex2_fast(m_run - bmax)) : 1.f;
-                        l_run *= alpha;
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            uint32_t o[16];
-                            tmem_ld16(o_addr + c * 16, o);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                            tmem_st16(o_addr + c * 16, o);
-                        }
-                    }
-                }
-                if (grow) m_run = bmax;
-                if (tid == 0) AT_STAMP(31 + 4 * (j & 3));
-                // P = 2^(s - reference) as packed fp16 over the first 32 score columns; the row sum is the sum of exactly
-                // the fp16 values that are multiplied with V.
-                const float nshift = (m_run == -INFINITY) ? 0.f : -m_run;
-#pragma unroll
-                for (int c = 0; c < kNCh; ++c) {
-                    uint32_t pk[16];
-                    if (plain && kScoresF16) {
-                        const half2 sc2 = __float2half2_rn(p.scale_log2), sh2 = __float2half2_rn(nshift);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const half2 a2 = __hfma2(*reinterpret_cast<const half2*>(&rp[c * 16 + i]), sc2, sh2);
-                            pk[i] = ex2_h2(*reinterpret_cast<const uint32_t*>(&a2));
-                        }
-                    } else if (plain) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2)
-                            pk[i >> 1] = ex2_h2(pack2(fmaf(__uint_as_float(rf[c][i]), p.scale_log2, nshift),
-                                                      fmaf(__uint_as_float(rf[c][i + 1]), p.scale_log2, nshift)));
-                    } else {
-                        float v[32];
-                        general_chunk(c, v);
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) pk[i >> 1] = ex2_h2(pack2(v[i] + nshift, v[i + 1] + nshift));
-                    }
-                    tmem_st16(p_addr + c * 16, pk);
-                    l_run += sum_packed(pk);
-                }
-                if (tid == 0) AT_STAMP(32 + 4 * (j & 3));
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (elect_one()) mbar_arrive(&sh->p_ready);
-                if (tid == 0) AT_STAMP(33 + 4 * (j & 3));
             }
-            // ---- epilogue: O / row sum -> fp16 -> global
-            const bool fin = ok && !sh->abort && mbar_wait(&sh->o_done, 0);
+            // O += P V of block g
+            const int vs = g % C::kVS;
+            ok = mbar_wait(&sh->p_full, g & 1) && mbar_wait(&sh->v_full[vs], (uint32_t)(g / C::kVS) & 1u);
+            if (!ok) break;
             tc_fence_after();
-            if (tid == 0) AT_STAMP(50);
-            if (fin) {
-                const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-                half* zrow = p.Z + (size_t)(tok0 + qr) * p.z_pitch + h * kHD;
+            if (elect_one()) {
+                const uint32_t va = smem_u32(sV + vs * kTile);
+                const int steps = half ? kBK / 32 : kBK / 16;
+                for (int ks = 0; ks < steps; ++ks)   // P of keys 16ks..16ks+15: 8 packed columns
+                    umma_f16_ts(tmem + kOCol, tmem + kPCol + (uint32_t)(ks * 8), make_smem_desc(va + ks * 2048, 0, 1024, 2), idesc_pv,
+                                (!first || ks > 0) ? 1u : 0u);
+                umma_commit(&sh->pv_done);
+                umma_commit(&sh->v_empty[vs]);
+            }
+            __syncwarp();
+            if (!issued) {
+                ok = next_item();
+                if (!ok || end) break;
+                const int qs = nq % C::kQS;
+                ok = mbar_wait(&sh->q_full[qs], (uint32_t)(nq / C::kQS) & 1u) && mbar_wait(&sh->k_full[kb1], kp1) &&
+                     mbar_wait(&sh->s_free, g & 1);
+                if (!ok) break;
+                issue_qk(g + 1, qs, is_half(0), nkb == 1);
+                ++nq;
+                j = -1;
+            }
+            ++j;
+            ++g;
+        }
+        if (!ok && lane == 0) {
+            atomicExch(p.err, 21);
+            sh->abort = 1;
+        }
+        __syncwarp();
+    } else if (warp < kSoftmaxWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+        // ---- softmax: one thread per query row (TMEM lane)
+        pdl_wait();
+        const int row = warp * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+        const uint32_t s_addr = tmem + lane_base + kSCol, p_addr = tmem + lane_base + kPCol, o_addr = tmem + lane_base + kOCol;
+        uint8_t* const mw = smem + C::kMaskAt + (size_t)warp * (32 * kMaskPitch);   // kMask: this warp's mask rows
+        const bool wide = (p.z_pitch & 15) == 0 && (reinterpret_cast<uintptr_t>(p.Z) & 31) == 0;
+        uint32_t g = 0;
+        bool ok = true;
+        int done_slot = -1;     // item whose P V is on its way and whose rows are still to be written
+        float done_sum = 0.f;   // its row sum
+        auto release = [&](int slot) {
+            __syncwarp();
+            if (elect_one()) mbar_arrive(&sh->item_empty[slot]);
+            __syncwarp();
+        };
+        // O / row sum -> fp16 -> global. Called when the item's last P V has completed: inside the
+        // next item's first block, whose scores and exponentials cover the wait.
+        auto finish = [&]() {
+            const Item& it = sh->item[done_slot];
+            const float inv = done_sum > 0.f ? 1.f / done_sum : 0.f;
+            const int qr = it.q0 + row;
+            const bool in = qr < it.len;
+            half* const zrow = p.Z + (size_t)(it.tok0 + qr) * p.z_pitch + it.head * kHD;
+            if constexpr (kPruneV) {
+                // a row is put together in shared memory (zeros where V was pruned) and written whole
+                half* const st = reinterpret_cast<half*>(smem + C::kScatterAt + row * kScatterPitch);
+                if (!it.v_add) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) reinterpret_cast<uint2*>(st)[i] = make_uint2(0u, 0u);
+                }
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t r[16];
+                    tmem_ld16(o_addr + c * 16, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const int k = c * 16 + i - it.v_off;
+                        if (k >= 0 && k < it.v_n) {   // the same for the whole warp
+                            const int col = __ldg(p.v_col_id + it.v_base + k) - it.head * kHD;
+                            const half z = __float2half_rn(__uint_as_float(r[i]) * inv);
+                            if (!it.v_add) st[col] = z;
+                            else if (in) zrow[col] = z;
+                        }
+                    }
+                }
+                if (!it.v_add && in) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint2* s2 = reinterpret_cast<const uint2*>(st) + 2 * i;
+                        *reinterpret_cast<uint4*>(zrow + i * 8) = make_uint4(s2[0].x, s2[0].y, s2[1].x, s2[1].y);
+                    }
+                }
+            } else {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     uint32_t r[16];
                     tmem_ld16(o_addr + c * 16, r);
                     tmem_ld_wait();
-                    if (qr < L) {
-                        uint4 o[2];
-                        uint32_t* ow = reinterpret_cast<uint32_t*>(o);
+                    if (in) {
+                        uint32_t ow[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
                             ow[i] = pack2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
-                        *reinterpret_cast<uint4*>(zrow + c * 16) = o[0];
-                        *reinterpret_cast<uint4*>(zrow + c * 16 + 8) = o[1];
+                        half* const z = zrow + c * 16;
+                        if (wide) {
+                            asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(z), "r"(ow[0]), "r"(ow[1]), "r"(ow[2]),
+                                         "r"(ow[3]), "r"(ow[4]), "r"(ow[5]), "r"(ow[6]), "r"(ow[7])
+                                         : "memory");
+                        } else {
+                            *reinterpret_cast<uint4*>(z) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                            *reinterpret_cast<uint4*>(z + 8) = make_uint4(ow[4], ow[5], ow[6], ow[7]);
+                        }
                     }
                 }
-            } else if (lane == 0 && !sh->abort) {
-                atomicExch(p.err, 22);
-                sh->abort = 1;
             }
-        }
-    } else if (b >= 0 && warp < 4) {
-        // no valid key: the output rows are zero
-        const int qr = q0 + warp * 32 + lane;
-        if (qr < L) {
-            uint4* z = reinterpret_cast<uint4*>(p.Z + (size_t)(tok0 + qr) * p.z_pitch + h * kHD);
+            release(done_slot);
+            done_slot = -1;
+        };
+        for (int ni = 0; ok; ++ni) {
+            const int slot = ni % kItemRing;
+            ok = mbar_wait(&sh->item_full[slot], (uint32_t)(ni / kItemRing) & 1u);
+            if (!ok) break;
+            const Item& it = sh->item[slot];   // stays in shared memory: registers are what limits this kernel
+            const int nkb = it.nkb;
+            if (nkb <= 0) {
+                if (done_slot >= 0) {   // (the ring could run out of slots if an item waited behind empty ones)
+                    ok = mbar_wait(&sh->pv_done, (g - 1) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                    finish();
+                }
+                if (nkb < 0) break;
+                const int qr = it.q0 + row;   // no valid key: the output rows are zero
+                if (qr < it.len) {
+                    uint4* z = reinterpret_cast<uint4*>(p.Z + (size_t)(it.tok0 + qr) * p.z_pitch + it.head * kHD);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) z[i] = make_uint4(0, 0, 0, 0);
+                    for (int i = 0; i < 8; ++i) z[i] = make_uint4(0, 0, 0, 0);
+                }
+                release(slot);
+                continue;
+            }
+            const int valid = it.valid;
+            // the mask rows of the warp's queries for a block of keys: seventeen granules per row, asynchronously
+            auto fetch_mask = [&](int j) {
+                const uint8_t* mend = reinterpret_cast<const uint8_t*>(p.mask + (size_t)(it.len - 1) * p.mask_ld + it.len);
+                for (int i = lane; i < 32 * 17; i += 32) {
+                    const int r = i / 17, c = i % 17;
+                    const int q = it.q0 + warp * 32 + r;
+                    const uintptr_t a = reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & ~(uintptr_t)15;
+                    const uint8_t* src = reinterpret_cast<const uint8_t*>(a) + c * 16;
+                    const long left = q < it.len ? (long)(mend - src) : 0;
+                    const int n = left >= 16 ? 16 : (left > 0 ? (int)left : 0);
+                    cp_async16(mw + r * kMaskPitch + c * 16, n > 0 ? src : reinterpret_cast<const uint8_t*>(p.mask), n);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            if constexpr (kMask) fetch_mask(0);
+            float m_run = -INFINITY;
+            float2 l2 = make_float2(0.f, 0.f);
+            for (int j = 0; j < nkb; ++j, ++g) {
+                const int left = valid - j * kBK;          // valid keys from here on
+                const bool full = left > kBK / 2;          // otherwise half a block: two 32-column chunks instead of four
+                ok = mbar_wait(&sh->s_full, g & 1);
+                if (!ok) break;
+                tc_fence_after();
+                float v[4][32];
+                {
+                    uint32_t(*raw)[32] = reinterpret_cast<uint32_t(*)[32]>(v);
+                    tmem_ld32(s_addr, raw[0]);
+                    tmem_ld32(s_addr + 32, raw[1]);
+                    if (full) {
+                        tmem_ld32(s_addr + 64, raw[2]);
+                        tmem_ld32(s_addr + 96, raw[3]);
+                    }
+                    tmem_ld_wait();
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&sh->s_free);
+                __syncwarp();
+                float sc = p.scale_log2;
+                if constexpr (kMask) {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                    __syncwarp();
+                    sc = 1.f;
+                    const int q = min(it.q0 + row, it.len - 1);
+                    const int shift = (int)((reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & 15) >> 1);
+                    const uint8_t* gr = mw + lane * kMaskPitch;
+                    uint4 cur = *reinterpret_cast<const uint4*>(gr);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (c < 2 || full) {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const uint4 nxt = *reinterpret_cast<const uint4*>(gr + (c * 4 + e + 1) * 16);
+                                uint32_t w[8] = {cur.x, cur.y, cur.z, cur.w, nxt.x, nxt.y, nxt.z, nxt.w};
+                                if (shift & 4)
+#pragma unroll
+                                    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+                                if (shift & 2)
+#pragma unroll
+                                    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const uint32_t mv = (shift & 1) ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
+                                    const float2 m = __half22float2(*reinterpret_cast<const half2*>(&mv));
+                                    const int k = e * 8 + 2 * i;
+                                    v[c][k] = fmaf(v[c][k], p.scale_log2, m.x * kLog2e);
+                                    v[c][k + 1] = fmaf(v[c][k + 1], p.scale_log2, m.y * kLog2e);
+                                }
+                                cur = nxt;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (j + 1 < nkb) fetch_mask(j + 1);
+                }
+                if (left < (full ? kBK : kBK / 2)) {   // keys beyond the valid length
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (c * 32 + i >= left) v[c][i] = -INFINITY;
+                }
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (c < 2 || full) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], v[c][i], v[c][i + 1]);
+                    }
+                const float bmax = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * sc;   // the scale is positive: scale the maximum once
+                // The reference point moves only when the row maximum has grown by more than 2^8 (P could leave the fp16
+                // range); the final division by the row sum makes the result independent of it.
+                const bool grow = bmax > m_run + kRescaleStep;   // also true for the first finite score of a row
+                const bool any = __any_sync(0xffffffffu, grow);
+                float alpha = 1.f;
+                if (grow) {
+                    alpha = m_run == -INFINITY ? 0.f : ex2_fast(m_run - bmax);
+                    m_run = bmax;
+                    l2.x *= alpha;
+                    l2.y *= alpha;
+                }
+                const float nshift = (m_run == -INFINITY) ? 0.f : -m_run;
+                const float2 sc2 = make_float2(sc, sc), sh2 = make_float2(nshift, nshift);
+                uint32_t pk[4][16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c < 2 || full) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            float2 e = fma2(make_float2(v[c][2 * i], v[c][2 * i + 1]), sc2, sh2);
+                            // spread over the chunk so that both pipes stay busy
+                            if ((i * kPolyPairs) / 16 != ((i + 1) * kPolyPairs) / 16) {
+                                e = ex2_poly2(e);
+                            } else {
+                                e.x = ex2_fast(e.x);
+                                e.y = ex2_fast(e.y);
+                            }
+                            l2 = add2(l2, e);
+                            pk[c][i] = pack2(e.x, e.y);
+                        }
+                    }
+                }
+                // P and O may be written once P V of the previous block has completed
+                if (g > 0) {
+                    ok = mbar_wait(&sh->pv_done, (g - 1) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+                if (j == 0) {
+                    if (done_slot >= 0) finish();
+                } else if (any) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t o[16];
+                        tmem_ld16(o_addr + c * 16, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st16(o_addr + c * 16, o);
+                    }
+                }
+                tmem_st16(p_addr, pk[0]);
+                tmem_st16(p_addr + 16, pk[1]);
+                if (full) {
+                    tmem_st16(p_addr + 32, pk[2]);
+                    tmem_st16(p_addr + 48, pk[3]);
+                }
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&sh->p_full);
+                __syncwarp();
+            }
+            if (!ok) break;
+            done_slot = slot;
+            done_sum = l2.x + l2.y;
         }
+        if constexpr (kMask) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (!ok && lane == 0) {
+            atomicExch(p.err, 22);
+            sh->abort = 1;
+        }
+        __syncwarp();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (tid == 0) AT_STAMP(51);
-    if (warp == kSoftmaxWarps) tmem_dealloc(tmem, kTmemCols);
+    if (warp == kSoftmaxWarps + 1) tmem_dealloc(tmem, kTmemCols);
 }
 
-long long* g_attn_prof = nullptr;
-bool g_scores_fp32 = false;   // how Q K^T is accumulated (see kScoresF16 above); process-wide, read at launch
+bool g_scores_fp32 = false;   // kept for et_attention_scores_fp32: Q K^T accumulates in fp32 either way
 
 // Error word of the kernel's bounded waits: a device variable of the library image (one copy per device that
 // loads the library, zero at load), so that no launch ever allocates. The kernel writes it only when a wait
@@ -546,6 +778,16 @@ int attn_err_address(int** out) {
     return ET_OK;
 }
 
+template <bool kMask, bool kPruneV>
+cudaError_t opt_in() {
+    return cudaFuncSetAttribute(attention_tc_kernel<kMask, kPruneV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+}
+template <bool kMask, bool kPruneV>
+cudaError_t launch(dim3 grid, cudaStream_t st, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const TcParams& p) {
+    const size_t smem = (size_t)Cfg<kMask, kPruneV>::kBytes + sizeof(TcShared) + 1024;
+    return launch_pdl(attention_tc_kernel<kMask, kPruneV>, grid, dim3(kThreads), smem, st, tq, tk, tv, p);
+}
+
 }  // namespace
 
 // Looks up the error word's address on the current device (encoder constructors call this so that the first
@@ -555,14 +797,17 @@ int attention_prepare_device() {
     return attn_err_address(&p);
 }
 
-// Fast path. Returns ET_ERR_UNSUPPORTED (without touching anything) when the case is outside its range, so the
-// caller can use the general kernel instead.
-int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch,
-                        const half* mask, int mask_ld, const int* cu_seqlens, const int* valid_lens, int batch,
-                        int uniform_len, int total_tokens, int max_len, int d_model, int nhead, cudaStream_t st) {
+// Returns ET_ERR_UNSUPPORTED (without touching anything) when the case is outside the kernel's range, so the caller can use
+// the general kernel instead. v_head_ptr / v_col_id: V is compact ([tokens x v_cols], row pitch v_pitch).
+int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch, int v_cols,
+                        const int* v_head_ptr, const int* v_col_id, const half* mask, int mask_ld, const int* cu_seqlens,
+                        const int* valid_lens, int batch, int uniform_len, int total_tokens, int max_len, int d_model, int nhead,
+                        cudaStream_t st) {
     if (d_model / nhead != kHD || d_model % nhead) return ET_ERR_UNSUPPORTED;
     if (max_len <= 0) return ET_ERR_UNSUPPORTED;   // longest sequence unknown: the caller uses the general kernel
-    if ((q_pitch & 7) || (v_pitch & 7) || (d_model & 7) || !aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(Z))
+    // TMA: operands and pitches in whole 16-byte units; the mask's granules are read from a 16-byte aligned start
+    if ((q_pitch & 7) || (v_pitch & 7) || (d_model & 7) || !aligned16(Q) || !aligned16(K) || !aligned16(V) || !aligned16(Z) ||
+        (mask && !aligned16(mask)))
         return ET_ERR_UNSUPPORTED;
     if (batch <= 0 || total_tokens <= 0) return ET_OK;
     int* err_word = nullptr;
@@ -575,29 +820,29 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     // the column extent covers all heads of the operand; Q/K/V may be slices of one fused [tokens x 3 d_model] buffer
     if (!make_tmap_2d_f16(&tq, Q, rows, (uint64_t)d_model, (uint64_t)q_pitch, kBQ, kHD, 128) ||
         !make_tmap_2d_f16(&tk, K, rows, (uint64_t)d_model, (uint64_t)q_pitch, kBK, kHD, 128) ||
-        !make_tmap_2d_f16(&tv, V, rows, (uint64_t)d_model, (uint64_t)v_pitch, kBK, kHD, 128))
+        !make_tmap_2d_f16(&tv, V, rows, (uint64_t)v_cols, (uint64_t)v_pitch, kBK, kHD, 128))
         return fail(ET_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed");
     TcParams p;
     p.Z = Z; p.mask = mask; p.cu_seqlens = cu_seqlens; p.valid_lens = valid_lens;
+    p.v_head_ptr = v_head_ptr; p.v_col_id = v_col_id;
     p.z_pitch = d_model; p.mask_ld = mask_ld; p.batch = batch; p.uniform_len = uniform_len;
     p.scale_log2 = kLog2e / sqrtf((float)kHD);
     p.err = err_word;
-    p.prof = g_attn_prof;
-    const size_t smem = (size_t)kTile + 4 * (size_t)kKVTile + sizeof(TcShared) + 1024;
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-        if (e != cudaSuccess) return e;
-        return cudaFuncSetAttribute(attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+        cudaError_t e = opt_in<false, false>();
+        if (e == cudaSuccess) e = opt_in<true, false>();
+        if (e == cudaSuccess) e = opt_in<false, true>();
+        if (e == cudaSuccess) e = opt_in<true, true>();
+        return e;
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "attention: shared memory opt-in");
     const int nblk = cu_seqlens ? (total_tokens + kBQ - 1) / kBQ + batch : batch * ((uniform_len + kBQ - 1) / kBQ);
-    auto kernel = g_scores_fp32 ? attention_tc_kernel<false> : attention_tc_kernel<true>;
-    return cuda_status(launch_pdl(kernel, dim3(nblk, nhead), dim3(kThreads), smem, st, tq, tk, tv, p),
-                       "attention (tcgen05) launch");
+    const dim3 grid(nblk, nhead);
+    const cudaError_t e = v_head_ptr ? (mask ? launch<true, true>(grid, st, tq, tk, tv, p) : launch<false, true>(grid, st, tq, tk, tv, p))
+                                     : (mask ? launch<true, false>(grid, st, tq, tk, tv, p) : launch<false, false>(grid, st, tq, tk, tv, p));
+    return cuda_status(e, "attention (tcgen05) launch");
 }
-
-void attention_tc_set_profile_buffer(long long* dev_buf) { g_attn_prof = dev_buf; }
 
 void attention_tc_set_scores_fp32(int on) { g_scores_fp32 = on != 0; }
 int attention_tc_scores_fp32() { return g_scores_fp32 ? 1 : 0; }

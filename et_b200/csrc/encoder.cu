@@ -573,7 +573,7 @@ int et_attention_prune(void* out, const void* Q, const void* K, const void* V, c
     return et::attention_launch(static_cast<half*>(out), static_cast<const half*>(Q), static_cast<const half*>(K),
                                 static_cast<const half*>(V), nullptr, d_model, nnz_col_v, nullptr, v_col_id,
                                 v_head_ptr, static_cast<const half*>(mask), seq_len, nullptr, nullptr, 1, seq_len,
-                                seq_len, d_model, nhead, static_cast<cudaStream_t>(stream));
+                                seq_len, d_model, nhead, static_cast<cudaStream_t>(stream), 0, nnz_col_v);
 }
 int et_qk_scores(void* QK, const void* Q, const void* K, int seq_len, int d_model, int nhead, void* stream) {
     return et::qk_scores_launch(static_cast<half*>(QK), static_cast<const half*>(Q), static_cast<const half*>(K), 1,

@@ -57,6 +57,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // iteration limit corresponds to a wall time far above any legitimate wait in these kernels.
 constexpr uint32_t kMbarSpinLimit = 1u << 20;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
     for (uint32_t i = 0; i < kMbarSpinLimit; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     return false;

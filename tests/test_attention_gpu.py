@@ -170,6 +170,64 @@ def test_attention_prune_scatter(et, orc):
     assert (got[:, dropped] == 0).all()          # pruned columns are exactly zero
 
 
+@pytest.mark.parametrize("L,mask", [(63, True), (64, False), (65, True), (127, False), (129, True), (192, True), (193, True), (383, True)])
+def test_attention_block_edges(et, orc, L, mask):
+    """Both sides of a half and of a whole block of 128 keys and queries, with mask rows at every alignment."""
+    d, H = 192, 3
+    Q, K, V = _qkv(51, L, d)
+    M = (util.rng(L).standard_normal((L, L))).astype(np.float16) if mask else None
+    out = torch.full((L, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_otf(out, dev(Q), dev(K), dev(V), None if M is None else dev(M), L, d, H)
+    torch.cuda.synchronize()
+    et.attention_check()
+    util.assert_close(host(out), orc.attention(Q, K, V, [L], d, H, mask=M), what=f"attention L={L}")
+
+
+@pytest.mark.parametrize("sparsity,L,mask", [(0.03, 129, False), (0.1, 77, True), (0.5, 65, True), (0.75, 200, False)])
+def test_attention_prune_window_widths(et, orc, sparsity, L, mask):
+    """Compact windows from a few columns to nearly the whole head: the wide ones do not fit one copied box of 64 columns at
+    their alignment and are done in two passes."""
+    d, H = 512, 8
+    row_id = orc.gen_sparse_row_mat(d, sparsity, seed=15, nhead=H)
+    row_id = row_id[:len(row_id) // 8 * 8]           # a row pitch in whole 16-byte units
+    hp = orc.head_ptr(row_id, H, d)
+    nnz = len(row_id)
+    Q, K, Vc = util.activations(1, (L, d)), util.activations(2, (L, d)), util.activations(3, (L, nnz))
+    M = util.rng(L).standard_normal((L, L)).astype(np.float16) if mask else None
+    out = torch.full((L, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_prune(out, dev(Q), dev(K), dev(Vc), dev(row_id), dev(hp), nnz, None if M is None else dev(M), L, d, H)
+    torch.cuda.synchronize()
+    et.attention_check()
+    got = host(out)
+    util.assert_close(got, orc.attention(Q, K, Vc, [L], d, H, mask=M, v_col_id=row_id, v_head_ptr=hp), what=f"pruned V, sparsity {sparsity}")
+    assert (got[:, np.setdiff1d(np.arange(d), row_id)] == 0).all()
+
+
+@pytest.mark.parametrize("mask", [False, True])
+def test_attention_ragged_batch_with_empty_and_padded_sequences(et, orc, mask):
+    """More items than CTAs that fit at once, sequences without tokens or without valid keys among them."""
+    d, H = 256, 4
+    rng = util.rng(99)
+    lens = [int(n) for n in rng.integers(1, 300, size=150)] + [0, 128, 0, 1]
+    valid = [int(rng.integers(0, n + 1)) if i % 3 == 0 else n for i, n in enumerate(lens)]
+    T, L = sum(lens), max(lens)
+    Q, K, V = _qkv(61, T, d)
+    M = util.rng(5).standard_normal((L, L)).astype(np.float16) if mask else None
+    cu = dev(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32))
+    out = torch.full((T, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_batch(out, dev(Q), dev(K), dev(V), d, H, cu_seqlens=cu, valid_lens=dev(np.array(valid, dtype=np.int32)),
+                       batch=len(lens), max_seq_len=L, mask=None if M is None else dev(M), mask_ld=L if mask else 0)
+    torch.cuda.synchronize()
+    et.attention_check()
+    want = np.zeros((T, d), dtype=np.float32)
+    o = 0
+    for n, v in zip(lens, valid):
+        if n:
+            want[o:o + n] = orc.attention(Q[o:o + n], K[o:o + n], V[o:o + n], [n], d, H, mask=None if M is None else M[:n, :n].copy(), valid_lens=[v])
+        o += n
+    util.assert_close(host(out), want, what="ragged batch")
+
+
 def test_attention_qk_and_v_pruned(et, orc):
     L, d, H = 100, 768, 12
     row_id = orc.gen_sparse_row_mat(d, 0.5, seed=6, nhead=H)

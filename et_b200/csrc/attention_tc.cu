@@ -35,6 +35,7 @@
 #include "common.h"
 #include "ptx.cuh"
 #include "tmap.h"
+#include "vec_math.cuh"
 
 namespace et {
 
@@ -107,35 +108,9 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
-__device__ __forceinline__ float ex2_fast(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
-}
-// Two fp32 operations per instruction.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n.reg .b64 x, y, z, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmov.b64 z, {%6, %7};\n"
-        "fma.rn.f32x2 w, x, y, z;\nmov.b64 {%0, %1}, w;\n}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("{\n.reg .b64 x, y, w;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 w, x, y;\nmov.b64 {%0, %1}, w;\n}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
 }
 // 2^x for two values on the FMA and ALU pipes, x <= 127: x = n + f with n the nearest whole number (adding 1.5 * 2^23 leaves
 // n in the low bits of the sum) and |f| <= 1/2; 2^f by the cubic that interpolates it at the Chebyshev nodes of [-1/2, 1/2]

@@ -3,41 +3,77 @@
 // the device function kernels/attention.cu:10-48 of the reference.
 //
 // Bandwidth kernel: 4*L*L bytes per score matrix (fp16 read + write); the [L x L] mask is
-// shared by every matrix and stays in L2. One warp per row, 16-byte accesses, the row held in
-// registers, fp32 max / sum, true row max (a fully masked row yields zeros), ex2 with log2(e)
-// folded into the argument. Keys at index >= valid_len are excluded and written as zero.
+// shared by every matrix and stays in L2. The row is held in registers, fp32 max / sum, true row max (a fully masked
+// row yields zeros), ex2 with log2(e) folded into the argument. Keys at index >= valid_len are excluded and written as zero.
+#include <algorithm>
+#include <type_traits>
 #include "common.h"
+#include "vec_math.cuh"
 
 namespace et {
 
-// 2^x on the special-function unit; inputs here are <= 0 or -inf, results flush to zero below 2^-126.
-__device__ __forceinline__ float ex2_fast(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
+constexpr float kLog2e = 1.4426950408889634f;
+
+// A row is a head of up to 7 elements, whole 16-byte granules of memory, and a tail of up to 7 elements, whatever its
+// length and alignment (sequence lengths are rarely multiples of 8). G lanes share a row: lane l holds granules l, l + G, ...
+// (CH of them) and, for l < 8, head element l and tail element l. Nothing but valid elements is ever read, so the granules
+// need no per-element checks; what lies beyond valid_len is only written. The mask row has an alignment of its own: a
+// granule's eight mask values come as the two granules that hold them, shifted into place (five 4-byte loads instead: 40 us against 30, L1 wavefronts).
+// Short rows leave lanes idle, hence G = 8 and 16; R rows per group are in flight at once. Bound by HBM for rows above ~256
+// elements, by instruction issue below (~60 per granule: two fp32 operations per instruction, 32-bit index arithmetic).
+// Measured with a mask: 1024 matrices of 512 x 512 229 -> 173 us (6.2 TB/s; 64-bit modulo and scalar fp32 before), 128 of
+// 500 x 500 101 us (three passes, 2-byte accesses) -> 30 us.
+template <int G>
+__device__ __forceinline__ float group_max(float v) {
+    if constexpr (G == 32) {
+        return warp_max(v);
+    } else {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        return v;
+    }
+}
+template <int G>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
-template <int CH, int R>  // CH 16-byte chunks per lane (L <= CH*256); R rows per warp and iteration
-__global__ void __launch_bounds__(256) softmax_mask_vec(half* __restrict__ scores,
-                                                        const half* __restrict__ mask, long nrow,
+__device__ __forceinline__ uint4 pack_row(const float2 (&v)[4], float inv) {
+    const float2 i2 = make_float2(inv, inv);
+    uint4 o;
+    half2* oh = reinterpret_cast<half2*>(&o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 p = mul2(v[j], i2);
+        oh[j] = __floats2half2_rn(p.x, p.y);
+    }
+    return o;
+}
+
+// Rows in whole granules on both sides (length a multiple of 8, aligned tensors).
+template <int G, int CH, int R>
+__global__ void __launch_bounds__(256) softmax_mask_vec(half* __restrict__ scores, const half* __restrict__ mask, unsigned nrow,
                                                         int L, int valid) {
     pdl_launch_dependents();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarp = ((long)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned group = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const unsigned ngroup = (gridDim.x * blockDim.x) / G;
     const int nchunk = L >> 3;
-    constexpr float kLog2e = 1.4426950408889634f;
-    for (long row0 = warp * R; row0 < nrow; row0 += nwarp * R) {
+    const unsigned rounds = (nrow + ngroup * R - 1) / (ngroup * R);   // the same for all groups of a warp
+    for (unsigned it = 0; it < rounds; ++it) {
+        const unsigned row0 = (it * ngroup + group) * R;
         uint4 sv[R][CH], mv[R][CH];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const long row = row0 + r;
-            const uint4* sr = reinterpret_cast<const uint4*>(scores + row * L);
-            const uint4* mr = mask ? reinterpret_cast<const uint4*>(mask + (size_t)(row % L) * L) : nullptr;
+            const unsigned row = row0 + r;
+            const uint4* sr = reinterpret_cast<const uint4*>(scores + (size_t)row * L);
+            const uint4* mr = mask ? reinterpret_cast<const uint4*>(mask + (size_t)(row % (unsigned)L) * L) : nullptr;
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
-                const int c = lane + 32 * i;
+                const int c = lane + G * i;
                 sv[r][i] = make_uint4(0, 0, 0, 0);
                 mv[r][i] = make_uint4(0, 0, 0, 0);
                 if (row < nrow && c < nchunk) {
@@ -48,166 +84,174 @@ __global__ void __launch_bounds__(256) softmax_mask_vec(half* __restrict__ score
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const long row = row0 + r;
-            float v[CH][8];
+            const unsigned row = row0 + r;
+            float2 v[CH][4];
             float mx = -INFINITY;
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
-                const int c = lane + 32 * i;
                 const half2* sh = reinterpret_cast<const half2*>(&sv[r][i]);
                 const half2* mh = reinterpret_cast<const half2*>(&mv[r][i]);
+                const int left = valid - (lane + G * i) * 8;   // valid elements from this granule's first one on (valid <= L)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float2 a = __half22float2(sh[j]), m = __half22float2(mh[j]);
-                    const int k = c * 8 + 2 * j;
-                    v[i][2 * j] = (c < nchunk && k < valid) ? a.x + m.x : -INFINITY;
-                    v[i][2 * j + 1] = (c < nchunk && k + 1 < valid) ? a.y + m.y : -INFINITY;
-                    mx = fmaxf(mx, fmaxf(v[i][2 * j], v[i][2 * j + 1]));
+                    v[i][j] = add2(__half22float2(sh[j]), __half22float2(mh[j]));
+                    if (2 * j >= left) v[i][j].x = -INFINITY;
+                    if (2 * j + 1 >= left) v[i][j].y = -INFINITY;
+                    mx = max3(mx, v[i][j].x, v[i][j].y);
                 }
             }
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
-            const float shift = (mx == -INFINITY) ? 0.f : mx * kLog2e;
-            float sum = 0.f;
+            mx = group_max<G>(mx);
+            const float shift = (mx == -INFINITY) ? 0.f : -mx * kLog2e;
+            const float2 l2 = make_float2(kLog2e, kLog2e), s2 = make_float2(shift, shift);
+            float2 sum2 = make_float2(0.f, 0.f);
 #pragma unroll
             for (int i = 0; i < CH; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    v[i][j] = ex2_fast(v[i][j] * kLog2e - shift);
-                    sum += v[i][j];
+                for (int j = 0; j < 4; ++j) {
+                    const float2 x = fma2(v[i][j], l2, s2);
+                    v[i][j] = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+                    sum2 = add2(sum2, v[i][j]);
                 }
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+            const float sum = group_sum<G>(sum2.x + sum2.y);
             const float inv = sum > 0.f ? 1.0f / sum : 0.f;
             if (row < nrow) {
-                uint4* sw = reinterpret_cast<uint4*>(scores + row * L);
+                uint4* sw = reinterpret_cast<uint4*>(scores + (size_t)row * L);
 #pragma unroll
                 for (int i = 0; i < CH; ++i) {
-                    const int c = lane + 32 * i;
-                    if (c < nchunk) {
-                        uint4 o;
-                        half2* oh = reinterpret_cast<half2*>(&o);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            oh[j] = __floats2half2_rn(v[i][2 * j] * inv, v[i][2 * j + 1] * inv);
-                        __stcs(sw + c, o);
-                    }
+                    const int c = lane + G * i;
+                    if (c < nchunk) __stcs(sw + c, pack_row(v[i], inv));
                 }
             }
         }
     }
 }
 
-// Rows of any length and alignment (sequence lengths are rarely multiples of 8), at most CH * 256 - 14 elements: the row is
-// covered by the 16-byte granules of memory that it touches, so that all of its traffic but the two edge granules moves in
-// aligned 16-byte accesses. Edge granules are read whole where the tensor's bounds allow (the neighbouring row's elements
-// are masked off) and written element by element. The mask row has an alignment of its own: the two granules that hold a
-// lane's eight mask values are read (the second one is the next lane's first: an L1 hit) and shifted into place.
-// HBM bound: 4 * L bytes per row. 128 matrices of 500 x 500 with a mask: 101 us by the three-pass kernel below, 25 us here.
-__device__ __forceinline__ uint4 granule(const half* p, const half* lo, const half* hi) {
-    if (p >= lo && p + 8 <= hi) return __ldg(reinterpret_cast<const uint4*>(p));
+struct RowShape { int head, granules, tail; };
+__device__ __forceinline__ RowShape row_shape(const half* row, int valid) {
+    RowShape s;
+    s.head = min((int)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) >> 1, valid);
+    s.granules = (valid - s.head) >> 3;
+    s.tail = (valid - s.head) & 7;
+    return s;
+}
+
+// The elements of a granule that lie inside [lo, hi); zeros for the others.
+__device__ __noinline__ uint4 edge_granule(const half* p, const half* lo, const half* hi) {
     __align__(16) half v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = (p + j >= lo && p + j < hi) ? p[j] : __float2half(0.f);
     return *reinterpret_cast<const uint4*>(v);
 }
-template <int CH, int R>
-__global__ void __launch_bounds__(256) softmax_mask_shift(half* __restrict__ scores, const half* __restrict__ mask, long nrow,
-                                                          int L, int valid) {
+
+template <int G, int CH, int R, bool kMask>
+__global__ void __launch_bounds__(256) softmax_mask_kernel(half* __restrict__ scores, const half* __restrict__ mask,
+                                                           unsigned nrow, int L, int valid) {
     pdl_launch_dependents();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarp = ((long)gridDim.x * blockDim.x) >> 5;
-    constexpr float kLog2e = 1.4426950408889634f;
-    const half* const send = scores + nrow * L;
-    const half* const mend = mask ? mask + (size_t)L * L : nullptr;
-    for (long row0 = warp * R; row0 < nrow; row0 += nwarp * R) {
-        uint4 sv[R][CH];
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned group = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const unsigned ngroup = (gridDim.x * blockDim.x) / G;
+    const half kNone = __ushort_as_half((unsigned short)0xfc00u);   // -inf
+    // all groups of a warp make the same number of rounds (the reductions use the whole warp)
+    const unsigned rounds = (nrow + ngroup * R - 1) / (ngroup * R);
+    for (unsigned it = 0; it < rounds; ++it) {
+        const unsigned row0 = (it * ngroup + group) * R;
+        uint4 sv[R][CH], ma[R][CH], mb[R][CH];
+        half se[R][2], me[R][2];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const half* sr = scores + (row0 + r) * L;
-            const int off = (int)((reinterpret_cast<uintptr_t>(sr) & 15) >> 1);   // elements of the first granule before the row
+            const unsigned row = row0 + r;
+            const half* sr = scores + (size_t)row * L;
+            const RowShape q = row_shape(sr, row < nrow ? valid : 0);
+            const half* const mg = mask + (size_t)(row % (unsigned)L) * L + q.head;
+            const half* const ml = reinterpret_cast<const half*>(reinterpret_cast<uintptr_t>(mg) & ~(uintptr_t)15);
+            const bool split = ml != mg;   // the second granule exists: it holds the values from the first boundary on
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
-                const int k = (lane + 32 * i) * 8 - off;
-                sv[r][i] = make_uint4(0, 0, 0, 0);
-                if (row0 + r < nrow && k < L) {
-                    const half* p = sr + k;
-                    if (p >= scores && p + 8 <= send) sv[r][i] = __ldcs(reinterpret_cast<const uint4*>(p));
-                    else sv[r][i] = granule(p, scores, send);
+                const int c = lane + G * i;
+                sv[r][i] = make_uint4(0xfc00fc00u, 0xfc00fc00u, 0xfc00fc00u, 0xfc00fc00u);
+                ma[r][i] = mb[r][i] = make_uint4(0u, 0u, 0u, 0u);
+                if (c < q.granules) {
+                    sv[r][i] = __ldcs(reinterpret_cast<const uint4*>(sr + q.head) + c);
+                    if constexpr (kMask) {
+                        // whole granules: the first one may begin in front of the row, with the previous row's end (for the
+                        // mask's first row: within the same 16 bytes as its first element), the second one end behind it
+                        if (c > 0 || row % (unsigned)L > 0 || !split) ma[r][i] = __ldg(reinterpret_cast<const uint4*>(ml) + c);
+                        else ma[r][i] = edge_granule(ml, mask, mask + (size_t)L * L);
+                        if (split) {
+                            const half* t = ml + 8 * c + 8;
+                            if (t + 8 <= mask + (size_t)L * L) mb[r][i] = __ldg(reinterpret_cast<const uint4*>(t));
+                            else mb[r][i] = edge_granule(t, mask, mask + (size_t)L * L);
+                        }
+                    }
                 }
+            }
+            se[r][0] = lane < q.head ? sr[lane] : kNone;
+            se[r][1] = lane < q.tail ? sr[q.head + 8 * q.granules + lane] : kNone;
+            me[r][0] = me[r][1] = __float2half(0.f);
+            if constexpr (kMask) {
+                if (lane < q.head) me[r][0] = __ldg(mg - q.head + lane);
+                if (lane < q.tail) me[r][1] = __ldg(mg + 8 * q.granules + lane);
             }
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const long row = row0 + r;
-            if (row >= nrow) break;
-            half* sr = scores + row * L;
-            const int off = (int)((reinterpret_cast<uintptr_t>(sr) & 15) >> 1);
-            float v[CH][8];
-            float mx = -INFINITY;
+            const unsigned row = row0 + r;
+            half* const sr = scores + (size_t)row * L;
+            const RowShape q = row_shape(sr, row < nrow ? valid : 0);
+            const int sh = !kMask ? 0
+                                         : (int)((reinterpret_cast<uintptr_t>(mask + (size_t)(row % (unsigned)L) * L + q.head) & 15) >> 1);
+            float2 v[CH][4];
+            float2 e = make_float2(__half2float(se[r][0]) + __half2float(me[r][0]), __half2float(se[r][1]) + __half2float(me[r][1]));
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
-                const int k = (lane + 32 * i) * 8 - off;
-                uint32_t m[4] = {0u, 0u, 0u, 0u};
-                if (mask && k < L) {
-                    const half* p = mask + (size_t)(row % L) * L + k;
-                    const int sh = (int)((reinterpret_cast<uintptr_t>(p) & 15) >> 1);   // the same for the whole row
-                    const uint4 a = granule(p - sh, mask, mend);
-                    const uint4 b = sh ? granule(p - sh + 8, mask, mend) : make_uint4(0, 0, 0, 0);
-                    uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                    if (sh & 4)
+                uint32_t w[8] = {ma[r][i].x, ma[r][i].y, ma[r][i].z, ma[r][i].w, mb[r][i].x, mb[r][i].y, mb[r][i].z, mb[r][i].w};
+                if constexpr (kMask) {   // the same shift for the whole row
+                    if (sh & 4) {
 #pragma unroll
-                        for (int q = 0; q < 6; ++q) w[q] = w[q + 2];
-                    if (sh & 2)
+                        for (int k = 0; k < 6; ++k) w[k] = w[k + 2];
+                    }
+                    if (sh & 2) {
 #pragma unroll
-                        for (int q = 0; q < 5; ++q) w[q] = w[q + 1];
+                        for (int k = 0; k < 5; ++k) w[k] = w[k + 1];
+                    }
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) m[q] = (sh & 1) ? __funnelshift_r(w[q], w[q + 1], 16) : w[q];
+                    for (int k = 0; k < 4; ++k) w[k] = __funnelshift_r(w[k], w[k + 1], (sh & 1) * 16);
                 }
                 const half2* xh = reinterpret_cast<const half2*>(&sv[r][i]);
-                const half2* mh = reinterpret_cast<const half2*>(m);
+                const half2* mh = reinterpret_cast<const half2*>(w);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 a = __half22float2(xh[j]), b = __half22float2(mh[j]);
-                    const int e = k + 2 * j;
-                    v[i][2 * j] = (e >= 0 && e < valid) ? a.x + b.x : -INFINITY;
-                    v[i][2 * j + 1] = (e + 1 >= 0 && e + 1 < valid) ? a.y + b.y : -INFINITY;
-                    mx = fmaxf(mx, fmaxf(v[i][2 * j], v[i][2 * j + 1]));
-                }
+                for (int j = 0; j < 4; ++j) v[i][j] = kMask ? add2(__half22float2(xh[j]), __half22float2(mh[j])) : __half22float2(xh[j]);
             }
+            float mx = fmaxf(e.x, e.y);
 #pragma unroll
-            for (int m = 16; m > 0; m >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
-            const float shift = (mx == -INFINITY) ? 0.f : mx * kLog2e;
-            float sum = 0.f;
+            for (int i = 0; i < CH; ++i)
+                mx = max3(mx, max3(v[i][0].x, v[i][0].y, fmaxf(v[i][1].x, v[i][1].y)), max3(v[i][2].x, v[i][2].y, fmaxf(v[i][3].x, v[i][3].y)));
+            mx = group_max<G>(mx);
+            const float shift = (mx == -INFINITY) ? 0.f : -mx * kLog2e;
+            const float2 l2 = make_float2(kLog2e, kLog2e), s2 = make_float2(shift, shift);
+            e = fma2(e, l2, s2);
+            e = make_float2(ex2_fast(e.x), ex2_fast(e.y));
+            float2 sum2 = e;
 #pragma unroll
             for (int i = 0; i < CH; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    v[i][j] = ex2_fast(v[i][j] * kLog2e - shift);
-                    sum += v[i][j];
+                for (int j = 0; j < 4; ++j) {
+                    const float2 x = fma2(v[i][j], l2, s2);
+                    v[i][j] = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+                    sum2 = add2(sum2, v[i][j]);
                 }
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+            const float sum = group_sum<G>(sum2.x + sum2.y);
             const float inv = sum > 0.f ? 1.0f / sum : 0.f;
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
-                const int k = (lane + 32 * i) * 8 - off;
-                if (k >= L) continue;
-                uint4 o;
-                half2* oh = reinterpret_cast<half2*>(&o);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) oh[j] = __floats2half2_rn(v[i][2 * j] * inv, v[i][2 * j + 1] * inv);
-                if (k >= 0 && k + 8 <= L) {
-                    __stcs(reinterpret_cast<uint4*>(sr + k), o);
-                } else {
-                    const half* ov = reinterpret_cast<const half*>(&o);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (k + j >= 0 && k + j < L) sr[k + j] = ov[j];
-                }
+                const int c = lane + G * i;
+                if (c < q.granules) __stcs(reinterpret_cast<uint4*>(sr + q.head) + c, pack_row(v[i], inv));
             }
+            if (lane < q.head) sr[lane] = __float2half_rn(e.x * inv);
+            if (lane < q.tail) sr[q.head + 8 * q.granules + lane] = __float2half_rn(e.y * inv);
+            if (valid < L && row < nrow)
+                for (int k = valid + lane; k < L; k += G) sr[k] = __float2half(0.f);
         }
     }
 }
@@ -215,16 +259,15 @@ __global__ void __launch_bounds__(256) softmax_mask_shift(half* __restrict__ sco
 // Rows above 2048 elements: one warp per row, three passes.
 __global__ void __launch_bounds__(256) softmax_mask_generic(half* __restrict__ scores,
                                                             const half* __restrict__ mask,
-                                                            long nrow, int L, int valid) {
+                                                            unsigned nrow, int L, int valid) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarp = ((long)gridDim.x * blockDim.x) >> 5;
-    constexpr float kLog2e = 1.4426950408889634f;
-    for (long row = warp; row < nrow; row += nwarp) {
-        half* s = scores + row * L;
-        const half* m = mask ? mask + (size_t)(row % L) * L : nullptr;
+    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned nwarp = (gridDim.x * blockDim.x) >> 5;
+    for (unsigned row = warp; row < nrow; row += nwarp) {
+        half* s = scores + (size_t)row * L;
+        const half* m = mask ? mask + (size_t)(row % (unsigned)L) * L : nullptr;
         float mx = -INFINITY;
         for (int k = lane; k < valid; k += 32)
             mx = fmaxf(mx, __half2float(s[k]) + (m ? __half2float(m[k]) : 0.f));
@@ -257,30 +300,41 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     half* s = static_cast<half*>(scores);
     const half* m = static_cast<const half*>(mask);
-    const long nrow = (long)nmat * seq_len;
-    long blocks = (nrow + 15) / 16;          // 8 warps per block, 2 rows per warp and iteration
-    const long cap = (long)sm_count() * 8;
-    if (blocks > cap) blocks = cap;
-    // Rows whose elements all sit in whole 16-byte granules take the plain form; the others the shifted one, up to the length
-    // that eight granules per lane hold wherever a row starts.
-    const bool vec = seq_len % 8 == 0 && seq_len <= 2048 && aligned16(s) && (!m || aligned16(m));
-    const int granules = (seq_len + 14) / 8;   // touched by a row at the worst alignment
-    if (!vec && granules <= 256 && (reinterpret_cast<uintptr_t>(s) & 1) == 0) {
-        if (granules <= 32) launch_pdl(softmax_mask_shift<1, 4>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
-        else if (granules <= 64) launch_pdl(softmax_mask_shift<2, 2>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
-        else if (granules <= 128) launch_pdl(softmax_mask_shift<4, 1>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
-        else launch_pdl(softmax_mask_shift<8, 1>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
-    } else if (vec) {
-        const int ch = (seq_len / 8 + 31) / 32;
-        switch (ch) {
-            case 1: launch_pdl(softmax_mask_vec<1, 2>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len); break;
-            case 2: launch_pdl(softmax_mask_vec<2, 2>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len); break;
-            case 3:
-            case 4: launch_pdl(softmax_mask_vec<4, 2>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len); break;
-            default: launch_pdl(softmax_mask_vec<8, 1>, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len); break;
-        }
-    } else {
+    ET_REQUIRE((long)nmat * seq_len < 0x7fffffffl, "et_softmax_mask: too many rows");   // 2^31 rows of one element are 4 GB
+    const unsigned nrow = (unsigned)nmat * (unsigned)seq_len;
+    // Rows in whole granules on both sides take the kernel without heads and tails. CH * G * 8 elements fit (beside a head and
+    // a tail in the other one). Two rows in flight where their registers leave enough warps: not with a shifted mask (44 us
+    // with two, 31 with one, at 128 x 500 x 500).
+    const bool vec = seq_len % 8 == 0 && aligned16(s) && (!m || aligned16(m));
+    auto run = [&](auto kernel, int group, int rows) {
+        const long groups = ((long)nrow + rows - 1) / rows;
+        const long blocks = std::min((groups * group + 255) / 256, (long)sm_count() * 8);
+        launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
+    };
+    auto pick = [&](auto masked) {
+        constexpr bool kMask = decltype(masked)::value;
+        constexpr int R = kMask ? 1 : 2;
+        if (seq_len <= 64) run(softmax_mask_kernel<8, 1, R, kMask>, 8, R);
+        else if (seq_len <= 128) run(softmax_mask_kernel<16, 1, R, kMask>, 16, R);
+        else if (seq_len <= 256) run(softmax_mask_kernel<32, 1, R, kMask>, 32, R);
+        else if (seq_len <= 512) run(softmax_mask_kernel<32, 2, R, kMask>, 32, R);
+        else if (seq_len <= 1024) run(softmax_mask_kernel<32, 4, 1, kMask>, 32, 1);
+        else run(softmax_mask_kernel<32, 8, 1, kMask>, 32, 1);
+    };
+    if (seq_len > 2048) {
+        const long blocks = std::min(((long)nrow + 7) / 8, (long)sm_count() * 8);
         launch_pdl(softmax_mask_generic, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
+    } else if (vec) {
+        if (seq_len <= 64) run(softmax_mask_vec<8, 1, 2>, 8, 2);
+        else if (seq_len <= 128) run(softmax_mask_vec<16, 1, 2>, 16, 2);
+        else if (seq_len <= 256) run(softmax_mask_vec<32, 1, 2>, 32, 2);
+        else if (seq_len <= 512) run(softmax_mask_vec<32, 2, 2>, 32, 2);
+        else if (seq_len <= 1024) run(softmax_mask_vec<32, 4, 2>, 32, 2);
+        else run(softmax_mask_vec<32, 8, 1>, 32, 1);
+    } else if (m) {
+        pick(std::true_type{});
+    } else {
+        pick(std::false_type{});
     }
     return cuda_status(cudaGetLastError(), "et_softmax_mask launch");
 }

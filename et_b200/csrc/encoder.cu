@@ -135,36 +135,95 @@ void row_spmm_cache_clear() {
 // ------------------------------------------------------------------------------ encoder layer
 enum EncoderKind { kTile = 0, kPrune = 1, kLength = 2, kPruneQKV = 3 };
 
-// The legacy default stream cannot be captured, so a layer launched there could not be replayed as a CUDA graph
-// (and its seven launches would cost the host three times as much). Calls on the legacy stream therefore run on a
-// stream of the object, ordered behind the caller's stream by one event and ahead of it by another.
-struct StreamBridge {
+// One instantiated CUDA graph per distinct call (buffers, lengths) of a layer or a stack: its launches replayed without the
+// host cost of each and without the gaps between them. The first call with a key runs directly, the second is captured, later
+// ones replay. Capture takes place on a stream of the cache's own (the legacy default stream cannot be captured); the graph is
+// launched into the caller's stream, the legacy one included.
+struct ReplayCache {
+    struct Entry {
+        std::vector<int64_t> key;
+        int seen = 0;
+        cudaGraphExec_t exec = nullptr;
+    };
+    static constexpr size_t kEntries = 8;
+    std::vector<Entry> entries;
+    std::vector<int64_t> key;      // of the call being made
+    bool on = true;
     cudaStream_t own = nullptr;
-    cudaEvent_t in = nullptr, out = nullptr;
-    ~StreamBridge() {
-        if (in) cudaEventDestroy(in);
-        if (out) cudaEventDestroy(out);
+    void drop() {
+        for (auto& r : entries)
+            if (r.exec) cudaGraphExecDestroy(r.exec);
+        entries.clear();
+    }
+    ~ReplayCache() {
+        drop();
         if (own) cudaStreamDestroy(own);
     }
-    static bool is_legacy(cudaStream_t st) { return st == nullptr || st == cudaStreamLegacy; }
-    // Returns the stream to run on, or nullptr if the bridge could not be set up (the caller then stays on `st`).
-    cudaStream_t begin(cudaStream_t st) {
-        if (!own) {
-            if (cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) != cudaSuccess ||
-                cudaEventCreateWithFlags(&in, cudaEventDisableTiming) != cudaSuccess ||
-                cudaEventCreateWithFlags(&out, cudaEventDisableTiming) != cudaSuccess) {
-                cudaGetLastError();
-                return nullptr;
+    // Runs `forward(stream)` directly or replays it, for the call that `key` describes.
+    template <typename F>
+    int run(cudaStream_t st, const char* what, F&& forward) {
+        Entry* slot = nullptr;
+        for (auto& r : entries)
+            if (r.key == key) { slot = &r; break; }
+        if (slot && slot->exec) return cuda_status(cudaGraphLaunch(slot->exec, st), what);
+        if (!slot) {
+            if (entries.size() >= kEntries) {
+                if (entries.front().exec) cudaGraphExecDestroy(entries.front().exec);
+                entries.erase(entries.begin());
             }
+            entries.push_back({key, 0, nullptr});
+            slot = &entries.back();
         }
-        if (cudaEventRecord(in, st) != cudaSuccess || cudaStreamWaitEvent(own, in, 0) != cudaSuccess) {
+        if (slot->seen++ == 0) return forward(st);
+        if ((!own && cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) != cudaSuccess) ||
+            cudaStreamBeginCapture(own, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
-            return nullptr;
+            return forward(st);
         }
-        return own;
+        const int frc = forward(own);
+        cudaGraph_t graph = nullptr;
+        const cudaError_t ce = cudaStreamEndCapture(own, &graph);
+        const bool good = frc == ET_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&slot->exec, graph, 0) == cudaSuccess;
+        if (graph) cudaGraphDestroy(graph);
+        if (!good) {
+            slot->exec = nullptr;
+            cudaGetLastError();
+            on = false;   // plain launches from now on
+            return forward(st);
+        }
+        return cuda_status(cudaGraphLaunch(slot->exec, st), what);
     }
-    void end(cudaStream_t st) {
-        if (cudaEventRecord(out, own) != cudaSuccess || cudaStreamWaitEvent(st, out, 0) != cudaSuccess) cudaGetLastError();
+};
+
+// Sequence offsets and key counts on the device (offsets of batch + 1, then counts of batch). The array grows geometrically; a
+// recorded graph holds its address as a kernel argument, so every graph recorded with the old array is dropped before it is
+// freed. A call with the lengths that the array holds already, on the stream that uploaded them, uploads nothing.
+struct LengthArray {
+    int* d = nullptr;
+    int cap = 0;
+    std::vector<int> held;
+    unsigned long long held_stream = 0;
+    ~LengthArray() { cudaFree(d); }
+    int upload(const std::vector<int>& meta, cudaStream_t st, bool captured, ReplayCache& graphs, const char* what) {
+        const int need = (int)meta.size();
+        if (captured) held.clear();   // the caller's graph uploads on every launch
+        if (cap < need) {
+            graphs.drop();
+            held.clear();
+            const int ncap = std::max(need, std::max(64, 2 * cap));
+            int* fresh = nullptr;
+            if (cudaMalloc(&fresh, sizeof(int) * (size_t)ncap) != cudaSuccess) return fail(ET_ERR_CUDA, "lengths: cudaMalloc failed");
+            cudaFree(d);   // synchronises with work still reading the old array
+            d = fresh;
+            cap = ncap;
+        }
+        unsigned long long id = 0;
+        const bool known = cudaStreamGetId(st, &id) == cudaSuccess;
+        if (known && id == held_stream && held == meta) return ET_OK;
+        const int rc = cuda_status(cudaMemcpyAsync(d, meta.data(), sizeof(int) * (size_t)need, cudaMemcpyHostToDevice, st), what);
+        held.clear();
+        if (rc == ET_OK && known && !captured) { held = meta; held_stream = id; }
+        return rc;
     }
 };
 
@@ -180,49 +239,19 @@ struct Encoder {
     half* d_ln[4] = {nullptr, nullptr, nullptr, nullptr};  // gamma1 beta1 gamma2 beta2
     std::vector<half> h_ln[4];                             // the same on the host (folded into weights by the layer stack)
     half* d_mask = nullptr;                                // [seq_len x seq_len] additive, may be null
-    int* d_lens = nullptr; int lens_cap = 0;               // cu_seqlens (batch+1) then valid_lens (batch)
+    LengthArray lens;
+    std::vector<int> meta;                                 // lengths of the call being made
     bool materialize_scores = false;
-    // Replay cache: one instantiated CUDA graph per distinct call (buffers, lengths). A layer is 7 short
-    // launches; replaying them as one graph removes the launch gaps between them.
-    struct Replay {
-        std::vector<int64_t> key;
-        int seen = 0;
-        cudaGraphExec_t exec = nullptr;
-    };
-    std::vector<Replay> replays;
-    bool use_graphs = true;
-    StreamBridge bridge;
-    void drop_replays() {
-        for (auto& r : replays)
-            if (r.exec) cudaGraphExecDestroy(r.exec);
-        replays.clear();
-    }
+    ReplayCache graphs;
     ~Encoder() {
-        drop_replays();
+        graphs.drop();
         for (auto* t : lin) tile_weight_free(t);
         tile_weight_free(qkv);
         delete rq; delete rk; delete rv;
         for (auto* p : d_ln) cudaFree(p);
         cudaFree(d_mask);
-        cudaFree(d_lens);
     }
 };
-
-// The device array of sequence offsets and key counts grows geometrically. A recorded graph holds the array's
-// address as a kernel argument, so every graph recorded with the old array is dropped before it is freed
-// (`drop` does that); the caller re-records on its next calls.
-template <typename Drop>
-static int grow_lens(int** d_lens, int* cap, int need, Drop&& drop) {
-    if (*cap >= need) return ET_OK;
-    drop();
-    int ncap = std::max(need, std::max(64, 2 * *cap));
-    int* fresh = nullptr;
-    if (cudaMalloc(&fresh, sizeof(int) * (size_t)ncap) != cudaSuccess) return fail(ET_ERR_CUDA, "lengths: cudaMalloc failed");
-    cudaFree(*d_lens);   // synchronises with work still reading the old array
-    *d_lens = fresh;
-    *cap = ncap;
-    return ET_OK;
-}
 
 static int upload_half(half** dst, const half* src_host, size_t n) {
     if (cudaMalloc(dst, n * sizeof(half)) != cudaSuccess) return fail(ET_ERR_CUDA, "encoder: cudaMalloc failed");
@@ -342,15 +371,9 @@ static int encoder_forward(Encoder* e, half* out, const half* in, half* scratch,
 struct Model {
     std::vector<Encoder*> layers;
     half* scratch = nullptr; size_t scratch_halfs = 0;
-    int* d_lens = nullptr; int lens_cap = 0;
-    struct Replay {
-        std::vector<int64_t> key;
-        int seen = 0;
-        cudaGraphExec_t exec = nullptr;
-    };
-    std::vector<Replay> replays;
-    bool use_graphs = true;
-    StreamBridge bridge;
+    LengthArray lens;
+    std::vector<int> meta;
+    ReplayCache graphs;
     // LayerNorm folded into the linears (tile and length layers): per layer the FFN1 weight folded with the layer's
     // first LayerNorm, the fused Q|K|V weight folded with the PREVIOUS layer's second LayerNorm, fp32 copies of
     // the four LayerNorm vectors; per row the partial sums that the output projection and FFN2 leave behind.
@@ -363,11 +386,6 @@ struct Model {
     std::vector<Fused> fused;
     bool fuse_ln = false;
     float* stats1 = nullptr; float* stats2 = nullptr; size_t stats_floats = 0;
-    void drop_replays() {
-        for (auto& r : replays)
-            if (r.exec) cudaGraphExecDestroy(r.exec);
-        replays.clear();
-    }
     void drop_fused() {
         for (auto& f : fused) {
             tile_weight_free(f.ffn1);
@@ -378,11 +396,10 @@ struct Model {
         fuse_ln = false;
     }
     ~Model() {
-        drop_replays();
+        graphs.drop();
         drop_fused();
         for (auto* e : layers) delete e;
         cudaFree(scratch);
-        cudaFree(d_lens);
         cudaFree(stats1);
         cudaFree(stats2);
     }
@@ -739,12 +756,24 @@ size_t et_encoder_batch_buffer_size(int kind, int d_model, int total_tokens, int
     return n * sizeof(half);
 }
 
+// Whether the stream is inside a capture of the caller's (or its state cannot be told): no graph of our own then.
+static bool in_capture(cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
 int et_encoder_run(et_encoder* enc, void* out, const void* in, void* stream) {
     ET_REQUIRE(enc && enc->e && out && in, "et_encoder_run: null pointer");
     Encoder* e = enc->e;
     ET_REQUIRE(e->buffer, "et_encoder_run: the encoder was created without a scratch buffer");
-    return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in), e->buffer, e->seq_len,
-                               nullptr, nullptr, 1, e->seq_len, static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    auto forward = [&](cudaStream_t s) {
+        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in), e->buffer, e->seq_len, nullptr,
+                                   nullptr, 1, e->seq_len, s);
+    };
+    if (!e->graphs.on || in_capture(st)) return forward(st);
+    e->graphs.key.assign({(int64_t)(intptr_t)out, (int64_t)(intptr_t)in, -1, (int64_t)e->materialize_scores});
+    return e->graphs.run(st, "et_encoder_run: graph launch", forward);
 }
 
 int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* seq_lens_host,
@@ -755,16 +784,8 @@ int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (batch == 0) return ET_OK;
     ET_REQUIRE(seq_lens_host, "et_encoder_run_batch: null seq_lens");
-    if (e->use_graphs && et::StreamBridge::is_legacy(st)) {
-        // the legacy default stream cannot be captured: run on the encoder's own stream, ordered by events
-        cudaStream_t own = e->bridge.begin(st);
-        if (own) {
-            const int rc = et_encoder_run_batch(enc, out, in, seq_lens_host, valid_lens_host, batch, scratch, scratch_bytes, own);
-            e->bridge.end(st);
-            return rc;
-        }
-    }
-    std::vector<int> meta(2 * batch + 1);
+    std::vector<int>& meta = e->meta;
+    meta.resize(2 * (size_t)batch + 1);
     meta[0] = 0;
     bool uniform = true;
     int max_len = 0;
@@ -784,67 +805,23 @@ int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* 
     ET_REQUIRE(scratch_bytes >= need * sizeof(half), "et_encoder_run_batch: scratch buffer too small");
     const int* cu = nullptr;
     const int* vl = nullptr;
+    const bool capturing = in_capture(st);
     if (!uniform || valid_lens_host) {
-        int rc = et::grow_lens(&e->d_lens, &e->lens_cap, 2 * batch + 1, [e] { e->drop_replays(); });
+        const int rc = e->lens.upload(meta, st, capturing, e->graphs, "et_encoder_run_batch: lengths upload");
         if (rc) return rc;
-        rc = et::cuda_status(cudaMemcpyAsync(e->d_lens, meta.data(), sizeof(int) * (2 * batch + 1),
-                                                 cudaMemcpyHostToDevice, st), "et_encoder_run_batch: lengths upload");
-        if (rc) return rc;
-        if (!uniform) cu = e->d_lens;
-        if (valid_lens_host) vl = e->d_lens + batch + 1;
+        if (!uniform) cu = e->lens.d;
+        if (valid_lens_host) vl = e->lens.d + batch + 1;
     }
-    // First call with given buffers and lengths runs directly, the second is captured into a graph, later ones
-    // replay it. Skipped while the caller's stream is itself being captured.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!e->use_graphs || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in),
-                                   static_cast<half*>(scratch), T, cu, vl, batch, uniform ? seq_lens_host[0] : 0, st, max_len);
-    std::vector<int64_t> key = {(int64_t)(intptr_t)out, (int64_t)(intptr_t)in, (int64_t)(intptr_t)scratch,
-                                (int64_t)batch, (int64_t)(valid_lens_host != nullptr), (int64_t)e->materialize_scores,
-                                (int64_t)(intptr_t)e->d_lens};
-    for (int v : meta) key.push_back(v);
-    Encoder::Replay* slot = nullptr;
-    for (auto& r : e->replays)
-        if (r.key == key) slot = &r;
-    if (!slot) {
-        if (e->replays.size() >= 8) {
-            if (e->replays.front().exec) cudaGraphExecDestroy(e->replays.front().exec);
-            e->replays.erase(e->replays.begin());
-        }
-        e->replays.push_back({key, 0, nullptr});
-        slot = &e->replays.back();
-    }
-    if (slot->exec) return et::cuda_status(cudaGraphLaunch(slot->exec, st), "et_encoder_run_batch: graph launch");
-    if (slot->seen++ == 0)
-        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in),
-                                   static_cast<half*>(scratch), T, cu, vl, batch, uniform ? seq_lens_host[0] : 0, st, max_len);
-    if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        cudaGetLastError();
-        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in),
-                                   static_cast<half*>(scratch), T, cu, vl, batch, uniform ? seq_lens_host[0] : 0, st, max_len);
-    }
-    const int frc = et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in),
-                                        static_cast<half*>(scratch), T, cu, vl, batch,
-                                        uniform ? seq_lens_host[0] : 0, st, max_len);
-    cudaGraph_t graph = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-    if (frc != ET_OK || ce != cudaSuccess || !graph) {
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
-        e->use_graphs = false;   // fall back to plain launches for this encoder
-        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in),
-                                   static_cast<half*>(scratch), T, cu, vl, batch, uniform ? seq_lens_host[0] : 0, st, max_len);
-    }
-    const cudaError_t ie = cudaGraphInstantiate(&slot->exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ie != cudaSuccess) {
-        slot->exec = nullptr;
-        cudaGetLastError();
-        e->use_graphs = false;
-        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in),
-                                   static_cast<half*>(scratch), T, cu, vl, batch, uniform ? seq_lens_host[0] : 0, st, max_len);
-    }
-    return et::cuda_status(cudaGraphLaunch(slot->exec, st), "et_encoder_run_batch: graph launch");
+    auto forward = [&](cudaStream_t s) {
+        return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in), static_cast<half*>(scratch), T, cu, vl,
+                                   batch, uniform ? seq_lens_host[0] : 0, s, max_len);
+    };
+    if (!e->graphs.on || capturing) return forward(st);
+    std::vector<int64_t>& key = e->graphs.key;
+    key.assign({(int64_t)(intptr_t)out, (int64_t)(intptr_t)in, (int64_t)(intptr_t)scratch, (int64_t)batch,
+                (int64_t)(valid_lens_host != nullptr), (int64_t)e->materialize_scores, (int64_t)(intptr_t)e->lens.d});
+    key.insert(key.end(), meta.begin(), meta.end());
+    return e->graphs.run(st, "et_encoder_run_batch: graph launch", forward);
 }
 
 // Reads and clears the error words of every kernel the layer launches: the tile GEMMs' (one per owned weight) and
@@ -893,7 +870,7 @@ int et_attention_check(int* code) {
 
 int et_encoder_set_graph_replay(et_encoder* enc, int on) {
     ET_REQUIRE(enc && enc->e, "et_encoder_set_graph_replay: null encoder");
-    enc->e->use_graphs = on != 0;
+    enc->e->graphs.on = on != 0;
     return ET_OK;
 }
 
@@ -923,7 +900,7 @@ int et_model_create(et_model** out, et_encoder* const* layers, int n_layers) {
 int et_model_set_layernorm_fusion(et_model* model, int on) {
     ET_REQUIRE(model && model->m, "et_model_set_layernorm_fusion: null model");
     et::Model* m = model->m;
-    m->drop_replays();
+    m->graphs.drop();
     if (!on) { m->drop_fused(); return ET_OK; }
     return et::model_prepare_fusion(m);
 }
@@ -961,7 +938,7 @@ int et_model_check(et_model* model, int* code) {
 
 int et_model_set_graph_replay(et_model* model, int on) {
     ET_REQUIRE(model && model->m, "et_model_set_graph_replay: null model");
-    model->m->use_graphs = on != 0;
+    model->m->graphs.on = on != 0;
     return ET_OK;
 }
 
@@ -975,14 +952,14 @@ int et_model_reserve(et_model* model, int total_tokens, int batch, int max_len) 
     size_t need_stats = 0;
     for (const auto& f : m->fused) need_stats = std::max(need_stats, (size_t)total_tokens * std::max(f.np1, f.np2) * 2);
     if (need > m->scratch_halfs) {
-        m->drop_replays();
+        m->graphs.drop();
         cudaFree(m->scratch);
         m->scratch = nullptr; m->scratch_halfs = 0;
         if (cudaMalloc(&m->scratch, need * sizeof(half)) != cudaSuccess) return et::fail(ET_ERR_CUDA, "et_model_reserve: cudaMalloc failed");
         m->scratch_halfs = need;
     }
     if (need_stats > m->stats_floats) {
-        m->drop_replays();
+        m->graphs.drop();
         cudaFree(m->stats1); cudaFree(m->stats2);
         m->stats1 = m->stats2 = nullptr; m->stats_floats = 0;
         if (cudaMalloc(&m->stats1, need_stats * sizeof(float)) != cudaSuccess || cudaMalloc(&m->stats2, need_stats * sizeof(float)) != cudaSuccess)
@@ -1000,16 +977,8 @@ int et_model_run_batch(et_model* model, void* out, const void* in, const int* se
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (batch == 0) return ET_OK;
     ET_REQUIRE(seq_lens_host, "et_model_run_batch: null seq_lens");
-    if (m->use_graphs && et::StreamBridge::is_legacy(st)) {
-        // the legacy default stream cannot be captured: run on the model's own stream, ordered by events
-        cudaStream_t own = m->bridge.begin(st);
-        if (own) {
-            const int rc = et_model_run_batch(model, out, in, seq_lens_host, valid_lens_host, batch, own);
-            m->bridge.end(st);
-            return rc;
-        }
-    }
-    std::vector<int> meta(2 * batch + 1);
+    std::vector<int>& meta = m->meta;
+    meta.resize(2 * (size_t)batch + 1);
     meta[0] = 0;
     bool uniform = true;
     int max_len = 0;
@@ -1024,8 +993,7 @@ int et_model_run_batch(et_model* model, void* out, const void* in, const int* se
     }
     const int T = meta[batch];
     if (T == 0) return ET_OK;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool capturing = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    const bool capturing = in_capture(st);
     if (capturing) {
         // inside the caller's own capture nothing may be allocated or uploaded from a temporary
         size_t need_stats = 0;
@@ -1040,58 +1008,22 @@ int et_model_run_batch(et_model* model, void* out, const void* in, const int* se
     const int* cu = nullptr;
     const int* vl = nullptr;
     if (!uniform || valid_lens_host) {
-        int rc = et::grow_lens(&m->d_lens, &m->lens_cap, 2 * batch + 1, [m] { m->drop_replays(); });
+        const int rc = m->lens.upload(meta, st, capturing, m->graphs, "et_model_run_batch: lengths upload");
         if (rc) return rc;
-        rc = et::cuda_status(cudaMemcpyAsync(m->d_lens, meta.data(), sizeof(int) * (2 * batch + 1),
-                                                 cudaMemcpyHostToDevice, st), "et_model_run_batch: lengths upload");
-        if (rc) return rc;
-        if (!uniform) cu = m->d_lens;
-        if (valid_lens_host) vl = m->d_lens + batch + 1;
+        if (!uniform) cu = m->lens.d;
+        if (valid_lens_host) vl = m->lens.d + batch + 1;
     }
-    half* o = static_cast<half*>(out);
-    const half* x = static_cast<const half*>(in);
-    const int ul = uniform ? seq_lens_host[0] : 0;
-    if (!m->use_graphs || capturing) return et::model_forward(m, o, x, T, cu, vl, batch, ul, st, max_len);
-    // First call with given buffers and lengths runs directly, the second is captured, later ones replay.
-    std::vector<int64_t> key = {(int64_t)(intptr_t)out, (int64_t)(intptr_t)in, (int64_t)batch,
-                                (int64_t)(valid_lens_host != nullptr), (int64_t)(intptr_t)m->d_lens};
+    auto forward = [&](cudaStream_t s) {
+        return et::model_forward(m, static_cast<half*>(out), static_cast<const half*>(in), T, cu, vl, batch,
+                                 uniform ? seq_lens_host[0] : 0, s, max_len);
+    };
+    if (!m->graphs.on || capturing) return forward(st);
+    std::vector<int64_t>& key = m->graphs.key;
+    key.assign({(int64_t)(intptr_t)out, (int64_t)(intptr_t)in, (int64_t)batch, (int64_t)(valid_lens_host != nullptr),
+                (int64_t)(intptr_t)m->lens.d});
     for (Encoder* e : m->layers) key.push_back((int64_t)e->materialize_scores);
-    for (int v : meta) key.push_back(v);
-    et::Model::Replay* slot = nullptr;
-    for (auto& r : m->replays)
-        if (r.key == key) slot = &r;
-    if (!slot) {
-        if (m->replays.size() >= 8) {
-            if (m->replays.front().exec) cudaGraphExecDestroy(m->replays.front().exec);
-            m->replays.erase(m->replays.begin());
-        }
-        m->replays.push_back({key, 0, nullptr});
-        slot = &m->replays.back();
-    }
-    if (slot->exec) return et::cuda_status(cudaGraphLaunch(slot->exec, st), "et_model_run_batch: graph launch");
-    if (slot->seen++ == 0) return et::model_forward(m, o, x, T, cu, vl, batch, ul, st, max_len);
-    if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        cudaGetLastError();
-        return et::model_forward(m, o, x, T, cu, vl, batch, ul, st, max_len);
-    }
-    const int frc = et::model_forward(m, o, x, T, cu, vl, batch, ul, st, max_len);
-    cudaGraph_t graph = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-    if (frc != ET_OK || ce != cudaSuccess || !graph) {
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
-        m->use_graphs = false;   // plain launches from now on
-        return et::model_forward(m, o, x, T, cu, vl, batch, ul, st, max_len);
-    }
-    const cudaError_t ie = cudaGraphInstantiate(&slot->exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ie != cudaSuccess) {
-        slot->exec = nullptr;
-        cudaGetLastError();
-        m->use_graphs = false;
-        return et::model_forward(m, o, x, T, cu, vl, batch, ul, st, max_len);
-    }
-    return et::cuda_status(cudaGraphLaunch(slot->exec, st), "et_model_run_batch: graph launch");
+    key.insert(key.end(), meta.begin(), meta.end());
+    return m->graphs.run(st, "et_model_run_batch: graph launch", forward);
 }
 
 }  // extern "C"

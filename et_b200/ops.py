@@ -3,11 +3,12 @@
 Tensors are torch CUDA fp16/int32 tensors; host arrays are numpy. Nothing here computes: every
 function forwards to `libet_b200.so`.
 """
+import array
 import ctypes
 
 import numpy as np
 
-from . import check, lib, ptr, stream_ptr
+from . import check, lib, ptr, raw_stream
 
 __all__ = [
     "skip_layernorm", "softmax_mask", "TileWeight", "tile_spmm_bias", "tile_spmm_cache_clear",
@@ -21,11 +22,65 @@ __all__ = [
 _i = ctypes.c_int
 
 
+# The entry points that are called per launch, with their argument types declared: ctypes then converts plain numbers by
+# itself, which costs a third of building a c_void_p / c_int object for every argument (p = pointer, i = int, s = size_t).
+_SIGNATURES = {
+    "et_skip_layernorm": "ppppiip", "et_softmax_mask": "ppiiip", "et_tile_linear": "pppiip", "et_row_linear": "pppip",
+    "et_tile_spmm_bias": "pppppiiipip", "et_attention_otf": "pppppiiip", "et_attention_prune": "ppppppipiiip",
+    "et_qk_scores": "pppiiip", "et_attention_sharedqk": "ppppiiip", "et_attention_static_scores": "pppppiiip",
+    "et_attention_batch": "ppppiippppippiiiiiip", "et_encoder_run": "pppp", "et_encoder_run_batch": "pppppipsp",
+    "et_model_run_batch": "pppppip",
+}
+
+
+class _Entries:
+    """One attribute per entry point of _SIGNATURES, bound on first use of the library."""
+    __slots__ = tuple(_SIGNATURES)
+
+    def __init__(self):
+        types = {"p": ctypes.c_void_p, "i": ctypes.c_int, "s": ctypes.c_size_t}
+        for name, signature in _SIGNATURES.items():
+            fn = lib()[name]   # a function object of its own: argument types of lib().<name> stay undeclared
+            fn.argtypes = [types[c] for c in signature]
+            fn.restype = ctypes.c_int
+            setattr(self, name, fn)
+
+
+_entries = None
+
+
+def _lib():
+    global _entries
+    if _entries is None:
+        _entries = _Entries()
+    return _entries
+
+
+def _a(t):
+    """Address of a torch tensor, a numpy array, or None."""
+    if t is None:
+        return None
+    try:
+        return t.data_ptr()
+    except AttributeError:
+        return ptr(t).value
+
+
+def _ints(values):
+    """(address, count, owner) of a sequence of whole numbers as C ints."""
+    if type(values) is list or type(values) is tuple:
+        a = array.array("i", values)
+        return a.buffer_info()[0], len(a), a
+    a = np.ascontiguousarray(values, dtype=np.int32)
+    return a.ctypes.data, len(a), a
+
+
 def skip_layernorm(in_out, skip, gamma, beta, stream=None):
     """in_out[num, size] <- LN(in_out + skip) * gamma + beta, in place."""
     num, size = in_out.shape
-    check(lib().et_skip_layernorm(ptr(in_out), ptr(skip), ptr(gamma), ptr(beta), _i(num), _i(size),
-                                  stream_ptr(stream)))
+    rc = (_entries or _lib()).et_skip_layernorm(_a(in_out), _a(skip), _a(gamma), _a(beta), num, size, raw_stream(stream))
+    if rc:
+        check(rc)
     return in_out
 
 
@@ -33,8 +88,10 @@ def softmax_mask(scores, mask=None, valid_len=None, stream=None):
     """scores[nmat, L, L] <- softmax(scores + mask) per row, in place."""
     nmat, L, L2 = scores.shape
     assert L == L2
-    check(lib().et_softmax_mask(ptr(scores), ptr(mask), _i(nmat), _i(L),
-                                _i(L if valid_len is None else valid_len), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_softmax_mask(_a(scores), _a(mask), nmat, L, L if valid_len is None else valid_len,
+                                              raw_stream(stream))
+    if rc:
+        check(rc)
     return scores
 
 
@@ -72,8 +129,9 @@ class TileWeight:
     def run(self, out, x, gelu=None, stream=None):
         tokens = x.shape[0]
         g = self.is_gelu if gelu is None else gelu
-        check(lib().et_tile_linear(self._h, ptr(out), ptr(x), _i(tokens), _i(1 if g else 0),
-                                   stream_ptr(stream)))
+        rc = (_entries or _lib()).et_tile_linear(self._h, _a(out), _a(x), tokens, 1 if g else 0, raw_stream(stream))
+        if rc:
+            check(rc)
         return out
 
     def check(self):
@@ -101,8 +159,10 @@ def tile_spmm_bias(Y, X, row_ptr, row_offset, data, bias, K=None, gelu=False, st
     """Launcher-level entry with device-resident tile arrays (packed form cached by address)."""
     M, N = Y.shape
     K = X.shape[1] if K is None else K
-    check(lib().et_tile_spmm_bias(ptr(Y), ptr(X), ptr(row_ptr), ptr(row_offset), ptr(data), _i(M),
-                                  _i(N), _i(K), ptr(bias), _i(1 if gelu else 0), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_tile_spmm_bias(_a(Y), _a(X), _a(row_ptr), _a(row_offset), _a(data), M, N, K, _a(bias),
+                                                1 if gelu else 0, raw_stream(stream))
+    if rc:
+        check(rc)
     return Y
 
 
@@ -132,7 +192,9 @@ class RowWeight:
         self.head_ptr = np.array(list(hph), dtype=np.int32)
 
     def run(self, out, x, stream=None):
-        check(lib().et_row_linear(self._h, ptr(out), ptr(x), _i(x.shape[0]), stream_ptr(stream)))
+        rc = (_entries or _lib()).et_row_linear(self._h, _a(out), _a(x), x.shape[0], raw_stream(stream))
+        if rc:
+            check(rc)
         return out
 
     def close(self):
@@ -149,33 +211,40 @@ class RowWeight:
 
 # ---------------------------------------------------------------------------------- attention
 def attention_otf(out, Q, K, V, mask, seq_len, d_model, nhead, stream=None):
-    check(lib().et_attention_otf(ptr(out), ptr(Q), ptr(K), ptr(V), ptr(mask), _i(seq_len), _i(d_model),
-                                 _i(nhead), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_attention_otf(_a(out), _a(Q), _a(K), _a(V), _a(mask), seq_len, d_model, nhead, raw_stream(stream))
+    if rc:
+        check(rc)
     return out
 
 
 def attention_prune(out, Q, K, V, v_col_id, v_head_ptr, nnz_col_v, mask, seq_len, d_model, nhead, stream=None):
-    check(lib().et_attention_prune(ptr(out), ptr(Q), ptr(K), ptr(V), ptr(v_col_id), ptr(v_head_ptr),
-                                   _i(nnz_col_v), ptr(mask), _i(seq_len), _i(d_model), _i(nhead),
-                                   stream_ptr(stream)))
+    rc = (_entries or _lib()).et_attention_prune(_a(out), _a(Q), _a(K), _a(V), _a(v_col_id), _a(v_head_ptr), nnz_col_v, _a(mask),
+                                                 seq_len, d_model, nhead, raw_stream(stream))
+    if rc:
+        check(rc)
     return out
 
 
 def qk_scores(QK, Q, K, seq_len, d_model, nhead, stream=None):
-    check(lib().et_qk_scores(ptr(QK), ptr(Q), ptr(K), _i(seq_len), _i(d_model), _i(nhead), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_qk_scores(_a(QK), _a(Q), _a(K), seq_len, d_model, nhead, raw_stream(stream))
+    if rc:
+        check(rc)
     return QK
 
 
 def attention_sharedqk(out, QK, V, mask, seq_len, d_model, nhead, stream=None):
-    check(lib().et_attention_sharedqk(ptr(out), ptr(QK), ptr(V), ptr(mask), _i(seq_len), _i(d_model),
-                                      _i(nhead), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_attention_sharedqk(_a(out), _a(QK), _a(V), _a(mask), seq_len, d_model, nhead, raw_stream(stream))
+    if rc:
+        check(rc)
     return out
 
 
 def attention_static_scores(out, Q, K, V, mask, seq_len, d_model, nhead, stream=None):
     """et_attention_otf's result through the library's built-in score buffer: allocates nothing."""
-    check(lib().et_attention_static_scores(ptr(out), ptr(Q), ptr(K), ptr(V), ptr(mask), _i(seq_len), _i(d_model),
-                                           _i(nhead), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_attention_static_scores(_a(out), _a(Q), _a(K), _a(V), _a(mask), seq_len, d_model, nhead,
+                                                         raw_stream(stream))
+    if rc:
+        check(rc)
     return out
 
 
@@ -190,12 +259,12 @@ def attention_batch(out, Q, K, V, d_model, nhead, cu_seqlens=None, valid_lens=No
                     max_seq_len=0, total_tokens=None, mask=None, mask_ld=0, qk_pitch=None, v_pitch=None, qk_head_ptr=None,
                     v_col_id=None, v_head_ptr=None, stream=None):
     total = Q.shape[0] if total_tokens is None else total_tokens
-    check(lib().et_attention_batch(ptr(out), ptr(Q), ptr(K), ptr(V),
-                                   _i(Q.shape[1] if qk_pitch is None else qk_pitch),
-                                   _i(V.shape[1] if v_pitch is None else v_pitch), ptr(qk_head_ptr),
-                                   ptr(v_col_id), ptr(v_head_ptr), ptr(mask), _i(mask_ld), ptr(cu_seqlens),
-                                   ptr(valid_lens), _i(batch), _i(uniform_len), _i(max_seq_len), _i(total), _i(d_model),
-                                   _i(nhead), stream_ptr(stream)))
+    rc = (_entries or _lib()).et_attention_batch(
+        _a(out), _a(Q), _a(K), _a(V), Q.shape[1] if qk_pitch is None else qk_pitch, V.shape[1] if v_pitch is None else v_pitch,
+        _a(qk_head_ptr), _a(v_col_id), _a(v_head_ptr), _a(mask), mask_ld, _a(cu_seqlens), _a(valid_lens), batch, uniform_len,
+        max_seq_len, total, d_model, nhead, raw_stream(stream))
+    if rc:
+        check(rc)
     return out
 
 
@@ -271,15 +340,18 @@ class Encoder:
             raise ValueError("unknown encoder kind")
 
     def run(self, out, x, stream=None):
-        check(lib().et_encoder_run(self._h, ptr(out), ptr(x), stream_ptr(stream)))
+        rc = (_entries or _lib()).et_encoder_run(self._h, _a(out), _a(x), raw_stream(stream))
+        if rc:
+            check(rc)
         return out
 
     def run_batch(self, out, x, seq_lens, scratch, valid_lens=None, stream=None):
-        seq_lens = np.ascontiguousarray(seq_lens, dtype=np.int32)
-        valid = None if valid_lens is None else np.ascontiguousarray(valid_lens, dtype=np.int32)
-        check(lib().et_encoder_run_batch(self._h, ptr(out), ptr(x), ptr(seq_lens), ptr(valid), _i(len(seq_lens)),
-                                         ptr(scratch), ctypes.c_size_t(scratch.numel() * scratch.element_size()),
-                                         stream_ptr(stream)))
+        lens, n, keep = _ints(seq_lens)
+        valid, _, keep_valid = (None, 0, None) if valid_lens is None else _ints(valid_lens)
+        rc = (_entries or _lib()).et_encoder_run_batch(self._h, _a(out), _a(x), lens, valid, n, _a(scratch),
+                                                       scratch.numel() * scratch.element_size(), raw_stream(stream))
+        if rc:
+            check(rc)
         return out
 
     def check(self):
@@ -323,10 +395,11 @@ class Model:
         check(lib().et_model_reserve(self._h, _i(total_tokens), _i(batch), _i(max_len)))
 
     def run_batch(self, out, x, seq_lens, valid_lens=None, stream=None):
-        seq_lens = np.ascontiguousarray(seq_lens, dtype=np.int32)
-        valid = None if valid_lens is None else np.ascontiguousarray(valid_lens, dtype=np.int32)
-        check(lib().et_model_run_batch(self._h, ptr(out), ptr(x), ptr(seq_lens), ptr(valid), _i(len(seq_lens)),
-                                       stream_ptr(stream)))
+        lens, n, keep = _ints(seq_lens)
+        valid, _, keep_valid = (None, 0, None) if valid_lens is None else _ints(valid_lens)
+        rc = (_entries or _lib()).et_model_run_batch(self._h, _a(out), _a(x), lens, valid, n, raw_stream(stream))
+        if rc:
+            check(rc)
         return out
 
     def set_layernorm_fusion(self, on):

@@ -1,0 +1,549 @@
+// Dense linear  Y[T x N] = X[T x K] . W^T + bias  (optional tanh-GELU) on tcgen05: what a tile-pruned or row-pruned weight
+// becomes when the multiplications with its zero tiles cost less than skipping them (the rule is in tile_gemm.cu).
+// Replaces, for those weights, kernels/linear.cu:5-34 (row-pruned) and :54-167 (tile-pruned) of the reference.
+//
+// Two kernels. Both keep X and W in panels of 64 K elements, 128-byte-swizzled in shared memory (one TMA copy each), one or two
+// panels to a stage, and accumulate in fp32 in tensor memory with both UMMA operands from shared memory. A stage costs the
+// issuing warp ~400 clocks beside its UMMAs (a wait that finds its barrier complete, fences, commits), hence two panels where
+// a panel's UMMAs are short; wide tiles take one, for more stages.
+//
+// dense_kernel, many tiles: persistent pairs of CTAs (cta_group::2, UMMAs 256 x BN x 16): each CTA of a pair copies its own 128
+// tokens and half of the weight's rows, so that a 256 x 256 tile needs 32 KB per CTA and 512 clocks of UMMA time. What bounds a
+// dense linear otherwise is the way from L2: with one CTA per 128 x 256 tile an SM asks for 94 bytes per clock and gets ~58
+// (measured, all SMs busy). Four warps copy, one (of the pair's first CTA) issues, eight convert and store; two accumulators,
+// so that a tile is stored while the next one is multiplied. 16384 x 4096 x 1024: tensor pipe 90 % busy.
+//
+// dense_split_kernel, few tiles (small batches): the K range is split over a thread-block cluster. Each CTA accumulates its
+// share, leaves the fp32 partial tile in its shared memory, and after a cluster barrier sums 1/cluster of the rows over
+// all partials in rank order (distributed shared memory, no atomics: results do not depend on timing). 128 tokens, 3072
+// inputs, 768 outputs: 12 CTAs walking 24 chunks of 128 each took 18.8 us in the tile kernel, 8.8 us here.
+//
+// The weight does not depend on the preceding kernel: its first copies are requested before griddepcontrol.wait.
+// Every mbarrier wait is bounded; a role that gives up records a code, and all threads reach the common exit (and the
+// cluster barriers) whatever happened.
+#include <algorithm>
+#include "common.h"
+#include "dense_gemm.h"
+#include "epilogue.cuh"
+#include "ptx.cuh"
+#include "tmap.h"
+
+namespace et {
+
+namespace {
+
+constexpr int kBM = 128;                  // tokens per CTA
+constexpr int kBK = 64;                   // K elements per panel: one 128-byte-swizzled row
+constexpr int kAPanel = kBM * kBK * 2;    // 16 KB
+constexpr int kEpiWarps = 8;
+constexpr int kUnitCols = 32;             // columns per epilogue store
+constexpr int kUnitBytes = 32 * kUnitCols * 2;
+constexpr int kMaxStages = 8;
+// Copying warps take the stages in turn. A stage must always fall to the same warp: a parity wait is only safe for a waiter
+// that has seen the barrier's previous phase, so the number of warps at work divides the number of stages (copy_warps).
+constexpr int kCopyWarps = 4;
+constexpr int kFirstEpi = kCopyWarps + 1;
+constexpr int kThreads = 32 * (kFirstEpi + kEpiWarps);
+constexpr int kSmemMax = 232448;
+constexpr int kMaxBN = 256;
+
+struct DenseParams {
+    const half* bias;
+    half* Y;
+    int T, N, k_panels, tiles_n, tiles, bn, stages, panels;   // panels: per stage; the last stage of a K range may hold fewer
+    int* err;
+};
+
+__host__ __device__ constexpr int copy_warps(int stages) {
+    return stages % 4 == 0 ? 4 : stages % 3 == 0 ? 3 : stages % 2 == 0 ? 2 : 1;
+}
+// The largest ring of at most n stages that several warps can share.
+inline int ring_stages(int n) { return n >= 8 ? 8 : n == 7 ? 6 : n == 5 ? 4 : n; }
+
+struct DenseShared {
+    uint64_t full[kMaxStages], empty[kMaxStages];
+    uint64_t acc_full[2], acc_empty[2];
+    uint32_t tmem_base;
+    volatile int abort;
+    __align__(16) half bias[2][kMaxBN];
+};
+
+// Columns to allocate for `n` (a power of two, at least 32).
+__device__ __forceinline__ uint32_t tmem_cols(int n) {
+    uint32_t c = 32;
+    while ((int)c < n) c <<= 1;
+    return c;
+}
+__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory"); }
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of the same shared-memory object in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t in_cta(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+// A copy into this CTA's shared memory that reports to a barrier of either CTA of the pair (cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(tmap), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Arrives on the barrier at this address in both CTAs of the pair once every UMMA issued so far has completed.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+template <bool kGelu>
+__global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
+                                                            const __grid_constant__ CUtensorMap tmY, const __grid_constant__ DenseParams p) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int S = p.stages, bn = p.bn;
+    const int b_panel = bn * kBK;   // bytes: half of the tile's features
+    const int stage_bytes = p.panels * (kAPanel + b_panel);
+    const int k_stages = (p.k_panels + p.panels - 1) / p.panels;
+    uint8_t* const epi = smem + (size_t)S * stage_bytes;
+    DenseShared* const sh = reinterpret_cast<DenseShared*>(epi + kEpiWarps * kUnitBytes);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_rank();
+    const int pair = (int)blockIdx.x >> 1, G = (int)gridDim.x >> 1;
+    const int my_tiles = (p.tiles - pair + G - 1) / G;
+    if (tid == 0) {
+        for (int i = 0; i < S; ++i) { mbar_init(&sh->full[i], 1); mbar_init(&sh->empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&sh->acc_full[i], 1); mbar_init(&sh->acc_empty[i], 2 * kEpiWarps); }
+        sh->abort = 0;
+        fence_mbar_init();
+        prefetch_tmap(&tmX);
+        prefetch_tmap(&tmW);
+    }
+    if (warp == kCopyWarps) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"(tmem_cols(2 * bn))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // the other CTA's barriers exist
+    tc_fence_after();
+    const uint32_t tmem = sh->tmem_base;
+
+    if (warp < kCopyWarps) {
+        // ---- copies, stages in turn; both CTAs' report to the first one's barriers
+        bool ok = true;
+        const int cw = copy_warps(S);
+        const int ahead = min(S, k_stages);   // weight panels of the first tile's first stages, requested before the wait
+        auto load_w = [&](int s, int kc, int tile) {
+            const int np = min(p.panels, p.k_panels - kc * p.panels);
+            const uint32_t bar = in_cta(&sh->full[s], 0);
+            if (rank == 0) mbar_expect_tx(&sh->full[s], 2 * np * (kAPanel + b_panel));
+            for (int i = 0; i < np; ++i)
+                tma_load_2d_pair(smem + (size_t)s * stage_bytes + p.panels * kAPanel + i * b_panel, &tmW, (kc * p.panels + i) * kBK,
+                                 (tile % p.tiles_n) * bn + (int)rank * (bn / 2), bar);
+        };
+        if (warp < cw && lane == 0)
+            for (int i = warp; i < ahead; i += cw) load_w(i, i, pair);
+        __syncwarp();
+        pdl_wait();
+        int tl = 0, kc = warp, s = warp;
+        uint32_t ph = 1;
+        for (int c = warp; warp < cw && c < my_tiles * k_stages; c += cw) {
+            while (kc >= k_stages) { kc -= k_stages; ++tl; }
+            if (s >= S) { s -= S; ph ^= 1u; }
+            const int tile = pair + tl * G;
+            ok = mbar_wait(&sh->empty[s], ph);
+            if (!ok) break;
+            if (lane == 0) {
+                if (c >= ahead) load_w(s, kc, tile);
+                const int np = min(p.panels, p.k_panels - kc * p.panels);
+                const uint32_t bar = in_cta(&sh->full[s], 0);
+                for (int i = 0; i < np; ++i)
+                    tma_load_2d_pair(smem + (size_t)s * stage_bytes + i * kAPanel, &tmX, (kc * p.panels + i) * kBK,
+                                     (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM, bar);
+            }
+            __syncwarp();
+            kc += cw;
+            s += cw;
+        }
+        // (On the normal way out every copy has been consumed: the accumulators of the last tile are complete. A wait that gives
+        // up has lasted far longer than any copy.)
+        if (!ok && lane == 0) {
+            atomicExch(p.err, 31);
+            sh->abort = 1;
+        }
+    } else if (warp == kCopyWarps && rank == 0) {
+        // ---- UMMAs of the pair
+        const uint32_t idesc = make_idesc_f16(2 * kBM, bn);
+        const uint64_t a0 = make_smem_desc(smem_u32(smem), 16, 1024, 2);
+        const uint64_t b0 = make_smem_desc(smem_u32(smem) + p.panels * kAPanel, 16, 1024, 2);
+        bool ok = true;
+        int s = 0;
+        uint32_t ph = 0;
+        for (int tl = 0; tl < my_tiles && ok; ++tl) {
+            const int buf = tl & 1;
+            ok = mbar_wait(&sh->acc_empty[buf], ((uint32_t)(tl >> 1) & 1u) ^ 1u);
+            if (!ok) break;
+            tc_fence_after();
+            for (int kc = 0; kc < k_stages; ++kc) {
+                ok = mbar_wait(&sh->full[s], ph);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t at = (uint64_t)(s * stage_bytes) >> 4;   // descriptors count 16-byte units
+                    const int np = min(p.panels, p.k_panels - kc * p.panels);
+                    for (int i = 0; i < np; ++i)
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_f16_pair(tmem + buf * bn, a0 + at + (i * kAPanel >> 4) + ks * 2, b0 + at + (i * b_panel >> 4) + ks * 2,
+                                          idesc, (kc > 0 || i > 0 || ks > 0) ? 1u : 0u);
+                    umma_commit_pair(&sh->empty[s]);
+                    if (kc + 1 == k_stages) umma_commit_pair(&sh->acc_full[buf]);
+                }
+                __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1u; }
+            }
+        }
+        if (!ok && lane == 0) {
+            atomicExch(p.err, 32);
+            sh->abort = 1;
+        }
+    } else if (warp >= kFirstEpi) {
+        // ---- convert and store this CTA's 128 tokens: two warps per 32 rows take the tile's 32-column units in turn
+        const int w = warp - kFirstEpi, q = warp & 3, h = w >> 2;
+        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        uint8_t* const buf = epi + (size_t)w * kUnitBytes;
+        const int units = bn / kUnitCols;
+        bool ok = true;
+        for (int tl = 0; tl < my_tiles; ++tl) {
+            const int tile = pair + tl * G;
+            const int m0 = (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM + q * 32, n0 = (tile % p.tiles_n) * bn;
+            const int a = tl & 1;
+            for (int i = tid - 32 * kFirstEpi; i < bn; i += 32 * kEpiWarps)
+                sh->bias[a][i] = n0 + i < p.N ? p.bias[n0 + i] : __float2half(0.f);
+            epi_barrier();
+            if (ok) ok = mbar_wait(&sh->acc_full[a], (uint32_t)(tl >> 1) & 1u);
+            if (!ok) continue;   // the barrier above needs every warp
+            tc_fence_after();
+            if (tl + 1 == my_tiles) pdl_launch_dependents();
+            auto accumulator_read = [&]() {
+                tc_fence_before();
+                __syncwarp();
+                if (elect_one()) mbar_arrive_cluster(in_cta(&sh->acc_empty[a], 0));
+                __syncwarp();
+            };
+            for (int u = h; u < units; u += kEpiWarps / 4) {
+                uint32_t acc[32];
+                tmem_ld32(tmem + a * bn + lane_base + u * kUnitCols, acc);
+                tmem_ld_wait();
+                if (u + kEpiWarps / 4 >= units) accumulator_read();   // this warp's share: it may be overwritten
+                uint4 ov[4];
+                epi_convert<kGelu>(acc, sh->bias[a] + u * kUnitCols, true, ov);
+                if (lane == 0) tma_store_wait_read();   // the buffer's previous store has read it
+                __syncwarp();
+                epi_write(buf, lane, ov);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if (n0 + u * kUnitCols < p.N && m0 < p.T) tma_store_2d(&tmY, buf, n0 + u * kUnitCols, m0);
+                    tma_store_commit();
+                }
+            }
+            if (h >= units) accumulator_read();
+        }
+        if (!ok && lane == 0) {
+            atomicExch(p.err, 33);
+            sh->abort = 1;
+        }
+        if (lane == 0) tma_store_wait_read();
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // nobody still reads this CTA's shared memory or signals its barriers
+    tc_fence_after();
+    if (warp == kCopyWarps) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(2 * bn)) : "memory");
+}
+
+// ------------------------------------------------------------------------------------------ K split over a cluster
+constexpr int kSplitThreads = 256;
+
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
+    float4 v;
+    asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %4, %5;\nld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [a];\n}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr), "r"(rank)
+                 : "memory");
+    return v;
+}
+
+template <bool kGelu>
+__global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __grid_constant__ CUtensorMap tmX,
+                                                                       const __grid_constant__ CUtensorMap tmW,
+                                                                       const __grid_constant__ DenseParams p, int split) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int S = p.stages, bn = p.bn;
+    const int b_panel = bn * kBK * 2;
+    const int stage_bytes = p.panels * (kAPanel + b_panel);
+    // the partial tile goes over the stages when they are done with
+    float* const part = reinterpret_cast<float*>(smem);
+    const int pitch = bn + 4;   // floats
+    DenseShared* const sh = reinterpret_cast<DenseShared*>(smem + max(S * stage_bytes, kBM * pitch * 4));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = (int)cluster_rank();
+    const int tile = (int)blockIdx.x / split;
+    const int m0 = (tile / p.tiles_n) * kBM, n0 = (tile % p.tiles_n) * bn;
+    const int kp0 = rank * p.k_panels / split, kp1 = (rank + 1) * p.k_panels / split;   // this CTA's panels
+    const int kn = (kp1 - kp0 + p.panels - 1) / p.panels;                               // in stages
+    if (tid == 0) {
+        for (int i = 0; i < S; ++i) { mbar_init(&sh->full[i], 1); mbar_init(&sh->empty[i], 1); }
+        mbar_init(&sh->acc_full[0], 1);
+        sh->abort = 0;
+        fence_mbar_init();
+    }
+    if (warp == kCopyWarps) {
+        tmem_alloc(&sh->tmem_base, tmem_cols(bn));
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh->tmem_base;
+    // the weight's first panels, before anything that depends on the preceding kernel
+    auto load_w = [&](int s, int kc) {
+        const int k0 = kp0 + kc * p.panels, np = min(p.panels, kp1 - k0);
+        mbar_expect_tx(&sh->full[s], np * (kAPanel + b_panel));
+        for (int i = 0; i < np; ++i)
+            tma_load_2d(smem + (size_t)s * stage_bytes + p.panels * kAPanel + i * b_panel, &tmW, (k0 + i) * kBK, n0, &sh->full[s]);
+    };
+    const int cw = copy_warps(S);
+    if (warp < cw && lane == 0)
+        for (int i = warp; i < min(S, kn); i += cw) load_w(i, i);
+    __syncwarp();
+    pdl_wait();
+    bool ok = true;
+    if (warp < cw) {
+        int s = warp;
+        uint32_t ph = 1;
+        for (int i = warp; i < kn; i += cw) {
+            if (s >= S) { s -= S; ph ^= 1u; }
+            ok = mbar_wait(&sh->empty[s], ph);
+            if (!ok) break;
+            if (lane == 0) {
+                if (i >= S) load_w(s, i);
+                const int k0 = kp0 + i * p.panels, np = min(p.panels, kp1 - k0);
+                for (int j = 0; j < np; ++j)
+                    tma_load_2d(smem + (size_t)s * stage_bytes + j * kAPanel, &tmX, (k0 + j) * kBK, m0, &sh->full[s]);
+            }
+            __syncwarp();
+            s += cw;
+        }
+    } else if (warp == kCopyWarps) {
+        const uint32_t idesc = make_idesc_f16(kBM, bn);
+        const uint64_t a0 = make_smem_desc(smem_u32(smem), 16, 1024, 2);
+        const uint64_t b0 = make_smem_desc(smem_u32(smem) + p.panels * kAPanel, 16, 1024, 2);
+        int s = 0;
+        uint32_t ph = 0;
+        for (int i = 0; i < kn; ++i) {
+            ok = mbar_wait(&sh->full[s], ph);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+                const uint64_t at = (uint64_t)(s * stage_bytes) >> 4;   // descriptors count 16-byte units
+                const int np = min(p.panels, kp1 - kp0 - i * p.panels);
+                for (int j = 0; j < np; ++j)
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        umma_f16(tmem, a0 + at + (j * kAPanel >> 4) + ks * 2, b0 + at + (j * b_panel >> 4) + ks * 2, idesc,
+                                 (i > 0 || j > 0 || ks > 0) ? 1u : 0u);
+                umma_commit(&sh->empty[s]);
+                if (i + 1 == kn) umma_commit(&sh->acc_full[0]);
+            }
+            __syncwarp();
+            if (++s == S) { s = 0; ph ^= 1u; }
+        }
+    }
+    // every copy has landed and every UMMA has read its operands when the accumulator is complete
+    const bool fin = mbar_wait(&sh->acc_full[0], 0);
+    if ((!ok || !fin) && lane == 0) {
+        atomicExch(p.err, 34);
+        sh->abort = 1;
+        if (warp < cw)   // copies in flight land before shared memory is given another use (bounded)
+            for (int i = 0; i < min(S, kn); ++i) mbar_wait(&sh->full[i], 0);
+    }
+    __syncwarp();
+    tc_fence_after();
+    pdl_launch_dependents();
+    {
+        const int q = warp & 3, h = warp >> 2;   // two warps per 32 rows
+        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        float* const row = part + (size_t)(q * 32 + lane) * pitch;
+        for (int c = h * 16; c < bn; c += 32) {
+            uint32_t r[16];
+            tmem_ld16(tmem + lane_base + c, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float4*>(row + c + 4 * i) = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
+                                                                          __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    cluster_sync();
+    tc_fence_after();
+    if (warp == kCopyWarps) tmem_dealloc(tmem, tmem_cols(bn));
+    const int rows = kBM / split;
+    const int segs = bn / 8;
+    for (int i = tid; i < rows * segs; i += kSplitThreads) {
+        const int r = rank * rows + i / segs, c = (i % segs) * 8;
+        if (m0 + r >= p.T || n0 + c >= p.N) continue;
+        const uint32_t at = smem_u32(part + (size_t)r * pitch + c);
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < split; ++k) {
+            const float4 x = ld_cluster(at, k), y = ld_cluster(at + 16, k);
+            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+            v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+        }
+        uint4 o;
+        half2* oh = reinterpret_cast<half2*>(&o);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float b0 = __half2float(p.bias[n0 + c + 2 * j]), b1 = __half2float(p.bias[n0 + c + 2 * j + 1]);
+            const half2 t = __floats2half2_rn(v[2 * j] + b0, v[2 * j + 1] + b1);
+            oh[j] = kGelu ? gelu_tanh_h2(t) : t;
+        }
+        *reinterpret_cast<uint4*>(p.Y + (size_t)(m0 + r) * p.N + n0 + c) = o;
+    }
+    __syncwarp();
+    cluster_sync();   // the other CTAs may still be reading this one's partial tile
+}
+
+}  // namespace
+
+// Panels per stage and stages that fit.
+static int panels_for(int bn, int split) { return split > 1 || bn <= 128 ? 2 : 1; }
+
+// CTAs of a cluster of `split` that run at once (one CTA per SM; clusters do not straddle the groups of 16-20 SMs, so that of
+// the larger ones fewer fit).
+static int split_capacity(int split) { return split == 8 ? 14 * 8 : split == 4 ? 33 * 4 : sm_count() / split * split; }
+
+// Cost in clocks of a launch over `tokens` with tile width bn and the K range split over `split` CTAs: waves of tiles, each
+// K panel taking its UMMAs (2 bn clocks) or its copies (an SM gets ~58 bytes per clock from L2 when all ask), plus what comes
+// before the first UMMA and after the last one. Fitted to launches of 64 to 32768 tokens (within 20 %).
+static double dense_cost(int tokens, int N, int K, int bn, int split) {
+    const int tiles_n = (N + bn - 1) / bn;
+    const int panels = (K + kBK - 1) / kBK;
+    if (split == 1) {
+        const int pairs = sm_count() / 2;
+        const int waves = ((tokens + 2 * kBM - 1) / (2 * kBM) * tiles_n + pairs - 1) / pairs;
+        const double panel = std::max({2.0 * bn, (kAPanel + bn * 64.0) / 58.0, 400.0 / panels_for(bn, 1)});
+        const double tile = std::max(panels * panel, bn * 9.0);   // the main loop, or the stores of the tile before
+        // a long launch of dense UMMAs runs at the power limit: 1.4e15 operations per second on the whole GPU
+        const double power = 2.0 * tokens * N * (double)K / 1.4e15 * 1.9e9;
+        return 9500.0 + std::max(waves * tile + bn * 9.0, power);
+    }
+    const int tiles = std::max(1, (tokens + kBM - 1) / kBM) * tiles_n;
+    const double panel = std::max({2.0 * bn, (kAPanel + bn * 128.0) / 58.0, 200.0});
+    const int waves = (tiles * split + split_capacity(split) - 1) / split_capacity(split);
+    return 7500.0 + waves * (3500.0 + ((panels + split - 1) / split) * panel + 900.0 + bn * 8.0);
+}
+
+DensePlan dense_plan(int tokens, int N, int K) {
+    DensePlan best;
+    for (int bn : {256, 192, 128, 96, 64, 32}) {
+        if (bn > 32 && bn - 32 >= N) continue;   // no narrower tile would leave columns out
+        for (int split : {1, 2, 4, 8}) {
+            const int panels = (K + kBK - 1) / kBK;
+            if (split > 1 && (split > panels || bn > 128)) continue;
+            const double c = dense_cost(tokens, N, K, bn, split);
+            if (best.bn == 0 || c < best.cost * 0.98) best = DensePlan{bn, split, c};
+        }
+    }
+    return best;
+}
+
+int dense_map_weight(CUtensorMap* map, const half* W, int N, int K, const DensePlan& plan) {
+    // a CTA of a pair copies half of the tile's rows
+    if (!make_tmap_2d_f16(map, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)(plan.split > 1 ? plan.bn : plan.bn / 2), kBK, 128))
+        return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
+    return ET_OK;
+}
+
+int dense_run(const CUtensorMap& tmW, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int N, int K, int gelu,
+              int* err, cudaStream_t st) {
+    CUtensorMap tmX, tmY;
+    if (!make_tmap_2d_f16(&tmX, X, (uint64_t)T, (uint64_t)K, (uint64_t)K, kBM, kBK, 128))
+        return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
+    static PerDeviceOnce once;
+    const cudaError_t attr_err = once.run([] {
+        cudaError_t e = cudaFuncSetAttribute(dense_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_split_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        return e;
+    });
+    if (attr_err != cudaSuccess) return cuda_status(attr_err, "dense linear: shared memory opt-in");
+    DenseParams p;
+    p.bias = bias; p.Y = Y; p.T = T; p.N = N; p.bn = plan.bn;
+    p.k_panels = (K + kBK - 1) / kBK;
+    p.tiles_n = (N + plan.bn - 1) / plan.bn;
+    p.panels = panels_for(plan.bn, plan.split);
+    p.err = err;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    if (plan.split > 1) {
+        const int stage = p.panels * (kAPanel + plan.bn * kBK * 2);
+        p.tiles = ((T + kBM - 1) / kBM) * p.tiles_n;
+        p.stages = ring_stages(std::min({kMaxStages, (kSmemMax - 1024 - (int)sizeof(DenseShared)) / stage,
+                                         ((p.k_panels + plan.split - 1) / plan.split + p.panels - 1) / p.panels}));
+        cfg.gridDim = dim3((unsigned)(p.tiles * plan.split));
+        cfg.blockDim = dim3(kSplitThreads);
+        cfg.dynamicSmemBytes = (size_t)std::max(p.stages * stage, kBM * (plan.bn + 4) * 4) + sizeof(DenseShared) + 1024;
+        attr[1].val.clusterDim.x = (unsigned)plan.split;
+        return cuda_status(gelu ? cudaLaunchKernelEx(&cfg, dense_split_kernel<true>, tmX, tmW, p, plan.split)
+                                : cudaLaunchKernelEx(&cfg, dense_split_kernel<false>, tmX, tmW, p, plan.split),
+                           "dense linear launch");
+    }
+    if (!make_tmap_2d_f16(&tmY, Y, (uint64_t)T, (uint64_t)N, (uint64_t)N, 32, kUnitCols, 64))
+        return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
+    const int stage = p.panels * (kAPanel + plan.bn * kBK);
+    p.tiles = ((T + 2 * kBM - 1) / (2 * kBM)) * p.tiles_n;
+    p.stages = ring_stages(std::min(kMaxStages, (kSmemMax - 1024 - (int)sizeof(DenseShared) - kEpiWarps * kUnitBytes) / stage));
+    cfg.gridDim = dim3((unsigned)(2 * std::min(p.tiles, sm_count() / 2)));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)p.stages * stage + kEpiWarps * kUnitBytes + sizeof(DenseShared) + 1024;
+    attr[1].val.clusterDim.x = 2;
+    return cuda_status(gelu ? cudaLaunchKernelEx(&cfg, dense_kernel<true>, tmX, tmW, tmY, p)
+                            : cudaLaunchKernelEx(&cfg, dense_kernel<false>, tmX, tmW, tmY, p),
+                       "dense linear launch");
+}
+
+}  // namespace et

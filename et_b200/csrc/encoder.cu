@@ -417,7 +417,9 @@ static int model_prepare_fusion(Model* m) {
     for (size_t l = 0; l < m->layers.size(); ++l) {
         Encoder* e = m->layers[l];
         Model::Fused& f = m->fused[l];
-        int rc = tile_weight_fold(&f.ffn1, e->lin[4], e->h_ln[0].data(), e->h_ln[1].data());
+        int rc = tile_weight_prepare_fusion(e->lin[3]);
+        if (rc == ET_OK) rc = tile_weight_prepare_fusion(e->lin[5]);
+        if (rc == ET_OK) rc = tile_weight_fold(&f.ffn1, e->lin[4], e->h_ln[0].data(), e->h_ln[1].data());
         if (rc == ET_OK && l > 0) {
             const Encoder* pe = m->layers[l - 1];
             rc = tile_weight_fold(&f.qkv, e->qkv, pe->h_ln[2].data(), pe->h_ln[3].data());

@@ -37,7 +37,10 @@
 #include <tuple>
 #include <vector>
 #include "common.h"
+#include "dense_gemm.h"
+#include "epilogue.cuh"
 #include "ptx.cuh"
+#include "resident_gemm.h"
 #include "tmap.h"
 #include "tile_gemm.h"
 
@@ -99,21 +102,6 @@ __device__ __forceinline__ void tmem_st16_zero(uint32_t taddr) {
         "r"(0u)
         : "memory");
 }
-// tanh-GELU of two values in packed fp16 arithmetic: 0.5 x (1 + tanh(x (c1 + c2 x^2))), six packed operations and
-// one special-function op per pair, no conversion. The epilogue is bound by the conversion unit (fp32 <-> fp16
-// conversions and special functions run at 16 per clock per SM): with the polynomial in fp32 and conversions
-// around the tanh a 128 x 384 GELU tile took ~9000 clocks against ~4400 without GELU. The result is stored as fp16
-// anyway; tanh saturates, so the rounding of its argument does not grow with |x| (an argument that overflows to
-// infinity gives tanh = +-1, the correct limit).
-__device__ __forceinline__ half2 gelu_tanh_h2(half2 x) {
-    const half2 c1 = __float2half2_rn(0.7978845608028654f), c2 = __float2half2_rn(0.7978845608028654f * 0.044715f);
-    const half2 u = __hmul2(x, __hfma2(__hmul2(x, x), c2, c1));
-    uint32_t t;
-    asm("tanh.approx.f16x2 %0, %1;" : "=r"(t) : "r"(*reinterpret_cast<const uint32_t*>(&u)));
-    const half2 hx = __hmul2(x, __float2half2_rn(0.5f));
-    return __hfma2(hx, *reinterpret_cast<const half2*>(&t), hx);
-}
-
 struct Shared {
     // Barrier rings (a parity wait is only safe for a waiter that has seen the barrier's previous phase complete and
     // cannot be a whole phase late, which fixes each ring's length):
@@ -139,47 +127,6 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
 }
 __device__ __forceinline__ void named_barrier_arrive(int id, int threads) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// One 32-column unit of the epilogue, in three steps so that two units can be in flight per warp.
-__device__ __forceinline__ void epi_load(uint32_t taddr, bool two, uint32_t (&acc)[32]) {
-    if (two) {
-        tmem_ld32(taddr, acc);
-    } else {
-        uint32_t lo[16];
-        tmem_ld16(taddr, lo);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            acc[i] = lo[i];
-            acc[16 + i] = 0u;
-        }
-    }
-}
-template <bool kGelu>
-__device__ __forceinline__ void epi_convert(const uint32_t (&acc)[32], const half* bias, bool two, uint4 (&ov)[4]) {
-    uint4 bv[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        bv[c] = (two || c < 2) ? reinterpret_cast<const uint4*>(bias)[c] : make_uint4(0u, 0u, 0u, 0u);
-    const half2* bh = reinterpret_cast<const half2*>(bv);
-    half2* oh = reinterpret_cast<half2*>(ov);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        if constexpr (kGelu) {
-            // one conversion per pair: the accumulator is packed first and the bias is added in packed fp16
-            oh[i] = gelu_tanh_h2(__hadd2(__floats2half2_rn(__uint_as_float(acc[2 * i]), __uint_as_float(acc[2 * i + 1])), bh[i]));
-        } else {
-            const float2 bb = __half22float2(bh[i]);
-            oh[i] = __floats2half2_rn(__uint_as_float(acc[2 * i]) + bb.x, __uint_as_float(acc[2 * i + 1]) + bb.y);
-        }
-    }
-}
-// Row `lane` of a 32 x 32 unit: four 16-byte chunks under the 64-byte swizzle (chunk ^= (row / 2) % 4).
-__device__ __forceinline__ void epi_write(uint8_t* buf, int lane, const uint4 (&ov)[4]) {
-    uint8_t* prow = buf + lane * 64;
-    const int x = (lane >> 1) & 3;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(prow + ((c ^ x) << 4)) = ov[c];
 }
 
 // ---- LayerNorm folded into the epilogue (the layer stack's fused path) --------------------------------------------
@@ -672,6 +619,13 @@ struct TileWeight {
     float* d_colc = nullptr; float* d_cold = nullptr;   // c_n, d_n of a weight folded with a LayerNorm's gamma / beta
     int* d_err = nullptr;
     size_t stream_bytes = 0;
+    // the dense form, where it is the faster one for the expected token count (packed_dense); the tile form is then built only
+    // when something needs it (the fused epilogues)
+    bool packed_dense = false;
+    ResidentWeight* resident = nullptr;   // the form with the activations resident in tensor memory, where that is the fastest
+    half* d_dense = nullptr;
+    CUtensorMap dense_map;
+    DensePlan dense;
 };
 
 // Ring depths for a chunk shape. The operands live for different times, so each has its own ring: an activation
@@ -704,7 +658,7 @@ static int g_goal = 0;
 constexpr int kThroughputTilesPerCta = 2;
 void tile_gemm_set_goal(int goal) { g_goal = goal == 1 ? 1 : 0; }
 
-static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double density) {
+static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double density, double* cost_out) {
     const int slabs = std::max(1, (size_hint + kSlab - 1) / kSlab);
     const int sms = std::max(1, sm_count());
     double best = 0;
@@ -728,39 +682,17 @@ static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double densi
         const double cost = g_goal == 1 ? (double)tiles * t_tile : per_cta * t_tile + 3000.0;
         if (best_nb == 0 || cost < best * 0.999) { best = cost; best_nb = nbe; }
     }
+    *cost_out = best_nb > 0 ? best : 1e30;
     return best_nb > 0 ? best_nb : std::min(8, std::max(n_block_rows, 1));
 }
 
-int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, const half* data,
-                     const int* row_ptr, const int* row_offset, const half* bias, int nb_override) {
-    if (!out) return fail(ET_ERR_INVALID, "tile weight: null output");
-    *out = nullptr;
-    if (K <= 0 || N <= 0 || K % 16 || N % 16) return fail(ET_ERR_INVALID, "tile weight: in/out features must be positive multiples of 16");
-    if (ntile < 0 || !row_ptr || (ntile > 0 && (!row_offset || !data))) return fail(ET_ERR_INVALID, "tile weight: null array");
-    const int NBR = N / 16;
-    if (row_ptr[0] != 0 || row_ptr[NBR] != ntile) return fail(ET_ERR_INVALID, "tile weight: row_ptr does not span ntile");
-    for (int r = 0; r < NBR; ++r)
-        if (row_ptr[r + 1] < row_ptr[r]) return fail(ET_ERR_INVALID, "tile weight: row_ptr not monotone");
-    for (long i = 0; i < ntile; ++i)
-        if (row_offset[i] < 0 || row_offset[i] % 16 || row_offset[i] + 16 > K) return fail(ET_ERR_INVALID, "tile weight: row_offset out of range or not a multiple of 16");
-
-    auto* w = new TileWeight();
-    w->K = K; w->N = N; w->ntile = ntile; w->size_hint = size_hint;
-    w->tiles_per_cta = g_goal == 1 ? kThroughputTilesPerCta : 1;
-    const double density = (double)ntile / std::max(1.0, (double)NBR * (K / 16));
-    w->nb = choose_nb(NBR, (K + kKC - 1) / kKC, size_hint, density);
-    if (nb_override > 0) {
-        const int nbo = std::min(nb_override, kMaxNB);
-        w->nb = NBR <= nbo ? NBR : std::max(4, nbo / 4 * 4);
-    }
-    w->h_row_ptr.assign(row_ptr, row_ptr + NBR + 1);
-    w->h_row_offset.assign(row_offset, row_offset + ntile);
-    w->h_data.assign(data, data + (size_t)ntile * 256);
-    w->h_bias.assign((size_t)N, __float2half(0.f));
-    if (bias) std::copy(bias, bias + N, w->h_bias.begin());
+// The tile form on the device: issue lists and tiles as the kernel reads them.
+static int build_tile_form(TileWeight* w) {
+    if (w->d_stream) return ET_OK;
+    const int NBR = w->N / 16;
     w->n_chunks = (NBR + w->nb - 1) / w->nb;
-    w->k_chunks = (K + kKC - 1) / kKC;
-    if (w->k_chunks > kMaxKChunks) { delete w; return fail(ET_ERR_UNSUPPORTED, "tile weight: in_feat above 32768"); }
+    w->k_chunks = (w->K + kKC - 1) / kKC;
+    if (w->k_chunks > kMaxKChunks) return fail(ET_ERR_UNSUPPORTED, "tile weight: in_feat above 32768");
 
     // Bucket tiles by (chunk, k-chunk, issuing warp).
     struct Ent { int tile; int slice; int lb; };
@@ -768,8 +700,8 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     std::vector<std::vector<Ent>> buckets(nblocks * kIssuers);
     for (int r = 0; r < NBR; ++r) {
         const int c = r / w->nb, lb = r % w->nb;
-        for (int i = row_ptr[r]; i < row_ptr[r + 1]; ++i) {
-            const int kc = row_offset[i] / kKC, sl = (row_offset[i] % kKC) / 16;
+        for (int i = w->h_row_ptr[r]; i < w->h_row_ptr[r + 1]; ++i) {
+            const int kc = w->h_row_offset[i] / kKC, sl = (w->h_row_offset[i] % kKC) / 16;
             buckets[((size_t)c * w->k_chunks + kc) * kIssuers + (lb % kIssuers)].push_back({i, sl, lb});
         }
     }
@@ -790,16 +722,15 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
         for (int wv = 0; wv < kIssuers; ++wv) {
             auto& v = buckets[b * kIssuers + wv];
             std::stable_sort(v.begin(), v.end(), [](const Ent& a, const Ent& c) { return a.slice < c.slice; });
-            if (e > 0xffff || v.size() > 0xffff) { delete w; return fail(ET_ERR_UNSUPPORTED, "tile weight: block too large"); }
+            if (e > 0xffff || v.size() > 0xffff) return fail(ET_ERR_UNSUPPORTED, "tile weight: block too large");
             hdr[wv] = e | ((uint32_t)v.size() << 16);
             for (const Ent& t : v) {
                 ent[e] = make_uint4(e * 32u, (uint32_t)t.slice * 8u, (uint32_t)t.lb * 16u, idesc16);
-                const half* src = data + (size_t)t.tile * 256;
+                const half* src = w->h_data.data() + (size_t)t.tile * 256;
                 uint8_t* dst = tiles + (size_t)e * 512;
                 for (int n = 0; n < 16; ++n)
-                    for (int k = 0; k < 16; ++k)
-                        std::memcpy(dst + (n / 8) * 256 + (k / 8) * 128 + (n % 8) * 16 + (k % 8) * 2,
-                                    src + n * 16 + k, 2);
+                    for (int k = 0; k < 16; k += 8)
+                        std::memcpy(dst + (n / 8) * 256 + (k / 8) * 128 + (n % 8) * 16, src + n * 16 + k, 16);
                 ++e;
             }
         }
@@ -813,26 +744,92 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
         const RingShape rs = ring_shape(w->nb, w->stage_b_bytes);
         w->nx = rs.nx; w->nw = rs.nw; w->a_slots = rs.a_slots;
     }
-    if (w->nx < 2 || w->a_slots < 1) { delete w; return fail(ET_ERR_UNSUPPORTED, "tile weight: weight block exceeds shared memory"); }
+    if (w->nx < 2 || w->a_slots < 1) return fail(ET_ERR_UNSUPPORTED, "tile weight: weight block exceeds shared memory");
     w->stream_bytes = stream.size();
 
-    cudaError_t e1 = cudaMalloc(&w->d_dir, dir.size() * sizeof(uint2));
-    cudaError_t e2 = cudaMalloc(&w->d_stream, std::max<size_t>(stream.size(), 16));
-    cudaError_t e3 = cudaMalloc(&w->d_bias, (size_t)N * sizeof(half));
-    cudaError_t e4 = cudaMalloc(&w->d_err, sizeof(int));
-    cudaError_t e5 = cudaMalloc(&w->d_bias_f32, (size_t)N * sizeof(float));
-    if (e1 || e2 || e3 || e4 || e5) { tile_weight_free(w); return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed"); }
-    {
-        std::vector<float> bf((size_t)N, 0.f);
-        if (bias) for (int i = 0; i < N; ++i) bf[i] = __half2float(bias[i]);
-        cudaMemcpy(w->d_bias_f32, bf.data(), (size_t)N * sizeof(float), cudaMemcpyHostToDevice);
-    }
+    if (cudaMalloc(&w->d_dir, dir.size() * sizeof(uint2)) != cudaSuccess ||
+        cudaMalloc(&w->d_stream, std::max<size_t>(stream.size(), 16)) != cudaSuccess)
+        return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed");
     cudaMemcpy(w->d_dir, dir.data(), dir.size() * sizeof(uint2), cudaMemcpyHostToDevice);
     cudaMemcpy(w->d_stream, stream.data(), stream.size(), cudaMemcpyHostToDevice);
-    if (bias) cudaMemcpy(w->d_bias, bias, (size_t)N * sizeof(half), cudaMemcpyHostToDevice);
-    else cudaMemset(w->d_bias, 0, (size_t)N * sizeof(half));
+    return cuda_status(cudaDeviceSynchronize(), "tile weight upload");
+}
+
+// The dense form: the weight as a row-major [N x K] matrix, zeros where tiles were pruned.
+static int build_dense_form(TileWeight* w) {
+    std::vector<half> dense((size_t)w->N * w->K, __float2half(0.f));
+    for (int r = 0; r < w->N / 16; ++r)
+        for (int i = w->h_row_ptr[r]; i < w->h_row_ptr[r + 1]; ++i)
+            for (int n = 0; n < 16; ++n)
+                std::memcpy(&dense[(size_t)(16 * r + n) * w->K + w->h_row_offset[i]], &w->h_data[(size_t)i * 256 + n * 16], 32);
+    if (cudaMalloc(&w->d_dense, dense.size() * sizeof(half)) != cudaSuccess) return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed");
+    cudaMemcpy(w->d_dense, dense.data(), dense.size() * sizeof(half), cudaMemcpyHostToDevice);
+    return dense_map_weight(&w->dense_map, w->d_dense, w->N, w->K, w->dense);
+}
+
+// Whether a block-row lists the same tile twice (legal: the contributions add up; the dense form could hold only their
+// rounded sum).
+static bool repeats_a_tile(const int* row_ptr, const int* row_offset, int block_rows) {
+    std::vector<int> seen;
+    for (int r = 0; r < block_rows; ++r) {
+        seen.assign(row_offset + row_ptr[r], row_offset + row_ptr[r + 1]);
+        std::sort(seen.begin(), seen.end());
+        if (std::adjacent_find(seen.begin(), seen.end()) != seen.end()) return true;
+    }
+    return false;
+}
+
+int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, const half* data,
+                     const int* row_ptr, const int* row_offset, const half* bias, int nb_override) {
+    if (!out) return fail(ET_ERR_INVALID, "tile weight: null output");
+    *out = nullptr;
+    if (K <= 0 || N <= 0 || K % 16 || N % 16) return fail(ET_ERR_INVALID, "tile weight: in/out features must be positive multiples of 16");
+    if (ntile < 0 || !row_ptr || (ntile > 0 && (!row_offset || !data))) return fail(ET_ERR_INVALID, "tile weight: null array");
+    const int NBR = N / 16;
+    if (row_ptr[0] != 0 || row_ptr[NBR] != ntile) return fail(ET_ERR_INVALID, "tile weight: row_ptr does not span ntile");
+    for (int r = 0; r < NBR; ++r)
+        if (row_ptr[r + 1] < row_ptr[r]) return fail(ET_ERR_INVALID, "tile weight: row_ptr not monotone");
+    for (long i = 0; i < ntile; ++i)
+        if (row_offset[i] < 0 || row_offset[i] % 16 || row_offset[i] + 16 > K) return fail(ET_ERR_INVALID, "tile weight: row_offset out of range or not a multiple of 16");
+
+    auto* w = new TileWeight();
+    w->K = K; w->N = N; w->ntile = ntile; w->size_hint = size_hint;
+    w->tiles_per_cta = g_goal == 1 ? kThroughputTilesPerCta : 1;
+    const double density = (double)ntile / std::max(1.0, (double)NBR * (K / 16));
+    double tile_cost = 0;
+    w->nb = choose_nb(NBR, (K + kKC - 1) / kKC, size_hint, density, &tile_cost);
+    if (nb_override > 0) {
+        const int nbo = std::min(nb_override, kMaxNB);
+        w->nb = NBR <= nbo ? NBR : std::max(4, nbo / 4 * 4);
+    }
+    w->h_row_ptr.assign(row_ptr, row_ptr + NBR + 1);
+    w->h_row_offset.assign(row_offset, row_offset + ntile);
+    w->h_data.assign(data, data + (size_t)ntile * 256);
+    w->h_bias.assign((size_t)N, __float2half(0.f));
+    if (bias) std::copy(bias, bias + N, w->h_bias.begin());
+    w->dense = dense_plan(size_hint, N, K);
+    // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's, which
+    // was made to compare its own shapes only, is 1.3 times too short). At 75 % sparsity and 32768 tokens, in us, tile / resident /
+    // dense: 768 -> 2304 84 / 63 / 83, 3072 -> 768 76 / - / 107, 1024 -> 3072 128 / 167 / 132; without zeros 160 / - / 96.
+    tile_cost = 1.3 * tile_cost + 1000.0;
+    const double resident = resident_cost(size_hint, N, K, density);
+    const bool plain = nb_override <= 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
+    w->packed_dense = plain && w->dense.cost < std::min(tile_cost, resident);
+    int rc = w->packed_dense ? build_dense_form(w)
+             : plain && resident < 0.97 * tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
+                                             : build_tile_form(w);
+    if (rc) { tile_weight_free(w); return rc; }
+    if (cudaMalloc(&w->d_bias, (size_t)N * sizeof(half)) != cudaSuccess || cudaMalloc(&w->d_err, sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&w->d_bias_f32, (size_t)N * sizeof(float)) != cudaSuccess) {
+        tile_weight_free(w);
+        return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed");
+    }
+    std::vector<float> bf((size_t)N);
+    for (int i = 0; i < N; ++i) bf[i] = __half2float(w->h_bias[i]);
+    cudaMemcpy(w->d_bias_f32, bf.data(), (size_t)N * sizeof(float), cudaMemcpyHostToDevice);
+    cudaMemcpy(w->d_bias, w->h_bias.data(), (size_t)N * sizeof(half), cudaMemcpyHostToDevice);
     cudaMemset(w->d_err, 0, sizeof(int));
-    int rc = cuda_status(cudaDeviceSynchronize(), "tile weight upload");
+    rc = cuda_status(cudaDeviceSynchronize(), "tile weight upload");
     if (rc) { tile_weight_free(w); return rc; }
     *out = w;
     return ET_OK;
@@ -861,7 +858,8 @@ int tile_weight_concat(TileWeight** out, const TileWeight* const* parts, int cou
 void tile_weight_free(TileWeight* w) {
     if (!w) return;
     cudaFree(w->d_dir); cudaFree(w->d_stream); cudaFree(w->d_bias); cudaFree(w->d_err);
-    cudaFree(w->d_bias_f32); cudaFree(w->d_colc); cudaFree(w->d_cold);
+    cudaFree(w->d_bias_f32); cudaFree(w->d_colc); cudaFree(w->d_cold); cudaFree(w->d_dense);
+    resident_free(w->resident);
     delete w;
 }
 
@@ -874,6 +872,10 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
     if (T < 0) return fail(ET_ERR_INVALID, "tile linear: negative token count");
     if (T == 0) return ET_OK;
     if (!aligned16(X) || !aligned16(Y)) return fail(ET_ERR_INVALID, "tile linear: X and Y must be 16-byte aligned");
+    if (w->packed_dense && !fusion)
+        return dense_run(w->dense_map, w->dense, Y, X, bias_dev ? bias_dev : w->d_bias, T, w->N, w->K, gelu, w->d_err, st);
+    if (w->resident && !fusion) return resident_run(w->resident, Y, X, bias_dev ? bias_dev : w->d_bias, T, gelu, w->d_err, st);
+    if (!w->d_stream) return fail(ET_ERR_INVALID, "tile linear: the tile form of this weight was not prepared");
     CUtensorMap tm, tmy;
     if (!make_tmap_panels_f16(&tm, X, (uint64_t)T, (uint64_t)w->K, (uint64_t)w->K, kSlab, kKC / kPanel) ||
         !make_tmap_2d_f16(&tmy, Y, (uint64_t)T, (uint64_t)w->N, (uint64_t)w->N, 32, kUnitCols, 64))
@@ -929,6 +931,7 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
     return cuda_status(cudaGetLastError(), "tile linear launch");
 }
 
+int tile_weight_prepare_fusion(TileWeight* w) { return build_tile_form(w); }
 int tile_weight_out_feat(const TileWeight* w) { return w->N; }
 int tile_weight_chunks(const TileWeight* w) { return w->n_chunks; }
 int tile_weight_stat_slots(const TileWeight* w) { return kEpiPerQuarter * w->n_chunks; }
@@ -958,6 +961,7 @@ int tile_weight_fold(TileWeight** out, const TileWeight* w, const half* gamma, c
     int rc = tile_weight_pack(&f, w->K, w->N, w->size_hint, w->ntile, data.data(), w->h_row_ptr.data(), w->h_row_offset.data(),
                               w->h_bias.data(), 0);
     if (rc) return rc;
+    if ((rc = build_tile_form(f))) { tile_weight_free(f); return rc; }
     std::vector<float> cf((size_t)w->N), df((size_t)w->N);
     for (int n = 0; n < w->N; ++n) {
         cf[n] = (float)c[n];
@@ -983,6 +987,17 @@ int tile_weight_error(const TileWeight* w, int* code) {
 }
 
 void tile_weight_info(const TileWeight* w, int* info) {
+    if (w->resident) {
+        const int v[6] = {4, (w->N + 63) / 64, (w->K + kKC - 1) / kKC, 0, 0, (int)std::min<size_t>(resident_bytes(w->resident), 0x7fffffff)};
+        std::copy(v, v + 6, info);
+        return;
+    }
+    if (!w->d_stream) {   // dense form only
+        const int v[6] = {w->dense.bn / 16, (w->N + w->dense.bn - 1) / w->dense.bn, (w->K + kKC - 1) / kKC, w->dense.split, 0,
+                          (int)std::min<size_t>((size_t)w->N * w->K * sizeof(half), 0x7fffffff)};
+        std::copy(v, v + 6, info);
+        return;
+    }
     info[0] = w->nb; info[1] = w->n_chunks; info[2] = w->k_chunks; info[3] = w->nx;   // activation slots (the weight ring has w->nw, chosen from the same memory)
     info[4] = w->stage_b_bytes; info[5] = (int)std::min<size_t>(w->stream_bytes, 0x7fffffff);
 }

@@ -41,6 +41,8 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
 // New weight = w with gamma multiplied into its input features and the column vectors c_n = sum_k gamma_k W_nk,
 // d_n = sum_k beta_k W_nk + bias_n that the mode-1 epilogue needs (gamma, beta: host, in_feat values).
 int tile_weight_fold(TileWeight** out, const TileWeight* w, const half* gamma, const half* beta);
+// Builds what the fused epilogues (GemmFusion) of this weight need, if it is not there yet.
+int tile_weight_prepare_fusion(TileWeight* w);
 // Column chunks of the packed weight, and the partial-sum slots per row that its residual epilogue writes.
 int tile_weight_chunks(const TileWeight* w);
 int tile_weight_stat_slots(const TileWeight* w);

@@ -150,6 +150,35 @@ def test_tile_linear(et, orc, T, K, N, sparsity, gelu):
     util.assert_close(got, want, what=f"tile linear T={T} K={K} N={N} s={sparsity}")
 
 
+@pytest.mark.parametrize("T,K,N,sparsity,gelu,size,form", [
+    (1, 3072, 768, 0.75, False, 128, "dense"),       # K split over a cluster, one row of a tile
+    (129, 3072, 784, 0.0, True, 512, "dense"),       # ragged tokens and features
+    (300, 1040, 1168, 0.0, False, 2048, "dense"),    # a K range of an odd number of panels, the last one partial
+    (511, 768, 2304, 0.0, True, 32768, "dense"),     # pairs of CTAs, second CTA's tokens partly outside
+    (1, 768, 2304, 0.75, False, 32768, "resident"),
+    (700, 768, 3088, 0.75, True, 32768, "resident"),     # last group of one block-row
+    (257, 752, 2320, 0.5, False, 32768, "resident"),     # a partial chunk of K
+    (20000, 768, 768, 0.9, False, 32768, "resident"),    # several items per CTA
+    (260, 1024, 1024, 0.9, False, 32768, "resident"),    # K beyond the tensor-memory part
+    (5000, 1024, 4096, 0.9, True, 32768, "resident"),
+    (300, 768, 2304, 0.995, False, 32768, "resident"),   # block-rows without tiles
+])
+def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
+    """The forms a weight is packed in for an expected token count (`size`), run with other token counts too: edges of the
+    slabs and tiles, partial chunks, and repeated calls give the same bits."""
+    got, want, w = _run_tile(et, orc, T, K, N, sparsity, seed=T + K + N, gelu=gelu, size=size)
+    info = w.info()
+    assert form == ("tile" if info["stage_bytes"] else "dense" if info["stages"] else "resident"), info
+    util.assert_close(got, want, what=f"{form} linear T={T} K={K} N={N} s={sparsity}")
+    X = dev(util.activations(7, (T, K)))
+    ys = [torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(3)]
+    for y in ys:
+        w.run(y, X)
+    torch.cuda.synchronize()
+    w.check()
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+
+
 def test_tile_linear_exact_count_shuffled_order_and_empty_rows(et, orc):
     # exact-count generator lists a block-row's tiles in shuffle order; at 95 % many block-rows are empty
     got, want, _ = _run_tile(et, orc, 256, 768, 768, 0.95, seed=77, bernoulli=False)

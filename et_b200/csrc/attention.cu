@@ -407,7 +407,7 @@ int attention_launch(half* Z, const half* Q, const half* K, const half* V, const
     if (!scores && !qk_head_ptr && (!v_head_ptr || v_cols > 0)) {
         // dense Q and K: tensor-core (tcgen05) kernel when the shape is in its range
         const int ml = cu_seqlens ? max_len : uniform_len;
-        const int rc = attention_tc_launch(Z, Q, K, V, q_pitch, v_pitch, v_head_ptr ? v_cols : d_model, v_head_ptr, v_col_id, mask,
+        const int rc = attention_tc_launch(Z, Q, K, V, q_pitch, v_pitch, d_model, v_head_ptr ? v_cols : d_model, nullptr, v_head_ptr, v_col_id, mask,
                                            mask_ld, cu_seqlens, valid_lens, batch, uniform_len, total_tokens, ml, d_model, nhead, st);
         if (rc != ET_ERR_UNSUPPORTED) return rc;
     }

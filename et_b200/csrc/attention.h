@@ -15,11 +15,12 @@ int attention_launch(half* Z, const half* Q, const half* K, const half* V, const
                      const int* v_head_ptr, const half* mask, int mask_ld, const int* cu_seqlens,
                      const int* valid_lens, int batch, int uniform_len, int total_tokens, int d_model,
                      int nhead, cudaStream_t st, int max_len = 0, int v_cols = 0);
-// tcgen05 path (head_dim 64, dense or column-pruned V, longest sequence known); ET_ERR_UNSUPPORTED outside its range.
-int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch, int v_cols,
-                        const int* v_head_ptr, const int* v_col_id, const half* mask, int mask_ld, const int* cu_seqlens,
-                        const int* valid_lens, int batch, int uniform_len, int total_tokens, int max_len, int d_model,
-                        int nhead, cudaStream_t st);
+// tcgen05 path (head_dim 64, dense or column-pruned operands, longest sequence known; see its definition for the forms);
+// ET_ERR_UNSUPPORTED outside its range.
+int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch, int qk_cols, int v_cols,
+                        const int* qk_head_ptr, const int* v_head_ptr, const int* v_col_id, const half* mask, int mask_ld,
+                        const int* cu_seqlens, const int* valid_lens, int batch, int uniform_len, int total_tokens, int max_len,
+                        int d_model, int nhead, cudaStream_t st);
 // Reads and clears the current device's error word of the tcgen05 kernel's bounded waits (synchronises).
 int attention_tc_error(int* code);
 // One-time per-device set-up of that error word (no allocation); safe to call repeatedly.
@@ -27,11 +28,6 @@ int attention_prepare_device();
 // pitch: row pitch of Q and K in elements (0 = d_model).
 int qk_scores_launch(half* S, const half* Q, const half* K, int batch, int L, int d_model, int nhead,
                      cudaStream_t st, int pitch = 0);
-
-// dst[o][t][p] = inv[o][p] >= 0 ? src[o][t][inv[o][p]] : 0 for n <= 3 operands in one launch: compact row-pruned
-// activations back at their original feature positions, zeros elsewhere (d a multiple of 8).
-int expand_rows_launch(int n, const half* const* src, const int* src_pitch, half* const* dst, const int* dst_pitch,
-                       const int* const* inv, int d, int T, cudaStream_t st);
 
 // Same result as the on-the-fly form for one sequence, through scores held in a device array that is part
 // of the library image (no allocation). seq_len*seq_len*nhead is limited to 16*512*512.

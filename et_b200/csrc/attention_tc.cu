@@ -1,5 +1,5 @@
-// On-the-fly attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA) for heads of 64, dense or with a compact,
-// column-pruned V: the path behind et_attention_otf / et_attention_batch / et_attention_prune and the encoder layers (the
+// On-the-fly attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA) for heads of 64, dense or with compact,
+// column-pruned operands: the path behind et_attention_otf / et_attention_batch / et_attention_prune and the encoder layers (the
 // mma.sync kernel in attention.cu covers the remaining variants).
 // Replaces kernels/attention.cu:51-134 and :149-271 of the reference for those cases.
 //
@@ -29,6 +29,11 @@
 // Measured against the form with 64-key blocks, fp16 scores and four CTAs per SM that it replaces (12 heads): 64 ragged
 // sequences of 32..512 tokens 71 -> 57 us, 256 x 128 tokens 47 -> 37, 32 x 256 19.8 -> 16.1, 64 x 512 87 -> 83; with an additive
 // mask (read twice there, one row per thread) 64 x 384 169 -> 117, 64 x 383 730 -> 121; scores are fp32 here.
+// Column-pruned operands come in two forms. kScatterV (the operator): V is compact, a head's columns start anywhere, results go
+// to their original columns with zeros between. kCompact (the encoder layers, which lay their weights out for it): every head's
+// columns of Q, K and V start at a multiple of 16 and are padded to one with zeros, so that Q K^T takes width / 16 steps, P V
+// a UMMA of the width, and the result is stored compact; the next linear has its input features gathered accordingly.
+//
 // Every mbarrier wait is bounded; a wait that gives up sets the error word and the CTA leaves through the common exit.
 #include <mutex>
 #include "attention.h"
@@ -65,6 +70,7 @@ struct TcParams {
     const half* mask;
     const int* cu_seqlens;
     const int* valid_lens;
+    const int* qk_head_ptr;
     const int* v_head_ptr;
     const int* v_col_id;
     int z_pitch, mask_ld, batch, uniform_len;
@@ -77,11 +83,15 @@ struct Item {
     int tok0, q0, len, valid, head;
     int nkb;               // key blocks; < 0: no more items
     int v_x, v_off, v_n, v_base;   // pruned V: first column of the copied box, of the head's window in it, width, index of its first column id
+    int qk_x, qk_steps;    // first column of the Q and K boxes, 16-wide steps of Q K^T
     int v_add;             // second part of a wide window: only its own columns are written
 };
 
-template <bool kMask, bool kPruneV>
+enum Form { kDense = 0, kScatterV = 1, kCompact = 2 };
+
+template <bool kMask, int kForm>
 struct Cfg {
+    static constexpr bool kPruneV = kForm == kScatterV;
     static constexpr int kQS = (kMask || kPruneV) ? 1 : 2;
     static constexpr int kKS = 2;
     static constexpr int kVS = (kMask || kPruneV) ? 1 : 2;
@@ -164,6 +174,7 @@ __device__ __forceinline__ Item find_item(const TcParams& p, int blk, int h, int
     Item it;
     it.tok0 = it.q0 = it.len = it.valid = 0;
     it.head = h;
+    it.qk_x = h * kHD; it.qk_steps = kHD / 16;
     it.v_x = h * kHD; it.v_off = 0; it.v_n = kHD; it.v_base = 0; it.v_add = 0;
     int b = -1;
     if (p.cu_seqlens) {
@@ -202,12 +213,13 @@ __device__ __forceinline__ Item find_item(const TcParams& p, int blk, int h, int
     return it;
 }
 
-template <bool kMask, bool kPruneV>
+template <bool kMask, int kForm>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                             const __grid_constant__ CUtensorMap tmK,
                                                                             const __grid_constant__ CUtensorMap tmV,
                                                                             const __grid_constant__ TcParams p) {
-    using C = Cfg<kMask, kPruneV>;
+    using C = Cfg<kMask, kForm>;
+    constexpr bool kPruneV = kForm == kScatterV;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* const sQ = smem;
@@ -261,6 +273,14 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 clc_try_cancel(&sh->clc, &sh->clc_full);
             }
             Item it = find_item(p, bx, by, lane);
+            if constexpr (kForm == kCompact) {
+                if (p.qk_head_ptr) {
+                    it.qk_x = p.qk_head_ptr[by];
+                    it.qk_steps = (p.qk_head_ptr[by + 1] - it.qk_x) >> 4;
+                }
+                it.v_x = p.v_head_ptr[by];
+                it.v_n = p.v_head_ptr[by + 1] - it.v_x;
+            }
             int vx0 = 0, vw = 0;
             if constexpr (kPruneV) {
                 vx0 = p.v_head_ptr[by];
@@ -291,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 if (!(ok = mbar_wait(&sh->q_empty[qs], ((uint32_t)(nq / C::kQS) & 1u) ^ 1u))) break;
                 if (lane == 0) {
                     mbar_expect_tx(&sh->q_full[qs], kTile);
-                    tma_load_2d(sQ + qs * kTile, &tmQ, it.head * kHD, it.tok0 + it.q0, &sh->q_full[qs]);
+                    tma_load_2d(sQ + qs * kTile, &tmQ, it.qk_x, it.tok0 + it.q0, &sh->q_full[qs]);
                 }
                 ++nq;
                 // K_0, then K_{j+1} ahead of V_j: the next Q K^T needs its block before this one's P V does
@@ -301,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                         if (!(ok = mbar_wait(&sh->k_empty[ks], ((uint32_t)(nk >> 1) & 1u) ^ 1u))) break;
                         if (lane == 0) {
                             mbar_expect_tx(&sh->k_full[ks], kTile);
-                            tma_load_2d(sK + ks * kTile, &tmK, it.head * kHD, it.tok0 + (j + 1) * kBK, &sh->k_full[ks]);
+                            tma_load_2d(sK + ks * kTile, &tmK, it.qk_x, it.tok0 + (j + 1) * kBK, &sh->k_full[ks]);
                         }
                         ++nk;
                     }
@@ -349,7 +369,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
         // ---- UMMAs: the warp stays converged (every lane waits), one elected lane issues. Blocks are numbered through
         // across items: Q K^T of block g + 1 is issued as soon as the scores of block g are in registers, ahead of P V of g.
         const uint32_t idesc_qk = make_idesc_f16(128, kBK), idesc_qk_half = make_idesc_f16(128, kBK / 2);
-        const uint32_t idesc_pv = make_idesc_f16(128, kHD, false, true);   // V is an MN-major B operand
+        uint32_t idesc_pv = make_idesc_f16(128, kHD, false, true);   // V is an MN-major B operand
+        uint32_t idesc_pv_next = idesc_pv;   // of the item whose Q K^T is being issued
+        int steps = kHD / 16;
         int ni = 0, nq = 0;
         uint32_t g = 0;
         bool ok = true, end = false;
@@ -361,6 +383,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 if (!mbar_wait(&sh->item_full[slot], (uint32_t)(ni / kItemRing) & 1u)) return false;
                 nkb = sh->item[slot].nkb;
                 valid = sh->item[slot].valid;
+                if constexpr (kForm == kCompact) {
+                    steps = sh->item[slot].qk_steps;
+                    idesc_pv_next = make_idesc_f16(128, sh->item[slot].v_n, false, true);
+                }
                 __syncwarp();
                 if (elect_one()) mbar_arrive(&sh->item_empty[slot]);
                 __syncwarp();
@@ -375,9 +401,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             if (elect_one()) {
                 const uint32_t qa = smem_u32(sQ + qs * kTile), ka = smem_u32(sK + (gg & 1) * kTile);
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks)
+                for (int ks = 0; ks < 4; ++ks) {
+                    if (kForm == kCompact && ks >= steps) break;
                     umma_f16(tmem + kSCol, make_smem_desc(qa + ks * 32, 16, 1024, 2), make_smem_desc(ka + ks * 32, 16, 1024, 2),
                              half ? idesc_qk_half : idesc_qk, ks > 0);
+                }
                 umma_commit(&sh->s_full);
                 umma_commit(&sh->k_empty[gg & 1]);
                 if (last) umma_commit(&sh->q_empty[qs]);
@@ -397,6 +425,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
         while (ok && !end) {
             const bool half = is_half(j);
             const bool first = j == 0;
+            if (first) idesc_pv = idesc_pv_next;
             bool issued = false;
             const uint32_t kb1 = (g + 1) & 1, kp1 = ((g + 1) >> 1) & 1;
             if (j + 1 < nkb) {
@@ -476,7 +505,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             const float inv = done_sum > 0.f ? 1.f / done_sum : 0.f;
             const int qr = it.q0 + row;
             const bool in = qr < it.len;
-            half* const zrow = p.Z + (size_t)(it.tok0 + qr) * p.z_pitch + it.head * kHD;
+            half* const zrow = p.Z + (size_t)(it.tok0 + qr) * p.z_pitch + (kForm == kCompact ? it.v_x : it.head * kHD);
             if constexpr (kPruneV) {
                 // a row is put together in shared memory (zeros where V was pruned) and written whole
                 half* const st = reinterpret_cast<half*>(smem + C::kScatterAt + row * kScatterPitch);
@@ -510,6 +539,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             } else {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
+                    if (kForm == kCompact && 16 * c >= it.v_n) break;   // the same for the whole CTA
                     uint32_t r[16];
                     tmem_ld16(o_addr + c * 16, r);
                     tmem_ld_wait();
@@ -549,9 +579,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 if (nkb < 0) break;
                 const int qr = it.q0 + row;   // no valid key: the output rows are zero
                 if (qr < it.len) {
-                    uint4* z = reinterpret_cast<uint4*>(p.Z + (size_t)(it.tok0 + qr) * p.z_pitch + it.head * kHD);
+                    uint4* z = reinterpret_cast<uint4*>(p.Z + (size_t)(it.tok0 + qr) * p.z_pitch + (kForm == kCompact ? it.v_x : it.head * kHD));
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) z[i] = make_uint4(0, 0, 0, 0);
+                    for (int i = 0; i < 8; ++i)
+                        if (kForm != kCompact || 8 * i < it.v_n) z[i] = make_uint4(0, 0, 0, 0);
                 }
                 release(slot);
                 continue;
@@ -753,14 +784,14 @@ int attn_err_address(int** out) {
     return ET_OK;
 }
 
-template <bool kMask, bool kPruneV>
+template <bool kMask, int kForm>
 cudaError_t opt_in() {
-    return cudaFuncSetAttribute(attention_tc_kernel<kMask, kPruneV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    return cudaFuncSetAttribute(attention_tc_kernel<kMask, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
 }
-template <bool kMask, bool kPruneV>
+template <bool kMask, int kForm>
 cudaError_t launch(dim3 grid, cudaStream_t st, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const TcParams& p) {
-    const size_t smem = (size_t)Cfg<kMask, kPruneV>::kBytes + sizeof(TcShared) + 1024;
-    return launch_pdl(attention_tc_kernel<kMask, kPruneV>, grid, dim3(kThreads), smem, st, tq, tk, tv, p);
+    const size_t smem = (size_t)Cfg<kMask, kForm>::kBytes + sizeof(TcShared) + 1024;
+    return launch_pdl(attention_tc_kernel<kMask, kForm>, grid, dim3(kThreads), smem, st, tq, tk, tv, p);
 }
 
 }  // namespace
@@ -773,11 +804,16 @@ int attention_prepare_device() {
 }
 
 // Returns ET_ERR_UNSUPPORTED (without touching anything) when the case is outside the kernel's range, so the caller can use
-// the general kernel instead. v_head_ptr / v_col_id: V is compact ([tokens x v_cols], row pitch v_pitch).
-int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch, int v_cols,
-                        const int* v_head_ptr, const int* v_col_id, const half* mask, int mask_ld, const int* cu_seqlens,
-                        const int* valid_lens, int batch, int uniform_len, int total_tokens, int max_len, int d_model, int nhead,
-                        cudaStream_t st) {
+// the general kernel instead.
+//   v_head_ptr and v_col_id: V is compact ([tokens x v_cols]), results are scattered to their original columns.
+//   v_head_ptr without v_col_id: V (and Q and K where qk_head_ptr is given) are compact, each head's columns start at a multiple
+//   of 16 and number 16 to 64, a multiple of 16; the result is [tokens x v_cols] in V's layout.
+int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, int q_pitch, int v_pitch, int qk_cols, int v_cols,
+                        const int* qk_head_ptr, const int* v_head_ptr, const int* v_col_id, const half* mask, int mask_ld,
+                        const int* cu_seqlens, const int* valid_lens, int batch, int uniform_len, int total_tokens, int max_len,
+                        int d_model, int nhead, cudaStream_t st) {
+    const bool compact = v_head_ptr && !v_col_id;
+    if (qk_head_ptr && !compact) return ET_ERR_UNSUPPORTED;
     if (d_model / nhead != kHD || d_model % nhead) return ET_ERR_UNSUPPORTED;
     if (max_len <= 0) return ET_ERR_UNSUPPORTED;   // longest sequence unknown: the caller uses the general kernel
     // TMA: operands and pitches in whole 16-byte units; the mask's granules are read from a 16-byte aligned start
@@ -792,30 +828,34 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     }
     CUtensorMap tq, tk, tv;
     const uint64_t rows = (uint64_t)total_tokens;
-    // the column extent covers all heads of the operand; Q/K/V may be slices of one fused [tokens x 3 d_model] buffer
-    if (!make_tmap_2d_f16(&tq, Q, rows, (uint64_t)d_model, (uint64_t)q_pitch, kBQ, kHD, 128) ||
-        !make_tmap_2d_f16(&tk, K, rows, (uint64_t)d_model, (uint64_t)q_pitch, kBK, kHD, 128) ||
+    // the column extent covers all heads of the operand; Q/K/V may be slices of one fused buffer
+    if (!make_tmap_2d_f16(&tq, Q, rows, (uint64_t)qk_cols, (uint64_t)q_pitch, kBQ, kHD, 128) ||
+        !make_tmap_2d_f16(&tk, K, rows, (uint64_t)qk_cols, (uint64_t)q_pitch, kBK, kHD, 128) ||
         !make_tmap_2d_f16(&tv, V, rows, (uint64_t)v_cols, (uint64_t)v_pitch, kBK, kHD, 128))
         return fail(ET_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed");
     TcParams p;
     p.Z = Z; p.mask = mask; p.cu_seqlens = cu_seqlens; p.valid_lens = valid_lens;
-    p.v_head_ptr = v_head_ptr; p.v_col_id = v_col_id;
-    p.z_pitch = d_model; p.mask_ld = mask_ld; p.batch = batch; p.uniform_len = uniform_len;
+    p.qk_head_ptr = qk_head_ptr; p.v_head_ptr = v_head_ptr; p.v_col_id = v_col_id;
+    p.z_pitch = compact ? v_cols : d_model; p.mask_ld = mask_ld; p.batch = batch; p.uniform_len = uniform_len;
     p.scale_log2 = kLog2e / sqrtf((float)kHD);
     p.err = err_word;
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] {
-        cudaError_t e = opt_in<false, false>();
-        if (e == cudaSuccess) e = opt_in<true, false>();
-        if (e == cudaSuccess) e = opt_in<false, true>();
-        if (e == cudaSuccess) e = opt_in<true, true>();
+        cudaError_t e = opt_in<false, kDense>();
+        if (e == cudaSuccess) e = opt_in<true, kDense>();
+        if (e == cudaSuccess) e = opt_in<false, kScatterV>();
+        if (e == cudaSuccess) e = opt_in<true, kScatterV>();
+        if (e == cudaSuccess) e = opt_in<false, kCompact>();
+        if (e == cudaSuccess) e = opt_in<true, kCompact>();
         return e;
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "attention: shared memory opt-in");
     const int nblk = cu_seqlens ? (total_tokens + kBQ - 1) / kBQ + batch : batch * ((uniform_len + kBQ - 1) / kBQ);
     const dim3 grid(nblk, nhead);
-    const cudaError_t e = v_head_ptr ? (mask ? launch<true, true>(grid, st, tq, tk, tv, p) : launch<false, true>(grid, st, tq, tk, tv, p))
-                                     : (mask ? launch<true, false>(grid, st, tq, tk, tv, p) : launch<false, false>(grid, st, tq, tk, tv, p));
+    const auto run = compact      ? (mask ? launch<true, kCompact> : launch<false, kCompact>)
+                     : v_head_ptr ? (mask ? launch<true, kScatterV> : launch<false, kScatterV>)
+                                  : (mask ? launch<true, kDense> : launch<false, kDense>);
+    const cudaError_t e = run(grid, st, tq, tk, tv, p);
     return cuda_status(e, "attention (tcgen05) launch");
 }
 

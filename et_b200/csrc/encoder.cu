@@ -6,6 +6,7 @@
 // a batch of packed variable-length sequences is a first-class input (run_batch); every failure is a
 // status code instead of exit(1).
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -30,13 +31,12 @@ struct RowWeight {
     TileWeight* tw = nullptr;
     int* d_row_id = nullptr;
     int* d_head_ptr = nullptr;
-    int* d_inv = nullptr;   // [out_feat]: compact column of an original feature, -1 where it was pruned
-    std::vector<int> h_head_ptr;
+    std::vector<int> h_head_ptr, h_row_id;
+    std::vector<half> h_weight, h_bias;   // as given, for layers that lay the rows out with padded heads
     ~RowWeight() {
         tile_weight_free(tw);
         cudaFree(d_row_id);
         cudaFree(d_head_ptr);
-        cudaFree(d_inv);
     }
 };
 
@@ -53,8 +53,7 @@ static int dense_to_tiles(const half* weight, int rows, int K, std::vector<half>
             const size_t i = (size_t)r * bcs + c;
             row_offset[i] = c * 16;
             for (int n = 0; n < 16 && 16 * r + n < rows; ++n)
-                for (int k = 0; k < 16; ++k)
-                    data[i * 256 + n * 16 + k] = weight[(size_t)(16 * r + n) * K + 16 * c + k];
+                std::memcpy(&data[i * 256 + n * 16], weight + (size_t)(16 * r + n) * K + 16 * c, 32);
         }
     }
     row_ptr[brs] = brs * bcs;
@@ -88,14 +87,28 @@ static int row_weight_create(RowWeight** out, int in_feat, int out_feat, int siz
         return fail(ET_ERR_CUDA, "row weight: cudaMalloc failed");
     cudaMemcpy(w->d_row_id, row_id, sizeof(int) * row_id_size, cudaMemcpyHostToDevice);
     cudaMemcpy(w->d_head_ptr, w->h_head_ptr.data(), sizeof(int) * (nhead + 1), cudaMemcpyHostToDevice);
-    {
-        std::vector<int> inv((size_t)(out_feat + 7) / 8 * 8, -1);
-        for (int i = 0; i < row_id_size; ++i) inv[row_id[i]] = i;
-        if (cudaMalloc(&w->d_inv, sizeof(int) * inv.size()) != cudaSuccess) return fail(ET_ERR_CUDA, "row weight: cudaMalloc failed");
-        cudaMemcpy(w->d_inv, inv.data(), sizeof(int) * inv.size(), cudaMemcpyHostToDevice);
-    }
+    w->h_row_id.assign(row_id, row_id + row_id_size);
+    w->h_weight.assign(weight, weight + (size_t)row_id_size * in_feat);
+    w->h_bias.assign(pbias.begin(), pbias.begin() + row_id_size);
     *out = w.release();
     return ET_OK;
+}
+
+// The same rows with every head's share padded with zero rows to a multiple of 16 (at least 16): the layout in which the
+// attention kernel can address a head's columns. ptr[h]: first row of head h.
+static int row_weight_padded(TileWeight** out, const RowWeight* w, int size, std::vector<int>& ptr) {
+    ptr.assign(1, 0);
+    for (int h = 0; h < w->nhead; ++h) ptr.push_back(ptr.back() + std::max(16, (w->h_head_ptr[h + 1] - w->h_head_ptr[h] + 15) / 16 * 16));
+    const int N = ptr.back(), K = w->in_feat;
+    std::vector<half> weight((size_t)N * K, __float2half(0.f)), bias((size_t)N, __float2half(0.f)), data;
+    for (int h = 0; h < w->nhead; ++h) {
+        const int r0 = w->h_head_ptr[h], n = w->h_head_ptr[h + 1] - r0;
+        std::copy_n(w->h_weight.begin() + (size_t)r0 * K, (size_t)n * K, weight.begin() + (size_t)ptr[h] * K);
+        std::copy_n(w->h_bias.begin() + r0, n, bias.begin() + ptr[h]);
+    }
+    std::vector<int> rp, ro;
+    dense_to_tiles(weight.data(), N, K, data, rp, ro);
+    return tile_weight_pack(out, K, N, size, (long)ro.size(), data.data(), rp.data(), ro.data(), bias.data(), 0);
 }
 
 namespace {
@@ -233,8 +246,11 @@ struct Encoder {
     TileWeight* lin[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // q k v o mlp1 mlp2
     TileWeight* qkv = nullptr;   // Q|K|V as one weight: one launch, one staging of the activations per CTA
     int qkv_cols[3] = {0, 0, 0}; // output columns of the three parts inside the fused result
-    bool expand_pruned = false;  // row-pruned operands are expanded to their original positions (zeros where pruned)
-                                 // and attention runs on the tensor-core kernel
+    // Row-pruned layers with heads of 64: the row-pruned linears are laid out with padded heads (row_weight_padded), attention
+    // works on and produces compact heads, and the output projection has its input features gathered to match. (Expanding the
+    // compact operands to 64 per head first, and the projection over all features: 20 us more of 123 at 32 x 256 tokens.)
+    TileWeight* o_compact = nullptr;
+    int* d_qk_ptr = nullptr; int* d_v_ptr = nullptr;   // first column of each head in Q and K (null: dense) and in V
     RowWeight* rq = nullptr; RowWeight* rk = nullptr; RowWeight* rv = nullptr;
     half* d_ln[4] = {nullptr, nullptr, nullptr, nullptr};  // gamma1 beta1 gamma2 beta2
     std::vector<half> h_ln[4];                             // the same on the host (folded into weights by the layer stack)
@@ -247,6 +263,9 @@ struct Encoder {
         graphs.drop();
         for (auto* t : lin) tile_weight_free(t);
         tile_weight_free(qkv);
+        tile_weight_free(o_compact);
+        cudaFree(d_qk_ptr);
+        cudaFree(d_v_ptr);
         delete rq; delete rk; delete rv;
         for (auto* p : d_ln) cudaFree(p);
         cudaFree(d_mask);
@@ -288,40 +307,13 @@ static int encoder_forward(Encoder* e, half* out, const half* in, half* scratch,
     int rc;
     int q_pitch = e->d_model, v_pitch = e->d_model;
     const int *qk_hp = nullptr, *v_hp = nullptr, *v_id = nullptr;
-    if (e->qkv && e->expand_pruned) {
-        // Row-pruned operands. One launch writes the compact Q | K | V side by side; one bandwidth-bound pass puts
-        // the row-pruned ones back at their original feature positions with zeros where a feature was pruned; the
-        // tensor-core attention kernel then runs on dense heads of 64: a zero column adds nothing to Q K^T, and a
-        // zero column of V gives a zero column of the result, which is the scatter with zero fill that the pruned
-        // attention means (kernels/attention.cu:242-248).
+    if (e->o_compact) {
+        if ((rc = tile_linear_run(e->qkv, b0, in, T, 0, st))) return rc;
         const int P = e->qkv_cols[0] + e->qkv_cols[1] + e->qkv_cols[2];
-        const int d = e->d_model;
-        half* b4 = scratch + 4 * td;
-        if (e->kind == kPruneQKV) {
-            // compact result in buffers 3-4 (P <= 2 d_model), expanded Q | K | V over buffers 0-2
-            half* comp = b3;
-            if ((rc = tile_linear_run(e->qkv, comp, in, T, 0, st))) return rc;
-            const half* src[3] = {comp, comp + e->qkv_cols[0], comp + e->qkv_cols[0] + e->qkv_cols[1]};
-            const int sp[3] = {P, P, P}, dp[3] = {3 * d, 3 * d, 3 * d};
-            half* dst[3] = {b0, b0 + d, b0 + 2 * d};
-            const int* inv[3] = {e->rq->d_inv, e->rk->d_inv, e->rv->d_inv};
-            if ((rc = expand_rows_launch(3, src, sp, dst, dp, inv, d, T, st))) return rc;
-            q_pitch = v_pitch = 3 * d;
-            b1 = b0 + d;
-            b2 = b0 + 2 * d;
-        } else {
-            // Q and K are dense already (inside the fused result); only V is expanded, into buffer 4
-            if ((rc = tile_linear_run(e->qkv, b0, in, T, 0, st))) return rc;
-            const half* src[1] = {b0 + e->qkv_cols[0] + e->qkv_cols[1]};
-            const int sp[1] = {P}, dp[1] = {d};
-            half* dst[1] = {b4};
-            const int* inv[1] = {e->rv->d_inv};
-            if ((rc = expand_rows_launch(1, src, sp, dst, dp, inv, d, T, st))) return rc;
-            q_pitch = P;
-            v_pitch = d;
-            b1 = b0 + e->qkv_cols[0];
-            b2 = b4;
-        }
+        if ((rc = attention_tc_launch(b3, b0, b0 + e->qkv_cols[0], b0 + e->qkv_cols[0] + e->qkv_cols[1], P, P, e->qkv_cols[0],
+                                      e->qkv_cols[2], e->d_qk_ptr, e->d_v_ptr, nullptr, e->d_mask, e->seq_len, cu_seqlens, valid_lens,
+                                      batch, uniform_len, T, cu_seqlens ? max_len : uniform_len, e->d_model, e->nheads, st)))
+            return rc == ET_ERR_UNSUPPORTED ? fail(ET_ERR_INVALID, "encoder: scratch must be 16-byte aligned") : rc;
     } else if (e->qkv) {
         // fused: one launch writes Q | K | V side by side, [T x (q + k + v columns)] over the first three scratch
         // buffers (row-pruned parts are compact, so the three widths may differ)
@@ -352,11 +344,11 @@ static int encoder_forward(Encoder* e, half* out, const half* in, half* scratch,
         if ((rc = qk_scores_launch(sbuf, b0, b1, batch, uniform_len, e->d_model, e->nheads, st, q_pitch))) return rc;
         scores = sbuf;
     }
-    if ((rc = attention_launch(b3, b0, b1, b2, scores, q_pitch, v_pitch, qk_hp, v_id, v_hp, e->d_mask, e->seq_len,
+    if (!e->o_compact && (rc = attention_launch(b3, b0, b1, b2, scores, q_pitch, v_pitch, qk_hp, v_id, v_hp, e->d_mask, e->seq_len,
                                cu_seqlens, valid_lens, batch, uniform_len, T, e->d_model, e->nheads, st, max_len)))
         return rc;
     b1 = scratch + td;
-    if ((rc = tile_linear_run(e->lin[3], b0, b3, T, 0, st))) return rc;
+    if ((rc = tile_linear_run(e->o_compact ? e->o_compact : e->lin[3], b0, b3, T, 0, st))) return rc;
     if ((rc = et_skip_layernorm(b0, in, e->d_ln[0], e->d_ln[1], T, e->d_model, st))) return rc;
     if ((rc = tile_linear_run(e->lin[4], b1, b0, T, 1, st))) return rc;
     if ((rc = tile_linear_run(e->lin[5], out, b1, T, 0, st))) return rc;
@@ -637,6 +629,41 @@ static int take_tiles(Encoder* e, et_tile_weight** t, int first, int count, int 
     return ET_OK;
 }
 
+// Lays a row-pruned layer out for compact heads (see Encoder::o_compact): q, k, v are the parts of the fused weight, rows[i] the
+// row-pruned linear behind part i or null. Leaves the encoder as it was where the output projection cannot be gathered.
+static int compact_heads(Encoder* e, const et::TileWeight* const* dense, RowWeight* const* rows) {
+    et::TileWeight* own[3] = {nullptr, nullptr, nullptr};
+    const et::TileWeight* parts[3];
+    std::vector<int> ptr[3];
+    int rc = ET_OK;
+    for (int i = 0; i < 3 && rc == ET_OK; ++i) {
+        if (rows[i]) rc = et::row_weight_padded(&own[i], rows[i], et::tile_weight_size(rows[i]->tw), ptr[i]);
+        parts[i] = rows[i] ? own[i] : dense[i];
+    }
+    if (rc == ET_OK) {
+        std::vector<int> src((size_t)ptr[2].back(), -1);
+        for (int h = 0; h < e->nheads; ++h)
+            for (int j = rows[2]->h_head_ptr[h]; j < rows[2]->h_head_ptr[h + 1]; ++j)
+                src[ptr[2][h] + j - rows[2]->h_head_ptr[h]] = rows[2]->h_row_id[j];
+        rc = et::tile_weight_gather_inputs(&e->o_compact, e->lin[3], src.data(), (int)src.size());
+        if (rc == ET_ERR_UNSUPPORTED) {
+            for (auto* t : own) et::tile_weight_free(t);
+            return ET_OK;
+        }
+    }
+    if (rc == ET_OK) rc = et::tile_weight_concat(&e->qkv, parts, 3, 0);
+    auto upload = [](int** d, const std::vector<int>& v) {
+        if (cudaMalloc(d, v.size() * sizeof(int)) != cudaSuccess) return et::fail(ET_ERR_CUDA, "encoder: cudaMalloc failed");
+        return et::cuda_status(cudaMemcpy(*d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice), "encoder: upload");
+    };
+    if (rc == ET_OK && rows[0]) rc = upload(&e->d_qk_ptr, ptr[0]);
+    if (rc == ET_OK) rc = upload(&e->d_v_ptr, ptr[2]);
+    if (rc == ET_OK) rc = et::cuda_status(cudaDeviceSynchronize(), "encoder: upload");
+    for (int i = 0; i < 3 && rc == ET_OK; ++i) e->qkv_cols[i] = rows[i] ? ptr[i].back() : e->d_model;
+    for (auto* t : own) et::tile_weight_free(t);
+    return rc;
+}
+
 static int finish_create(et_encoder** out, std::unique_ptr<Encoder>& e) {
     *out = new et_encoder{e.release()};
     return ET_OK;
@@ -692,10 +719,14 @@ int et_encoder_prune_create(et_encoder** out, int d_model, int seq_len, int nhea
         e->rv->in_feat == d_model) {
         // Q | K | compact V in one launch
         const et::TileWeight* parts[3] = {e->lin[0], e->lin[1], e->rv->tw};
+        if (d_model == 64 * nheads && e->rv->out_feat == d_model && e->rv->nhead == nheads) {
+            RowWeight* const rows[3] = {nullptr, nullptr, e->rv};
+            if ((rc = compact_heads(e.get(), parts, rows))) return rc;
+            if (e->o_compact) return finish_create(out, e);
+        }
         if ((rc = et::tile_weight_concat(&e->qkv, parts, 3, 0))) return rc;
         e->qkv_cols[0] = e->qkv_cols[1] = d_model;
         e->qkv_cols[2] = e->rv->nrow;
-        e->expand_pruned = d_model / nheads == 64 && e->rv->out_feat == d_model;   // the tensor-core kernel's head width
     }
     return finish_create(out, e);
 }
@@ -722,14 +753,19 @@ int et_encoder_prune_qkv_create(et_encoder** out, int d_model, int seq_len, int 
     e->rq = q->w; q->w = nullptr;
     e->rk = k->w; k->w = nullptr;
     e->rv = v->w; v->w = nullptr;
+    if (e->rq->in_feat == d_model && e->rk->in_feat == d_model && e->rv->in_feat == d_model && d_model == 64 * nheads &&
+        e->rq->out_feat == d_model && e->rk->out_feat == d_model && e->rv->out_feat == d_model && e->rq->nhead == nheads &&
+        e->rk->nhead == nheads && e->rv->nhead == nheads) {
+        RowWeight* const rows[3] = {e->rq, e->rk, e->rv};
+        if ((rc = compact_heads(e.get(), nullptr, rows))) return rc;
+        if (e->o_compact) return finish_create(out, e);
+    }
     if (e->rq->in_feat == d_model && e->rk->in_feat == d_model && e->rv->in_feat == d_model &&
         e->rq->nrow + e->rk->nrow + e->rv->nrow <= 3 * d_model) {
         // compact Q | K | V in one launch
         const et::TileWeight* parts[3] = {e->rq->tw, e->rk->tw, e->rv->tw};
         if ((rc = et::tile_weight_concat(&e->qkv, parts, 3, 0))) return rc;
         e->qkv_cols[0] = e->rq->nrow; e->qkv_cols[1] = e->rk->nrow; e->qkv_cols[2] = e->rv->nrow;
-        e->expand_pruned = d_model / nheads == 64 && e->rq->out_feat == d_model && e->rk->out_feat == d_model &&
-                           e->rv->out_feat == d_model && e->rq->nrow + e->rk->nrow + e->rv->nrow <= 2 * d_model;
     }
     return finish_create(out, e);
 }
@@ -831,6 +867,7 @@ int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* 
 static int encoder_check(Encoder* e, int* code) {
     std::vector<et::TileWeight*> ws(e->lin, e->lin + 6);
     ws.push_back(e->qkv);
+    ws.push_back(e->o_compact);
     for (RowWeight* r : {e->rq, e->rk, e->rv})
         if (r) ws.push_back(r->tw);
     for (et::TileWeight* w : ws) {

@@ -614,6 +614,7 @@ struct TileWeight {
     std::vector<uint2> h_first;   // directory entry of each chunk's first block
     uint2* d_dir = nullptr;
     uint8_t* d_stream = nullptr;
+    uint8_t* d_small = nullptr;                  // holds the next two and the error word
     half* d_bias = nullptr;
     float* d_bias_f32 = nullptr;                 // the bias as fp32 (fused epilogues)
     float* d_colc = nullptr; float* d_cold = nullptr;   // c_n, d_n of a weight folded with a LayerNorm's gamma / beta
@@ -751,8 +752,7 @@ static int build_tile_form(TileWeight* w) {
         cudaMalloc(&w->d_stream, std::max<size_t>(stream.size(), 16)) != cudaSuccess)
         return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed");
     cudaMemcpy(w->d_dir, dir.data(), dir.size() * sizeof(uint2), cudaMemcpyHostToDevice);
-    cudaMemcpy(w->d_stream, stream.data(), stream.size(), cudaMemcpyHostToDevice);
-    return cuda_status(cudaDeviceSynchronize(), "tile weight upload");
+    return cuda_status(cudaMemcpy(w->d_stream, stream.data(), stream.size(), cudaMemcpyHostToDevice), "tile weight upload");
 }
 
 // The dense form: the weight as a row-major [N x K] matrix, zeros where tiles were pruned.
@@ -819,17 +819,20 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
              : plain && resident < 0.97 * tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);
     if (rc) { tile_weight_free(w); return rc; }
-    if (cudaMalloc(&w->d_bias, (size_t)N * sizeof(half)) != cudaSuccess || cudaMalloc(&w->d_err, sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&w->d_bias_f32, (size_t)N * sizeof(float)) != cudaSuccess) {
+    // the bias in both types and the error word in one allocation and one copy
+    const size_t at_half = (size_t)N * sizeof(float), at_err = at_half + (size_t)N * sizeof(half);   // N is a multiple of 16
+    std::vector<uint8_t> small(at_err + sizeof(int), 0);
+    for (int i = 0; i < N; ++i) reinterpret_cast<float*>(small.data())[i] = __half2float(w->h_bias[i]);
+    std::memcpy(small.data() + at_half, w->h_bias.data(), (size_t)N * sizeof(half));
+    if (cudaMalloc(&w->d_small, small.size()) != cudaSuccess) {
         tile_weight_free(w);
         return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed");
     }
-    std::vector<float> bf((size_t)N);
-    for (int i = 0; i < N; ++i) bf[i] = __half2float(w->h_bias[i]);
-    cudaMemcpy(w->d_bias_f32, bf.data(), (size_t)N * sizeof(float), cudaMemcpyHostToDevice);
-    cudaMemcpy(w->d_bias, w->h_bias.data(), (size_t)N * sizeof(half), cudaMemcpyHostToDevice);
-    cudaMemset(w->d_err, 0, sizeof(int));
-    rc = cuda_status(cudaDeviceSynchronize(), "tile weight upload");
+    w->d_bias_f32 = reinterpret_cast<float*>(w->d_small);
+    w->d_bias = reinterpret_cast<half*>(w->d_small + at_half);
+    w->d_err = reinterpret_cast<int*>(w->d_small + at_err);
+    rc = cuda_status(cudaMemcpy(w->d_small, small.data(), small.size(), cudaMemcpyHostToDevice), "tile weight upload");
+    if (rc == ET_OK) rc = cuda_status(cudaDeviceSynchronize(), "tile weight upload");   // launches on any stream may follow
     if (rc) { tile_weight_free(w); return rc; }
     *out = w;
     return ET_OK;
@@ -855,10 +858,41 @@ int tile_weight_concat(TileWeight** out, const TileWeight* const* parts, int cou
                             bias.data(), 0);
 }
 
+int tile_weight_gather_inputs(TileWeight** out, const TileWeight* w, const int* src, int n) {
+    *out = nullptr;
+    const int NBR = w->N / 16;
+    if (n <= 0 || n % 16) return fail(ET_ERR_INVALID, "tile weight gather: the number of features must be a positive multiple of 16");
+    if (repeats_a_tile(w->h_row_ptr.data(), w->h_row_offset.data(), NBR)) return fail(ET_ERR_UNSUPPORTED, "tile weight gather: a tile is listed twice");
+    std::vector<int> rp(1, 0), ro;
+    std::vector<half> data, rows((size_t)16 * w->K);
+    for (int r = 0; r < NBR; ++r) {
+        std::fill(rows.begin(), rows.end(), __float2half(0.f));
+        for (int i = w->h_row_ptr[r]; i < w->h_row_ptr[r + 1]; ++i)
+            for (int m = 0; m < 16; ++m)
+                std::memcpy(&rows[(size_t)m * w->K + w->h_row_offset[i]], &w->h_data[(size_t)i * 256 + m * 16], 32);
+        for (int c = 0; c < n / 16; ++c) {
+            uint16_t tile[256], any = 0;   // as bits: only zeros are told apart
+            const uint16_t* in = reinterpret_cast<const uint16_t*>(rows.data());
+            for (int m = 0; m < 16; ++m)
+                for (int k = 0; k < 16; ++k) {
+                    const int f = src[16 * c + k];
+                    const uint16_t v = f >= 0 ? in[(size_t)m * w->K + f] : 0;
+                    tile[m * 16 + k] = v;
+                    any |= v & 0x7fff;
+                }
+            if (!any) continue;
+            ro.push_back(16 * c);
+            const half* t = reinterpret_cast<const half*>(tile);
+            data.insert(data.end(), t, t + 256);
+        }
+        rp.push_back((int)ro.size());
+    }
+    return tile_weight_pack(out, n, w->N, w->size_hint, (long)ro.size(), data.data(), rp.data(), ro.data(), w->h_bias.data(), 0);
+}
+
 void tile_weight_free(TileWeight* w) {
     if (!w) return;
-    cudaFree(w->d_dir); cudaFree(w->d_stream); cudaFree(w->d_bias); cudaFree(w->d_err);
-    cudaFree(w->d_bias_f32); cudaFree(w->d_colc); cudaFree(w->d_cold); cudaFree(w->d_dense);
+    cudaFree(w->d_dir); cudaFree(w->d_stream); cudaFree(w->d_small); cudaFree(w->d_colc); cudaFree(w->d_cold); cudaFree(w->d_dense);
     resident_free(w->resident);
     delete w;
 }
@@ -933,6 +967,7 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
 
 int tile_weight_prepare_fusion(TileWeight* w) { return build_tile_form(w); }
 int tile_weight_out_feat(const TileWeight* w) { return w->N; }
+int tile_weight_size(const TileWeight* w) { return w->size_hint; }
 int tile_weight_chunks(const TileWeight* w) { return w->n_chunks; }
 int tile_weight_stat_slots(const TileWeight* w) { return kEpiPerQuarter * w->n_chunks; }
 

@@ -34,6 +34,7 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
 // New weight = the parts' output features back to back (equal in_feat); the parts stay valid.
 int tile_weight_concat(TileWeight** out, const TileWeight* const* parts, int count, int size_hint);
 int tile_weight_out_feat(const TileWeight* w);
+int tile_weight_size(const TileWeight* w);   // the token count that the weight was made for
 void tile_weight_free(TileWeight* w);
 // bias_dev != null replaces the weight's own bias for this launch (device pointer, N halfs).
 int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu, cudaStream_t st,
@@ -41,6 +42,9 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
 // New weight = w with gamma multiplied into its input features and the column vectors c_n = sum_k gamma_k W_nk,
 // d_n = sum_k beta_k W_nk + bias_n that the mode-1 epilogue needs (gamma, beta: host, in_feat values).
 int tile_weight_fold(TileWeight** out, const TileWeight* w, const half* gamma, const half* beta);
+// New weight whose input feature j is input feature src[j] of `w`, or zero where src[j] < 0 (n: a multiple of 16; tiles that
+// become all zero are dropped). ET_ERR_UNSUPPORTED when a block-row lists a tile twice.
+int tile_weight_gather_inputs(TileWeight** out, const TileWeight* w, const int* src, int n);
 // Builds what the fused epilogues (GemmFusion) of this weight need, if it is not there yet.
 int tile_weight_prepare_fusion(TileWeight* w);
 // Column chunks of the packed weight, and the partial-sum slots per row that its residual epilogue writes.

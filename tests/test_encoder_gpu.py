@@ -349,3 +349,44 @@ def test_run_batch_on_the_legacy_stream_and_on_a_side_stream_agree(et, orc):
         torch.cuda.synchronize()
         assert torch.equal(out, ref_out), f"call {call}"
         assert torch.equal(doubled, ref_out * 2)
+
+
+@pytest.mark.parametrize("qk_keep,v_keep", [(None, [1, 17, 64, 16]), ([15, 64, 1, 33], [64, 2, 48, 31])])
+@pytest.mark.parametrize("mask", [False, True])
+def test_prune_layers_with_heads_of_any_width(et, orc, qk_keep, v_keep, mask):
+    """Heads that keep one feature, all of them and counts around the multiples of 16 that the layer pads them to; Q/K and V keep
+    different ones. Tolerance as for the other layers with unit-scale weights: fp16 storage of O(1) values through five stages."""
+    d, H, S = 256, 4, 130
+    lin, ln = make_layer(orc, d, 1024, 0.5, seed=80, unit_scale=True)
+    ol = orc_lin(lin)
+    lens = [130, 1, 65]
+    T = sum(lens)
+    X = util.activations(81, (T, d))
+    M = util.activations(82, (S, S)) if mask else None
+    rng = np.random.default_rng(83)
+
+    def ids(keep):
+        return np.concatenate([h * 64 + np.sort(rng.choice(64, n, replace=False)) for h, n in enumerate(keep)]).astype(np.int32)
+
+    rows = {n: ids(k) for n, k in zip("qv", (qk_keep or [64] * H, v_keep))}
+    rows["k"] = rows["q"]
+    std = 1.0 / np.sqrt(d)
+    Wr = {n: util.weights(320 + i, (len(rows[n]), d), std) for i, n in enumerate("qkv")}
+    br = {n: util.weights(330 + i, (len(rows[n]),), 0.02) for i, n in enumerate("qkv")}
+    Xf = X.astype(np.float32)
+    q, k, v = (orc.row_linear(Xf, Wr[n], br[n]) if qk_keep or n == "v" else orc.tile_linear(Xf, *ol[n][:4], ol[n][4]) for n in "qkv")
+    z = orc.attention(q, k, v, lens, d, H, mask=M, qk_head_ptr=orc.head_ptr(rows["q"], H, d) if qk_keep else None, v_col_id=rows["v"],
+                      v_head_ptr=orc.head_ptr(rows["v"], H, d))
+    h1 = orc.skip_layernorm(orc.tile_linear(z, *ol["o"][:4], ol["o"][4]), Xf, *ln[0])
+    f = orc.tile_linear(h1, *ol["ffn1"][:4], ol["ffn1"][4], gelu=True)
+    want = orc.skip_layernorm(orc.tile_linear(f, *ol["ffn2"][:4], ol["ffn2"][4]), h1, *ln[1])
+    w = tile_weights(et, lin, T)
+    r = {n: et.RowWeight(d, d, T, Wr[n], rows[n], br[n], H) for n in ("qkv" if qk_keep else "v")}
+    enc = et.Encoder(et.KIND_PRUNE_QKV if qk_keep else et.KIND_PRUNE, d, S, H, None, r.get("q", w["q"]), r.get("k", w["k"]), r["v"],
+                     w["o"], w["ffn1"], w["ffn2"], (ln[0][0], ln[0][1], ln[1][0], ln[1][1]), mask=M)
+    scratch = torch.zeros(et.encoder_batch_buffer_size(et.KIND_PRUNE, d, T, len(lens), S, H) // 2, dtype=torch.float16, device="cuda")
+    out = torch.zeros((T, d), dtype=torch.float16, device="cuda")
+    enc.run_batch(out, dev(X), lens, scratch)
+    torch.cuda.synchronize()
+    util.assert_close(host(out), want, what="row-pruned layer", max_abs=4e-2, mean_abs=4e-3)
+    enc.check()

@@ -79,7 +79,7 @@ struct GemmParams {
     const uint8_t* stream;   // packed blocks
     half* Y;
     const half* bias;
-    int T, N, k_chunks, n_chunks, n_tiles, nb, stage_b_bytes, nx, nw, a_slots, gelu;
+    int T, N, k_chunks, n_chunks, n_tiles, nb, nx, w_ring, w_room, a_slots, gelu;   // bytes of the weight ring, and of it for a block at least
     int* err;
     uint2 first[kDirInParams];   // dir[chunk][0] for chunk < kDirInParams: no global load before the first TMA
     GemmFusion fz;           // LayerNorm folded into the epilogue (modes 1-3 of the kernel template)
@@ -107,12 +107,13 @@ struct Shared {
     // cannot be a whole phase late, which fixes each ring's length):
     uint64_t full_x[kMaxRing];    // [chunk % FX]  the chunk's activations have landed (TMA); FX = nx, doubled when odd, so
                                   //               that a barrier always falls to the same one of the two movers
-    uint64_t full_w[kMaxRing];    // [chunk % FW]  the chunk's weight block has landed (bulk copy); FW from nw likewise
+    uint64_t full_w[kMaxRing];    // [chunk % kMaxRing]  the chunk's weight block has landed (bulk copy)
     uint64_t a_ready[kMaxRing];   // [chunk % kMaxRing]  the chunk's activations are in tensor memory (mover commit): read by
                                   //               the issuers, and by the activation producer as "shared-memory slot free"
     uint64_t a_issued[kMaxRing];  // [chunk % a_slots]  every issuer has issued (not completed) its UMMAs on the chunk
-    uint64_t done[kMaxRing];      // [chunk % nw]  every issuer's UMMAs on the chunk have completed (8 commits)
+    uint64_t done[kMaxRing];      // [chunk % kMaxRing]  every issuer's UMMAs on the chunk have completed (8 commits)
     uint64_t acc_done;            // 8 issuer commits after a tile's last chunk
+    int w_at[kMaxRing];           // [chunk % kMaxRing]  where in the weight ring the block starts (valid with full_w)
     uint32_t tmem_base;
     volatile int abort;            // any role gave up: everybody winds down
     volatile int issuer_abort[2];  // [tile parity]: set by an issuer warp that gives up during a tile, read by
@@ -245,11 +246,11 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                  const __grid_constant__ GemmParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int NX = p.nx, NW = p.nw, RA = p.a_slots;
-    const int FX = (NX & 1) ? 2 * NX : NX, FW = (NW & 1) ? 2 * NW : NW;
+    const int NX = p.nx, RA = p.a_slots;
+    const int FX = (NX & 1) ? 2 * NX : NX;
     uint8_t* const xring = smem;                                       // NX x 32 KB of activations
-    uint8_t* const wring = smem + (size_t)NX * kXStageBytes;           // NW weight blocks
-    uint8_t* const epi = wring + (size_t)NW * p.stage_b_bytes;         // 16 warps x 2 KB
+    uint8_t* const wring = smem + (size_t)NX * kXStageBytes;           // weight blocks
+    uint8_t* const epi = wring + p.w_ring;                             // 16 warps x 2 KB
     Shared* sh = reinterpret_cast<Shared*>(epi + kEpiWarps * kUnitBytes);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = gridDim.x;
@@ -319,11 +320,15 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 mbar_wait(&sh->full_x[kk % FX], (uint32_t)(kk / FX) & 1u);
     } else if (warp == 1) {
         // ---------------- weight producer: the packed weight does not depend on the preceding kernel, so these copies
-        // start as soon as the barriers exist. A slot is free when the UMMAs that read it have completed.
+        // start as soon as the barriers exist. The ring holds blocks one behind the other (lane l knows the bounds of the block
+        // in barrier slot l); a block that does not fit before the end starts at the beginning. It may be copied once the UMMAs
+        // on every block that it overlaps, and on all before those, have completed.
         named_barrier_sync(4, 64);
         named_barrier_arrive(2, kThreads);
-        int issued = 0, ws = 0, fw = 0;
-        uint32_t phw = 0;
+        int issued = 0, ws = 0;            // blocks requested, barrier slot of the next
+        int oldest = 0, os = 0, head = 0;  // first block not known to be done, its slot; end of the last block
+        uint32_t pho = 0;
+        int from = 0, to = 0;
         bool alive = true;
         for (int tl = 0; tl < my_tiles && alive; ++tl) {
             const int tile = (int)blockIdx.x + tl * G;
@@ -331,11 +336,19 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             const uint2* gdir = p.dir + (size_t)chunk * p.k_chunks;
             // directory entries: the first one of the first tile comes from the kernel parameters, the others are
             // fetched one chunk ahead
-            uint2 dnext = (tl == 0 && chunk < kDirInParams) ? p.first[chunk] : (lane == 0 ? __ldg(gdir) : make_uint2(0, 0));
+            uint2 dnext = (tl == 0 && chunk < kDirInParams) ? p.first[chunk] : __ldg(gdir);
             for (int kc = 0; kc < p.k_chunks; ++kc) {
                 const uint2 d = dnext;
-                if (lane == 0 && kc + 1 < p.k_chunks) dnext = __ldg(gdir + kc + 1);
-                const bool go = mbar_wait(&sh->done[ws], phw ^ 1u);
+                if (kc + 1 < p.k_chunks) dnext = __ldg(gdir + kc + 1);
+                const int bytes = (int)(d.y * 16u), room = max((bytes + 127) & ~127, p.w_room);
+                const int at = head + room <= p.w_ring ? head : 0;
+                bool go = true;
+                while (go && (issued - oldest == kMaxRing || __any_sync(0xffffffffu, from < at + room && to > at))) {
+                    go = mbar_wait(&sh->done[os], pho);
+                    if (lane == os) from = to = 0;
+                    ++oldest;
+                    if (++os == kMaxRing) { os = 0; pho ^= 1u; }
+                }
                 if (!go) {
                     if (lane == 0 && !sh->abort) {
                         atomicExch(p.err, 15);
@@ -345,19 +358,20 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                     break;
                 }
                 if (lane == 0) {
-                    const uint32_t bbytes = d.y * 16u;
-                    mbar_expect_tx(&sh->full_w[fw], bbytes);
-                    bulk_load(wring + (size_t)ws * p.stage_b_bytes, p.stream + (size_t)d.x * 16u, bbytes, &sh->full_w[fw]);
+                    sh->w_at[ws] = at;
+                    mbar_expect_tx(&sh->full_w[ws], (uint32_t)bytes);
+                    bulk_load(wring + at, p.stream + (size_t)d.x * 16u, (uint32_t)bytes, &sh->full_w[ws]);
                     if (issued < 64) ET_STAMP(1100 + issued);
                 }
+                head = at + room;
+                if (lane == ws) { from = at; to = head; }
                 ++issued;
-                if (++fw == FW) fw = 0;
-                if (++ws == NW) { ws = 0; phw ^= 1u; }
+                if (++ws == kMaxRing) ws = 0;
             }
         }
         if (lane == 1 && sh->abort)
-            for (int kk = issued > NW ? issued - NW : 0; kk < issued; ++kk)
-                mbar_wait(&sh->full_w[kk % FW], (uint32_t)(kk / FW) & 1u);
+            for (int kk = issued > kMaxRing ? issued - kMaxRing : 0; kk < issued; ++kk)
+                mbar_wait(&sh->full_w[kk % kMaxRing], (uint32_t)(kk / kMaxRing) & 1u);
     } else {
         if (warp == kFirstMover) {
             tmem_alloc(&sh->tmem_base, 512);
@@ -428,7 +442,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 fx += kMovers;
                 if (fx >= FX) { fx -= FX; phx ^= 1u; }
                 fw += kMovers;
-                if (fw >= FW) { fw -= FW; phw ^= 1u; }
+                if (fw >= kMaxRing) { fw -= kMaxRing; phw ^= 1u; }
                 ar += kMovers;
                 if (ar >= kMaxRing) ar -= kMaxRing;
             }
@@ -475,7 +489,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                             break;
                         }
                         tc_fence_after();
-                        const uint8_t* blk = wring + (size_t)ws * p.stage_b_bytes;
+                        const uint8_t* blk = wring + sh->w_at[ws];
                         const uint32_t hw = reinterpret_cast<const uint32_t*>(blk)[w];
                         const int e0 = hw & 0xffff, ne = hw >> 16;
                         const uint32_t n_entries = reinterpret_cast<const uint32_t*>(blk)[8];
@@ -496,7 +510,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                         }
                         if (w == 0 && lane == 0 && tl * p.k_chunks + kc < 64) ET_STAMP(600 + tl * p.k_chunks + kc);
                         __syncwarp();
-                        if (++ws == NW) ws = 0;
+                        if (++ws == kMaxRing) ws = 0;
                         if (++a == RA) a = 0;
                         if (++ar == kMaxRing) { ar = 0; pha ^= 1u; }
                     }
@@ -604,7 +618,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 // --------------------------------------------------------------------------------- host side
 
 struct TileWeight {
-    int K = 0, N = 0, nb = 0, n_chunks = 0, k_chunks = 0, stage_b_bytes = 0, nx = 0, nw = 0, a_slots = 0;
+    int K = 0, N = 0, nb = 0, n_chunks = 0, k_chunks = 0, stage_b_bytes = 0, nx = 0, w_ring = 0, w_room = 0, a_slots = 0;   // stage_b_bytes: the largest weight block
     int tiles_per_cta = 1;   // > 1 when packed for SM time: a CTA takes that many tiles even when SMs are free
     long ntile = 0;
     int size_hint = 0;
@@ -631,22 +645,28 @@ struct TileWeight {
 
 // Ring depths for a chunk shape. The operands live for different times, so each has its own ring: an activation
 // slot (32 KB) goes round in ~2700 clocks (free when copied on to tensor memory -> seen by the producer -> TMA ->
-// landed -> copied), a weight slot in ~2500 (free when its UMMAs have completed -> seen -> bulk copy -> landed ->
+// landed -> copied), a weight block in ~2500 (free when its UMMAs have completed -> seen -> bulk copy -> landed ->
 // the issuers reach it), a tensor-memory slot in ~1400 (UMMAs issued -> seen by the mover -> eight tcgen05.cp ->
 // seen by the issuers). The period of a chunk is the largest cycle / depth; shared memory is shared out to make
-// that smallest (at most four slots per ring: beyond that the cycles above no longer bound the period).
-struct RingShape { int nx, nw, a_slots; double period; };
-static RingShape ring_shape(int nb, int stage_b_bytes) {
+// that smallest (at most four slots of activations: beyond that the cycles above no longer bound the period). Weight blocks
+// vary in size: they lie back to back where clearly more fit than slots for the largest one (24 block-rows, 75 % sparsity: 3.8
+// instead of 2, and 3072 -> 768 chunks of 1230 clocks instead of 1480). They count for 0.7: room is lost at the ring's end, and a
+// block waits for every one that it overlaps (50 % sparsity, two blocks: 16 % slower back to back).
+struct RingShape { int nx, w_ring, w_room, a_slots; double period; };
+static RingShape ring_shape(int nb, int largest, double mean) {
     const int tmem_slots = std::min(4, (512 - nb * 16) / kSlotCols);
     const int avail = kSmemMax - 1024 - (int)sizeof(Shared) - kEpiWarps * kUnitBytes;
-    static_assert(kMovers == 2 && 2 * 3 <= kMaxRing && 4 <= kMaxRing, "the full-barrier rings must fit");
-    RingShape best{0, 0, tmem_slots, 1e30};
-    for (int nx = 2; nx <= 4; ++nx)
-        for (int nw = 2; nw <= 4; ++nw) {
-            if (nx * kXStageBytes + nw * stage_b_bytes > avail || tmem_slots < 1) continue;
-            const double period = std::max({2700.0 / nx, 2500.0 / nw, 1400.0 / tmem_slots});
-            if (period < best.period * 0.999) best = RingShape{nx, nw, tmem_slots, period};
-        }
+    static_assert(kMovers == 2 && 2 * 3 <= kMaxRing && 4 <= kMaxRing && kMaxRing % kMovers == 0, "a full barrier falls to one mover");
+    RingShape best{0, 0, 0, tmem_slots, 1e30};
+    for (int nx = 2; nx <= 4; ++nx) {
+        const int ring = std::min((avail - nx * kXStageBytes) / 1024, kMaxRing * largest / 1024) * 1024;
+        if (ring < 2 * largest || tmem_slots < 1) continue;
+        const int slots = std::min(4, ring / largest);
+        const double packed = std::min((double)kMaxRing, 0.7 * ring / mean);
+        const bool pack = packed > 1.2 * slots;
+        const double period = std::max({2700.0 / nx, 2500.0 / (pack ? packed : slots), 1400.0 / tmem_slots});
+        if (period < best.period * 0.999) best = RingShape{nx, pack ? ring : slots * largest, pack ? 0 : largest, tmem_slots, period};
+    }
     return best;
 }
 // Block-rows per CTA from a model of the persistent kernel: a chunk takes the ring period, or its UMMAs (~10
@@ -673,7 +693,7 @@ static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double densi
         const double tiles_max = std::min((double)nbe * kSlices,
                                           tiles_per_chunk + 3.0 * std::sqrt(nbe * kSlices * density * (1.0 - density)));
         const int stage_b = (int)((kHeaderBytes + tiles_max * 528.0 + 1023) / 1024) * 1024;
-        const RingShape rs = ring_shape(nbe, stage_b);
+        const RingShape rs = ring_shape(nbe, stage_b, kHeaderBytes + tiles_per_chunk * 528.0);
         if (rs.nx < 2 || rs.a_slots < 1) continue;
         const long tiles = (long)slabs * ((n_block_rows + nbe - 1) / nbe);
         const double per_cta = (double)((tiles + sms - 1) / sms);
@@ -742,8 +762,8 @@ static int build_tile_form(TileWeight* w) {
     for (int c = 0; c < w->n_chunks && c < kDirInParams; ++c) w->h_first.push_back(dir[(size_t)c * w->k_chunks]);
     w->stage_b_bytes = (int)((max_block + 1023) / 1024 * 1024);
     {
-        const RingShape rs = ring_shape(w->nb, w->stage_b_bytes);
-        w->nx = rs.nx; w->nw = rs.nw; w->a_slots = rs.a_slots;
+        const RingShape rs = ring_shape(w->nb, w->stage_b_bytes, (double)stream.size() / nblocks);
+        w->nx = rs.nx; w->w_ring = rs.w_ring; w->w_room = rs.w_room; w->a_slots = rs.a_slots;
     }
     if (w->nx < 2 || w->a_slots < 1) return fail(ET_ERR_UNSUPPORTED, "tile weight: weight block exceeds shared memory");
     w->stream_bytes = stream.size();
@@ -810,13 +830,14 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's, which
     // was made to compare its own shapes only, is 1.3 times too short). At 75 % sparsity and 32768 tokens, in us, tile / resident /
-    // dense: 768 -> 2304 84 / 63 / 83, 3072 -> 768 76 / - / 107, 1024 -> 3072 128 / 167 / 132; without zeros 160 / - / 96.
+    // dense: 768 -> 2304 74 / 63 / 83, 3072 -> 768 75 / - / 107, 1024 -> 3072 109 / 167 / 132; without zeros 160 / - / 96.
+    // (1.08: where the first two come this close, the resident kernel was the faster one in seven of ten measured launches.)
     tile_cost = 1.3 * tile_cost + 1000.0;
     const double resident = resident_cost(size_hint, N, K, density);
     const bool plain = nb_override <= 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
     w->packed_dense = plain && w->dense.cost < std::min(tile_cost, resident);
     int rc = w->packed_dense ? build_dense_form(w)
-             : plain && resident < 0.97 * tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
+             : plain && resident < 1.08 * tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);
     if (rc) { tile_weight_free(w); return rc; }
     // the bias in both types and the error word in one allocation and one copy
@@ -934,10 +955,10 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
     p.T = T; p.N = w->N; p.k_chunks = w->k_chunks; p.nb = w->nb;
     p.n_chunks = w->n_chunks;
     p.n_tiles = ((T + kSlab - 1) / kSlab) * w->n_chunks;
-    p.stage_b_bytes = w->stage_b_bytes; p.nx = w->nx; p.nw = w->nw; p.a_slots = w->a_slots; p.gelu = gelu; p.err = w->d_err;
+    p.nx = w->nx; p.w_ring = w->w_ring; p.w_room = w->w_room; p.a_slots = w->a_slots; p.gelu = gelu; p.err = w->d_err;
     p.prof = g_prof;
     for (size_t c = 0; c < w->h_first.size(); ++c) p.first[c] = w->h_first[c];
-    const size_t smem = (size_t)w->nx * kXStageBytes + (size_t)w->nw * w->stage_b_bytes +
+    const size_t smem = (size_t)w->nx * kXStageBytes + (size_t)w->w_ring +
                         (size_t)kEpiWarps * kUnitBytes + sizeof(Shared) + 1024;
     // Packed for SM time (several batches in flight): a CTA takes several tiles in a row even when SMs are free,
     // so that set-up and pipeline fill are paid once and the next tile's loads run under an epilogue.
@@ -1033,7 +1054,7 @@ void tile_weight_info(const TileWeight* w, int* info) {
         std::copy(v, v + 6, info);
         return;
     }
-    info[0] = w->nb; info[1] = w->n_chunks; info[2] = w->k_chunks; info[3] = w->nx;   // activation slots (the weight ring has w->nw, chosen from the same memory)
+    info[0] = w->nb; info[1] = w->n_chunks; info[2] = w->k_chunks; info[3] = w->nx;   // activation slots
     info[4] = w->stage_b_bytes; info[5] = (int)std::min<size_t>(w->stream_bytes, 0x7fffffff);
 }
 

@@ -162,6 +162,8 @@ def test_tile_linear(et, orc, T, K, N, sparsity, gelu):
     (260, 1024, 1024, 0.9, False, 32768, "resident"),    # K beyond the tensor-memory part
     (5000, 1024, 4096, 0.9, True, 32768, "resident"),
     (300, 768, 2304, 0.995, False, 32768, "resident"),   # block-rows without tiles
+    (700, 3072, 768, 0.75, False, 17792, "tile"),        # weight blocks back to back in their ring, many times round
+    (701, 3072, 768, 0.6, False, 17792, "tile"),         # weight blocks in slots
 ])
 def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     """The forms a weight is packed in for an expected token count (`size`), run with other token counts too: edges of the

@@ -73,8 +73,9 @@ struct TcParams {
     const int* qk_head_ptr;
     const int* v_head_ptr;
     const int* v_col_id;
-    int z_pitch, mask_ld, batch, uniform_len;
+    int z_pitch, mask_ld, batch, uniform_len, nhead;
     float scale_log2;
+    bool take_over;   // CTAs ask for items that have not started
     int* err;
 };
 
@@ -153,18 +154,16 @@ __device__ __forceinline__ void clc_try_cancel(uint4* answer, uint64_t* bar) {
                  "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ bool clc_query(const uint4* answer, int& x, int& y) {
-    uint32_t ok, cx, cy;
+__device__ __forceinline__ bool clc_query(const uint4* answer, int& x) {
+    uint32_t ok, cx;
     asm volatile(
-        "{\n.reg .b128 h;\n.reg .pred p;\nld.shared.b128 h, [%3];\n"
-        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\nselp.u32 %0, 1, 0, p;\nmov.u32 %1, 0;\nmov.u32 %2, 0;\n"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, h;\n}"
-        : "=r"(ok), "=r"(cx), "=r"(cy)
+        "{\n.reg .b128 h;\n.reg .pred p;\nld.shared.b128 h, [%2];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\nselp.u32 %0, 1, 0, p;\nmov.u32 %1, 0;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n}"
+        : "=r"(ok), "=r"(cx)
         : "r"(smem_u32(answer))
         : "memory");
     x = (int)cx;
-    y = (int)cy;
     return ok != 0;
 }
 
@@ -263,16 +262,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
     if (warp == kSoftmaxWarps) {
         // ---- items and loads (all lanes stay together; lane 0 issues)
         pdl_wait();   // lengths and activations come from the preceding kernels
-        int bx = blockIdx.x, by = blockIdx.y;
+        int id = blockIdx.x;   // heads fastest: what a ragged batch has too many lies at the end of the grid
         int ni = 0, nq = 0, nk = 0, nv = 0;   // items handed out, tiles requested
         uint32_t clc_phase = 0;
         bool ok = true;
         for (;;) {
-            if (lane == 0) {
+            if (lane == 0 && p.take_over) {
                 mbar_expect_tx(&sh->clc_full, 16);
                 clc_try_cancel(&sh->clc, &sh->clc_full);
             }
-            Item it = find_item(p, bx, by, lane);
+            const int by = id % p.nhead;
+            Item it = find_item(p, id / p.nhead, by, lane);
             if constexpr (kForm == kCompact) {
                 if (p.qk_head_ptr) {
                     it.qk_x = p.qk_head_ptr[by];
@@ -336,12 +336,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     }
                 }
             }
+            if (!p.take_over) break;
             // the answer is awaited even on the way out: nothing may be in flight towards shared memory when the CTA leaves
             const bool answered = mbar_wait(&sh->clc_full, clc_phase);
             clc_phase ^= 1u;
             ok = ok && answered;
             if (!ok) break;
-            const bool more = clc_query(&sh->clc, bx, by);
+            const bool more = clc_query(&sh->clc, id);
             fence_proxy_async_smem();   // the answer has been read before the next one may be written
             __syncwarp();
             if (!more) break;
@@ -851,7 +852,12 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "attention: shared memory opt-in");
     const int nblk = cu_seqlens ? (total_tokens + kBQ - 1) / kBQ + batch : batch * ((uniform_len + kBQ - 1) / kBQ);
-    const dim3 grid(nblk, nhead);
+    const dim3 grid(nblk * nhead);
+    p.nhead = nhead;
+    // CTAs that all fit are left to the hardware: one that starts early would take an item for which a place is still free. (Of a
+    // ragged batch only the tokens are known here: at least this many blocks. 4 x 512 tokens, 16 heads: 18.2 -> 11.3 us.)
+    const long items = cu_seqlens ? (total_tokens + kBQ - 1) / kBQ : nblk;
+    p.take_over = items * nhead > (long)kCtasPerSm * sm_count();
     const auto run = compact      ? (mask ? launch<true, kCompact> : launch<false, kCompact>)
                      : v_head_ptr ? (mask ? launch<true, kScatterV> : launch<false, kScatterV>)
                                   : (mask ? launch<true, kDense> : launch<false, kDense>);

@@ -834,7 +834,9 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     // (1.08: where the first two come this close, the resident kernel was the faster one in seven of ten measured launches.)
     tile_cost = 1.3 * tile_cost + 1000.0;
     const double resident = resident_cost(size_hint, N, K, density);
-    const bool plain = nb_override <= 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
+    // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
+    // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
+    const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
     w->packed_dense = plain && w->dense.cost < std::min(tile_cost, resident);
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < 1.08 * tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)

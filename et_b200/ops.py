@@ -102,8 +102,7 @@ def set_tuning_goal(goal):
 
 
 def set_attention_scores_fp32(on):
-    """False (default): the tcgen05 attention kernel accumulates Q K^T in fp16, as the reference's kernels do; True: in
-    fp32 (for models whose attention logits are large; ~1.5 times the time). Process-wide, read at launch."""
+    """Whether attention must accumulate Q K^T in fp32. The tcgen05 kernel always does: kept for callers that set it."""
     check(lib().et_set_attention_scores_fp32(_i(1 if on else 0)))
 
 

@@ -66,11 +66,9 @@ int et_tile_weight_check(const et_tile_weight* w, int* code);
 #define ET_GOAL_LATENCY 0
 #define ET_GOAL_THROUGHPUT 1
 int et_set_tuning_goal(int goal);
-/* Extension: how the tcgen05 attention kernel accumulates Q K^T. 0 (default): in fp16, as the reference's kernels
- * accumulate their scores (kernels/attention.cu:82, `c_t<half>`); the error against exact arithmetic grows with the
- * size of the scores (worst output element: 2e-3 for |q.k| up to 50, 1.4e-2 up to 165, 3e-2 up to 390). 1: in fp32
- * (2e-3 throughout, ~1.5 times the time). Process-wide, read when a launch is issued: graphs recorded earlier by
- * et_encoder_run_batch / et_model_run_batch keep the kernel they were recorded with. */
+/* Extension: whether the caller needs Q K^T accumulated in fp32 (the reference's kernels accumulate their scores in fp16,
+ * kernels/attention.cu:82, `c_t<half>`). The tcgen05 attention kernel always does, so both settings give the same result (worst
+ * output element 2e-3 for |q.k| up to 390); the setting is kept and read back for callers that make it. Process-wide. */
 int et_set_attention_scores_fp32(int on);
 int et_attention_scores_fp32(void);
 /* info[6] = {block_rows_per_cta, n_chunks, k_chunks, stages, stage_bytes, packed_bytes}. The form the weight was packed in
@@ -154,8 +152,8 @@ int et_attention_check(int* code);
  * for `batch` sequences of uniform_len tokens. valid_lens (device, may be NULL) excludes keys at or beyond
  * valid_lens[b] (key padding). Q and K share qk_pitch; qk_head_ptr / v_head_ptr + v_col_id (device, may be
  * NULL) select compact per-head column windows as in et_attention_prune. max_seq_len: the longest sequence
- * when cu_seqlens is given (0 = unknown); it only selects between the tensor-core kernel for dense heads of
- * 64 with at most 512 keys and the general kernel. */
+ * when cu_seqlens is given (0 = unknown); it only selects between the tcgen05 kernel for heads of 64 and the general
+ * kernel. */
 int et_attention_batch(void* out, const void* Q, const void* K, const void* V, int qk_pitch, int v_pitch,
                        const int* qk_head_ptr, const int* v_col_id, const int* v_head_ptr, const void* mask,
                        int mask_ld, const int* cu_seqlens, const int* valid_lens, int batch, int uniform_len,

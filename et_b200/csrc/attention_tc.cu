@@ -494,6 +494,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
         bool ok = true;
         int done_slot = -1;     // item whose P V is on its way and whose rows are still to be written
         float done_sum = 0.f;   // its row sum
+        // Output columns of the window's features `lane` and `lane` + 32, of this item and of the one still to be written: read
+        // when the item is taken up (one by one in the epilogue they cost more than everything else of a short item).
+        int cols[2] = {0, 0}, done_cols[2] = {0, 0};
         auto release = [&](int slot) {
             __syncwarp();
             if (elect_one()) mbar_arrive(&sh->item_empty[slot]);
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     for (int i = 0; i < 16; ++i) {
                         const int k = c * 16 + i - it.v_off;
                         if (k >= 0 && k < it.v_n) {   // the same for the whole warp
-                            const int col = __ldg(p.v_col_id + it.v_base + k) - it.head * kHD;
+                            const int col = __shfl_sync(0xffffffffu, k < 32 ? done_cols[0] : done_cols[1], k & 31) - it.head * kHD;
                             const half z = __float2half_rn(__uint_as_float(r[i]) * inv);
                             if (!it.v_add) st[col] = z;
                             else if (in) zrow[col] = z;
@@ -589,6 +592,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 continue;
             }
             const int valid = it.valid;
+            if constexpr (kPruneV) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) cols[i] = lane + 32 * i < it.v_n ? __ldg(p.v_col_id + it.v_base + lane + 32 * i) : 0;
+            }
             // the mask rows of the warp's queries for a block of keys: seventeen granules per row, asynchronously
             auto fetch_mask = [&](int j) {
                 const uint8_t* mend = reinterpret_cast<const uint8_t*>(p.mask + (size_t)(it.len - 1) * p.mask_ld + it.len);
@@ -745,6 +752,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             if (!ok) break;
             done_slot = slot;
             done_sum = l2.x + l2.y;
+            if constexpr (kPruneV) {
+                done_cols[0] = cols[0];
+                done_cols[1] = cols[1];
+            }
         }
         if constexpr (kMask) asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok && lane == 0) {

@@ -108,7 +108,7 @@ static int row_weight_padded(TileWeight** out, const RowWeight* w, int size, std
     }
     std::vector<int> rp, ro;
     dense_to_tiles(weight.data(), N, K, data, rp, ro);
-    return tile_weight_pack(out, K, N, size, (long)ro.size(), data.data(), rp.data(), ro.data(), bias.data(), 0);
+    return tile_weight_pack(out, K, N, size, (long)ro.size(), data.data(), rp.data(), ro.data(), bias.data(), 0, true);
 }
 
 namespace {

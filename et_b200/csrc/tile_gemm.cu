@@ -800,7 +800,7 @@ static bool repeats_a_tile(const int* row_ptr, const int* row_offset, int block_
 }
 
 int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, const half* data,
-                     const int* row_ptr, const int* row_offset, const half* bias, int nb_override) {
+                     const int* row_ptr, const int* row_offset, const half* bias, int nb_override, bool part) {
     if (!out) return fail(ET_ERR_INVALID, "tile weight: null output");
     *out = nullptr;
     if (K <= 0 || N <= 0 || K % 16 || N % 16) return fail(ET_ERR_INVALID, "tile weight: in/out features must be positive multiples of 16");
@@ -827,6 +827,10 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     w->h_data.assign(data, data + (size_t)ntile * 256);
     w->h_bias.assign((size_t)N, __float2half(0.f));
     if (bias) std::copy(bias, bias + N, w->h_bias.begin());
+    if (part) {
+        *out = w;
+        return ET_OK;
+    }
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's, which
     // was made to compare its own shapes only, is 1.3 times too short). At 75 % sparsity and 32768 tokens, in us, tile / resident /
@@ -929,6 +933,7 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
     if (T < 0) return fail(ET_ERR_INVALID, "tile linear: negative token count");
     if (T == 0) return ET_OK;
     if (!aligned16(X) || !aligned16(Y)) return fail(ET_ERR_INVALID, "tile linear: X and Y must be 16-byte aligned");
+    if (!w->d_small) return fail(ET_ERR_INVALID, "tile linear: this weight is a part for concatenation only");
     if (w->packed_dense && !fusion)
         return dense_run(w->dense_map, w->dense, Y, X, bias_dev ? bias_dev : w->d_bias, T, w->N, w->K, gelu, w->d_err, st);
     if (w->resident && !fusion) return resident_run(w->resident, Y, X, bias_dev ? bias_dev : w->d_bias, T, gelu, w->d_err, st);

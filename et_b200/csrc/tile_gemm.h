@@ -28,9 +28,10 @@ struct GemmFusion {
 };
 
 // Validates the BSR arrays (host pointers), re-packs them for the kernel and uploads.
-// nb_override > 0 forces the block-rows-per-CTA choice (tests); 0 picks it from size_hint.
+// nb_override > 0 forces the block-rows-per-CTA choice (tests); 0 picks it from size_hint. part: only the host arrays, for
+// tile_weight_concat (nothing is uploaded, the weight cannot be run).
 int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, const half* data,
-                     const int* row_ptr, const int* row_offset, const half* bias, int nb_override);
+                     const int* row_ptr, const int* row_offset, const half* bias, int nb_override, bool part = false);
 // New weight = the parts' output features back to back (equal in_feat); the parts stay valid.
 int tile_weight_concat(TileWeight** out, const TileWeight* const* parts, int count, int size_hint);
 int tile_weight_out_feat(const TileWeight* w);

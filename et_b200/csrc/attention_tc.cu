@@ -434,11 +434,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 if (!ok) break;
                 issue_qk(g + 1, (nq - 1) % C::kQS, is_half(j + 1), j + 2 == nkb);
                 issued = true;
-            } else if (mbar_try_wait(&sh->item_full[ni % kItemRing], (uint32_t)(ni / kItemRing) & 1u) &&
+            } else if (mbar_poll_warp(&sh->item_full[ni % kItemRing], (uint32_t)(ni / kItemRing) & 1u) &&
                        sh->item[ni % kItemRing].nkb > 0) {
                 // the next item's first block, if its operands are there already: P V of this block does not wait for them
                 const int qs = nq % C::kQS;
-                if (C::kQS > 1 && mbar_try_wait(&sh->q_full[qs], (uint32_t)(nq / C::kQS) & 1u) && mbar_try_wait(&sh->k_full[kb1], kp1)) {
+                if (C::kQS > 1 && mbar_poll_warp(&sh->q_full[qs], (uint32_t)(nq / C::kQS) & 1u) && mbar_poll_warp(&sh->k_full[kb1], kp1)) {
                     ok = mbar_wait(&sh->s_free, g & 1) && next_item();
                     if (!ok) break;
                     issue_qk(g + 1, qs, is_half(0), nkb == 1);

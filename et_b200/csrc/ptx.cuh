@@ -62,6 +62,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
+// Whether a phase has completed, asked without waiting by a whole warp that branches on the answer: the barrier may complete
+// between the lanes' queries, so they vote (lanes that went different ways would meet in different warp-wide operations).
+__device__ __forceinline__ bool mbar_poll_warp(uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_try_wait(bar, parity));
+}
 // ------------------------------------------------------------------ TMA
 __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, int y,
                                             uint64_t* bar) {

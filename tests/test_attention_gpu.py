@@ -228,6 +228,23 @@ def test_attention_ragged_batch_with_empty_and_padded_sequences(et, orc, mask):
     util.assert_close(host(out), want, what="ragged batch")
 
 
+@pytest.mark.parametrize("L", [40, 128, 200])
+def test_attention_many_items_per_cta_repeat_exactly(et, orc, L):
+    """Items of one or two key blocks taken over one after the other, so that the next item's first block is often, but not
+    always, there when the current one's last is multiplied: the same bits on every launch."""
+    d, H, B = 256, 4, 400
+    Q, K, V = _qkv(71, B * L, d)
+    dq, dk, dv = dev(Q), dev(K), dev(V)
+    outs = [torch.full((B * L, d), float("nan"), dtype=torch.float16, device="cuda") for _ in range(8)]
+    for out in outs:
+        et.attention_batch(out, dq, dk, dv, d, H, batch=B, uniform_len=L)
+    torch.cuda.synchronize()
+    et.attention_check()
+    assert all(torch.equal(outs[0], out) for out in outs[1:])
+    n = 3 * L
+    util.assert_close(host(outs[0])[-n:], orc.attention(Q[-n:], K[-n:], V[-n:], [L] * 3, d, H), what=f"last sequences of {B} x {L}")
+
+
 def test_attention_qk_and_v_pruned(et, orc):
     L, d, H = 100, 768, 12
     row_id = orc.gen_sparse_row_mat(d, 0.5, seed=6, nhead=H)

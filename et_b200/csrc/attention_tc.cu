@@ -126,9 +126,10 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // 2^x for two values on the FMA and ALU pipes, x <= 127: x = n + f with n the nearest whole number (adding 1.5 * 2^23 leaves
 // n in the low bits of the sum) and |f| <= 1/2; 2^f by the cubic that interpolates it at the Chebyshev nodes of [-1/2, 1/2]
 // (largest relative error 1.0e-4, below half a unit of the fp16 that the result is rounded to); n goes into the exponent.
+// Not a number stays so: the maximum keeps it, and as the arithmetic on the exponent would make a number of it, x * 0 is added.
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
-    x.x = fmaxf(x.x, -126.f);
-    x.y = fmaxf(x.y, -126.f);
+    x.x = max_nan(x.x, -126.f);
+    x.y = max_nan(x.y, -126.f);
     const float2 big = make_float2(12582912.f, 12582912.f), nbig = make_float2(-12582912.f, -12582912.f);
     const float2 t = add2(x, big);
     const float2 n = add2(t, nbig);
@@ -139,7 +140,7 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
     float2 y;
     y.x = __int_as_float(__float_as_int(r.x) + (__float_as_int(t.x) << 23));
     y.y = __int_as_float(__float_as_int(r.y) + (__float_as_int(t.y) << 23));
-    return y;
+    return fma2(x, make_float2(0.f, 0.f), y);
 }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {   // bytes < 16: the rest is zero-filled

@@ -228,6 +228,30 @@ def test_attention_ragged_batch_with_empty_and_padded_sequences(et, orc, mask):
     util.assert_close(host(out), want, what="ragged batch")
 
 
+@pytest.mark.parametrize("mask,prune", [(False, False), (True, False), (False, True)])
+def test_attention_keys_that_are_not_numbers_reach_every_query(et, orc, mask, prune):
+    """A key that is not a number makes every score with it, and so every row of the result, not a number, wherever in a block
+    the key lies (exponentials are taken in different ways by position); other heads stay clean."""
+    L, d, H = 136, 128, 2
+    Q, K, V = (dev(x) for x in _qkv(91, L, d))
+    M = dev(util.rng(92).standard_normal((L, L)).astype(np.float16)) if mask else None
+    ids = np.arange(0, d, 2, dtype=np.int32)
+    lost = []
+    for key in range(L):
+        Kn = K.clone()
+        Kn[key, 5] = float("nan")
+        out = torch.zeros((L, d), dtype=torch.float16, device="cuda")
+        if prune:
+            et.attention_prune(out, Q, Kn, V[:, :len(ids)].contiguous(), dev(ids), dev(orc.head_ptr(ids, H, d)), len(ids), M, L, d, H)
+        else:
+            et.attention_otf(out, Q, Kn, V, M, L, d, H)
+        cols = ids[ids < 64] if prune else np.arange(64)
+        if not torch.isnan(out[:, cols.tolist()]).all() or not torch.isfinite(out[:, 64:]).all():
+            lost.append(key)
+    et.attention_check()
+    assert not lost, lost
+
+
 @pytest.mark.parametrize("L", [40, 128, 200])
 def test_attention_many_items_per_cta_repeat_exactly(et, orc, L):
     """Items of one or two key blocks taken over one after the other, so that the next item's first block is often, but not

@@ -93,6 +93,11 @@ enum Form { kDense = 0, kScatterV = 1, kCompact = 2 };
 template <bool kMask, int kForm>
 struct Cfg {
     static constexpr bool kPruneV = kForm == kScatterV;
+    // The operator with compact V replaced a kernel that takes every exponential on the special-function unit, relative to the
+    // row's true maximum (the largest P is then exactly 1); it keeps that, as its results would be further from exact ones
+    // otherwise (up to 1.12 times with a mask and 1000 tokens). The other forms replaced packed fp16 exponentials, three times as far off.
+    static constexpr int kPolyPairs = kPruneV ? 0 : et::kPolyPairs;
+    static constexpr float kRescaleStep = kPruneV ? 0.f : et::kRescaleStep;
     static constexpr int kQS = (kMask || kPruneV) ? 1 : 2;
     static constexpr int kKS = 2;
     static constexpr int kVS = (kMask || kPruneV) ? 1 : 2;
@@ -688,8 +693,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     }
                 const float bmax = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * sc;   // the scale is positive: scale the maximum once
                 // The reference point moves only when the row maximum has grown by more than 2^8 (P could leave the fp16
-                // range); the final division by the row sum makes the result independent of it.
-                const bool grow = bmax > m_run + kRescaleStep;   // also true for the first finite score of a row
+                // range; with each growth where kRescaleStep is 0); the final division by the row sum makes the result independent of it.
+                const bool grow = bmax > m_run + C::kRescaleStep;   // also true for the first finite score of a row
                 const bool any = __any_sync(0xffffffffu, grow);
                 float alpha = 1.f;
                 if (grow) {
@@ -708,7 +713,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                         for (int i = 0; i < 16; ++i) {
                             float2 e = fma2(make_float2(v[c][2 * i], v[c][2 * i + 1]), sc2, sh2);
                             // spread over the chunk so that both pipes stay busy
-                            if ((i * kPolyPairs) / 16 != ((i + 1) * kPolyPairs) / 16) {
+                            if ((i * C::kPolyPairs) / 16 != ((i + 1) * C::kPolyPairs) / 16) {
                                 e = ex2_poly2(e);
                             } else {
                                 e.x = ex2_fast(e.x);

@@ -269,6 +269,31 @@ def test_attention_many_items_per_cta_repeat_exactly(et, orc, L):
     util.assert_close(host(outs[0])[-n:], orc.attention(Q[-n:], K[-n:], V[-n:], [L] * 3, d, H), what=f"last sequences of {B} x {L}")
 
 
+@pytest.mark.parametrize("mask,bound", [(False, 2.84e-4), (True, 2.7e-4)])
+def test_attention_prune_precision(et, orc, mask, bound):
+    """Against 64 bits over many key blocks. What the data types give is the rounding of the probabilities, of which the largest
+    is exactly 1, and of the result, ~2e-4 each: 2.78e-4 and 2.60e-4 (with the mask the largest probabilities weigh more).
+    Probabilities taken relative to an earlier block's maximum gave 2.90e-4 and 2.89e-4."""
+    L, d, H = 1000, 768, 12
+    ids = orc.gen_sparse_row_mat(d, 0.5, seed=6, nhead=H)
+    hp = orc.head_ptr(ids, H, d)
+    ids, hp = ids[:len(ids) // 8 * 8], np.minimum(hp, len(ids) // 8 * 8)
+    Q, K, V = (util.activations(s, (L, n)) for s, n in ((1, d), (2, d), (3, len(ids))))
+    M = util.activations(4, (L, L)) if mask else None
+    out = torch.zeros((L, d), dtype=torch.float16, device="cuda")
+    et.attention_prune(out, dev(Q), dev(K), dev(V), dev(ids), dev(hp.astype(np.int32)), len(ids), None if M is None else dev(M), L, d, H)
+    et.attention_check()
+    q, k, v = (torch.from_numpy(x).double().cuda() for x in (Q, K, V))
+    want = torch.zeros((L, d), dtype=torch.float64, device="cuda")
+    for h in range(H):
+        s = q[:, 64 * h:64 * h + 64] @ k[:, 64 * h:64 * h + 64].T / 8
+        if mask:
+            s = s + torch.from_numpy(M).double().cuda()
+        want[:, ids[hp[h]:hp[h + 1]].tolist()] = torch.softmax(s, -1) @ v[:, hp[h]:hp[h + 1]]
+    rel = float((out.double() - want).norm() / want.norm())
+    assert rel <= bound, rel
+
+
 def test_attention_qk_and_v_pruned(et, orc):
     L, d, H = 100, 768, 12
     row_id = orc.gen_sparse_row_mat(d, 0.5, seed=6, nhead=H)

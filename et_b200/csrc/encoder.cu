@@ -210,16 +210,21 @@ struct ReplayCache {
 
 // Sequence offsets and key counts on the device (offsets of batch + 1, then counts of batch). The array grows geometrically; a
 // recorded graph holds its address as a kernel argument, so every graph recorded with the old array is dropped before it is
-// freed. A call with the lengths that the array holds already, on the stream that uploaded them, uploads nothing.
+// freed. A call with the lengths that the array holds already, on the stream that uploaded them, uploads nothing. A call inside
+// the caller's own capture gets an array that is filled then and there and never written again: the caller's graph may be
+// launched at any time, between direct calls with other lengths and beside them.
 struct LengthArray {
     int* d = nullptr;
     int cap = 0;
     std::vector<int> held;
     unsigned long long held_stream = 0;
-    ~LengthArray() { cudaFree(d); }
-    int upload(const std::vector<int>& meta, cudaStream_t st, bool captured, ReplayCache& graphs, const char* what) {
+    std::map<std::vector<int>, int*> captured;   // by content; as long-lived as the object, as the graphs hold them
+    ~LengthArray() {
+        cudaFree(d);
+        for (auto& kv : captured) cudaFree(kv.second);
+    }
+    int upload(const std::vector<int>& meta, cudaStream_t st, ReplayCache& graphs, const char* what) {
         const int need = (int)meta.size();
-        if (captured) held.clear();   // the caller's graph uploads on every launch
         if (cap < need) {
             graphs.drop();
             held.clear();
@@ -235,8 +240,30 @@ struct LengthArray {
         if (known && id == held_stream && held == meta) return ET_OK;
         const int rc = cuda_status(cudaMemcpyAsync(d, meta.data(), sizeof(int) * (size_t)need, cudaMemcpyHostToDevice, st), what);
         held.clear();
-        if (rc == ET_OK && known && !captured) { held = meta; held_stream = id; }
+        if (rc == ET_OK && known) { held = meta; held_stream = id; }
         return rc;
+    }
+    // For a call inside the caller's capture: allocates and fills on a stream beside it (the capture mode of this thread is
+    // relaxed meanwhile; nothing of this becomes part of the caller's graph).
+    int in_capture(const std::vector<int>& meta, const int** out, const char* what) {
+        auto it = captured.find(meta);
+        if (it != captured.end()) { *out = it->second; return ET_OK; }
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return cuda_status(e, what);
+        int* fresh = nullptr;
+        cudaStream_t side = nullptr;
+        e = cudaMalloc(&fresh, sizeof(int) * meta.size());
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(fresh, meta.data(), sizeof(int) * meta.size(), cudaMemcpyHostToDevice, side);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(side);
+        if (side) cudaStreamDestroy(side);
+        if (e != cudaSuccess) cudaFree(fresh);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return cuda_status(e, what);
+        captured[meta] = fresh;
+        *out = fresh;
+        return ET_OK;
     }
 };
 
@@ -845,10 +872,13 @@ int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* 
     const int* vl = nullptr;
     const bool capturing = in_capture(st);
     if (!uniform || valid_lens_host) {
-        const int rc = e->lens.upload(meta, st, capturing, e->graphs, "et_encoder_run_batch: lengths upload");
+        const int* lens = nullptr;
+        const int rc = capturing ? e->lens.in_capture(meta, &lens, "et_encoder_run_batch: lengths upload")
+                                 : e->lens.upload(meta, st, e->graphs, "et_encoder_run_batch: lengths upload");
         if (rc) return rc;
-        if (!uniform) cu = e->lens.d;
-        if (valid_lens_host) vl = e->lens.d + batch + 1;
+        if (!capturing) lens = e->lens.d;
+        if (!uniform) cu = lens;
+        if (valid_lens_host) vl = lens + batch + 1;
     }
     auto forward = [&](cudaStream_t s) {
         return et::encoder_forward(e, static_cast<half*>(out), static_cast<const half*>(in), static_cast<half*>(scratch), T, cu, vl,
@@ -1047,7 +1077,7 @@ int et_model_run_batch(et_model* model, void* out, const void* in, const int* se
     const int* cu = nullptr;
     const int* vl = nullptr;
     if (!uniform || valid_lens_host) {
-        const int rc = m->lens.upload(meta, st, capturing, m->graphs, "et_model_run_batch: lengths upload");
+        const int rc = m->lens.upload(meta, st, m->graphs, "et_model_run_batch: lengths upload");
         if (rc) return rc;
         if (!uniform) cu = m->lens.d;
         if (valid_lens_host) vl = m->lens.d + batch + 1;

@@ -390,3 +390,45 @@ def test_prune_layers_with_heads_of_any_width(et, orc, qk_keep, v_keep, mask):
     torch.cuda.synchronize()
     util.assert_close(host(out), want, what="row-pruned layer", max_abs=4e-2, mean_abs=4e-3)
     enc.check()
+
+
+@pytest.mark.parametrize("padded", [False, True])
+def test_captured_ragged_call_and_direct_calls_keep_their_own_lengths(et, orc, padded):
+    """A ragged batch inside the caller's own graph: its lengths belong to the graph. Direct calls in between, with other lengths
+    of the same and of a larger batch (the layer's array grows), change nothing for the graph, nor the graph for them."""
+    d, H, dff = 256, 4, 512
+    lin, ln = make_layer(orc, d, dff, 0.5, seed=71)
+    a, b, c = [70, 3, 64], [5, 100, 32], [9] * 30 + [40] * 3 + [1] * 30
+    T = max(map(sum, (a, b, c)))
+    enc = build_encoder(et, et.KIND_TILE, lin, ln, d, 128, H, T)
+    scratch = torch.zeros(et.encoder_batch_buffer_size(et.KIND_TILE, d, T, len(c), 128, H) // 2, dtype=torch.float16, device="cuda")
+    x = dev(util.activations(72, (T, d)))
+
+    def valid(lens):
+        return [max(1, n - 2) for n in lens] if padded else None
+
+    def call(lens, out, layer=enc):
+        layer.run_batch(out, x[:sum(lens)], lens, scratch, valid_lens=valid(lens))
+        return out
+
+    def empty(lens):
+        return torch.zeros((sum(lens), d), dtype=torch.float16, device="cuda")
+
+    other = build_encoder(et, et.KIND_TILE, lin, ln, d, 128, H, T)   # never captured
+    other.set_graph_replay(False)
+    want = {i: call(n, empty(n), other).clone() for i, n in enumerate((a, b, c))}
+    outs = [empty(n) for n in (a, b, c)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(a, outs[0])
+    for step in range(3):                                # the direct call's own graph is captured and replayed meanwhile
+        assert torch.equal(call(b, outs[1].zero_()), want[1]), step
+        outs[0].zero_()
+        graph.replay()
+        assert torch.equal(outs[0], want[0]), step
+        assert torch.equal(call(b, outs[1].zero_()), want[1]), step
+        assert torch.equal(call(c, outs[2].zero_()), want[2]), step
+        outs[0].zero_()
+        graph.replay()
+        assert torch.equal(outs[0], want[0]), step
+    enc.check()

@@ -283,7 +283,6 @@ struct Encoder {
     std::vector<half> h_ln[4];                             // the same on the host (folded into weights by the layer stack)
     half* d_mask = nullptr;                                // [seq_len x seq_len] additive, may be null
     LengthArray lens;
-    std::vector<int> meta;                                 // lengths of the call being made
     bool materialize_scores = false;
     ReplayCache graphs;
     ~Encoder() {
@@ -849,8 +848,9 @@ int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (batch == 0) return ET_OK;
     ET_REQUIRE(seq_lens_host, "et_encoder_run_batch: null seq_lens");
-    std::vector<int>& meta = e->meta;
-    meta.resize(2 * (size_t)batch + 1);
+    // The call's own: with equal lengths and without graph replay a layer may be run by several threads at once, each with its
+    // own stream and buffers.
+    std::vector<int> meta(2 * (size_t)batch + 1);
     meta[0] = 0;
     bool uniform = true;
     int max_len = 0;

@@ -432,3 +432,39 @@ def test_captured_ragged_call_and_direct_calls_keep_their_own_lengths(et, orc, p
         graph.replay()
         assert torch.equal(outs[0], want[0]), step
     enc.check()
+
+
+def test_threads_share_a_layer_that_keeps_nothing_of_a_call(et, orc):
+    """Equal lengths, no graph replay: several host threads run one layer at once, each with its own stream, buffers and batch."""
+    import threading
+    d, H, dff, S = 256, 4, 512, 32
+    lin, ln = make_layer(orc, d, dff, 0.5, seed=75)
+    batches = [1, 7, 40, 3]
+    enc = build_encoder(et, et.KIND_TILE, lin, ln, d, S, H, max(batches) * S)
+    enc.set_graph_replay(False)
+    xs = [dev(util.activations(76 + i, (b * S, d))) for i, b in enumerate(batches)]
+    scratch = [torch.zeros(et.encoder_batch_buffer_size(et.KIND_TILE, d, b * S, b, S, H) // 2, dtype=torch.float16, device="cuda") for b in batches]
+    outs = [torch.zeros_like(x) for x in xs]
+    for i, b in enumerate(batches):
+        enc.run_batch(outs[i], xs[i], [S] * b, scratch[i])
+    torch.cuda.synchronize()
+    want = [o.clone() for o in outs]
+    failed = []
+
+    def work(i):
+        try:
+            stream = torch.cuda.Stream()
+            for _ in range(100):
+                enc.run_batch(outs[i], xs[i], [S] * batches[i], scratch[i], stream=stream)
+            stream.synchronize()
+        except Exception as e:   # noqa: BLE001 - reported by the main thread
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(batches))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
+    enc.check()

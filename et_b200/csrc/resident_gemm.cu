@@ -66,8 +66,7 @@ struct ResidentShared {
     uint64_t x_full[kMaxRing], x_empty[kMaxRing];   // chunk slots: landed / copied on to tensor memory
     uint64_t w_full[kSets][kMaxRing], w_empty[kSets][kMaxRing];   // weight blocks: landed / their UMMAs have completed (4 commits)
     uint64_t a_ready[kMaxChunks];                   // per chunk, once per item: in place for the UMMAs
-    uint64_t a_free;                                // every issuer has issued the item's last UMMA
-    uint64_t tail_free;                             // the item's UMMAs have completed: the shared-memory part may be overwritten
+    uint64_t a_free, tail_free;                     // the item's UMMAs have completed: its activations in tensor memory, in shared memory may be overwritten
     uint64_t acc_full[2], acc_empty[2];
     uint32_t tmem_base;
     volatile int abort;
@@ -191,8 +190,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
         }
         if (!ok) give_up(42);
     } else if (warp == 1) {
-        // ---- shared memory -> tensor memory. The columns are free when the previous item's UMMAs have been issued: tcgen05
-        // operations execute in issue order (across threads: fence, barrier, fence).
+        // ---- shared memory -> tensor memory. The columns are free when the previous item's UMMAs have completed: a copy is
+        // guaranteed to run ahead of UMMAs issued after it, but not behind those issued before it.
         bool ok = true;
         int xs = 0, n = 0;
         uint32_t ph = 0;
@@ -289,8 +288,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
             for (; ready < chunks && ok; ++ready) ok = mbar_wait(&sh->a_ready[ready], (uint32_t)n & 1u);
             if (leader) {
                 if (tchunks < chunks) umma_commit(&sh->tail_free);
-                tc_fence_before();
-                mbar_arrive(&sh->a_free);
+                umma_commit(&sh->a_free);
             }
             __syncwarp();
         }

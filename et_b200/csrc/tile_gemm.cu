@@ -17,9 +17,8 @@
 //     cp.async.bulk brings a block into shared memory. The sparsity pattern is kept exactly.
 //   * Persistent CTAs (grid = min(tiles, SMs)); one chunk counter runs on across a CTA's tiles and indexes three
 //     rings, one per resource, because the operands live for different times: shared-memory slots for activations
-//     (free once copied on to tensor memory), shared-memory slots for weight blocks (free once their UMMAs have
-//     completed), tensor-memory A slots (free once the UMMAs that read them have been issued: tcgen05 operations
-//     execute in issue order). Roles: warp 0 copies activations, warp 1 weight blocks, warps 2-3 move activations
+//     (free once copied on to tensor memory), shared-memory slots for weight blocks and tensor-memory A
+//     slots (free once the UMMAs that read them have completed). Roles: warp 0 copies activations, warp 1 weight blocks, warps 2-3 move activations
 //     to tensor memory, warps 4-11 issue UMMAs. (Every asynchronous operation costs the issuing warp 100-250
 //     clocks, so the hops per chunk are what the loop time is made of.)
 //   * Epilogue, warp by warp, by sixteen warps (the eight issuers and eight helpers that sleep on a hardware
@@ -110,8 +109,8 @@ struct Shared {
     uint64_t full_w[kMaxRing];    // [chunk % kMaxRing]  the chunk's weight block has landed (bulk copy)
     uint64_t a_ready[kMaxRing];   // [chunk % kMaxRing]  the chunk's activations are in tensor memory (mover commit): read by
                                   //               the issuers, and by the activation producer as "shared-memory slot free"
-    uint64_t a_issued[kMaxRing];  // [chunk % a_slots]  every issuer has issued (not completed) its UMMAs on the chunk
-    uint64_t done[kMaxRing];      // [chunk % kMaxRing]  every issuer's UMMAs on the chunk have completed (8 commits)
+    uint64_t done[kMaxRing];      // [chunk % kMaxRing]  every issuer's UMMAs on the chunk have completed (8 commits): read by the
+                                  //               weight producer, and by the mover of the chunk a_slots later
     uint64_t acc_done;            // 8 issuer commits after a tile's last chunk
     int w_at[kMaxRing];           // [chunk % kMaxRing]  where in the weight ring the block starts (valid with full_w)
     uint32_t tmem_base;
@@ -233,8 +232,8 @@ __device__ __forceinline__ void epi_fused(const uint32_t (&acc)[32], const uint3
 //     chunk have completed (the movers' one commit per chunk, `a_ready`, is read by the issuers and by the
 //     activation producer);
 //   * nw shared-memory slots for the weight block of a chunk, free when the chunk's UMMAs have completed (`done`);
-//   * a_slots tensor-memory slots for the A operand, free when the UMMAs of the chunk a_slots earlier have been
-//     issued (`a_issued`).
+//   * a_slots tensor-memory slots for the A operand, free when the UMMAs of the chunk a_slots earlier have
+//     completed (`done` as well).
 // What bounds the chunk period is bytes in flight per clock of lifetime; each operand gets the slots its own
 // lifetime needs. Every role does as few serial barrier operations per chunk as possible: on this part a wait on a
 // completed mbarrier, a tcgen05.cp or a TMA issue each cost a warp 100-250 clocks.
@@ -267,11 +266,10 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (lane < kMaxRing) mbar_init(&sh->full_x[lane], 1);
         else if (lane < 2 * kMaxRing) mbar_init(&sh->full_w[lane - kMaxRing], 1);
         else if (lane < 3 * kMaxRing) mbar_init(&sh->a_ready[lane - 2 * kMaxRing], 1);
-        else if (lane < 4 * kMaxRing) mbar_init(&sh->a_issued[lane - 3 * kMaxRing], kIssuers);
-        else if (lane < 5 * kMaxRing) mbar_init(&sh->done[lane - 4 * kMaxRing], kIssuers);
-        else if (lane == 5 * kMaxRing) mbar_init(&sh->acc_done, kIssuers);
-        static_assert(5 * kMaxRing < 32, "one lane per barrier");
-        if (lane <= 5 * kMaxRing) fence_mbar_init();
+        else if (lane < 4 * kMaxRing) mbar_init(&sh->done[lane - 3 * kMaxRing], kIssuers);
+        else if (lane == 4 * kMaxRing) mbar_init(&sh->acc_done, kIssuers);
+        static_assert(4 * kMaxRing < 32, "one lane per barrier");
+        if (lane <= 4 * kMaxRing) fence_mbar_init();
         if (lane == 0) {
             sh->abort = 0;
             sh->issuer_abort[0] = 0;
@@ -397,18 +395,22 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 
         if (warp < kFirstIssuer) {
             // ---------------- movers: shared memory -> tensor memory copy of the A operand. The mover warps take
-            // chunks in turn; lane 1 polls, lane 0 issues and commits. The tensor-memory slot is free as soon as the
-            // issuers have ISSUED the UMMAs of the chunk a_slots earlier: tcgen05 operations execute in issue order
-            // (the order across threads being established by the fence + barrier pair), so the copy cannot overtake
-            // the UMMAs that still read the slot, and the hop "UMMAs completed -> seen by the mover" (~500 clocks)
-            // leaves the slot's cycle. The one commit per chunk tells the issuers that A is in place and the
-            // activation producer that the shared-memory slot may be overwritten.
+            // chunks in turn; lane 1 polls, lane 0 issues and commits. The tensor-memory slot is free when the
+            // UMMAs of the chunk a_slots earlier have completed: a tcgen05.cp is guaranteed to run ahead of UMMAs issued
+            // after it, but not behind those issued before it (waiting for their issue alone saved nothing measurable:
+            // 4096 -> 1024 at 80 % sparsity, 8192 tokens 35.3 and 35.4 us). The one commit per chunk tells the issuers that
+            // A is in place and the activation producer that the shared-memory slot may be overwritten.
             const int m = warp - kFirstMover;
             int xs = m % NX, a = m % RA, fx = m, fw = m, ar = m;
-            uint32_t phx = 0, phw = 0;
+            uint32_t phx = 0, phw = 0, phd = 0;
+            int ds = (m + RA) & 1;   // of the chunk RA before this one, from the first that has one
             for (int it = m; it < n_items; it += kMovers) {
                 bool got = mbar_wait(&sh->full_x[fx], phx);
-                if (got && it >= RA) got = mbar_wait(&sh->a_issued[a], (uint32_t)(it / RA - 1) & 1u);
+                if (got && it >= RA) {
+                    got = mbar_wait(&sh->done[ds], phd);
+                    ds += kMovers;
+                    if (ds >= kMaxRing) { ds -= kMaxRing; phd ^= 1u; }
+                }
                 if (lane == 0 && it < 64) ET_STAMP(700 + it);
                 if (!got) {
                     if (lane == 0) atomicExch(p.err, 12);
@@ -503,9 +505,6 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                                 umma_f16_ts(tmem + en.z, abuf + en.y, b_desc0 | (uint64_t)((tiles16 + en.x) & 0x3fff), en.w, 1u);
                         }
                         if (elect_one()) {
-                            // issued: the tensor-memory slot may be refilled behind these UMMAs; completed: the weight slot
-                            tc_fence_before();
-                            mbar_arrive(&sh->a_issued[a]);
                             umma_commit(&sh->done[ws]);
                         }
                         if (w == 0 && lane == 0 && tl * p.k_chunks + kc < 64) ET_STAMP(600 + tl * p.k_chunks + kc);

@@ -50,8 +50,11 @@ constexpr int kMaxBN = 256;
 struct DenseParams {
     const half* bias;
     half* Y;
-    int T, N, k_panels, tiles_n, tiles, bn, stages, panels;   // panels: per stage; the last stage of a K range may hold fewer
+    int T, N, K, k_panels, tiles_n, tiles, bn, stages, panels;   // panels: per stage; the last stage of a K range may hold fewer
     int* err;
+    const half* X;
+    const half* W;
+    const uint32_t* kept;   // one bit per 16 x 16 tile, rows of whole words; null when no tile was pruned
 };
 
 __host__ __device__ constexpr int copy_warps(int stages) {
@@ -112,6 +115,60 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// A pruned tile takes no part in the product, but 0 x infinity does here. Results that are not finite are therefore computed
+// again from the kept tiles alone (one that really leaves the fp16 range comes out the same). Finding them costs one operation
+// per two results; `kept` is null, and nothing is looked for, where no tile was pruned.
+struct NotFinite {   // zeros, until a value came that is not finite
+    half2 s[4];
+    __device__ __forceinline__ NotFinite() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i] = __float2half2_rn(0.f);
+    }
+    __device__ __forceinline__ void note(const uint4& v) {
+        const half2* h = reinterpret_cast<const half2*>(&v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i] = __hfma2(h[i], __float2half2_rn(0.f), s[i]);
+    }
+    __device__ __forceinline__ bool any() const {
+        const half2 t = __hadd2(__hadd2(s[0], s[1]), __hadd2(s[2], s[3]));
+        return !(__low2float(t) + __high2float(t) == 0.f);
+    }
+};
+
+// Those of the eight results of `row` from column n0 on (all of one block-row) that are not finite, in place.
+template <bool kGelu>
+__device__ __forceinline__ void recompute_segment(const DenseParams& p, int row, int n0) {
+    half* const y = p.Y + (size_t)row * p.N + n0;
+    uint4 held = __ldcg(reinterpret_cast<const uint4*>(y));
+    half* const h = reinterpret_cast<half*>(&held);
+    NotFinite odd;
+    odd.note(held);
+    if (!odd.any()) return;
+    const uint32_t* kept = p.kept + (size_t)(n0 / 16) * ((p.K / 16 + 31) / 32);
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int t = 0; t < p.K / 16; ++t) {
+        if (!((kept[t >> 5] >> (t & 31)) & 1u)) continue;
+        const uint4* xs = reinterpret_cast<const uint4*>(p.X + (size_t)row * p.K + 16 * t);
+        const uint4 x2[2] = {__ldcg(xs), __ldcg(xs + 1)};
+        const half* x = reinterpret_cast<const half*>(x2);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const uint4* ws = reinterpret_cast<const uint4*>(p.W + (size_t)(n0 + c) * p.K + 16 * t);
+            const uint4 w2[2] = {__ldg(ws), __ldg(ws + 1)};
+            const half* w = reinterpret_cast<const half*>(w2);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) acc[c] = fmaf(__half2float(x[k]), __half2float(w[k]), acc[c]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        if ((__half_as_ushort(h[c]) & 0x7c00u) != 0x7c00u) continue;
+        const half v = __float2half_rn(acc[c] + __half2float(p.bias[n0 + c]));
+        h[c] = kGelu ? __low2half(gelu_tanh_h2(__half2half2(v))) : v;
+    }
+    *reinterpret_cast<uint4*>(y) = held;
 }
 
 template <bool kGelu>
@@ -251,6 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 if (elect_one()) mbar_arrive_cluster(in_cta(&sh->acc_empty[a], 0));
                 __syncwarp();
             };
+            NotFinite odd;
             for (int u = h; u < units; u += kEpiWarps / 4) {
                 uint32_t acc[32];
                 tmem_ld32(tmem + a * bn + lane_base + u * kUnitCols, acc);
@@ -261,6 +319,10 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 if (lane == 0) tma_store_wait_read();   // the buffer's previous store has read it
                 __syncwarp();
                 epi_write(buf, lane, ov);
+                if (p.kept) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) odd.note(ov[c]);
+                }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
@@ -269,6 +331,14 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 }
             }
             if (h >= units) accumulator_read();
+            if (p.kept && __any_sync(0xffffffffu, odd.any())) {
+                if (lane == 0) tma_store_wait();   // the results are in memory
+                __syncwarp();
+                fence_proxy_async_global();
+                for (int u = h; u < units && odd.any() && m0 + lane < p.T; u += kEpiWarps / 4)
+                    for (int c = n0 + u * kUnitCols; c < min(n0 + (u + 1) * kUnitCols, p.N); c += 8) recompute_segment<kGelu>(p, m0 + lane, c);
+                __syncwarp();
+            }
         }
         if (!ok && lane == 0) {
             atomicExch(p.err, 33);
@@ -434,6 +504,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
             oh[j] = kGelu ? gelu_tanh_h2(t) : t;
         }
         *reinterpret_cast<uint4*>(p.Y + (size_t)(m0 + r) * p.N + n0 + c) = o;
+        if (p.kept) {
+            NotFinite odd;
+            odd.note(o);
+            if (odd.any()) recompute_segment<kGelu>(p, m0 + r, n0 + c);
+        }
     }
     __syncwarp();
     cluster_sync();   // the other CTAs may still be reading this one's partial tile
@@ -490,8 +565,8 @@ int dense_map_weight(CUtensorMap* map, const half* W, int N, int K, const DenseP
     return ET_OK;
 }
 
-int dense_run(const CUtensorMap& tmW, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int N, int K, int gelu,
-              int* err, cudaStream_t st) {
+int dense_run(const CUtensorMap& tmW, const half* W, const uint32_t* kept, const DensePlan& plan, half* Y, const half* X, const half* bias,
+              int T, int N, int K, int gelu, int* err, cudaStream_t st) {
     CUtensorMap tmX, tmY;
     if (!make_tmap_2d_f16(&tmX, X, (uint64_t)T, (uint64_t)K, (uint64_t)K, kBM, kBK, 128))
         return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
@@ -505,7 +580,8 @@ int dense_run(const CUtensorMap& tmW, const DensePlan& plan, half* Y, const half
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "dense linear: shared memory opt-in");
     DenseParams p;
-    p.bias = bias; p.Y = Y; p.T = T; p.N = N; p.bn = plan.bn;
+    p.bias = bias; p.Y = Y; p.T = T; p.N = N; p.K = K; p.bn = plan.bn;
+    p.X = X; p.W = W; p.kept = kept;
     p.k_panels = (K + kBK - 1) / kBK;
     p.tiles_n = (N + plan.bn - 1) / plan.bn;
     p.panels = panels_for(plan.bn, plan.split);

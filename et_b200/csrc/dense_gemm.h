@@ -15,7 +15,8 @@ struct DensePlan {
 DensePlan dense_plan(int tokens, int N, int K);
 // W: dense [N x K] on the device; the map holds its address.
 int dense_map_weight(CUtensorMap* map, const half* W, int N, int K, const DensePlan& plan);
-int dense_run(const CUtensorMap& tmW, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int N, int K, int gelu,
-              int* err, cudaStream_t st);
+// kept: device bitmap of the kept tiles ([N / 16] rows of whole 32-bit words, a bit per 16 inputs), null when none was pruned.
+int dense_run(const CUtensorMap& tmW, const half* W, const uint32_t* kept, const DensePlan& plan, half* Y, const half* X, const half* bias,
+              int T, int N, int K, int gelu, int* err, cudaStream_t st);
 
 }  // namespace et

@@ -95,6 +95,9 @@ __device__ __forceinline__ void tma_store_commit() {
 __device__ __forceinline__ void tma_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
+// The stores of this thread are complete: their results may be read back (by other threads after a barrier and the fence below).
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 // All but the most recent store group of this thread have finished reading shared memory.
 __device__ __forceinline__ void tma_store_wait_read1() {
     asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");

@@ -57,6 +57,7 @@ struct ResidentParams {
     const uint2* dir;         // [group][part]: {offset, size} in 16-byte units
     const uint8_t* stream;
     const half* bias;
+    const uint8_t* empty;     // per group, a bit per block-row without tiles; null when there is none
     int T, N, K, groups, parts, ranges, items, slabs;
     int nx, nw, block_bytes;   // nw: weight slots per set
     int* err;
@@ -91,7 +92,8 @@ __device__ __forceinline__ void cp_128x256b(uint32_t taddr, uint64_t sdesc) {
     asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
 
-template <bool kGelu>
+// kEmpty: some block-row has no tiles.
+template <bool kGelu, bool kEmpty>
 __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY,
                                                                const __grid_constant__ ResidentParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -319,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
 #pragma unroll
                     for (int c = 0; c < 32; ++c) b[c] = c < cols ? __ldg(p.bias + col + c) : __float2half(0.f);
                 }
+                const uint32_t e2 = kEmpty ? (__ldg(p.empty + g) >> (2 * half_of)) & 3u : 0u;
                 ok = mbar_wait(&sh->acc_full[set], (gs >> 1) & 1u);
                 if (!ok) break;
                 tc_fence_after();
@@ -330,6 +333,11 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
                 __syncwarp();
                 if (elect_one()) mbar_arrive(&sh->acc_empty[set]);
                 __syncwarp();
+                if (kEmpty && e2) {   // what the zero tile of a block-row without tiles left is the bias alone, whatever the activations are
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if ((e2 >> (i >> 4)) & 1u) acc[i] = 0u;
+                }
                 uint4 ov[4];
                 epi_convert_regs<kGelu>(acc, bv, ov);
                 if (lane == 0) tma_store_wait_read();   // the buffer's previous store has read it
@@ -360,6 +368,7 @@ struct ResidentWeight {
     double group_clocks = 0;   // modelled, per group of 64 features and slab
     uint2* d_dir = nullptr;
     uint8_t* d_stream = nullptr;
+    const uint8_t* d_empty = nullptr;   // behind the stream
     size_t bytes = 0;
 };
 
@@ -451,6 +460,11 @@ int resident_pack(ResidentWeight** out, int K, int N, const half* data, const in
     }
     if (!w->nx) { delete w; return fail(ET_ERR_UNSUPPORTED, "resident linear: weight blocks exceed shared memory"); }
     w->bytes = stream.size();
+    std::vector<uint8_t> empty(w->groups, 0);
+    for (int r = 0; r < NBR; ++r)
+        if (row_ptr[r] == row_ptr[r + 1]) empty[r / kGroupRows] |= (uint8_t)(1u << (r % kGroupRows));
+    const bool any_empty = std::any_of(empty.begin(), empty.end(), [](uint8_t e) { return e != 0; });
+    if (any_empty) stream.insert(stream.end(), empty.begin(), empty.end());
     if (cudaMalloc(&w->d_dir, dir.size() * sizeof(uint2)) != cudaSuccess || cudaMalloc(&w->d_stream, stream.size()) != cudaSuccess) {
         resident_free(w);
         return fail(ET_ERR_CUDA, "resident linear: cudaMalloc failed");
@@ -458,6 +472,7 @@ int resident_pack(ResidentWeight** out, int K, int N, const half* data, const in
     cudaMemcpy(w->d_dir, dir.data(), dir.size() * sizeof(uint2), cudaMemcpyHostToDevice);
     const int rc = cuda_status(cudaMemcpy(w->d_stream, stream.data(), stream.size(), cudaMemcpyHostToDevice), "resident linear: upload");
     if (rc) { resident_free(w); return rc; }
+    if (any_empty) w->d_empty = w->d_stream + w->bytes;
     *out = w;
     return ET_OK;
 }
@@ -477,13 +492,18 @@ int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bi
         !make_tmap_2d_f16(&tmy, Y, (uint64_t)T, (uint64_t)w->N, (uint64_t)w->N, 32, 32, 64))
         return fail(ET_ERR_CUDA, "resident linear: cuTensorMapEncodeTiled failed");
     static PerDeviceOnce once;
+    using KernelFn = void (*)(CUtensorMap, CUtensorMap, ResidentParams);
+    static const KernelFn kernels[2][2] = {{resident_kernel<false, false>, resident_kernel<false, true>},
+                                           {resident_kernel<true, false>, resident_kernel<true, true>}};
     const cudaError_t attr_err = once.run([] {
-        const cudaError_t e = cudaFuncSetAttribute(resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-        return e != cudaSuccess ? e : cudaFuncSetAttribute(resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < 4 && e == cudaSuccess; ++i)
+            e = cudaFuncSetAttribute(kernels[i >> 1][i & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        return e;
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "resident linear: shared memory opt-in");
     ResidentParams p;
-    p.dir = w->d_dir; p.stream = w->d_stream; p.bias = bias;
+    p.dir = w->d_dir; p.stream = w->d_stream; p.bias = bias; p.empty = w->d_empty;
     p.T = T; p.N = w->N; p.K = w->K; p.groups = w->groups; p.parts = w->parts;
     p.slabs = (T + kSlab - 1) / kSlab;
     launch_clocks(p.slabs, w->groups, w->K, w->group_clocks, &p.ranges);
@@ -491,7 +511,7 @@ int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bi
     p.nx = w->nx; p.nw = w->nw; p.block_bytes = w->block_bytes; p.err = err;
     const int chunks = (w->K + kKC - 1) / kKC;
     const size_t smem = (size_t)(std::max(0, chunks - kTmemChunks) + w->nx) * kChunkBytes + (size_t)kSets * w->nw * w->block_bytes + kEpiWarps * kUnitBytes + sizeof(ResidentShared) + 1024;
-    return cuda_status(launch_pdl(gelu ? resident_kernel<true> : resident_kernel<false>, dim3((unsigned)std::min(p.items, sm_count())),
+    return cuda_status(launch_pdl(kernels[gelu ? 1 : 0][w->d_empty ? 1 : 0], dim3((unsigned)std::min(p.items, sm_count())),
                                   dim3(kThreads), smem, st, tm, tmy, p),
                        "resident linear launch");
 }

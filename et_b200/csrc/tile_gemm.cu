@@ -638,6 +638,7 @@ struct TileWeight {
     bool packed_dense = false;
     ResidentWeight* resident = nullptr;   // the form with the activations resident in tensor memory, where that is the fastest
     half* d_dense = nullptr;
+    const uint32_t* d_kept = nullptr;   // behind the matrix: a bit per kept tile; null when every tile is kept
     CUtensorMap dense_map;
     DensePlan dense;
 };
@@ -774,15 +775,22 @@ static int build_tile_form(TileWeight* w) {
     return cuda_status(cudaMemcpy(w->d_stream, stream.data(), stream.size(), cudaMemcpyHostToDevice), "tile weight upload");
 }
 
-// The dense form: the weight as a row-major [N x K] matrix, zeros where tiles were pruned.
+// The dense form: the weight as a row-major [N x K] matrix, zeros where tiles were pruned, and which tiles were kept.
 static int build_dense_form(TileWeight* w) {
-    std::vector<half> dense((size_t)w->N * w->K, __float2half(0.f));
+    const size_t words = (w->K / 16 + 31) / 32, matrix = (size_t)w->N * w->K;   // N and K are multiples of 16
+    const bool pruned = w->ntile < (long)(w->N / 16) * (w->K / 16);
+    std::vector<half> dense(matrix + (pruned ? w->N / 16 * words * 2 : 0), __float2half(0.f));
+    uint32_t* kept = reinterpret_cast<uint32_t*>(dense.data() + matrix);
     for (int r = 0; r < w->N / 16; ++r)
-        for (int i = w->h_row_ptr[r]; i < w->h_row_ptr[r + 1]; ++i)
+        for (int i = w->h_row_ptr[r]; i < w->h_row_ptr[r + 1]; ++i) {
             for (int n = 0; n < 16; ++n)
                 std::memcpy(&dense[(size_t)(16 * r + n) * w->K + w->h_row_offset[i]], &w->h_data[(size_t)i * 256 + n * 16], 32);
+            const int t = w->h_row_offset[i] / 16;
+            if (pruned) kept[r * words + t / 32] |= 1u << (t % 32);
+        }
     if (cudaMalloc(&w->d_dense, dense.size() * sizeof(half)) != cudaSuccess) return fail(ET_ERR_CUDA, "tile weight: cudaMalloc failed");
     cudaMemcpy(w->d_dense, dense.data(), dense.size() * sizeof(half), cudaMemcpyHostToDevice);
+    if (pruned) w->d_kept = reinterpret_cast<const uint32_t*>(w->d_dense + matrix);
     return dense_map_weight(&w->dense_map, w->d_dense, w->N, w->K, w->dense);
 }
 
@@ -934,7 +942,7 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
     if (!aligned16(X) || !aligned16(Y)) return fail(ET_ERR_INVALID, "tile linear: X and Y must be 16-byte aligned");
     if (!w->d_small) return fail(ET_ERR_INVALID, "tile linear: this weight is a part for concatenation only");
     if (w->packed_dense && !fusion)
-        return dense_run(w->dense_map, w->dense, Y, X, bias_dev ? bias_dev : w->d_bias, T, w->N, w->K, gelu, w->d_err, st);
+        return dense_run(w->dense_map, w->d_dense, w->d_kept, w->dense, Y, X, bias_dev ? bias_dev : w->d_bias, T, w->N, w->K, gelu, w->d_err, st);
     if (w->resident && !fusion) return resident_run(w->resident, Y, X, bias_dev ? bias_dev : w->d_bias, T, gelu, w->d_err, st);
     if (!w->d_stream) return fail(ET_ERR_INVALID, "tile linear: the tile form of this weight was not prepared");
     CUtensorMap tm, tmy;

@@ -181,6 +181,42 @@ def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
+@pytest.mark.parametrize("T,K,N,sparsity,gelu,size,form", [
+    (200, 3072, 768, 0.75, False, 128, "dense"),         # K split over a cluster
+    (200, 3072, 784, 0.75, True, 128, "dense"),
+    (700, 768, 2304, 0.5, False, 4096, "dense"),         # pairs of CTAs
+    (700, 768, 2320, 0.5, True, 4096, "dense"),
+    (300, 768, 2304, 0.98, False, 32768, "resident"),    # block-rows without tiles among them
+    (300, 1024, 1040, 0.9, True, 32768, "resident"),
+    (300, 3072, 768, 0.9, False, 17792, "tile"),
+])
+def test_tile_linear_activations_that_are_not_finite_pass_pruned_tiles_by(et, orc, T, K, N, sparsity, gelu, size, form):
+    """An activation that is infinite or not a number reaches the outputs whose block-row keeps a tile at its input feature, and
+    those of its token alone; every other output is what it is without that activation, in whichever form the weight is packed."""
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, T + K, True, 0.05)
+    w = et.TileWeight(K, N, size, data, rp, ro, bias, is_gelu=gelu)
+    info = w.info()
+    assert form == ("tile" if info["stage_bytes"] else "dense" if info["stages"] else "resident"), info
+    X = util.activations(5, (T, K))
+    clean, reached = X.copy(), np.zeros((T, N), dtype=bool)
+    for t, k, v in ((0, 3, np.inf), (1, K - 1, np.nan), (T // 2, 100, -np.inf), (T - 1, 7, np.nan), (T - 1, 500, np.inf)):
+        X[t, k], clean[t, k] = v, 0
+        for r in range(N // 16):
+            reached[t, 16 * r:16 * r + 16] |= (ro[rp[r]:rp[r + 1]] == k // 16 * 16).any()
+    assert reached.any() and not reached.all(axis=1).any()
+    Y = torch.zeros((T, N), dtype=torch.float16, device="cuda")
+    w.run(Y, dev(X))
+    torch.cuda.synchronize()
+    w.check()
+    got, want = host(Y), orc.tile_linear(clean, rp, ro, data, bias, N, gelu=gelu)
+    finite = np.isfinite(got)
+    if not gelu:   # (GELU turns minus infinity into not a number, and an infinite sum of either sign may come)
+        assert (finite == ~reached).all()
+    assert finite[~reached].all()
+    got[reached] = want[reached]
+    util.assert_close(got, want, what=f"{form} linear, activations that are not finite")
+
+
 def test_tile_linear_exact_count_shuffled_order_and_empty_rows(et, orc):
     # exact-count generator lists a block-row's tiles in shuffle order; at 95 % many block-rows are empty
     got, want, _ = _run_tile(et, orc, 256, 768, 768, 0.95, seed=77, bernoulli=False)

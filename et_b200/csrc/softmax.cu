@@ -300,16 +300,20 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     half* s = static_cast<half*>(scores);
     const half* m = static_cast<const half*>(mask);
-    ET_REQUIRE((long)nmat * seq_len < 0x7fffffffl, "et_softmax_mask: too many rows");   // 2^31 rows of one element are 4 GB
-    const unsigned nrow = (unsigned)nmat * (unsigned)seq_len;
+    // The kernels count rows in 32 bits: launches of whole matrices with at most 2^30 rows.
+    const int per_launch = std::max(1, (1 << 30) / seq_len);
     // Rows in whole granules on both sides take the kernel without heads and tails. CH * G * 8 elements fit (beside a head and
     // a tail in the other one). Two rows in flight where their registers leave enough warps: not with a shifted mask (44 us
     // with two, 31 with one, at 128 x 500 x 500).
     const bool vec = seq_len % 8 == 0 && aligned16(s) && (!m || aligned16(m));
     auto run = [&](auto kernel, int group, int rows) {
-        const long groups = ((long)nrow + rows - 1) / rows;
-        const long blocks = std::min((groups * group + 255) / 256, (long)sm_count() * 8);
-        launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
+        for (int at = 0, n; at < nmat; at += n) {
+            n = std::min(per_launch, nmat - at);
+            const unsigned nrow = (unsigned)n * (unsigned)seq_len;
+            const long groups = ((long)nrow + rows - 1) / rows;
+            const long blocks = std::min((groups * group + 255) / 256, (long)sm_count() * 8);
+            launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, st, s + (size_t)at * seq_len * seq_len, m, nrow, seq_len, valid_len);
+        }
     };
     auto pick = [&](auto masked) {
         constexpr bool kMask = decltype(masked)::value;
@@ -322,8 +326,7 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
         else run(softmax_mask_kernel<32, 8, 1, kMask>, 32, 1);
     };
     if (seq_len > 2048) {
-        const long blocks = std::min(((long)nrow + 7) / 8, (long)sm_count() * 8);
-        launch_pdl(softmax_mask_generic, dim3((unsigned)blocks), dim3(256), 0, st, s, m, nrow, seq_len, valid_len);
+        run(softmax_mask_generic, 32, 1);
     } else if (vec) {
         if (seq_len <= 64) run(softmax_mask_vec<8, 1, 2>, 8, 2);
         else if (seq_len <= 128) run(softmax_mask_vec<16, 1, 2>, 16, 2);

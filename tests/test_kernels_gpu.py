@@ -121,6 +121,25 @@ def test_softmax_mask_rows_of_any_alignment(et, orc, L, offset):
     assert (buf[:offset] == 7).all() and (buf[offset + nmat * L * L:] == 7).all()
 
 
+def test_softmax_mask_more_rows_than_31_bits_count(et):
+    """2^30 + 3 matrices of 2 x 2 (8.6 GB): of two scores the softmax is known."""
+    nmat, L = (1 << 30) + 3, 2
+    if torch.cuda.mem_get_info()[0] < 30 << 30:
+        pytest.skip("needs 30 GB of device memory")
+    S = torch.zeros((nmat, L, L), dtype=torch.float16, device="cuda")
+    S[:, :, 1] = 1.0
+    S[-1, 1, 0] = 2.0
+    et.softmax_mask(S)
+    torch.cuda.synchronize()
+    p = 1.0 / (1.0 + np.exp(1.0))
+    half_unit = 2.0 ** -12                     # of fp16 between 0.25 and 1
+    for at in range(0, nmat - 1, 1 << 28):
+        assert float((S[at:min(at + (1 << 28), nmat - 1), :, 0].float() - p).abs().max()) <= half_unit, at
+    assert abs(float(S[-1, 0, 0]) - p) <= half_unit and abs(float(S[-1, 1, 0]) - (1 - p)) <= half_unit
+    del S
+    torch.cuda.empty_cache()
+
+
 # ------------------------------------------------------------------ tile-pruned linear
 def _run_tile(et, orc, T, K, N, sparsity, seed, gelu=False, bernoulli=True, bias_std=0.05, size=None):
     rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, seed, bernoulli, bias_std)

@@ -658,6 +658,7 @@ static int take_tiles(Encoder* e, et_tile_weight** t, int first, int count, int 
 // Lays a row-pruned layer out for compact heads (see Encoder::o_compact): q, k, v are the parts of the fused weight, rows[i] the
 // row-pruned linear behind part i or null. Leaves the encoder as it was where the output projection cannot be gathered.
 static int compact_heads(Encoder* e, const et::TileWeight* const* dense, RowWeight* const* rows) {
+    if (et::tile_weight_in_feat(e->lin[3]) != e->d_model) return et::fail(ET_ERR_INVALID, "encoder: the output projection's in_feat must be d_model");
     et::TileWeight* own[3] = {nullptr, nullptr, nullptr};
     const et::TileWeight* parts[3];
     std::vector<int> ptr[3];

@@ -896,6 +896,8 @@ int tile_weight_gather_inputs(TileWeight** out, const TileWeight* w, const int* 
     *out = nullptr;
     const int NBR = w->N / 16;
     if (n <= 0 || n % 16) return fail(ET_ERR_INVALID, "tile weight gather: the number of features must be a positive multiple of 16");
+    for (int i = 0; i < n; ++i)
+        if (src[i] >= w->K) return fail(ET_ERR_INVALID, "tile weight gather: no such input feature");
     if (repeats_a_tile(w->h_row_ptr.data(), w->h_row_offset.data(), NBR)) return fail(ET_ERR_UNSUPPORTED, "tile weight gather: a tile is listed twice");
     std::vector<int> rp(1, 0), ro;
     std::vector<half> data, rows((size_t)16 * w->K);
@@ -1001,6 +1003,7 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
 }
 
 int tile_weight_prepare_fusion(TileWeight* w) { return build_tile_form(w); }
+int tile_weight_in_feat(const TileWeight* w) { return w->K; }
 int tile_weight_out_feat(const TileWeight* w) { return w->N; }
 int tile_weight_size(const TileWeight* w) { return w->size_hint; }
 int tile_weight_chunks(const TileWeight* w) { return w->n_chunks; }

@@ -34,6 +34,7 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
                      const int* row_ptr, const int* row_offset, const half* bias, int nb_override, bool part = false);
 // New weight = the parts' output features back to back (equal in_feat); the parts stay valid.
 int tile_weight_concat(TileWeight** out, const TileWeight* const* parts, int count, int size_hint);
+int tile_weight_in_feat(const TileWeight* w);
 int tile_weight_out_feat(const TileWeight* w);
 int tile_weight_size(const TileWeight* w);   // the token count that the weight was made for
 void tile_weight_free(TileWeight* w);
@@ -44,7 +45,7 @@ int tile_linear_run(const TileWeight* w, half* Y, const half* X, int T, int gelu
 // d_n = sum_k beta_k W_nk + bias_n that the mode-1 epilogue needs (gamma, beta: host, in_feat values).
 int tile_weight_fold(TileWeight** out, const TileWeight* w, const half* gamma, const half* beta);
 // New weight whose input feature j is input feature src[j] of `w`, or zero where src[j] < 0 (n: a multiple of 16; tiles that
-// become all zero are dropped). ET_ERR_UNSUPPORTED when a block-row lists a tile twice.
+// become all zero are dropped). ET_ERR_UNSUPPORTED when a block-row lists a tile twice, ET_ERR_INVALID for a feature that `w` lacks.
 int tile_weight_gather_inputs(TileWeight** out, const TileWeight* w, const int* src, int n);
 // Builds what the fused epilogues (GemmFusion) of this weight need, if it is not there yet.
 int tile_weight_prepare_fusion(TileWeight* w);

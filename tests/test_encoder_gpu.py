@@ -468,3 +468,24 @@ def test_threads_share_a_layer_that_keeps_nothing_of_a_call(et, orc):
     assert not failed, failed
     assert all(torch.equal(o, w) for o, w in zip(outs, want))
     enc.check()
+
+
+@pytest.mark.parametrize("kind", ["prune", "prune_qkv"])
+@pytest.mark.parametrize("width", [128, 512])
+def test_prune_layers_refuse_an_output_projection_of_another_width(et, orc, kind, width):
+    """The layer gathers the projection's inputs by feature: a projection that has not as many as the model is an error."""
+    d, H = 256, 4
+    ids = np.arange(0, d, 2, dtype=np.int32)
+    ln = [np.ones(d, np.float16), np.zeros(d, np.float16)] * 2
+
+    def tile(K, N):
+        rp, ro, data, bias = util.make_tile_linear(orc, K, N, 0.5, K + N)
+        return et.TileWeight(K, N, 64, data, rp, ro, bias)
+
+    def row():
+        return et.RowWeight(d, d, 64, util.weights(1, (len(ids), d)), ids, None, H)
+
+    q, k = (row(), row()) if kind == "prune_qkv" else (tile(d, d), tile(d, d))
+    with pytest.raises(et.EtError, match="in_feat"):
+        et.Encoder(et.KIND_PRUNE_QKV if kind == "prune_qkv" else et.KIND_PRUNE, d, 64, H, None, q, k, row(), tile(width, d), tile(d, 4 * d),
+                   tile(4 * d, d), ln)

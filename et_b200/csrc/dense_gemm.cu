@@ -558,15 +558,21 @@ DensePlan dense_plan(int tokens, int N, int K) {
     return best;
 }
 
-int dense_map_weight(CUtensorMap* map, const half* W, int N, int K, const DensePlan& plan) {
-    // a CTA of a pair copies half of the tile's rows
-    if (!make_tmap_2d_f16(map, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)(plan.split > 1 ? plan.bn : plan.bn / 2), kBK, 128))
-        return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
+// Weight rows per copy: a tile's width, or half of it for each CTA of a pair.
+constexpr int kBoxRows[6] = {16, 32, 48, 64, 96, 128};
+
+int dense_map_weight(DenseWeight* w) {
+    for (int i = 0; i < 6; ++i)
+        if (!make_tmap_2d_f16(&w->maps[i], w->W, (uint64_t)w->N, (uint64_t)w->K, (uint64_t)w->K, (uint32_t)kBoxRows[i], kBK, 128))
+            return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
     return ET_OK;
 }
 
-int dense_run(const CUtensorMap& tmW, const half* W, const uint32_t* kept, const DensePlan& plan, half* Y, const half* X, const half* bias,
-              int T, int N, int K, int gelu, int* err, cudaStream_t st) {
+int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int gelu, int* err, cudaStream_t st) {
+    const int N = w.N, K = w.K;
+    const int box = (int)(std::find(kBoxRows, kBoxRows + 6, plan.split > 1 ? plan.bn : plan.bn / 2) - kBoxRows);
+    if (box == 6) return fail(ET_ERR_INVALID, "dense linear: no such tile width");
+    const CUtensorMap& tmW = w.maps[box];
     CUtensorMap tmX, tmY;
     if (!make_tmap_2d_f16(&tmX, X, (uint64_t)T, (uint64_t)K, (uint64_t)K, kBM, kBK, 128))
         return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
@@ -581,7 +587,7 @@ int dense_run(const CUtensorMap& tmW, const half* W, const uint32_t* kept, const
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "dense linear: shared memory opt-in");
     DenseParams p;
     p.bias = bias; p.Y = Y; p.T = T; p.N = N; p.K = K; p.bn = plan.bn;
-    p.X = X; p.W = W; p.kept = kept;
+    p.X = X; p.W = w.W; p.kept = w.kept;
     p.k_panels = (K + kBK - 1) / kBK;
     p.tiles_n = (N + plan.bn - 1) / plan.bn;
     p.panels = panels_for(plan.bn, plan.split);

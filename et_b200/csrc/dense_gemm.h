@@ -13,10 +13,16 @@ struct DensePlan {
     double cost = 0;
 };
 DensePlan dense_plan(int tokens, int N, int K);
-// W: dense [N x K] on the device; the map holds its address.
-int dense_map_weight(CUtensorMap* map, const half* W, int N, int K, const DensePlan& plan);
-// kept: device bitmap of the kept tiles ([N / 16] rows of whole 32-bit words, a bit per 16 inputs), null when none was pruned.
-int dense_run(const CUtensorMap& tmW, const half* W, const uint32_t* kept, const DensePlan& plan, half* Y, const half* X, const half* bias,
-              int T, int N, int K, int gelu, int* err, cudaStream_t st);
+
+// W: [N x K] on the device. kept: bitmap of the kept tiles ([N / 16] rows of whole 32-bit words, a bit per 16 inputs), null when
+// none was pruned.
+struct DenseWeight {
+    const half* W = nullptr;
+    const uint32_t* kept = nullptr;
+    int N = 0, K = 0;
+    CUtensorMap maps[6];   // one per number of weight rows that a CTA may copy at once
+};
+int dense_map_weight(DenseWeight* w);   // fills in the maps
+int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int gelu, int* err, cudaStream_t st);
 
 }  // namespace et

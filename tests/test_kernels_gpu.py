@@ -200,6 +200,24 @@ def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
+@pytest.mark.parametrize("K,N", [(3072, 768), (4096, 1040)])
+def test_dense_weights_run_alike_whatever_count_they_were_made_for(et, orc, K, N):
+    """How a dense weight is cut into tiles and shares of the K range is chosen for the tokens of the call: the same bits from
+    weights made for few and for many, at both sides of where the choice changes."""
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, 0.0, K, True, 0.05)
+    made = [et.TileWeight(K, N, size, data, rp, ro, bias) for size in (1, 64, 512, 2048, 32768)]
+    assert all(w.info()["stage_bytes"] == 0 and w.info()["stages"] for w in made)
+    for T in (1, 64, 300, 1025, 5000):
+        X = util.activations(T, (T, K))
+        ys = [w.run(torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda"), dev(X)) for w in made]
+        torch.cuda.synchronize()
+        assert all(torch.equal(ys[0], y) for y in ys[1:]), T
+        rows = slice(max(0, T - 130), T)
+        util.assert_close(host(ys[0])[rows], orc.tile_linear(X[rows], rp, ro, data, bias, N), what=f"dense linear T={T}")
+    for w in made:
+        w.check()
+
+
 @pytest.mark.parametrize("T,K,N,sparsity,gelu,size,form", [
     (200, 3072, 768, 0.75, False, 128, "dense"),         # K split over a cluster
     (200, 3072, 784, 0.75, True, 128, "dense"),

@@ -5,6 +5,7 @@
 // it with 16-byte loads into registers, reduces with shuffles only (no shared memory, no block
 // barrier), does all arithmetic in fp32 (sum, two-pass variance, eps 1e-6 as the reference) and
 // writes 16 bytes per lane. gamma/beta are re-read per row through the read-only cache.
+#include <algorithm>
 #include "common.h"
 
 namespace et {
@@ -142,14 +143,17 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
     if (num == 0) return ET_OK;
     const int warps_needed = num;
     int blocks = (warps_needed + 7) / 8;
-    // Three blocks of eight warps are resident per SM (registers), so the grid is a multiple of three per SM: two waves, or eight
-    // where a warp would have more than six rows, as shorter shares even out the SMs' shares of the bandwidth. Eight blocks per SM,
-    // 2.7 waves, before: 17771 x 768 12.2 -> 11.5 us, 32768 x 768 20.8 -> 19.2, 131072 x 1024 139 -> 132 (6.1 TB/s).
-    const int per_sm = num / 12 > sm_count() * 3 * 8 ? 24 : 6;
-    const int cap = sm_count() * per_sm;
-    if (blocks > cap) blocks = cap;
     const bool vec = size % 8 == 0 && size <= 2048 && aligned16(x) && (!s || aligned16(s)) &&
                      aligned16(g) && aligned16(b);
+    // Blocks per SM, by what is resident there. Of the kernel for 257 to 1024 elements three blocks of eight warps are (registers): a
+    // multiple of three, two waves, or eight where a warp would have more than six rows, as shorter shares even out the SMs'
+    // shares of the bandwidth. Eight blocks per SM, 2.7 waves, before: 17771 x 768 12.2 -> 11.5 us, 32768 x 768 20.8 -> 19.2,
+    // 131072 x 1024 139 -> 132 (6.1 TB/s). Narrower rows and the kernel for any size leave room for eight blocks: with six, 17771 x
+    // 770 took 47 us instead of 33, and with 24, 60000 x 128 13.9 instead of 13.2 (but 131072 x 770 334 instead of 387). Wider
+    // rows: 24 cost 60000 x 2048 151 us instead of 142 with eight.
+    const bool long_share = num / 12 > sm_count() * 3 * 8;
+    const int per_sm = !vec ? (long_share ? 24 : 8) : size <= 256 ? 8 : size <= 1024 ? (long_share ? 24 : 6) : (long_share ? 8 : 6);
+    blocks = std::min(blocks, sm_count() * per_sm);
     if (vec) {
         const int ch = (size / 8 + 31) / 32;
         switch (ch) {

@@ -69,8 +69,11 @@ def _a(t):
 def _ints(values):
     """(address, count, owner) of a sequence of whole numbers as C ints."""
     if type(values) is list or type(values) is tuple:
-        a = array.array("i", values)
-        return a.buffer_info()[0], len(a), a
+        try:
+            a = array.array("i", values)
+            return a.buffer_info()[0], len(a), a
+        except TypeError:
+            pass   # not all of them are ints: as numpy converts them
     a = np.ascontiguousarray(values, dtype=np.int32)
     return a.ctypes.data, len(a), a
 

@@ -72,6 +72,15 @@ def test_generator_argument_checks(lib):
         et.build_head_ptr(np.array([5, 3], dtype=np.int32), 2, 64)   # not ascending
 
 
+def test_lengths_may_be_any_numbers_that_numpy_makes_ints_of(lib):
+    """Ints of any kind, numpy scalars and whole floats, in lists, tuples and arrays."""
+    import ctypes
+    from et_b200.ops import _ints
+    for values in ([3, 5], (3, 5), [3.0, 5.0], [np.float32(3), 5], [np.int64(3), np.int32(5)], np.array([3, 5]), np.array([3.0, 5.0])):
+        address, count, owner = _ints(values)
+        assert count == 2 and list((ctypes.c_int * 2).from_address(address)) == [3, 5], (values, owner)
+
+
 def test_tile_weight_validation_happens_before_any_device_work(lib):
     import et_b200 as et
     data = np.zeros((2, 256), dtype=np.float16)

@@ -87,6 +87,8 @@ static int row_weight_create(RowWeight** out, int in_feat, int out_feat, int siz
         return fail(ET_ERR_CUDA, "row weight: cudaMalloc failed");
     cudaMemcpy(w->d_row_id, row_id, sizeof(int) * row_id_size, cudaMemcpyHostToDevice);
     cudaMemcpy(w->d_head_ptr, w->h_head_ptr.data(), sizeof(int) * (nhead + 1), cudaMemcpyHostToDevice);
+    rc = cuda_status(cudaDeviceSynchronize(), "row weight: upload");   // launches on any stream may follow
+    if (rc) return rc;
     w->h_row_id.assign(row_id, row_id + row_id_size);
     w->h_weight.assign(weight, weight + (size_t)row_id_size * in_feat);
     w->h_bias.assign(pbias.begin(), pbias.begin() + row_id_size);
@@ -319,8 +321,11 @@ static int encoder_common(Encoder* e, int d_model, int seq_len, int nheads, half
         if (rc) return rc;
         e->h_ln[i].assign(src[i], src[i] + d_model);
     }
-    if (mask) return upload_half(&e->d_mask, mask, (size_t)seq_len * seq_len);
-    return ET_OK;
+    if (mask) {
+        const int rc = upload_half(&e->d_mask, mask, (size_t)seq_len * seq_len);
+        if (rc) return rc;
+    }
+    return cuda_status(cudaDeviceSynchronize(), "encoder: upload");   // launches on any stream may follow
 }
 
 // One layer over `T` packed tokens (op order of encoder/encoder.cu:20-45). scratch holds 5*T*d_model halfs:
@@ -452,6 +457,8 @@ static int model_prepare_fusion(Model* m) {
         f.np1 = tile_weight_stat_slots(e->lin[3]);
         f.np2 = tile_weight_stat_slots(e->lin[5]);
     }
+    const int rc = cuda_status(cudaDeviceSynchronize(), "model: upload");   // launches on any stream may follow
+    if (rc) { m->drop_fused(); return rc; }
     m->fuse_ln = true;
     return ET_OK;
 }

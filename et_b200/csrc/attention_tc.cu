@@ -5,7 +5,7 @@
 //
 // A work item is 128 queries of one head of one sequence; a block is 128 keys of it:
 //   S = Q K^T        SS UMMAs 128x128x16 (x4), Q and K_j in shared memory (TMA, 128-byte swizzle), fp32 in 128 TMEM columns
-//   softmax          eight warps, two threads per query row: a thread takes its 64 scores into registers in one go, which
+//   softmax          four warps, one thread per query row: a thread takes its 128 scores into registers in one go, which
 //                    frees the score columns at once: Q K^T of the NEXT block (of the next item, at the end of one) runs
 //                    while this block's exponentials are taken. Reference point and sum in fp32 (log2 domain); if the
 //                    maximum has grown by more than 2^8 the reference point moves and O is rescaled in place.
@@ -114,7 +114,6 @@ struct TcShared {
     uint64_t item_full[kItemRing], item_empty[kItemRing];
     Item item[kItemRing];
     uint32_t tmem_base;
-    volatile int abort;
 };
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -250,7 +249,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 mbar_init(&sh->item_full[i], 1);
                 mbar_init(&sh->item_empty[i], kSoftmaxWarps + 1);
             }
-            sh->abort = 0;
             fence_mbar_init();
             prefetch_tmap(&tmQ);
             prefetch_tmap(&tmK);
@@ -362,10 +360,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             }
         }
         if (!ok) {
-            if (lane == 0) {
-                atomicExch(p.err, 21);
-                sh->abort = 1;
-            }
+            if (lane == 0) atomicExch(p.err, 21);
             // copies still in flight land before the CTA leaves (bounded)
             for (int i = max(nq - C::kQS, 0); i < nq; ++i) mbar_wait(&sh->q_full[i % C::kQS], (uint32_t)(i / C::kQS) & 1u);
             for (int i = max(nk - 2, 0); i < nk; ++i) mbar_wait(&sh->k_full[i & 1], (uint32_t)(i >> 1) & 1u);
@@ -482,10 +477,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             ++j;
             ++g;
         }
-        if (!ok && lane == 0) {
-            atomicExch(p.err, 21);
-            sh->abort = 1;
-        }
+        if (!ok && lane == 0) atomicExch(p.err, 21);
         __syncwarp();
     } else if (warp < kSoftmaxWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
@@ -764,10 +756,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             }
         }
         if constexpr (kMask) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (!ok && lane == 0) {
-            atomicExch(p.err, 22);
-            sh->abort = 1;
-        }
+        if (!ok && lane == 0) atomicExch(p.err, 22);
         __syncwarp();
     }
     tc_fence_before();

@@ -67,7 +67,6 @@ struct DenseShared {
     uint64_t full[kMaxStages], empty[kMaxStages];
     uint64_t acc_full[2], acc_empty[2];
     uint32_t tmem_base;
-    volatile int abort;
     __align__(16) half bias[2][kMaxBN];
 };
 
@@ -189,7 +188,6 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
     if (tid == 0) {
         for (int i = 0; i < S; ++i) { mbar_init(&sh->full[i], 1); mbar_init(&sh->empty[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&sh->acc_full[i], 1); mbar_init(&sh->acc_empty[i], 2 * kEpiWarps); }
-        sh->abort = 0;
         fence_mbar_init();
         prefetch_tmap(&tmX);
         prefetch_tmap(&tmW);
@@ -244,10 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
         }
         // (On the normal way out every copy has been consumed: the accumulators of the last tile are complete. A wait that gives
         // up has lasted far longer than any copy.)
-        if (!ok && lane == 0) {
-            atomicExch(p.err, 31);
-            sh->abort = 1;
-        }
+        if (!ok && lane == 0) atomicExch(p.err, 31);
     } else if (warp == kCopyWarps && rank == 0) {
         // ---- UMMAs of the pair
         const uint32_t idesc = make_idesc_f16(2 * kBM, bn);
@@ -280,10 +275,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
-        if (!ok && lane == 0) {
-            atomicExch(p.err, 32);
-            sh->abort = 1;
-        }
+        if (!ok && lane == 0) atomicExch(p.err, 32);
     } else if (warp >= kFirstEpi) {
         // ---- convert and store this CTA's 128 tokens: two warps per 32 rows take the tile's 32-column units in turn
         const int w = warp - kFirstEpi, q = warp & 3, h = w >> 2;
@@ -340,10 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 __syncwarp();
             }
         }
-        if (!ok && lane == 0) {
-            atomicExch(p.err, 33);
-            sh->abort = 1;
-        }
+        if (!ok && lane == 0) atomicExch(p.err, 33);
         if (lane == 0) tma_store_wait_read();
     }
     __syncwarp();
@@ -388,7 +377,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     if (tid == 0) {
         for (int i = 0; i < S; ++i) { mbar_init(&sh->full[i], 1); mbar_init(&sh->empty[i], 1); }
         mbar_init(&sh->acc_full[0], 1);
-        sh->abort = 0;
         fence_mbar_init();
     }
     if (warp == kCopyWarps) {
@@ -457,7 +445,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     const bool fin = mbar_wait(&sh->acc_full[0], 0);
     if ((!ok || !fin) && lane == 0) {
         atomicExch(p.err, 34);
-        sh->abort = 1;
         if (warp < cw)   // copies in flight land before shared memory is given another use (bounded)
             for (int i = 0; i < min(S, kn); ++i) mbar_wait(&sh->full[i], 0);
     }
@@ -520,7 +507,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
 static int panels_for(int bn, int split) { return split > 1 || bn <= 128 ? 2 : 1; }
 
 // CTAs of a cluster of `split` that run at once (one CTA per SM; clusters do not straddle the groups of 16-20 SMs, so that of
-// the larger ones fewer fit).
+// the larger ones fewer fit: 74, 33 and 15 of two, four and eight by cudaOccupancyMaxActiveClusters; the model is fitted with 14).
 static int split_capacity(int split) { return split == 8 ? 14 * 8 : split == 4 ? 33 * 4 : sm_count() / split * split; }
 
 // Cost in clocks of a launch over `tokens` with tile width bn and the K range split over `split` CTAs: waves of tiles, each

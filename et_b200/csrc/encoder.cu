@@ -24,8 +24,8 @@ namespace et {
 // ------------------------------------------------------------------------------ row-pruned linear
 // Only `row_id_size` output features survive (sorted original indices in row_id); the weight is the
 // compact [row_id_size x in_feat] matrix. Output is [tokens x nrow] with nrow = row_id_size rounded up
-// to 16 (zero columns beyond row_id_size), the pitch every consumer uses. The contraction runs on the
-// tile kernel with every tile kept.
+// to 16 (zero columns beyond row_id_size), the pitch every consumer uses. The contraction is a
+// tile weight with every tile kept, in whichever form is the shortest launch for it (tile_weight_pack).
 struct RowWeight {
     int in_feat = 0, out_feat = 0, nhead = 0, row_id_size = 0, nrow = 0;
     TileWeight* tw = nullptr;

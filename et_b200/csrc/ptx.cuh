@@ -98,10 +98,6 @@ __device__ __forceinline__ void tma_store_wait_read() {
 // The stores of this thread are complete: their results may be read back (by other threads after a barrier and the fence below).
 __device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-// All but the most recent store group of this thread have finished reading shared memory.
-__device__ __forceinline__ void tma_store_wait_read1() {
-    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-}
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
                                           uint64_t* bar) {
@@ -169,20 +165,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
-// 64 consecutive columns that hold one 16-bit value each (an fp16 accumulator), two to a register.
-__device__ __forceinline__ void tmem_ld32_pack16(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.pack::16b.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
-        "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -219,10 +201,10 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo,
     d |= (uint64_t)(swizzle & 7) << 61;
     return d;
 }
-// Instruction descriptor for kind::f16 with fp16 A/B (both K-major unless flagged) and fp32 D (fp16 D when asked for).
+// Instruction descriptor for kind::f16 with fp16 A/B (both K-major unless flagged) and fp32 D.
 __host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, bool a_mn_major = false,
-                                                      bool b_mn_major = false, bool d_f16 = false) {
-    return ((d_f16 ? 0u : 1u) << 4)        // D format: f16 / f32
+                                                      bool b_mn_major = false) {
+    return (1u << 4)                       // D format: f32
            | (0u << 7) | (0u << 10)        // A, B format: f16
            | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
            ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);

@@ -12,7 +12,7 @@
 // What bounds it: for half-empty weights the UMMAs; at 75 % sparsity and above the stores, ~30 bytes per clock and SM
 // (546 clocks per 128 x 64 tile), which is about what L2 takes from all SMs together.
 //
-// The weight is re-packed once into blocks of 64 features (x a part of the K range, so that three blocks fit): per issuing warp
+// The weight is re-packed once into blocks of 64 features (x a part of the K range, so that two blocks per accumulator fit): per issuing warp
 // a list of K slices, one byte per tile, then the tiles in UMMA layout. Roles: warp 0 copies activations, warps 2-3 weight
 // blocks (a warp that has requested a copy goes on only after ~700 clocks), warp 1 moves activations to tensor memory, warps
 // 4-11 issue and warps 12-27 convert and store. Copies of weights, issuing and converting come in two sets, one per accumulator: four issuing warps (one block-row of 16 features each), eight converting ones. Issuing a UMMA costs a

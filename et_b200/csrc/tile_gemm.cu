@@ -397,9 +397,9 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             // ---------------- movers: shared memory -> tensor memory copy of the A operand. The mover warps take
             // chunks in turn; lane 1 polls, lane 0 issues and commits. The tensor-memory slot is free when the
             // UMMAs of the chunk a_slots earlier have completed: a tcgen05.cp is guaranteed to run ahead of UMMAs issued
-            // after it, but not behind those issued before it (waiting for their issue alone saved nothing measurable:
-            // 4096 -> 1024 at 80 % sparsity, 8192 tokens 35.3 and 35.4 us). The one commit per chunk tells the issuers that
-            // A is in place and the activation producer that the shared-memory slot may be overwritten.
+            // after it, but not behind those issued before it (going by their issue saved 2-3 % with two
+            // slots, 4096 -> 1024 at 75 % sparsity and 32768 tokens 130.3 us against 133.3, and nothing with more). The one commit per
+            // chunk tells the issuers that A is in place and the activation producer that the shared-memory slot may be overwritten.
             const int m = warp - kFirstMover;
             int xs = m % NX, a = m % RA, fx = m, fw = m, ar = m;
             uint32_t phx = 0, phw = 0, phd = 0;
@@ -1010,7 +1010,6 @@ int tile_weight_prepare_fusion(TileWeight* w) { return build_tile_form(w); }
 int tile_weight_in_feat(const TileWeight* w) { return w->K; }
 int tile_weight_out_feat(const TileWeight* w) { return w->N; }
 int tile_weight_size(const TileWeight* w) { return w->size_hint; }
-int tile_weight_chunks(const TileWeight* w) { return w->n_chunks; }
 int tile_weight_stat_slots(const TileWeight* w) { return kEpiPerQuarter * w->n_chunks; }
 
 // The weight with a LayerNorm folded in: tile values multiplied by gamma of their input feature (rounded to fp16

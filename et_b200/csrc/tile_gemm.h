@@ -49,8 +49,7 @@ int tile_weight_fold(TileWeight** out, const TileWeight* w, const half* gamma, c
 int tile_weight_gather_inputs(TileWeight** out, const TileWeight* w, const int* src, int n);
 // Builds what the fused epilogues (GemmFusion) of this weight need, if it is not there yet.
 int tile_weight_prepare_fusion(TileWeight* w);
-// Column chunks of the packed weight, and the partial-sum slots per row that its residual epilogue writes.
-int tile_weight_chunks(const TileWeight* w);
+// The partial-sum slots per row that the residual epilogue of the packed weight writes.
 int tile_weight_stat_slots(const TileWeight* w);
 // Reads and clears the device error word (0 = no bounded wait gave up). Synchronises.
 int tile_weight_error(const TileWeight* w, int* code);

@@ -328,9 +328,9 @@ def test_encoder_rejects_bad_arguments(et, orc):
 
 
 def test_run_batch_on_the_legacy_stream_and_on_a_side_stream_agree(et, orc):
-    """On the legacy default stream the layer runs on a stream of the encoder (ordered by events) so that the graph
-    replay still engages; results are bit-identical to a caller-provided stream, and ordered with the caller's
-    other work on the legacy stream."""
+    """On the legacy default stream, which cannot be captured, the layer's graph is recorded on a stream of its own and launched
+    into the caller's; results are bit-identical to a caller-provided stream, and ordered with the caller's other work on
+    the legacy stream."""
     d, H, dff, B, S = 256, 4, 512, 3, 64
     lin, ln = make_layer(orc, d, dff, 0.5, seed=61)
     enc = build_encoder(et, et.KIND_TILE, lin, ln, d, S, H, B * S)

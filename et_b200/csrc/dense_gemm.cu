@@ -54,7 +54,7 @@ struct DenseParams {
     int* err;
     const half* X;
     const half* W;
-    const uint32_t* kept;   // one bit per 16 x 16 tile, rows of whole words; null when no tile was pruned
+    const uint32_t* kept;   // kPruned: one bit per 16 x 16 tile, rows of whole words
 };
 
 __host__ __device__ constexpr int copy_warps(int stages) {
@@ -118,7 +118,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
 
 // A pruned tile takes no part in the product, but 0 x infinity does here. Results that are not finite are therefore computed
 // again from the kept tiles alone (one that really leaves the fp16 range comes out the same). Finding them costs one operation
-// per two results; `kept` is null, and nothing is looked for, where no tile was pruned.
+// per two results, in kernels of their own (kPruned) that weights without pruned tiles do not take.
 struct NotFinite {   // zeros, until a value came that is not finite
     half2 s[4];
     __device__ __forceinline__ NotFinite() {
@@ -170,7 +170,7 @@ __device__ __forceinline__ void recompute_segment(const DenseParams& p, int row,
     *reinterpret_cast<uint4*>(y) = held;
 }
 
-template <bool kGelu>
+template <bool kGelu, bool kPruned>
 __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                                                             const __grid_constant__ CUtensorMap tmY, const __grid_constant__ DenseParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 if (lane == 0) tma_store_wait_read();   // the buffer's previous store has read it
                 __syncwarp();
                 epi_write(buf, lane, ov);
-                if (p.kept) {
+                if constexpr (kPruned) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) odd.note(ov[c]);
                 }
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 }
             }
             if (h >= units) accumulator_read();
-            if (p.kept && __any_sync(0xffffffffu, odd.any())) {
+            if (kPruned && __any_sync(0xffffffffu, odd.any())) {
                 if (lane == 0) tma_store_wait();   // the results are in memory
                 __syncwarp();
                 fence_proxy_async_global();
@@ -355,7 +355,7 @@ __device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
     return v;
 }
 
-template <bool kGelu>
+template <bool kGelu, bool kPruned>
 __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __grid_constant__ CUtensorMap tmX,
                                                                        const __grid_constant__ CUtensorMap tmW,
                                                                        const __grid_constant__ DenseParams p, int split) {
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
             oh[j] = kGelu ? gelu_tanh_h2(t) : t;
         }
         *reinterpret_cast<uint4*>(p.Y + (size_t)(m0 + r) * p.N + n0 + c) = o;
-        if (p.kept) {
+        if constexpr (kPruned) {
             NotFinite odd;
             odd.note(o);
             if (odd.any()) recompute_segment<kGelu>(p, m0 + r, n0 + c);
@@ -563,12 +563,20 @@ int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* 
     CUtensorMap tmX, tmY;
     if (!make_tmap_2d_f16(&tmX, X, (uint64_t)T, (uint64_t)K, (uint64_t)K, kBM, kBK, 128))
         return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
+    // [gelu][pruned]
+    using PairFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, DenseParams);
+    using SplitFn = void (*)(CUtensorMap, CUtensorMap, DenseParams, int);
+    static const PairFn pair[2][2] = {{dense_kernel<false, false>, dense_kernel<false, true>}, {dense_kernel<true, false>, dense_kernel<true, true>}};
+    static const SplitFn split[2][2] = {{dense_split_kernel<false, false>, dense_split_kernel<false, true>},
+                                        {dense_split_kernel<true, false>, dense_split_kernel<true, true>}};
+    const int g = gelu ? 1 : 0, pruned = w.kept ? 1 : 0;
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] {
-        cudaError_t e = cudaFuncSetAttribute(dense_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_split_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+            e = cudaFuncSetAttribute(pair[i >> 1][i & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(split[i >> 1][i & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        }
         return e;
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "dense linear: shared memory opt-in");
@@ -597,9 +605,7 @@ int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* 
         cfg.blockDim = dim3(kSplitThreads);
         cfg.dynamicSmemBytes = (size_t)std::max(p.stages * stage, kBM * (plan.bn + 4) * 4) + sizeof(DenseShared) + 1024;
         attr[1].val.clusterDim.x = (unsigned)plan.split;
-        return cuda_status(gelu ? cudaLaunchKernelEx(&cfg, dense_split_kernel<true>, tmX, tmW, p, plan.split)
-                                : cudaLaunchKernelEx(&cfg, dense_split_kernel<false>, tmX, tmW, p, plan.split),
-                           "dense linear launch");
+        return cuda_status(cudaLaunchKernelEx(&cfg, split[g][pruned], tmX, tmW, p, plan.split), "dense linear launch");
     }
     if (!make_tmap_2d_f16(&tmY, Y, (uint64_t)T, (uint64_t)N, (uint64_t)N, 32, kUnitCols, 64))
         return fail(ET_ERR_CUDA, "dense linear: cuTensorMapEncodeTiled failed");
@@ -610,9 +616,7 @@ int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* 
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = (size_t)p.stages * stage + kEpiWarps * kUnitBytes + sizeof(DenseShared) + 1024;
     attr[1].val.clusterDim.x = 2;
-    return cuda_status(gelu ? cudaLaunchKernelEx(&cfg, dense_kernel<true>, tmX, tmW, tmY, p)
-                            : cudaLaunchKernelEx(&cfg, dense_kernel<false>, tmX, tmW, tmY, p),
-                       "dense linear launch");
+    return cuda_status(cudaLaunchKernelEx(&cfg, pair[g][pruned], tmX, tmW, tmY, p), "dense linear launch");
 }
 
 }  // namespace et

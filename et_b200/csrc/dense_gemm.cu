@@ -118,7 +118,8 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
 
 // A pruned tile takes no part in the product, but 0 x infinity does here. Results that are not finite are therefore computed
 // again from the kept tiles alone (one that really leaves the fp16 range comes out the same). Finding them costs one operation
-// per two results, in kernels of their own (kPruned) that weights without pruned tiles do not take.
+// per two results (3072 -> 768 at 75 %, 128 tokens 8.86 -> 8.98 us, at 50 %, 4096 tokens 18.8 -> 19.3), in kernels of their own
+// (kPruned) that weights without pruned tiles do not take.
 struct NotFinite {   // zeros, until a value came that is not finite
     half2 s[4];
     __device__ __forceinline__ NotFinite() {

@@ -228,10 +228,10 @@ int et_encoder_run_batch(et_encoder* enc, void* out, const void* in, const int* 
  * *code when a bounded device-side wait gave up since the last check: the output of that run is then
  * incomplete. The status a caller reads where the reference would have exited (encoder/utils.h:4-12). */
 int et_encoder_check(et_encoder* enc, int* code);
-/* et_encoder_run_batch replays a CUDA graph of the layer's launches from the third call on with the same
- * buffers and lengths (no counterpart in the reference, whose run() blocks the host three times per layer).
+/* et_encoder_run and et_encoder_run_batch replay a CUDA graph of the layer's launches from the third call on with the
+ * same buffers and lengths (no counterpart in the reference, whose run() blocks the host three times per layer).
  * on = 0 turns that off (plain launches every call). It is skipped by itself while the caller's stream is
- * being captured. */
+ * being captured (a ragged batch captured there keeps its own lengths, whatever is run between the graph's launches). */
 int et_encoder_set_graph_replay(et_encoder* enc, int on);
 /* Length encoder only: route attention through scores materialised in HBM (the reference's structure,
  * encoder/encoder.cu:126-136) instead of the default on-the-fly kernel. Equal-length batches only. */

@@ -25,10 +25,13 @@
 // clocks in the middle of a block (94 us); two threads per row and sixteen softmax warps at 96 registers: 102 us.
 // CTAs are persistent: the grid has one CTA per item, and a running CTA takes over the next one that has not started (cluster
 // launch control), so that ragged batches balance themselves and an item's loads and first Q K^T are under way while the
-// previous one is finished; its rows are written inside the next item's first block.
-// Measured against the form with 64-key blocks, fp16 scores and four CTAs per SM that it replaces (12 heads): 64 ragged
-// sequences of 32..512 tokens 71 -> 57 us, 256 x 128 tokens 47 -> 37, 32 x 256 19.8 -> 16.1, 64 x 512 87 -> 83; with an additive
-// mask (read twice there, one row per thread) 64 x 384 169 -> 117, 64 x 383 730 -> 121; scores are fp32 here.
+// previous one is finished; its rows are written inside the next item's first block. Ragged batches that outlast a wave are taken
+// longest first (sort_sequences).
+// An additive mask is added to the scores as score + 8 x mask, one mixed-precision multiply-add per element (8 is 1 / scale). It comes
+// by TMA where the rows allow it, otherwise two warps copy granules; with an SM per item two blocks' masks are held. Before, the
+// softmax warps copied it and spent 3400 of 7700 clocks of a block on it: 1 x 384 tokens 14.1 -> 9.1 us, 1 x 701 (16 heads, rows
+// anywhere) 25.7 -> 20.5, 1 x 600 with compact V 28.9 -> 20.8, 64 x 384 116 -> 112, 64 x 383 121 -> 117.
+// Measured (12 heads): 64 ragged sequences of 32..512 tokens 49 us, 64 x 512 84, 256 x 128 in a ragged call 46 (64 before the sort).
 // Column-pruned operands come in two forms. kScatterV (the operator): V is compact, a head's columns start anywhere, results go
 // to their original columns with zeros between. kCompact (the encoder layers, which lay their weights out for it): every head's
 // columns of Q, K and V start at a multiple of 16 and are padded to one with zeros, so that Q K^T takes width / 16 steps, P V
@@ -49,7 +52,8 @@ namespace {
 constexpr int kBQ = 128, kBK = 128, kHD = 64;
 constexpr int kTile = kBQ * kHD * 2;      // 16 KB: a Q tile, a key block of K or of V
 constexpr int kSoftmaxWarps = 4;          // one thread per query row
-constexpr int kThreads = 256;             // + a warp that requests the loads and hands out items, one that issues UMMAs, two idle
+constexpr int kMaskWarps = 2;             // copy masks that do not come by TMA
+constexpr int kThreads = 256;             // + a warp that requests the loads and hands out items, one that issues UMMAs, kMaskWarps
 // A thread of the softmax warps holds 128 scores. Registers are handed over between the two warpgroups: 256 threads start
 // with 128 each, 8 x 128 = 4 x 216 + 4 x 40.
 constexpr int kSoftmaxRegs = 216, kOtherRegs = 40;
@@ -59,6 +63,8 @@ constexpr uint32_t kSCol = 0, kPCol = 128, kOCol = 192;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleStep = 8.f;       // log2 units by which a row maximum must grow before O is rescaled
 constexpr int kItemRing = 4;
+constexpr int kMaxSorted = 256;           // sequences of a ragged batch that a CTA keeps in order of length
+constexpr int kLenClasses = 9;            // 8 or more key blocks, 7, ..., none
 constexpr int kMaskPitch = 272;           // bytes: seventeen 16-byte granules hold 128 mask values at any alignment; conflict-free
 constexpr int kMaskBytes = kSoftmaxWarps * 32 * kMaskPitch;
 constexpr int kScatterPitch = 136;        // bytes per staged output row (64 halfs + 8 bytes against bank conflicts)
@@ -76,6 +82,8 @@ struct TcParams {
     int z_pitch, mask_ld, batch, uniform_len, nhead;
     float scale_log2;
     bool take_over;   // CTAs ask for items that have not started
+    bool mask_two;    // two places for masks: where a CTA has an SM to itself
+    bool mask_rows;   // equal lengths, and every row of the mask starts on a 16-byte boundary: it comes by TMA
     int* err;
 };
 
@@ -104,6 +112,8 @@ struct Cfg {
     static constexpr int kMaskAt = (kQS + kKS + kVS) * kTile;
     static constexpr int kScatterAt = kMaskAt + (kMask ? kMaskBytes : 0);
     static constexpr int kBytes = kScatterAt + (kPruneV ? kScatterBytes : 0);
+    template <bool kSorted>
+    __host__ __device__ static constexpr int second_mask_at();   // what a second mask takes begins there
 };
 
 struct TcShared {
@@ -111,10 +121,23 @@ struct TcShared {
     uint64_t clc_full;
     uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2];
     uint64_t s_full, s_free, p_full, pv_done;
+    uint64_t m_full[2], m_empty[2];       // kMask: blocks' masks
     uint64_t item_full[kItemRing], item_empty[kItemRing];
     Item item[kItemRing];
     uint32_t tmem_base;
 };
+// A ragged batch in order of length: the sequences, and how many query blocks lie before each.
+struct SeqTable {
+    int tok0[kMaxSorted], len[kMaxSorted], valid[kMaxSorted], before[kMaxSorted + 1];
+    int class_at[kLenClasses + 1];
+    int given_tok0[kMaxSorted], given_len[kMaxSorted], given_valid[kMaxSorted];   // in the caller's order
+};
+
+template <bool kMask, int kForm>
+template <bool kSorted>
+__host__ __device__ constexpr int Cfg<kMask, kForm>::second_mask_at() {
+    return (kBytes + (int)sizeof(TcShared) + (kSorted ? (int)sizeof(SeqTable) : 0) + 1023) / 1024 * 1024;
+}
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
@@ -172,16 +195,97 @@ __device__ __forceinline__ bool clc_query(const uint4* answer, int& x) {
     return ok != 0;
 }
 
-// Which queries block `blk` of head `h` is (whole warp): 32 sequences per round, each lane takes one, a prefix sum of their
-// query-block counts locates the block. nkb = -1: the block lies beyond the batch (the grid of a ragged batch has slack).
-__device__ __forceinline__ Item find_item(const TcParams& p, int blk, int h, int lane) {
+// Sorts a ragged batch by key blocks, the longest first (whole warp; sequences of one class keep their order): what is left when CTAs
+// run out of items are then short ones, and an item is found without reading memory. In the caller's order, with two rounds of loads per
+// item, the CTAs of 64 sequences of 32..512 tokens, 12 heads, finished between 43 and 52.5 us, and 256 x 128 tokens waited for items:
+// 51.7 -> 49.4 and 64 -> 46 us. It takes ~1 us before the first item, so only batches that outlast one wave of CTAs are sorted (16 x 128
+// tokens would take 7.7 us instead of 6.1).
+__device__ __forceinline__ void sort_sequences(const TcParams& p, SeqTable* t, int lane) {
+    if (lane <= kLenClasses) t->class_at[lane] = 0;
+    __syncwarp();
+    const unsigned below = (1u << lane) - 1u;
+    for (int pass = 0; pass < 2; ++pass) {   // count, place
+        for (int base = 0; base < p.batch; base += 32) {
+            const int i = base + lane;
+            const bool in = i < p.batch;
+            int tok0 = 0, len = 0, valid = 0;
+            if (in && pass == 0) {
+                tok0 = p.cu_seqlens[i];
+                len = p.cu_seqlens[i + 1] - tok0;
+                valid = p.valid_lens ? max(0, min(p.valid_lens[i], len)) : len;
+                t->given_tok0[i] = tok0;
+                t->given_len[i] = len;
+                t->given_valid[i] = valid;
+            } else if (in) {
+                tok0 = t->given_tok0[i];
+                len = t->given_len[i];
+                valid = t->given_valid[i];
+            }
+            const int c = in ? 8 - min((valid + kBK - 1) / kBK, 8) : kLenClasses;
+            const unsigned same = __match_any_sync(0xffffffffu, c);
+            const int at = t->class_at[c];
+            __syncwarp();
+            if ((same & below) == 0) t->class_at[c] = at + __popc(same);
+            __syncwarp();
+            if (pass == 1 && in) {
+                const int pos = at + __popc(same & below);
+                t->tok0[pos] = tok0;
+                t->len[pos] = len;
+                t->valid[pos] = valid;
+            }
+        }
+        if (pass == 0) {   // counts -> where each class starts
+            const int n = lane < kLenClasses ? t->class_at[lane] : 0;
+            int incl = n;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane < kLenClasses) t->class_at[lane] = incl - n;
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+    int before = 0;
+    for (int base = 0; base < p.batch; base += 32) {
+        const int i = base + lane;
+        int incl = i < p.batch ? (t->len[i] + kBQ - 1) / kBQ : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (i < p.batch) t->before[i + 1] = before + incl;
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) t->before[0] = 0;
+    __syncwarp();
+}
+
+// Which queries block `blk` of head `h` is (whole warp). nkb = -1: the block lies beyond the batch (the grid of a ragged batch has
+// slack). A ragged batch that is not sorted is searched in memory: 32 sequences per round, each lane takes one, a prefix sum of their
+// query-block counts locates the block.
+template <bool kSorted>
+__device__ __forceinline__ Item find_item(const TcParams& p, const SeqTable* t, int blk, int h, int lane) {
     Item it;
     it.tok0 = it.q0 = it.len = it.valid = 0;
     it.head = h;
     it.qk_x = h * kHD; it.qk_steps = kHD / 16;
     it.v_x = h * kHD; it.v_off = 0; it.v_n = kHD; it.v_base = 0; it.v_add = 0;
     int b = -1;
-    if (p.cu_seqlens) {
+    if constexpr (kSorted) {
+        for (int base = 0; base < p.batch; base += 32) {
+            const unsigned hit = __ballot_sync(0xffffffffu, base + lane < p.batch && blk < t->before[min(base + lane, kMaxSorted - 1) + 1]);
+            if (!hit) continue;
+            b = base + __ffs(hit) - 1;
+            it.tok0 = t->tok0[b];
+            it.len = t->len[b];
+            it.valid = t->valid[b];
+            it.q0 = (blk - t->before[b]) * kBQ;
+            break;
+        }
+    } else if (p.cu_seqlens) {
         for (int base = 0; base < p.batch && b < 0; base += 32) {
             const int i = base + lane;
             const int t0 = i < p.batch ? p.cu_seqlens[i] : 0;
@@ -211,16 +315,18 @@ __device__ __forceinline__ Item find_item(const TcParams& p, int blk, int h, int
     }
     it.nkb = -1;
     if (b >= 0) {
-        it.valid = p.valid_lens ? min(p.valid_lens[b], it.len) : it.len;
+        if (!kSorted) it.valid = p.valid_lens ? min(p.valid_lens[b], it.len) : it.len;
         it.nkb = it.valid > 0 ? (it.valid + kBK - 1) / kBK : 0;
     }
     return it;
 }
 
-template <bool kMask, int kForm>
+// kSorted: a ragged batch of at most kMaxSorted sequences, taken longest first.
+template <bool kMask, int kForm, bool kSorted>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                             const __grid_constant__ CUtensorMap tmK,
                                                                             const __grid_constant__ CUtensorMap tmV,
+                                                                            const __grid_constant__ CUtensorMap tmM,
                                                                             const __grid_constant__ TcParams p) {
     using C = Cfg<kMask, kForm>;
     constexpr bool kPruneV = kForm == kScatterV;
@@ -230,8 +336,15 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
     uint8_t* const sK = sQ + C::kQS * kTile;
     uint8_t* const sV = sK + C::kKS * kTile;
     TcShared* const sh = reinterpret_cast<TcShared*>(smem + C::kBytes);
+    SeqTable* const table = reinterpret_cast<SeqTable*>(sh + 1);   // kSorted
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
+    // The place of block g's mask, and how often it has been used before. The second place lies behind everything else.
+    auto mask_place = [&](uint32_t g) {
+        return smem + (p.mask_two && (g & 1u) ? C::template second_mask_at<kSorted>() : C::kMaskAt);
+    };
+    auto mask_slot = [&](uint32_t g) { return p.mask_two ? g & 1u : 0u; };
+    auto mask_turn = [&](uint32_t g) { return p.mask_two ? g >> 1 : g; };
 
     if (warp == kSoftmaxWarps) {
         if (lane == 0) {
@@ -245,9 +358,16 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             mbar_init(&sh->s_free, kSoftmaxWarps);
             mbar_init(&sh->p_full, kSoftmaxWarps);
             mbar_init(&sh->pv_done, 1);
+            if constexpr (kMask) {
+                for (int i = 0; i < 2; ++i) {
+                    mbar_init(&sh->m_full[i], p.mask_rows ? 1 : 32 * kMaskWarps);
+                    mbar_init(&sh->m_empty[i], kSoftmaxWarps);
+                }
+                if (p.mask_rows) prefetch_tmap(&tmM);
+            }
             for (int i = 0; i < kItemRing; ++i) {
                 mbar_init(&sh->item_full[i], 1);
-                mbar_init(&sh->item_empty[i], kSoftmaxWarps + 1);
+                mbar_init(&sh->item_empty[i], kSoftmaxWarps + 1 + (kMask && !p.mask_rows ? kMaskWarps : 0));
             }
             fence_mbar_init();
             prefetch_tmap(&tmQ);
@@ -266,6 +386,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
     if (warp == kSoftmaxWarps) {
         // ---- items and loads (all lanes stay together; lane 0 issues)
         pdl_wait();   // lengths and activations come from the preceding kernels
+        if constexpr (kSorted) sort_sequences(p, table, lane);
         int id = blockIdx.x;   // heads fastest: what a ragged batch has too many lies at the end of the grid
         int ni = 0, nq = 0, nk = 0, nv = 0;   // items handed out, tiles requested
         uint32_t clc_phase = 0;
@@ -276,7 +397,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 clc_try_cancel(&sh->clc, &sh->clc_full);
             }
             const int by = id % p.nhead;
-            Item it = find_item(p, id / p.nhead, by, lane);
+            Item it = find_item<kSorted>(p, table, id / p.nhead, by, lane);
             if constexpr (kForm == kCompact) {
                 if (p.qk_head_ptr) {
                     it.qk_x = p.qk_head_ptr[by];
@@ -318,7 +439,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     tma_load_2d(sQ + qs * kTile, &tmQ, it.qk_x, it.tok0 + it.q0, &sh->q_full[qs]);
                 }
                 ++nq;
-                // K_0, then K_{j+1} ahead of V_j: the next Q K^T needs its block before this one's P V does
+                // K_0, then K_{j+1} ahead of V_j: the next Q K^T needs its block before this one's P V does. The mask of a block follows:
+                // its place is free when the previous block's has been added.
                 for (int j = -1; j < it.nkb && ok; ++j) {
                     if (j + 1 < it.nkb) {
                         const int ks = nk & 1;
@@ -337,6 +459,15 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                             tma_load_2d(sV + vs * kTile, &tmV, it.v_x, it.tok0 + j * kBK, &sh->v_full[vs]);
                         }
                         ++nv;
+                    }
+                    if (kMask && j + 1 < it.nkb && p.mask_rows) {   // block number nk - 1
+                        const uint32_t g = (uint32_t)nk - 1u, ms = mask_slot(g);
+                        if (!(ok = mbar_wait(&sh->m_empty[ms], (mask_turn(g) & 1u) ^ 1u))) break;
+                        if (lane == 0) {
+                            mbar_expect_tx(&sh->m_full[ms], 2 * kTile);
+                            tma_load_2d(mask_place(g), &tmM, (j + 1) * kBK, it.q0, &sh->m_full[ms]);
+                            tma_load_2d(mask_place(g) + kTile, &tmM, (j + 1) * kBK + 64, it.q0, &sh->m_full[ms]);
+                        }
                     }
                 }
             }
@@ -365,8 +496,51 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             for (int i = max(nq - C::kQS, 0); i < nq; ++i) mbar_wait(&sh->q_full[i % C::kQS], (uint32_t)(i / C::kQS) & 1u);
             for (int i = max(nk - 2, 0); i < nk; ++i) mbar_wait(&sh->k_full[i & 1], (uint32_t)(i >> 1) & 1u);
             for (int i = max(nv - C::kVS, 0); i < nv; ++i) mbar_wait(&sh->v_full[i % C::kVS], (uint32_t)(i / C::kVS) & 1u);
+            if (kMask && p.mask_rows)
+                for (int g = max(nk - 2, 0); g < nk; ++g) mbar_wait(&sh->m_full[mask_slot(g)], mask_turn(g) & 1u);
         }
         __syncwarp();
+    } else if (kMask && warp >= kSoftmaxWarps + 2) {
+        // ---- masks that do not come by TMA: the seventeen granules that a row of a block touches, asynchronously
+        if (!p.mask_rows) {
+            pdl_wait();
+            const int t = tid - 32 * (kSoftmaxWarps + 2);
+            uint32_t g = 0;
+            bool ok = true;
+            for (int ni = 0;; ++ni) {
+                const int slot = ni % kItemRing;
+                ok = mbar_wait(&sh->item_full[slot], (uint32_t)(ni / kItemRing) & 1u);
+                if (!ok) break;
+                const int nkb = sh->item[slot].nkb, q0 = sh->item[slot].q0, len = sh->item[slot].len;
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&sh->item_empty[slot]);
+                __syncwarp();
+                if (nkb < 0) break;
+                const uint8_t* const mend = reinterpret_cast<const uint8_t*>(p.mask + (size_t)(len - 1) * p.mask_ld + len);
+                for (int j = 0; j < nkb; ++j, ++g) {
+                    ok = mbar_wait(&sh->m_empty[mask_slot(g)], (mask_turn(g) & 1u) ^ 1u);
+                    if (!ok) break;
+                    uint8_t* const place = mask_place(g);
+                    const uint8_t* const m0 = reinterpret_cast<const uint8_t*>(p.mask + (size_t)q0 * p.mask_ld + j * kBK);
+                    const int rows = min(kBQ, len - q0);   // (what is not copied belongs to rows that are not stored, or to keys beyond the length)
+                    auto granule = [&](const uint8_t* row, int r, int c) {
+                        const uint8_t* src = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(row) & ~(uintptr_t)15) + c * 16;
+                        const long left = (long)(mend - src);
+                        if (left > 0) cp_async16(place + r * kMaskPitch + c * 16, src, left >= 16 ? 16 : (int)left);
+                    };
+                    // sixteen granules of a row by sixteen threads, then the seventeenth ones
+                    const uint8_t* row = m0 + (size_t)(t >> 4) * p.mask_ld * 2;
+#pragma unroll 4
+                    for (int r = t >> 4; r < rows; r += kMaskWarps * 2, row += (size_t)p.mask_ld * (kMaskWarps * 4)) granule(row, r, t & 15);
+                    for (int r = t; r < rows; r += 32 * kMaskWarps) granule(m0 + (size_t)r * p.mask_ld * 2, r, 16);
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&sh->m_full[mask_slot(g)])) : "memory");
+                }
+                if (!ok) break;
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            if (!ok && lane == 0) atomicExch(p.err, 23);
+            __syncwarp();
+        }
     } else if (warp == kSoftmaxWarps + 1) {
         // ---- UMMAs: the warp stays converged (every lane waits), one elected lane issues. Blocks are numbered through
         // across items: Q K^T of block g + 1 is issued as soon as the scores of block g are in registers, ahead of P V of g.
@@ -486,7 +660,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
         const int row = warp * 32 + lane;
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         const uint32_t s_addr = tmem + lane_base + kSCol, p_addr = tmem + lane_base + kPCol, o_addr = tmem + lane_base + kOCol;
-        uint8_t* const mw = smem + C::kMaskAt + (size_t)warp * (32 * kMaskPitch);   // kMask: this warp's mask rows
         const bool wide = (p.z_pitch & 15) == 0 && (reinterpret_cast<uintptr_t>(p.Z) & 31) == 0;
         uint32_t g = 0;
         bool ok = true;
@@ -594,21 +767,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
 #pragma unroll
                 for (int i = 0; i < 2; ++i) cols[i] = lane + 32 * i < it.v_n ? __ldg(p.v_col_id + it.v_base + lane + 32 * i) : 0;
             }
-            // the mask rows of the warp's queries for a block of keys: seventeen granules per row, asynchronously
-            auto fetch_mask = [&](int j) {
-                const uint8_t* mend = reinterpret_cast<const uint8_t*>(p.mask + (size_t)(it.len - 1) * p.mask_ld + it.len);
-                for (int i = lane; i < 32 * 17; i += 32) {
-                    const int r = i / 17, c = i % 17;
-                    const int q = it.q0 + warp * 32 + r;
-                    const uintptr_t a = reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & ~(uintptr_t)15;
-                    const uint8_t* src = reinterpret_cast<const uint8_t*>(a) + c * 16;
-                    const long left = q < it.len ? (long)(mend - src) : 0;
-                    const int n = left >= 16 ? 16 : (left > 0 ? (int)left : 0);
-                    cp_async16(mw + r * kMaskPitch + c * 16, n > 0 ? src : reinterpret_cast<const uint8_t*>(p.mask), n);
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            };
-            if constexpr (kMask) fetch_mask(0);
             float m_run = -INFINITY;
             float2 l2 = make_float2(0.f, 0.f);
             for (int j = 0; j < nkb; ++j, ++g) {
@@ -632,42 +790,63 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 __syncwarp();
                 if (elect_one()) mbar_arrive(&sh->s_free);
                 __syncwarp();
-                float sc = p.scale_log2;
+                const float sc = p.scale_log2;
                 if constexpr (kMask) {
-                    asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    __syncwarp();
-                    sc = 1.f;
-                    const int q = min(it.q0 + row, it.len - 1);
-                    const int shift = (int)((reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & 15) >> 1);
-                    const uint8_t* gr = mw + lane * kMaskPitch;
-                    uint4 cur = *reinterpret_cast<const uint4*>(gr);
+                    // scale x score + mask = scale x (score + mask x 8): eight is 1 / scale, and the product with it exact
+                    ok = mbar_wait(&sh->m_full[mask_slot(g)], mask_turn(g) & 1u);
+                    if (!ok) break;
+                    auto add_mask = [&](float& score, uint32_t two, bool high) {
+                        asm("{\n.reg .b16 l, h, e;\nmov.b32 {l, h}, %1;\nmov.b16 e, 0x4800;\nfma.rn.f32.f16 %0, l, e, %0;\n}" : "+f"(score) : "r"(high ? two >> 16 : two));
+                    };
+                    if (p.mask_rows) {
+                        const uint8_t* const mr = mask_place(g) + row * 128;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (c < 2 || full) {
+                        for (int c = 0; c < 4; ++c) {
+                            if (c < 2 || full) {
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const uint4 nxt = *reinterpret_cast<const uint4*>(gr + (c * 4 + e + 1) * 16);
-                                uint32_t w[8] = {cur.x, cur.y, cur.z, cur.w, nxt.x, nxt.y, nxt.z, nxt.w};
-                                if (shift & 4)
+                                for (int e = 0; e < 4; ++e) {
+                                    const uint4 m4 = *reinterpret_cast<const uint4*>(mr + (c >> 1) * kTile + ((((c & 1) * 4 + e) ^ (row & 7)) << 4));
+                                    const uint32_t w[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
-                                    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
-                                if (shift & 2)
-#pragma unroll
-                                    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const uint32_t mv = (shift & 1) ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
-                                    const float2 m = __half22float2(*reinterpret_cast<const half2*>(&mv));
-                                    const int k = e * 8 + 2 * i;
-                                    v[c][k] = fmaf(v[c][k], p.scale_log2, m.x * kLog2e);
-                                    v[c][k + 1] = fmaf(v[c][k + 1], p.scale_log2, m.y * kLog2e);
+                                    for (int i = 0; i < 4; ++i) {
+                                        add_mask(v[c][e * 8 + 2 * i], w[i], false);
+                                        add_mask(v[c][e * 8 + 2 * i + 1], w[i], true);
+                                    }
                                 }
-                                cur = nxt;
+                            }
+                        }
+                    } else {
+                        const int q = min(it.q0 + row, it.len - 1);
+                        const int shift = (int)((reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & 15) >> 1);
+                        const uint8_t* gr = mask_place(g) + row * kMaskPitch;
+                        uint4 cur = *reinterpret_cast<const uint4*>(gr);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            if (c < 2 || full) {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const uint4 nxt = *reinterpret_cast<const uint4*>(gr + (c * 4 + e + 1) * 16);
+                                    uint32_t w[8] = {cur.x, cur.y, cur.z, cur.w, nxt.x, nxt.y, nxt.z, nxt.w};
+                                    if (shift & 4)
+#pragma unroll
+                                        for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+                                    if (shift & 2)
+#pragma unroll
+                                        for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        const uint32_t mv = (shift & 1) ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
+                                        add_mask(v[c][e * 8 + 2 * i], mv, false);
+                                        add_mask(v[c][e * 8 + 2 * i + 1], mv, true);
+                                    }
+                                    cur = nxt;
+                                }
                             }
                         }
                     }
                     __syncwarp();
-                    if (j + 1 < nkb) fetch_mask(j + 1);
+                    if (elect_one()) mbar_arrive(&sh->m_empty[mask_slot(g)]);
+                    __syncwarp();
                 }
                 if (left < (full ? kBK : kBK / 2)) {   // keys beyond the valid length
 #pragma unroll
@@ -755,7 +934,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 done_cols[1] = cols[1];
             }
         }
-        if constexpr (kMask) asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok && lane == 0) atomicExch(p.err, 22);
         __syncwarp();
     }
@@ -791,14 +969,15 @@ int attn_err_address(int** out) {
     return ET_OK;
 }
 
-template <bool kMask, int kForm>
+template <bool kMask, int kForm, bool kSorted>
 cudaError_t opt_in() {
-    return cudaFuncSetAttribute(attention_tc_kernel<kMask, kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    return cudaFuncSetAttribute(attention_tc_kernel<kMask, kForm, kSorted>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
 }
-template <bool kMask, int kForm>
-cudaError_t launch(dim3 grid, cudaStream_t st, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const TcParams& p) {
-    const size_t smem = (size_t)Cfg<kMask, kForm>::kBytes + sizeof(TcShared) + 1024;
-    return launch_pdl(attention_tc_kernel<kMask, kForm>, grid, dim3(kThreads), smem, st, tq, tk, tv, p);
+template <bool kMask, int kForm, bool kSorted = false>
+cudaError_t launch(dim3 grid, cudaStream_t st, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tm, const TcParams& p) {
+    using C = Cfg<kMask, kForm>;
+    const size_t smem = (p.mask_two ? (size_t)C::template second_mask_at<kSorted>() + kMaskBytes : C::kBytes + sizeof(TcShared) + (kSorted ? sizeof(SeqTable) : 0)) + 1024;
+    return launch_pdl(attention_tc_kernel<kMask, kForm, kSorted>, grid, dim3(kThreads), smem, st, tq, tk, tv, tm, p);
 }
 
 }  // namespace
@@ -846,14 +1025,23 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     p.z_pitch = compact ? v_cols : d_model; p.mask_ld = mask_ld; p.batch = batch; p.uniform_len = uniform_len;
     p.scale_log2 = kLog2e / sqrtf((float)kHD);
     p.err = err_word;
+    // (Of a ragged batch max_len may be more than the mask has rows: only the kernel knows how far it may read.)
+    p.mask_rows = mask && !cu_seqlens && mask_ld % 8 == 0;
+    CUtensorMap tm = tq;
+    if (p.mask_rows && !make_tmap_2d_f16(&tm, mask, (uint64_t)uniform_len, (uint64_t)uniform_len, (uint64_t)mask_ld, kBQ, 64, 128))
+        return fail(ET_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed");
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] {
-        cudaError_t e = opt_in<false, kDense>();
-        if (e == cudaSuccess) e = opt_in<true, kDense>();
-        if (e == cudaSuccess) e = opt_in<false, kScatterV>();
-        if (e == cudaSuccess) e = opt_in<true, kScatterV>();
-        if (e == cudaSuccess) e = opt_in<false, kCompact>();
-        if (e == cudaSuccess) e = opt_in<true, kCompact>();
+        cudaError_t e = opt_in<false, kDense, false>();
+        if (e == cudaSuccess) e = opt_in<true, kDense, false>();
+        if (e == cudaSuccess) e = opt_in<false, kDense, true>();
+        if (e == cudaSuccess) e = opt_in<true, kDense, true>();
+        if (e == cudaSuccess) e = opt_in<false, kScatterV, false>();
+        if (e == cudaSuccess) e = opt_in<true, kScatterV, false>();
+        if (e == cudaSuccess) e = opt_in<false, kCompact, false>();
+        if (e == cudaSuccess) e = opt_in<true, kCompact, false>();
+        if (e == cudaSuccess) e = opt_in<false, kCompact, true>();
+        if (e == cudaSuccess) e = opt_in<true, kCompact, true>();
         return e;
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "attention: shared memory opt-in");
@@ -864,10 +1052,15 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     // ragged batch only the tokens are known here: at least this many blocks. 4 x 512 tokens, 16 heads: 18.2 -> 11.3 us.)
     const long items = cu_seqlens ? (total_tokens + kBQ - 1) / kBQ : nblk;
     p.take_over = items * nhead > (long)kCtasPerSm * sm_count();
-    const auto run = compact      ? (mask ? launch<true, kCompact> : launch<false, kCompact>)
+    p.mask_two = mask && items * nhead <= sm_count() && !cu_seqlens;
+    // (The form that scatters V is not sorted: the table takes registers that it does not have.)
+    const bool sorted = p.take_over && cu_seqlens && batch <= kMaxSorted;
+    const auto run = compact      ? (sorted ? (mask ? launch<true, kCompact, true> : launch<false, kCompact, true>)
+                                            : (mask ? launch<true, kCompact> : launch<false, kCompact>))
                      : v_head_ptr ? (mask ? launch<true, kScatterV> : launch<false, kScatterV>)
+                     : sorted     ? (mask ? launch<true, kDense, true> : launch<false, kDense, true>)
                                   : (mask ? launch<true, kDense> : launch<false, kDense>);
-    const cudaError_t e = run(grid, st, tq, tk, tv, p);
+    const cudaError_t e = run(grid, st, tq, tk, tv, tm, p);
     return cuda_status(e, "attention (tcgen05) launch");
 }
 

@@ -227,6 +227,40 @@ def test_attention_ragged_batch_with_empty_and_padded_sequences(et, orc, mask):
     util.assert_close(host(out), want, what="ragged batch")
 
 
+@pytest.mark.parametrize("batch,mask,pruned_keys", [(150, False, False), (160, True, True), (256, False, True), (257, False, False)])
+def test_attention_ragged_batch_longer_than_a_wave(et, orc, batch, mask, pruned_keys):
+    """More items than places: sequences are taken longest first (up to 256 of them; 257 are searched in order). The caller's
+    bound on the length may exceed the longest sequence, and the mask ends with that sequence's last key."""
+    d, H = 128, 2
+    lens = [int(n) for n in util.rng(batch).integers(0, 140, size=batch)]
+    lens[3], lens[batch - 2], lens[7] = 261, 129, 0
+    T, L = sum(lens), max(lens)
+    valid = [int(n) for n in util.rng(batch + 1).integers(0, 270, size=batch)] if pruned_keys else None
+    Q, K, V = _qkv(batch, T, d)
+    m = (util.rng(5).standard_normal((L, L)) * 0.5).astype(np.float16) if mask else None
+    want = orc.attention(Q, K, V, lens, d, H, mask=m, valid_lens=None if valid is None else [min(v, n) for v, n in zip(valid, lens)])
+    out = torch.full((T, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_batch(out, dev(Q), dev(K), dev(V), d, H, cu_seqlens=dev(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)), batch=batch,
+                       max_seq_len=L + 100, mask=None if m is None else dev(m), mask_ld=L if mask else 0,
+                       valid_lens=None if valid is None else dev(np.array(valid, dtype=np.int32)))
+    torch.cuda.synchronize()
+    util.assert_close(host(out), want, what=f"{batch} ragged sequences")
+
+
+@pytest.mark.parametrize("batch,L,ld", [(1, 136, 136), (1, 200, 208), (40, 136, 136), (40, 130, 130), (3, 300, 301)])
+def test_attention_masks_of_every_row_alignment(et, orc, batch, L, ld):
+    """Rows on 16-byte boundaries come by TMA, others in granules; with an SM per item two blocks' masks are held."""
+    d, H = 256, 4
+    Q, K, V = _qkv(L + batch, batch * L, d)
+    m = (util.rng(L).standard_normal((L, ld)) * 0.5).astype(np.float16)
+    m[:, L // 3] = -np.inf
+    want = orc.attention(Q, K, V, [L] * batch, d, H, mask=m[:, :L])
+    out = torch.full((batch * L, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_batch(out, dev(Q), dev(K), dev(V), d, H, batch=batch, uniform_len=L, mask=dev(m), mask_ld=ld)
+    torch.cuda.synchronize()
+    util.assert_close(host(out), want, what=f"mask of pitch {ld}")
+
+
 @pytest.mark.parametrize("mask,prune", [(False, False), (True, False), (False, True)])
 def test_attention_keys_that_are_not_numbers_reach_every_query(et, orc, mask, prune):
     """A key that is not a number makes every score with it, and so every row of the result, not a number, wherever in a block

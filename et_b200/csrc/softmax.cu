@@ -19,7 +19,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 // (CH of them) and, for l < 8, head element l and tail element l. Nothing but valid elements is ever read, so the granules
 // need no per-element checks; what lies beyond valid_len is only written. The mask row has an alignment of its own: a
 // granule's eight mask values come as the two granules that hold them, shifted into place (five 4-byte loads instead: 40 us against 30, L1 wavefronts).
-// Short rows leave lanes idle, hence G = 8 and 16; R rows per group are in flight at once. Bound by HBM for rows above ~256
+// Short rows leave lanes idle, hence G = 8 and 16; R rows per group are in flight at once (softmax_many_kernel, below, takes over where a
+// group has many). Bound by HBM for rows above ~256
 // elements, by instruction issue below (~60 per granule: two fp32 operations per instruction, 32-bit index arithmetic).
 // Measured with a mask: 1024 matrices of 512 x 512 229 -> 173 us (6.2 TB/s; 64-bit modulo and scalar fp32 before), 128 of
 // 500 x 500 101 us (three passes, 2-byte accesses) -> 30 us.
@@ -126,6 +127,13 @@ __global__ void __launch_bounds__(256) softmax_mask_vec(half* __restrict__ score
     }
 }
 
+// Two scores plus two mask values, in fp32.
+__device__ __forceinline__ float2 scores_plus(uint32_t two, uint32_t mask) {
+    float2 v = __half22float2(*reinterpret_cast<const half2*>(&two));
+    asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %2;\nadd.rn.f32.f16 %0, l, %0;\nadd.rn.f32.f16 %1, h, %1;\n}" : "+f"(v.x), "+f"(v.y) : "r"(mask));
+    return v;
+}
+
 struct RowShape { int head, granules, tail; };
 __device__ __forceinline__ RowShape row_shape(const half* row, int valid) {
     RowShape s;
@@ -136,11 +144,15 @@ __device__ __forceinline__ RowShape row_shape(const half* row, int valid) {
 }
 
 // The elements of a granule that lie inside [lo, hi); zeros for the others.
-__device__ __noinline__ uint4 edge_granule(const half* p, const half* lo, const half* hi) {
-    __align__(16) half v[8];
+__device__ __forceinline__ uint4 edge_granule(const half* p, const half* lo, const half* hi) {
+    uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = (p + j >= lo && p + j < hi) ? p[j] : __float2half(0.f);
-    return *reinterpret_cast<const uint4*>(v);
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t l = p + 2 * j >= lo && p + 2 * j < hi ? __half_as_ushort(p[2 * j]) : 0u;
+        const uint32_t h = p + 2 * j + 1 >= lo && p + 2 * j + 1 < hi ? __half_as_ushort(p[2 * j + 1]) : 0u;
+        w[j] = l | (h << 16);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 template <int G, int CH, int R, bool kMask>
@@ -256,6 +268,170 @@ __global__ void __launch_bounds__(256) softmax_mask_kernel(half* __restrict__ sc
     }
 }
 
+constexpr int kManyBlocks = 3;   // per SM
+
+// The order in which the rows of any alignment are taken: a row index of the matrices c, c + 8, c + 16, ... (whose rows have the same
+// alignment whatever the length, so the mask row stays in registers), the next row index, the next c.
+struct RowWalk {
+    half* at;
+    int r, n, c;
+    __device__ __forceinline__ RowWalk(half* scores, unsigned index, int nmat, int L) {
+        const unsigned full = (unsigned)nmat / 8, more = (unsigned)nmat % 8;   // classes below `more` have full + 1 matrices
+        const unsigned split = more * (full + 1) * (unsigned)L;
+        unsigned in, deep;
+        if (index < split) {
+            deep = full + 1;
+            c = (int)(index / (deep * (unsigned)L));
+            in = index - (unsigned)c * deep * (unsigned)L;
+        } else {
+            deep = max(full, 1u);
+            const unsigned past = index - split;
+            c = (int)(more + past / (deep * (unsigned)L));
+            in = past % (deep * (unsigned)L);
+        }
+        r = (int)(in / deep);
+        n = c + 8 * (int)(in % deep);
+        at = scores + (size_t)n * L * L + (size_t)r * L;
+    }
+    __device__ __forceinline__ void next(half* scores, int nmat, int L) {
+        n += 8;
+        at += (size_t)8 * L * L;
+        if (n < nmat) return;
+        if (++r == L) { r = 0; ++c; }
+        n = c;
+        at = scores + (size_t)n * L * L + (size_t)r * L;
+    }
+};
+
+// Many rows of any length and alignment: a group takes `rows / groups` of them in the order above, D of them in flight. A mask row is
+// fetched, shifted and put in place once for all matrices of its class, and added by mixed-precision additions. What bounds it is the
+// memory system at that size (aligned rows of 504 elements take 25.6 us, 128 matrices) and D times the registers; the kernel above, with
+// the next row requested when one is done, is the faster one where a group has few rows or a mask row few matrices.
+// 128 x 500 x 500 with a mask 33.6 -> 30.6 us, without 33.3 -> 27.8; 1024 x 500 x 500 with one 246 -> 212; 512 x 77 x 77 10.3 -> 8.7.
+template <int G, int CH, int D, bool kMask>
+__global__ void __launch_bounds__(256, kManyBlocks) softmax_many_kernel(half* __restrict__ scores, const half* __restrict__ mask, int nmat, int L,
+                                                                            int valid, unsigned rows) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned group = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const unsigned ngroup = (gridDim.x * blockDim.x) / G;
+    const unsigned first = (unsigned)((unsigned long long)group * rows / ngroup);
+    const int count = (int)((unsigned long long)(group + 1) * rows / ngroup - first);
+    const int rounds = (int)((rows + ngroup - 1) / ngroup);   // the same for all groups of a warp (the reductions use the whole warp)
+    RowWalk cur(scores, min(first, rows - 1), nmat, L), ahead = cur;
+    uint4 slot[D][CH];
+    half slot_e[D][2];
+    auto load = [&](int d, bool there) {
+        const RowShape q = row_shape(ahead.at, there ? valid : 0);
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            slot[d][i] = make_uint4(0xfc00fc00u, 0xfc00fc00u, 0xfc00fc00u, 0xfc00fc00u);   // -inf
+            if (lane + G * i < q.granules) slot[d][i] = __ldcs(reinterpret_cast<const uint4*>(ahead.at + q.head) + lane + G * i);
+        }
+        slot_e[d][0] = slot_e[d][1] = __ushort_as_half((unsigned short)0xfc00u);
+        if (lane < q.head) slot_e[d][0] = ahead.at[lane];
+        if (lane < q.tail) slot_e[d][1] = ahead.at[q.head + 8 * q.granules + lane];
+        if (there) ahead.next(scores, nmat, L);
+    };
+    uint32_t m[CH][4];
+    float me[2] = {0.f, 0.f};
+    auto load_mask = [&](const RowShape& q) {
+        const half* const mg = mask + (size_t)cur.r * L + q.head;
+        const half* const ml = reinterpret_cast<const half*>(reinterpret_cast<uintptr_t>(mg) & ~(uintptr_t)15);
+        const bool split = ml != mg;   // the second granule exists: it holds the values from the first boundary on
+        const int sh = (int)((reinterpret_cast<uintptr_t>(mg) & 15) >> 1);
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const int c = lane + G * i;
+            uint4 ma = make_uint4(0u, 0u, 0u, 0u), mb = ma;
+            if (c < q.granules) {
+                // whole granules: the first one may begin in front of the row, with the previous row's end (for the
+                // mask's first row: within the same 16 bytes as its first element), the second one end behind it
+                if (c > 0 || cur.r > 0 || !split) ma = __ldg(reinterpret_cast<const uint4*>(ml) + c);
+                else ma = edge_granule(ml, mask, mask + (size_t)L * L);
+                if (split) {
+                    const half* t = ml + 8 * c + 8;
+                    if (t + 8 <= mask + (size_t)L * L) mb = __ldg(reinterpret_cast<const uint4*>(t));
+                    else mb = edge_granule(t, mask, mask + (size_t)L * L);
+                }
+            }
+            uint32_t w[8] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
+            if (sh & 4) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) w[k] = w[k + 2];
+            }
+            if (sh & 2) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k) w[k] = w[k + 1];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                m[i][k] = __funnelshift_r(w[k], w[k + 1], (sh & 1) * 16);
+            }
+        }
+        me[0] = lane < q.head ? __half2float(__ldg(mg - q.head + lane)) : 0.f;
+        me[1] = lane < q.tail ? __half2float(__ldg(mg + 8 * q.granules + lane)) : 0.f;
+    };
+    // one row: slot d, then the slot is filled with the row D later
+    auto row = [&](int d, bool there, bool more) {
+        const RowShape q = row_shape(cur.at, there ? valid : 0);
+        float2 v[CH][4];
+        float2 e = make_float2(__half2float(slot_e[d][0]) + me[0], __half2float(slot_e[d][1]) + me[1]);
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const uint32_t w[4] = {slot[d][i].x, slot[d][i].y, slot[d][i].z, slot[d][i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = kMask ? scores_plus(w[j], m[i][j]) : __half22float2(*reinterpret_cast<const half2*>(&w[j]));
+        }
+        load(d, more);
+        float mx = fmaxf(e.x, e.y);
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+            mx = max3(mx, max3(v[i][0].x, v[i][0].y, fmaxf(v[i][1].x, v[i][1].y)), max3(v[i][2].x, v[i][2].y, fmaxf(v[i][3].x, v[i][3].y)));
+        mx = group_max<G>(mx);
+        const float shift = (mx == -INFINITY) ? 0.f : -mx * kLog2e;
+        const float2 l2 = make_float2(kLog2e, kLog2e), s2 = make_float2(shift, shift);
+        e = fma2(e, l2, s2);
+        e = make_float2(ex2_fast(e.x), ex2_fast(e.y));
+        float2 sum2 = e;
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 x = fma2(v[i][j], l2, s2);
+                v[i][j] = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+                sum2 = add2(sum2, v[i][j]);
+            }
+        const float sum = group_sum<G>(sum2.x + sum2.y);
+        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+            if (lane + G * i < q.granules) __stcs(reinterpret_cast<uint4*>(cur.at + q.head) + lane + G * i, pack_row(v[i], inv));
+        if (lane < q.head) cur.at[lane] = __float2half_rn(e.x * inv);
+        if (lane < q.tail) cur.at[q.head + 8 * q.granules + lane] = __float2half_rn(e.y * inv);
+        if (valid < L && there)
+            for (int z = valid + lane; z < L; z += G) cur.at[z] = __float2half(0.f);
+        if (there) cur.next(scores, nmat, L);
+    };
+#pragma unroll
+    for (int d = 0; d < D; ++d) load(d, d < count);
+    int mask_r = -1, mask_c = -1;
+    for (int k0 = 0; k0 < rounds; k0 += D) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            if (k0 + d >= rounds) break;
+            const bool there = k0 + d < count;
+            if (kMask && (cur.r != mask_r || cur.c != mask_c)) {
+                mask_r = cur.r;
+                mask_c = cur.c;
+                load_mask(row_shape(cur.at, there ? valid : 0));
+            }
+            row(d, there, k0 + d + D < count);
+        }
+    }
+}
+
 // Rows above 2048 elements: one warp per row, three passes.
 __global__ void __launch_bounds__(256) softmax_mask_generic(half* __restrict__ scores,
                                                             const half* __restrict__ mask,
@@ -315,9 +491,27 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
             launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, st, s + (size_t)at * seq_len * seq_len, m, nrow, seq_len, valid_len);
         }
     };
+    // Five rows a group, and for a mask six matrices of a class (30 x 509 x 509, four rows: 10.4 us here, 10.7 there; 500 x 45 x 45,
+    // two rows: 3.1 and 4.0; 16 x 1001 x 1001, two matrices: 18.8 and 24.4).
+    auto run_many = [&](auto kernel, int group) {
+        if ((long)nmat * seq_len < 5L * sm_count() * kManyBlocks * (256 / group) || (m && nmat < 48)) return false;
+        const int most = std::max(8, per_launch / 8 * 8);   // a launch begins with a matrix of the first one's alignment
+        for (int at = 0, n; at < nmat; at += n) {
+            n = std::min(most, nmat - at);
+            const unsigned rows = (unsigned)n * (unsigned)seq_len;
+            launch_pdl(kernel, dim3((unsigned)std::min(((long)rows * group + 255) / 256, (long)sm_count() * kManyBlocks)), dim3(256), 0, st,
+                       s + (size_t)at * seq_len * seq_len, m, n, seq_len, valid_len, rows);
+        }
+        return true;
+    };
     auto pick = [&](auto masked) {
         constexpr bool kMask = decltype(masked)::value;
         constexpr int R = kMask ? 1 : 2;
+        if (seq_len <= 64 ? run_many(softmax_many_kernel<8, 1, 3, kMask>, 8)
+            : seq_len <= 128 ? run_many(softmax_many_kernel<16, 1, 3, kMask>, 16)
+            : seq_len <= 256 ? run_many(softmax_many_kernel<32, 1, 3, kMask>, 32)
+            : seq_len <= 512 ? run_many(softmax_many_kernel<32, 2, kMask ? 2 : 3, kMask>, 32) : false)
+            return;
         if (seq_len <= 64) run(softmax_mask_kernel<8, 1, R, kMask>, 8, R);
         else if (seq_len <= 128) run(softmax_mask_kernel<16, 1, R, kMask>, 16, R);
         else if (seq_len <= 256) run(softmax_mask_kernel<32, 1, R, kMask>, 32, R);

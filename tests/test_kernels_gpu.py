@@ -120,6 +120,25 @@ def test_softmax_fully_masked_row_is_zero(et):
     assert (host(S) == 0).all()
 
 
+@pytest.mark.parametrize("nmat,L,offset,use_mask,cut", [(1131, 63, 1, True, 0), (5000, 15, 0, False, 2), (283, 127, 3, True, 30), (280, 127, 0, False, 0),
+                                                         (71, 255, 5, True, 0), (51, 509, 0, True, 9), (49, 365, 7, True, 0), (36, 500, 0, False, 1)])
+def test_softmax_many_rows_of_any_alignment(et, orc, nmat, L, offset, use_mask, cut):
+    """Enough rows that a group of lanes takes several, and with a mask several matrices for each of its rows."""
+    S = (util.rng(L).standard_normal((nmat, L, L)) * 3).astype(np.float16)
+    mask = util.rng(L + 1).standard_normal((L, L)).astype(np.float16) if use_mask else None
+    buf = torch.full((nmat * L * L + 16,), 7.0, dtype=torch.float16, device="cuda")
+    buf[offset:offset + nmat * L * L] = dev(S).reshape(-1)
+    view = buf[offset:offset + nmat * L * L].view(nmat, L, L)
+    mbuf = torch.zeros(L * L + 8, dtype=torch.float16, device="cuda")
+    if use_mask:
+        mbuf[offset:offset + L * L] = dev(mask).reshape(-1)
+    et.softmax_mask(view, mbuf[offset:offset + L * L].view(L, L) if use_mask else None, L - cut)
+    torch.cuda.synchronize()
+    util.assert_close(host(view), orc.softmax_mask(S, mask, L - cut), what=f"softmax {nmat}x{L}")
+    assert (host(view)[:, :, L - cut:] == 0).all()
+    assert (buf[:offset] == 7).all() and (buf[offset + nmat * L * L:] == 7).all()
+
+
 @pytest.mark.parametrize("L", [1, 7, 241, 242, 243, 499, 1017, 1019, 2034, 2035])
 @pytest.mark.parametrize("offset", [0, 3])
 def test_softmax_mask_rows_of_any_alignment(et, orc, L, offset):

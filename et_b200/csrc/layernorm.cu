@@ -90,6 +90,80 @@ __global__ void __launch_bounds__(256, (CH <= 4 ? 3 : 1)) skip_layernorm_vec(hal
     }
 }
 
+// Rows of exactly CH * 256 elements (768, 1024): the next row is requested before this one's reductions, by as many blocks as an SM holds
+// without spills (at 1024 elements a third one spilled 144 bytes: 17.8 us instead of 12.3 for 16384 rows); sizes known at compile time
+// leave the registers for it. What bounds it is memory, or L2 where the operands come from the linear before. Against the kernel above, with
+// operands in L2: 8192 x 768 6.3 -> 5.3 us, 17771 x 768 11.8 -> 9.2, 4096 x 1024 6.3 -> 3.9, 16384 x 1024 17.5 -> 12.3; from memory:
+// 17771 x 768 15.3 -> 14.4, 131072 x 1024 131 -> 123 (6.5 TB/s).
+constexpr int row_blocks(int ch) { return ch <= 3 ? 3 : 2; }   // per SM
+template <int CH>
+__global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half* __restrict__ in_out, const half* __restrict__ skip,
+                                                                       const half* __restrict__ gamma, const half* __restrict__ beta, int num) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int kSize = CH * 256;
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarp = (gridDim.x * blockDim.x) >> 5;
+    const size_t step = (size_t)nwarp * (kSize / 8);
+    uint4* xr = reinterpret_cast<uint4*>(in_out) + (size_t)warp * (kSize / 8) + lane;
+    const uint4* sr = reinterpret_cast<const uint4*>(skip) + (size_t)warp * (kSize / 8) + lane;
+    uint4 xv[CH], sv[CH];
+    auto load = [&]() {
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            xv[i] = xr[32 * i];
+            sv[i] = __ldcs(sr + 32 * i);
+        }
+    };
+    if (warp < num) load();
+    for (int row = warp; row < num; row += nwarp) {
+        uint4* const out = xr;
+        float v[CH][8];
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const half2* xh = reinterpret_cast<const half2*>(&xv[i]);
+            const half2* sh = reinterpret_cast<const half2*>(&sv[i]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 a = __half22float2(xh[j]), s = __half22float2(sh[j]);
+                v[i][2 * j] = a.x + s.x;
+                v[i][2 * j + 1] = a.y + s.y;
+                sum += v[i][2 * j] + v[i][2 * j + 1];
+            }
+        }
+        xr += step;
+        sr += step;
+        if (row + nwarp < num) load();
+        const float mean = warp_sum(sum) * (1.0f / kSize);
+        float sq = 0.f;
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float d = v[i][j] - mean;
+                sq += d * d;
+            }
+        const float rstd = rsqrtf(warp_sum(sq) * (1.0f / kSize) + 1e-6f);
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const uint4 g = __ldg(reinterpret_cast<const uint4*>(gamma) + lane + 32 * i);
+            const uint4 b = __ldg(reinterpret_cast<const uint4*>(beta) + lane + 32 * i);
+            const half2* gh = reinterpret_cast<const half2*>(&g);
+            const half2* bh = reinterpret_cast<const half2*>(&b);
+            uint4 o;
+            half2* oh = reinterpret_cast<half2*>(&o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 gg = __half22float2(gh[j]), bb = __half22float2(bh[j]);
+                oh[j] = __floats2half2_rn((v[i][2 * j] - mean) * rstd * gg.x + bb.x, (v[i][2 * j + 1] - mean) * rstd * gg.y + bb.y);
+            }
+            out[32 * i] = o;
+        }
+    }
+}
+
 // Any even size, any alignment of 4 bytes: one warp per row, three passes over the row.
 __global__ void __launch_bounds__(256) skip_layernorm_generic(half* __restrict__ in_out,
                                                               const half* __restrict__ skip,
@@ -145,7 +219,7 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
     int blocks = (warps_needed + 7) / 8;
     const bool vec = size % 8 == 0 && size <= 2048 && aligned16(x) && (!s || aligned16(s)) &&
                      aligned16(g) && aligned16(b);
-    // Blocks per SM, by what is resident there. Of the kernel for 257 to 1024 elements three blocks of eight warps are (registers): a
+    // (skip_layernorm_rows aside:) blocks per SM, by what is resident there. Of the kernel for 257 to 1024 elements three blocks of eight warps are (registers): a
     // multiple of three, two waves, or eight where a warp would have more than six rows, as shorter shares even out the SMs'
     // shares of the bandwidth. Eight blocks per SM, 2.7 waves, before: 17771 x 768 12.2 -> 11.5 us, 32768 x 768 20.8 -> 19.2,
     // 131072 x 1024 139 -> 132 (6.1 TB/s). Narrower rows and the kernel for any size leave room for eight blocks: with six, 17771 x
@@ -154,7 +228,11 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
     const bool long_share = num / 12 > sm_count() * 3 * 8;
     const int per_sm = !vec ? (long_share ? 24 : 8) : size <= 256 ? 8 : size <= 1024 ? (long_share ? 24 : 6) : (long_share ? 8 : 6);
     blocks = std::min(blocks, sm_count() * per_sm);
-    if (vec) {
+    if (vec && s && (size == 768 || size == 1024)) {
+        const dim3 grid(std::min((warps_needed + 7) / 8, sm_count() * row_blocks(size / 256)));
+        if (size == 768) launch_pdl(skip_layernorm_rows<3>, grid, dim3(256), 0, st, x, s, g, b, num);
+        else launch_pdl(skip_layernorm_rows<4>, grid, dim3(256), 0, st, x, s, g, b, num);
+    } else if (vec) {
         const int ch = (size / 8 + 31) / 32;
         switch (ch) {
             case 1: launch_pdl(skip_layernorm_vec<1>, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size); break;

@@ -46,6 +46,19 @@ def test_skip_layernorm(et, orc, num, size):
     util.assert_close(host(xd), want, what=f"skip_layernorm {num}x{size}")
 
 
+@pytest.mark.parametrize("num,size", [(1, 1024), (9, 768), (148 * 24, 768), (148 * 24 + 1, 768), (148 * 48 + 5, 768), (148 * 16 + 1, 1024), (5003, 1024)])
+def test_skip_layernorm_rows_beyond_a_wave(et, num, size):
+    """Warps that take one row, two, and one fewer than their neighbours, each requested while the one before is reduced."""
+    gen = torch.Generator(device="cuda").manual_seed(num)
+    x, s = (torch.randn((num, size), generator=gen, device="cuda").half() for _ in range(2))
+    g, b = (torch.randn((size,), generator=gen, device="cuda").half() for _ in range(2))
+    want = torch.nn.functional.layer_norm(x.double() + s.double(), (size,), g.double(), b.double(), 1e-6)
+    et.skip_layernorm(x, s, g, b)
+    torch.cuda.synchronize()
+    # one fp16 rounding of values up to ~20 (half a unit: 8e-3)
+    util.assert_close(host(x), want.float().cpu().numpy(), max_abs=1e-2, mean_abs=4e-4, what=f"skip_layernorm {num}x{size}")
+
+
 def test_skip_layernorm_matches_reference_kernels(et, orc, ref):
     for num, size in [(128, 768), (2048, 768), (1024, 1024)]:   # v1 and v2 kernels of the reference
         x, s = util.activations(1, (num, size)), util.activations(2, (num, size))

@@ -14,9 +14,12 @@
 // so that a tile is stored while the next one is multiplied. 16384 x 4096 x 1024: tensor pipe 90 % busy.
 //
 // dense_split_kernel, few tiles (small batches): the K range is split over a thread-block cluster. Each CTA accumulates its
-// share, leaves the fp32 partial tile in its shared memory, and after a cluster barrier sums 1/cluster of the rows over
-// all partials in rank order (distributed shared memory, no atomics: results do not depend on timing). 128 tokens, 3072
-// inputs, 768 outputs: 12 CTAs walking 24 chunks of 128 each took 18.8 us in the tile kernel, 8.8 us here.
+// share and finishes 1/cluster of the tile's columns: it sends the other CTAs the fp32 parts of theirs (stores to distributed shared
+// memory), and after a cluster barrier adds what it was sent to its own, in rank order (no atomics: results do not depend on timing).
+// Until then each left its whole part in its own memory and loaded rows of the others': 128 x 3072 -> 768 8.5 -> 6.6 us, 4096 -> 1024
+// 10.6 -> 7.7, 256 x 3072 -> 768 12.0 -> 8.1. 128 tokens, 768 (1024) inputs and outputs, which were faster in the tile kernel, 6.4 -> 4.4
+// (8.2 -> 4.6).
+// (A K share per pair of CTAs with tiles of 256 tokens: 1024 x 3072 -> 768 12.4 against 12.1 us, 2048 16.8 against 13.9.)
 //
 // The weight does not depend on the preceding kernel: its first copies are requested before griddepcontrol.wait.
 // Every mbarrier wait is bounded; a role that gives up records a code, and all threads reach the common exit (and the
@@ -137,24 +140,28 @@ struct NotFinite {   // zeros, until a value came that is not finite
     }
 };
 
-// Those of the eight results of `row` from column n0 on (all of one block-row) that are not finite, in place.
-template <bool kGelu>
+// Those of the kCols results of `row` from column n0 on (all of one block-row) that are not finite, in place.
+template <bool kGelu, int kCols = 8>
 __device__ __forceinline__ void recompute_segment(const DenseParams& p, int row, int n0) {
     half* const y = p.Y + (size_t)row * p.N + n0;
-    uint4 held = __ldcg(reinterpret_cast<const uint4*>(y));
-    half* const h = reinterpret_cast<half*>(&held);
-    NotFinite odd;
-    odd.note(held);
-    if (!odd.any()) return;
+    __align__(16) half h[kCols];
+    bool odd = false;
+#pragma unroll
+    for (int c = 0; c < kCols; c += 4) {
+        *reinterpret_cast<uint2*>(h + c) = __ldcg(reinterpret_cast<const uint2*>(y + c));
+#pragma unroll
+        for (int i = c; i < c + 4; ++i) odd = odd || (__half_as_ushort(h[i]) & 0x7c00u) == 0x7c00u;
+    }
+    if (!odd) return;
     const uint32_t* kept = p.kept + (size_t)(n0 / 16) * ((p.K / 16 + 31) / 32);
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float acc[kCols] = {};
     for (int t = 0; t < p.K / 16; ++t) {
         if (!((kept[t >> 5] >> (t & 31)) & 1u)) continue;
         const uint4* xs = reinterpret_cast<const uint4*>(p.X + (size_t)row * p.K + 16 * t);
         const uint4 x2[2] = {__ldcg(xs), __ldcg(xs + 1)};
         const half* x = reinterpret_cast<const half*>(x2);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < kCols; ++c) {
             const uint4* ws = reinterpret_cast<const uint4*>(p.W + (size_t)(n0 + c) * p.K + 16 * t);
             const uint4 w2[2] = {__ldg(ws), __ldg(ws + 1)};
             const half* w = reinterpret_cast<const half*>(w2);
@@ -163,12 +170,13 @@ __device__ __forceinline__ void recompute_segment(const DenseParams& p, int row,
         }
     }
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 0; c < kCols; ++c) {
         if ((__half_as_ushort(h[c]) & 0x7c00u) != 0x7c00u) continue;
         const half v = __float2half_rn(acc[c] + __half2float(p.bias[n0 + c]));
         h[c] = kGelu ? __low2half(gelu_tanh_h2(__half2half2(v))) : v;
     }
-    *reinterpret_cast<uint4*>(y) = held;
+#pragma unroll
+    for (int c = 0; c < kCols; c += 4) *reinterpret_cast<uint2*>(y + c) = *reinterpret_cast<const uint2*>(h + c);
 }
 
 template <bool kGelu, bool kPruned>
@@ -347,13 +355,11 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
 // ------------------------------------------------------------------------------------------ K split over a cluster
 constexpr int kSplitThreads = 256;
 
-__device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
-    float4 v;
-    asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %4, %5;\nld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [a];\n}"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(addr), "r"(rank)
+// Four words to the address `addr` of CTA `rank` of the cluster.
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, const uint32_t* v) {
+    asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, %1;\nst.shared::cluster.v4.b32 [a], {%2,%3,%4,%5};\n}" ::"r"(addr), "r"(rank),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
                  : "memory");
-    return v;
 }
 
 template <bool kGelu, bool kPruned>
@@ -365,10 +371,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     const int S = p.stages, bn = p.bn;
     const int b_panel = bn * kBK * 2;
     const int stage_bytes = p.panels * (kAPanel + b_panel);
-    // the partial tile goes over the stages when they are done with
-    float* const part = reinterpret_cast<float*>(smem);
-    const int pitch = bn + 4;   // floats
-    DenseShared* const sh = reinterpret_cast<DenseShared*>(smem + max(S * stage_bytes, kBM * pitch * 4));
+    // What the other shares send of this CTA's columns: [share][four columns][row], this CTA's own share left out.
+    const int own_cols = bn / split;
+    float4* const recv = reinterpret_cast<float4*>(smem + (size_t)S * stage_bytes);
+    DenseShared* const sh = reinterpret_cast<DenseShared*>(recv + (size_t)(split - 1) * (own_cols / 4) * kBM);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)cluster_rank();
     const int tile = (int)blockIdx.x / split;
@@ -380,12 +386,17 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
         mbar_init(&sh->acc_full[0], 1);
         fence_mbar_init();
     }
+    for (int i = tid; i < own_cols; i += kSplitThreads) {
+        const int n = n0 + rank * own_cols + i;
+        sh->bias[0][i] = n < p.N ? p.bias[n] : __float2half(0.f);
+    }
     if (warp == kCopyWarps) {
         tmem_alloc(&sh->tmem_base, tmem_cols(bn));
         tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this CTA runs: its memory may be written to
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
     // the weight's first panels, before anything that depends on the preceding kernel
@@ -446,60 +457,96 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     const bool fin = mbar_wait(&sh->acc_full[0], 0);
     if ((!ok || !fin) && lane == 0) {
         atomicExch(p.err, 34);
-        if (warp < cw)   // copies in flight land before shared memory is given another use (bounded)
+        if (warp < cw)   // copies in flight land before the CTA leaves (bounded)
             for (int i = 0; i < min(S, kn); ++i) mbar_wait(&sh->full[i], 0);
     }
     __syncwarp();
     tc_fence_after();
     pdl_launch_dependents();
-    {
-        const int q = warp & 3, h = warp >> 2;   // two warps per 32 rows
-        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-        float* const row = part + (size_t)(q * 32 + lane) * pitch;
-        for (int c = h * 16; c < bn; c += 32) {
-            uint32_t r[16];
-            tmem_ld16(tmem + lane_base + c, r);
-            tmem_ld_wait();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA of the cluster runs
+    const int q = warp & 3, h = warp >> 2;   // two warps per 32 rows
+    const int row = q * 32 + lane;
+    const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16);
+    // Every CTA finishes own_cols of the tile's columns and sends the others theirs, straight from tensor memory: stores into the
+    // other CTAs' shared memory go on without waiting, loads from it (a round trip each) took 2 us more.
+    for (int c = h * 16; c < bn; c += 32) {
+        uint32_t r[16];
+        tmem_ld16(acc + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int dst = (c + 4 * i) / own_cols, g = (c + 4 * i - dst * own_cols) / 4;
+            if (dst == rank) continue;   // the same for the whole CTA
+            const int from = rank < dst ? rank : rank - 1;
+            st_cluster(smem_u32(recv + ((size_t)from * (own_cols / 4) + g) * kBM + row), dst, r + 4 * i);
+        }
+    }
+    cluster_sync();   // what was sent has arrived (nobody touches another CTA's memory from here on)
+    auto finish = [&](const uint32_t* own, int c, uint32_t* out) {   // four of the own columns, from c on
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < split; ++k) {   // in the order of the shares
+            float4 x = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
+            if (k != rank) x = recv[((size_t)(k < rank ? k : k - 1) * (own_cols / 4) + c / 4) * kBM + row];
+            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+        }
+        const half2* bias = reinterpret_cast<const half2*>(sh->bias[0] + c);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float2 b = __half22float2(bias[j]);
+            half2 t = __floats2half2_rn(v[2 * j] + b.x, v[2 * j + 1] + b.y);
+            if constexpr (kGelu) t = gelu_tanh_h2(t);
+            out[j] = *reinterpret_cast<const uint32_t*>(&t);
+        }
+    };
+    auto not_finite = [&](const uint32_t* out, int n) {   // any of 2 n results
+        half2 t = __float2half2_rn(0.f);
+        for (int i = 0; i < n; ++i) t = __hfma2(*reinterpret_cast<const half2*>(out + i), __float2half2_rn(0.f), t);
+        return !(__low2float(t) + __high2float(t) == 0.f);
+    };
+    half* const y = p.Y + (size_t)(m0 + row) * p.N + n0 + rank * own_cols;
+    const int left = m0 + row < p.T ? p.N - n0 - rank * own_cols : 0;   // columns of this row that exist
+    const bool wide = (reinterpret_cast<uintptr_t>(p.Y) & 31) == 0 && ((n0 + rank * own_cols) & 15) == 0;
+    for (int c = h * 16; c + 16 <= own_cols; c += 32) {
+        uint32_t own[16], out[8];
+        tmem_ld16(acc + rank * own_cols + c, own);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) finish(own + 4 * i, c + 4 * i, out + 2 * i);
+        if (wide && c + 16 <= left) {   // a whole sector
+            asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(y + c), "r"(out[0]), "r"(out[1]), "r"(out[2]), "r"(out[3]), "r"(out[4]),
+                         "r"(out[5]), "r"(out[6]), "r"(out[7])
+                         : "memory");
+        } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                *reinterpret_cast<float4*>(row + c + 4 * i) = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
-                                                                          __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+                if (c + 4 * i < left) *reinterpret_cast<uint2*>(y + c + 4 * i) = make_uint2(out[2 * i], out[2 * i + 1]);
         }
+        if constexpr (kPruned) {
+            if (not_finite(out, 8))
+                for (int i = c; i < min(c + 16, left); i += 4) recompute_segment<kGelu, 4>(p, m0 + row, n0 + rank * own_cols + i);
+        }
+        __syncwarp();   // the next load from tensor memory needs every lane
+    }
+    for (int c = own_cols / 16 * 16 + h * 4; c < own_cols; c += 8) {
+        uint32_t own[4], out[2];
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(own[0]), "=r"(own[1]), "=r"(own[2]), "=r"(own[3])
+                     : "r"(acc + rank * own_cols + c)
+                     : "memory");
+        tmem_ld_wait();
+        finish(own, c, out);
+        if (c < left) {
+            *reinterpret_cast<uint2*>(y + c) = make_uint2(out[0], out[1]);
+            if constexpr (kPruned) {
+                if (not_finite(out, 2)) recompute_segment<kGelu, 4>(p, m0 + row, n0 + rank * own_cols + c);
+            }
+        }
+        __syncwarp();
     }
     tc_fence_before();
-    __syncwarp();
-    cluster_sync();
+    __syncthreads();
     tc_fence_after();
     if (warp == kCopyWarps) tmem_dealloc(tmem, tmem_cols(bn));
-    const int rows = kBM / split;
-    const int segs = bn / 8;
-    for (int i = tid; i < rows * segs; i += kSplitThreads) {
-        const int r = rank * rows + i / segs, c = (i % segs) * 8;
-        if (m0 + r >= p.T || n0 + c >= p.N) continue;
-        const uint32_t at = smem_u32(part + (size_t)r * pitch + c);
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < split; ++k) {
-            const float4 x = ld_cluster(at, k), y = ld_cluster(at + 16, k);
-            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-            v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
-        }
-        uint4 o;
-        half2* oh = reinterpret_cast<half2*>(&o);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float b0 = __half2float(p.bias[n0 + c + 2 * j]), b1 = __half2float(p.bias[n0 + c + 2 * j + 1]);
-            const half2 t = __floats2half2_rn(v[2 * j] + b0, v[2 * j + 1] + b1);
-            oh[j] = kGelu ? gelu_tanh_h2(t) : t;
-        }
-        *reinterpret_cast<uint4*>(p.Y + (size_t)(m0 + r) * p.N + n0 + c) = o;
-        if constexpr (kPruned) {
-            NotFinite odd;
-            odd.note(o);
-            if (odd.any()) recompute_segment<kGelu>(p, m0 + r, n0 + c);
-        }
-    }
-    __syncwarp();
-    cluster_sync();   // the other CTAs may still be reading this one's partial tile
 }
 
 }  // namespace
@@ -529,7 +576,8 @@ static double dense_cost(int tokens, int N, int K, int bn, int split) {
     const int tiles = std::max(1, (tokens + kBM - 1) / kBM) * tiles_n;
     const double panel = std::max({2.0 * bn, (kAPanel + bn * 128.0) / 58.0, 200.0});
     const int waves = (tiles * split + split_capacity(split) - 1) / split_capacity(split);
-    return 7500.0 + waves * (3500.0 + ((panels + split - 1) / split) * panel + 900.0 + bn * 8.0);
+    const double full = tiles * split > 132 ? 1500.0 : tiles * split > 100 ? 300.0 : 0.0;   // clusters on nearly all SMs: the last ones start late
+    return 5500.0 + full + waves * (3500.0 + ((panels + split - 1) / split) * panel + bn * 45.0);
 }
 
 DensePlan dense_plan(int tokens, int N, int K) {
@@ -600,11 +648,12 @@ int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* 
     if (plan.split > 1) {
         const int stage = p.panels * (kAPanel + plan.bn * kBK * 2);
         p.tiles = ((T + kBM - 1) / kBM) * p.tiles_n;
-        p.stages = ring_stages(std::min({kMaxStages, (kSmemMax - 1024 - (int)sizeof(DenseShared)) / stage,
+        const int recv = (plan.split - 1) * (plan.bn / plan.split) * kBM * 4;
+        p.stages = ring_stages(std::min({kMaxStages, (kSmemMax - 1024 - (int)sizeof(DenseShared) - recv) / stage,
                                          ((p.k_panels + plan.split - 1) / plan.split + p.panels - 1) / p.panels}));
         cfg.gridDim = dim3((unsigned)(p.tiles * plan.split));
         cfg.blockDim = dim3(kSplitThreads);
-        cfg.dynamicSmemBytes = (size_t)std::max(p.stages * stage, kBM * (plan.bn + 4) * 4) + sizeof(DenseShared) + 1024;
+        cfg.dynamicSmemBytes = (size_t)p.stages * stage + recv + sizeof(DenseShared) + 1024;
         attr[1].val.clusterDim.x = (unsigned)plan.split;
         return cuda_status(cudaLaunchKernelEx(&cfg, split[g][pruned], tmX, tmW, p, plan.split), "dense linear launch");
     }

@@ -196,6 +196,51 @@ __global__ void __launch_bounds__(256) skip_layernorm_generic(half* __restrict__
     }
 }
 
+// The same for even sizes on 4-byte boundaries, two elements per access (17771 x 770: 34 us with 2-byte accesses).
+__global__ void __launch_bounds__(256) skip_layernorm_pairs(half* __restrict__ in_out, const half* __restrict__ skip, const half* __restrict__ gamma,
+                                                            const half* __restrict__ beta, int num, int size) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarp = (gridDim.x * blockDim.x) >> 5;
+    const float inv_n = 1.0f / (float)size;
+    const half2* const g2 = reinterpret_cast<const half2*>(gamma);
+    const half2* const b2 = reinterpret_cast<const half2*>(beta);
+    for (int row = warp; row < num; row += nwarp) {
+        half2* x = reinterpret_cast<half2*>(in_out + (size_t)row * size);
+        const half2* s = reinterpret_cast<const half2*>(skip + (size_t)row * size);
+        auto value = [&](int i) {
+            float2 v = __half22float2(x[i]);
+            if (skip) {
+                const float2 t = __half22float2(s[i]);
+                v.x += t.x;
+                v.y += t.y;
+            }
+            return v;
+        };
+        float sum = 0.f;
+#pragma unroll 4
+        for (int i = lane; i < size / 2; i += 32) {
+            const float2 v = value(i);
+            sum += v.x + v.y;
+        }
+        const float mean = warp_sum(sum) * inv_n;
+        float sq = 0.f;
+#pragma unroll 4
+        for (int i = lane; i < size / 2; i += 32) {
+            const float2 v = value(i);
+            sq += (v.x - mean) * (v.x - mean) + (v.y - mean) * (v.y - mean);
+        }
+        const float rstd = rsqrtf(warp_sum(sq) * inv_n + 1e-6f);
+#pragma unroll 4
+        for (int i = lane; i < size / 2; i += 32) {
+            const float2 v = value(i), g = __half22float2(g2[i]), b = __half22float2(b2[i]);
+            x[i] = __floats2half2_rn((v.x - mean) * rstd * g.x + b.x, (v.y - mean) * rstd * g.y + b.y);
+        }
+    }
+}
+
 }  // namespace et
 
 namespace et {
@@ -243,6 +288,8 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
             case 6: launch_pdl(skip_layernorm_vec<6>, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size); break;
             default: launch_pdl(skip_layernorm_vec<8>, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size); break;
         }
+    } else if (size % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
+        launch_pdl(skip_layernorm_pairs, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size);
     } else {
         launch_pdl(skip_layernorm_generic, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size);
     }

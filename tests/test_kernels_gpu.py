@@ -270,6 +270,32 @@ def test_dense_weights_run_alike_whatever_count_they_were_made_for(et, orc, K, N
         w.check()
 
 
+@pytest.mark.parametrize("T,K,N,gelu", [(1, 3072, 16, False), (64, 4096, 48, True), (130, 1024, 784, False), (257, 3072, 1040, True), (400, 2048, 272, False),
+                                        (128, 768, 768, True), (700, 3072, 768, False)])
+def test_dense_shares_meet_at_every_width(et, orc, T, K, N, gelu):
+    """The K range in shares over a cluster: widths of 4 to 64 columns per CTA, outputs that begin between two sectors, and results
+    that are not finite (found per column group and computed again)."""
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, 0.5, T + N, bernoulli=True, bias_std=0.1)
+    X = util.activations(T, (T, K))
+    w = et.TileWeight(K, N, T, data, rp, ro, bias, is_gelu=gelu)
+    x = dev(X)
+    buf = torch.full((T * N + 24,), 7.0, dtype=torch.float16, device="cuda")
+    y = buf[8:8 + T * N].view(T, N)
+    w.run(y, x)
+    torch.cuda.synchronize()
+    util.assert_close(host(y), orc.tile_linear(X, rp, ro, data, bias, N, gelu), what=f"dense linear {T} x {K} -> {N}")
+    assert (buf[:8] == 7).all() and (buf[8 + T * N:] == 7).all()
+    k0 = 16 * (K // 32)
+    x[T // 2, k0:k0 + 16] = float("inf")   # one tile's inputs of one token
+    z = torch.empty_like(y)
+    w.run(z, x)
+    torch.cuda.synchronize()
+    dropped = torch.tensor([k0 not in ro[rp[r]:rp[r + 1]].tolist() for r in range(N // 16)]).repeat_interleave(16).cuda()
+    assert torch.isfinite(z[T // 2][dropped]).all()
+    keep = torch.arange(T, device="cuda") != T // 2
+    assert torch.equal(z[keep], y[keep])
+
+
 @pytest.mark.parametrize("T,K,N,sparsity,gelu,size,form", [
     (200, 3072, 768, 0.75, False, 128, "dense"),         # K split over a cluster
     (200, 3072, 784, 0.75, True, 128, "dense"),

@@ -142,7 +142,8 @@ int et_attention_sharedqk(void* out, const void* QK, const void* V, const void* 
 int et_attention_static_scores(void* out, const void* Q, const void* K, const void* V, const void* mask,
                                int seq_len, int d_model, int nhead, void* stream);
 /* Reads and clears the current device's error word of the tensor-core attention kernel (synchronises):
- * ET_ERR_DEVICE_TIMEOUT and the code in *code (21: the issuing thread's wait, 22: the final accumulator wait)
+ * ET_ERR_DEVICE_TIMEOUT and the code in *code (21: the issuing thread's wait, 22: the final accumulator wait, 23: a warp
+ * that copies masks)
  * when a bounded wait inside the kernel gave up since the last check; the rows of that CTA are then not
  * written. The word is one per device, shared by every launch on it. No counterpart in the reference, whose
  * only error handling is cudaChk's exit(1) (encoder/utils.h:4-12). */

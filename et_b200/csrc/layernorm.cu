@@ -16,6 +16,17 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// Which operations round together is stated, not left to the compiler, so that a row's result does not depend on the kernel that
+// reduces it: the subtraction of the mean is one rounding with sum / size, and so are the squares of a lane's first chunk with their
+// sum; the products of the other chunks are rounded before they are added. (Left to the compiler, sizes known at compile time
+// changed 1e-5 of the results by one fp16 rounding, and 24 layers made of that a relative difference of 1e-3.)
+__device__ __forceinline__ float centred(float v, float sum, float inv_n) { return __fmaf_rn(-sum, inv_n, v); }
+__device__ __forceinline__ float plus_square(float sq, float d, int chunk) {
+    return chunk == 0 ? __fmaf_rn(d, d, sq) : __fadd_rn(sq, __fmul_rn(d, d));
+}
+__device__ __forceinline__ float inv_std(float sq, float inv_n) { return rsqrtf(__fmaf_rn(sq, inv_n, 1e-6f)); }
+__device__ __forceinline__ float scaled(float d, float rstd, float g, float b) { return __fmaf_rn(__fmul_rn(d, rstd), g, b); }
+
 template <int CH>  // 16-byte chunks per lane; covers size <= CH*256
 __global__ void __launch_bounds__(256, (CH <= 4 ? 3 : 1)) skip_layernorm_vec(half* __restrict__ in_out,
                                                           const half* __restrict__ skip,
@@ -56,18 +67,16 @@ __global__ void __launch_bounds__(256, (CH <= 4 ? 3 : 1)) skip_layernorm_vec(hal
                 sum += v[i][2 * j] + v[i][2 * j + 1];
             }
         }
-        const float mean = warp_sum(sum) * inv_n;
+        sum = warp_sum(sum);
         float sq = 0.f;
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
             const int c = lane + 32 * i;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float d = v[i][j] - mean;
-                sq += c < nchunk ? d * d : 0.f;
-            }
+            for (int j = 0; j < 8; ++j)
+                if (c < nchunk) sq = plus_square(sq, centred(v[i][j], sum, inv_n), i);
         }
-        const float rstd = rsqrtf(warp_sum(sq) * inv_n + 1e-6f);
+        const float rstd = inv_std(warp_sum(sq), inv_n);
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
             const int c = lane + 32 * i;
@@ -81,8 +90,8 @@ __global__ void __launch_bounds__(256, (CH <= 4 ? 3 : 1)) skip_layernorm_vec(hal
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 gg = __half22float2(gh[j]), bb = __half22float2(bh[j]);
-                    oh[j] = __floats2half2_rn((v[i][2 * j] - mean) * rstd * gg.x + bb.x,
-                                              (v[i][2 * j + 1] - mean) * rstd * gg.y + bb.y);
+                    oh[j] = __floats2half2_rn(scaled(centred(v[i][2 * j], sum, inv_n), rstd, gg.x, bb.x),
+                                              scaled(centred(v[i][2 * j + 1], sum, inv_n), rstd, gg.y, bb.y));
                 }
                 xr[c] = o;
             }
@@ -136,16 +145,13 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
         xr += step;
         sr += step;
         if (row + nwarp < num) load();
-        const float mean = warp_sum(sum) * (1.0f / kSize);
+        sum = warp_sum(sum);
         float sq = 0.f;
 #pragma unroll
         for (int i = 0; i < CH; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float d = v[i][j] - mean;
-                sq += d * d;
-            }
-        const float rstd = rsqrtf(warp_sum(sq) * (1.0f / kSize) + 1e-6f);
+            for (int j = 0; j < 8; ++j) sq = plus_square(sq, centred(v[i][j], sum, 1.0f / kSize), i);
+        const float rstd = inv_std(warp_sum(sq), 1.0f / kSize);
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
             const uint4 g = __ldg(reinterpret_cast<const uint4*>(gamma) + lane + 32 * i);
@@ -157,7 +163,8 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float2 gg = __half22float2(gh[j]), bb = __half22float2(bh[j]);
-                oh[j] = __floats2half2_rn((v[i][2 * j] - mean) * rstd * gg.x + bb.x, (v[i][2 * j + 1] - mean) * rstd * gg.y + bb.y);
+                oh[j] = __floats2half2_rn(scaled(centred(v[i][2 * j], sum, 1.0f / kSize), rstd, gg.x, bb.x),
+                                          scaled(centred(v[i][2 * j + 1], sum, 1.0f / kSize), rstd, gg.y, bb.y));
             }
             out[32 * i] = o;
         }

@@ -59,6 +59,48 @@ def test_skip_layernorm_rows_beyond_a_wave(et, num, size):
     util.assert_close(host(x), want.float().cpu().numpy(), max_abs=1e-2, mean_abs=4e-4, what=f"skip_layernorm {num}x{size}")
 
 
+def _fma(a, b, c):
+    """One rounding (the product of two fp32 numbers is exact in 64 bits)."""
+    return (a.double() * b.double() + c.double()).float()
+
+
+def _layernorm_in_fp32(x, s, g, b):
+    """skip LayerNorm operation by operation: 32 lanes with chunks of 8 elements, sums over the lanes in pairs."""
+    rows, size = x.shape
+    chunks = size // 256
+    lay = lambda t: t.view(-1, chunks, 32, 8).float()
+    lanes = torch.arange(32, device="cuda")
+
+    def over_lanes(t):
+        for m in (16, 8, 4, 2, 1):
+            t = t + t[:, lanes ^ m]
+        return t[:, :1, None, None].view(rows, 1, 1, 1)
+    v = lay(x) + lay(s)
+    inv = torch.ones((), device="cuda") / torch.full((), float(size), device="cuda")
+    total, sq = (torch.zeros((rows, 32), device="cuda") for _ in range(2))
+    for i in range(chunks):
+        for j in range(0, 8, 2):
+            total = total + (v[:, i, :, j] + v[:, i, :, j + 1])
+    d = _fma(-over_lanes(total), inv, v)
+    for i in range(chunks):
+        for j in range(8):
+            sq = _fma(d[:, i, :, j], d[:, i, :, j], sq) if i == 0 else sq + d[:, i, :, j] * d[:, i, :, j]
+    rstd = torch.rsqrt(_fma(over_lanes(sq), inv, torch.full((), 1e-6, device="cuda")))
+    return _fma(d * rstd, lay(g[None]), lay(b[None])).half().view(rows, size)
+
+
+@pytest.mark.parametrize("num,size", [(3000, 256), (3000, 512), (3000, 768), (3000, 1024), (3000, 1280), (3000, 2048)])
+def test_skip_layernorm_rounds_alike_in_every_kernel(et, num, size):
+    """The bits of a row do not depend on which kernel reduces it: stacks of layers amplify a different rounding."""
+    gen = torch.Generator(device="cuda").manual_seed(size)
+    x, s = (torch.randn((num, size), generator=gen, device="cuda").half() for _ in range(2))
+    g, b = (torch.randn((size,), generator=gen, device="cuda").half() for _ in range(2))
+    want = _layernorm_in_fp32(x, s, g, b)
+    et.skip_layernorm(x, s, g, b)
+    torch.cuda.synchronize()
+    assert torch.equal(x, want), f"{int((x != want).sum())} results differ"
+
+
 def test_skip_layernorm_matches_reference_kernels(et, orc, ref):
     for num, size in [(128, 768), (2048, 768), (1024, 1024)]:   # v1 and v2 kernels of the reference
         x, s = util.activations(1, (num, size)), util.activations(2, (num, size))

@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
         uint8_t* const buf = epi + (size_t)w * kUnitBytes;
         const int units = bn / kUnitCols;
         bool ok = true;
+        pdl_wait();   // the bias may be the caller's and the preceding kernel's result
         for (int tl = 0; tl < my_tiles; ++tl) {
             const int tile = pair + tl * G;
             const int m0 = (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM + q * 32, n0 = (tile % p.tiles_n) * bn;
@@ -386,10 +387,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
         mbar_init(&sh->acc_full[0], 1);
         fence_mbar_init();
     }
-    for (int i = tid; i < own_cols; i += kSplitThreads) {
-        const int n = n0 + rank * own_cols + i;
-        sh->bias[0][i] = n < p.N ? p.bias[n] : __float2half(0.f);
-    }
     if (warp == kCopyWarps) {
         tmem_alloc(&sh->tmem_base, tmem_cols(bn));
         tmem_relinquish();
@@ -451,6 +448,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
             }
             __syncwarp();
             if (++s == S) { s = 0; ph ^= 1u; }
+        }
+    } else {
+        // the bias, which may be the caller's and the preceding kernel's result (read after the second cluster barrier)
+        for (int i = tid - 32 * (kCopyWarps + 1); i < own_cols; i += kSplitThreads - 32 * (kCopyWarps + 1)) {
+            const int n = n0 + rank * own_cols + i;
+            sh->bias[0][i] = n < p.N ? p.bias[n] : __float2half(0.f);
         }
     }
     // every copy has landed and every UMMA has read its operands when the accumulator is complete

@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
         uint8_t* const buf = epi + (size_t)e * kUnitBytes;
         bool ok = true;
         uint32_t gs = 0;
+        pdl_wait();   // the bias may be the caller's and the preceding kernel's result
         for (int item = blockIdx.x; item < p.items && ok; item += G) {
             const int r = item % p.ranges;
             const int g0 = r * p.groups / p.ranges, g1 = (r + 1) * p.groups / p.ranges;

@@ -465,6 +465,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             bool ok = true;
             int ws = 0, a = 0, ar = 0;
             uint32_t pha = 0;
+            pdl_wait();   // the bias may be the caller's and the preceding kernel's result; so are the fused modes' operands
             for (int tl = 0; tl < my_tiles; ++tl) {
                 const int tile = (int)blockIdx.x + tl * G;
                 const int slab = tile / p.n_chunks, chunk = tile - slab * p.n_chunks;

@@ -457,6 +457,38 @@ def test_tile_spmm_raw_launcher(et, orc):
     et.tile_spmm_cache_clear()
 
 
+@pytest.mark.parametrize("T,K,N,sparsity,form", [(128, 3072, 768, 0.0, "shares"), (4096, 768, 768, 0.0, "pairs"), (32768, 768, 2304, 0.75, "resident"),
+                                                 (17792, 3072, 768, 0.75, "tile")])
+def test_tile_spmm_bias_may_be_the_preceding_kernels_result(et, orc, T, K, N, sparsity, form):
+    """The caller's bias is read in the order of the stream: a LayerNorm of one long row, which lets the next kernel start at once
+    and ends long after, writes it right before the call."""
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, T + K, bernoulli=True)
+    info = et.TileWeight(K, N, T, data, rp, ro, bias).info()
+    assert form == ("tile" if info["stage_bytes"] else "resident" if not info["stages"] else "shares" if info["stages"] > 1 else "pairs"), info
+    drp, dro, dd, X = dev(rp), dev(ro), dev(data), dev(util.activations(7, (T, K)))
+    size = 60001
+    before, s = (torch.randn((1, size), device="cuda").half() for _ in range(2))
+    g, b = torch.full((size,), 3.0, device="cuda").half(), torch.ones(size, device="cuda").half()
+    row = before.clone()
+    at = (size - N) // 8 * 8
+    Y, want = (torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2))
+    et.tile_spmm_bias(Y, X, drp, dro, dd, row[0, at:at + N], K=K)   # (the weight is packed here)
+    torch.cuda.synchronize()
+    try:
+        for _ in range(3):
+            row.copy_(before)
+            torch.cuda.synchronize()
+            et.skip_layernorm(row, s, g, b)
+            et.tile_spmm_bias(Y, X, drp, dro, dd, row[0, at:at + N], K=K)
+            torch.cuda.synchronize()
+            assert not torch.equal(row, before)
+            et.tile_spmm_bias(want, X, drp, dro, dd, row[0, at:at + N], K=K)
+            torch.cuda.synchronize()
+            assert torch.equal(Y, want)
+    finally:
+        et.tile_spmm_cache_clear()
+
+
 def test_tile_weight_rejects_malformed_format(et):
     data = np.zeros((2, 256), dtype=np.float16)
     ok_rp = np.array([0, 1, 2], dtype=np.int32)

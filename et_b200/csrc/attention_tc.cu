@@ -83,7 +83,7 @@ struct TcParams {
     float scale_log2;
     bool take_over;   // CTAs ask for items that have not started
     bool mask_two;    // two places for masks: where a CTA has an SM to itself
-    bool mask_rows;   // equal lengths, and every row of the mask starts on a 16-byte boundary: it comes by TMA
+    bool mask_rows;   // equal lengths, and every row of the mask starts on a 16-byte boundary behind the one before: it comes by TMA
     int* err;
 };
 
@@ -1025,8 +1025,9 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     p.z_pitch = compact ? v_cols : d_model; p.mask_ld = mask_ld; p.batch = batch; p.uniform_len = uniform_len;
     p.scale_log2 = kLog2e / sqrtf((float)kHD);
     p.err = err_word;
-    // (Of a ragged batch max_len may be more than the mask has rows: only the kernel knows how far it may read.)
-    p.mask_rows = mask && !cu_seqlens && mask_ld % 8 == 0;
+    // (Of a ragged batch max_len may be more than the mask has rows: only the kernel knows how far it may read. Rows that overlap,
+    // as those of a mask that depends on key - query alone may, are no matrix for a tensor map.)
+    p.mask_rows = mask && !cu_seqlens && mask_ld % 8 == 0 && mask_ld >= uniform_len;
     CUtensorMap tm = tq;
     if (p.mask_rows && !make_tmap_2d_f16(&tm, mask, (uint64_t)uniform_len, (uint64_t)uniform_len, (uint64_t)mask_ld, kBQ, 64, 128))
         return fail(ET_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed");

@@ -261,6 +261,20 @@ def test_attention_masks_of_every_row_alignment(et, orc, batch, L, ld):
     util.assert_close(host(out), want, what=f"mask of pitch {ld}")
 
 
+@pytest.mark.parametrize("batch,L,ld", [(2, 200, 8), (1, 136, 64), (3, 72, 16)])
+def test_attention_masks_whose_rows_overlap(et, orc, batch, L, ld):
+    """A pitch below the length: each row begins inside the one before."""
+    d, H = 128, 2
+    Q, K, V = _qkv(L + ld, batch * L, d)
+    flat = (util.rng(ld).standard_normal((L - 1) * ld + L) * 0.5).astype(np.float16)
+    m = np.lib.stride_tricks.as_strided(flat, (L, L), (2 * ld, 2))
+    want = orc.attention(Q, K, V, [L] * batch, d, H, mask=np.ascontiguousarray(m))
+    out = torch.full((batch * L, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_batch(out, dev(Q), dev(K), dev(V), d, H, batch=batch, uniform_len=L, mask=dev(flat), mask_ld=ld)
+    torch.cuda.synchronize()
+    util.assert_close(host(out), want, what=f"mask of pitch {ld} below {L}")
+
+
 @pytest.mark.parametrize("mask,prune", [(False, False), (True, False), (False, True)])
 def test_attention_keys_that_are_not_numbers_reach_every_query(et, orc, mask, prune):
     """A key that is not a number makes every score with it, and so every row of the result, not a number, wherever in a block

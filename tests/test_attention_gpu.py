@@ -229,13 +229,19 @@ def test_attention_ragged_batch_with_empty_and_padded_sequences(et, orc, mask):
 
 @pytest.mark.parametrize("batch,mask,pruned_keys", [(150, False, False), (160, True, True), (256, False, True), (257, False, False)])
 def test_attention_ragged_batch_longer_than_a_wave(et, orc, batch, mask, pruned_keys):
-    """More items than places: sequences are taken longest first (up to 256 of them; 257 are searched in order). The caller's
-    bound on the length may exceed the longest sequence, and the mask ends with that sequence's last key."""
-    d, H = 128, 2
+    """More items than places: sequences are taken longest first (up to 256 of them; 257 are searched in order), every class of
+    lengths among them. The caller's bound on the length may exceed the longest sequence, and the mask ends with that sequence's
+    last key."""
     lens = [int(n) for n in util.rng(batch).integers(0, 140, size=batch)]
     lens[3], lens[batch - 2], lens[7] = 261, 129, 0
+    lens[20:27] = [1100, 128, 900, 500, 700, 385, 1024]
     T, L = sum(lens), max(lens)
+    places = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    H = places // -(-T // 128) + 1   # heads enough that the blocks of 128 tokens known to exist outnumber the places
+    d = 64 * H
     valid = [int(n) for n in util.rng(batch + 1).integers(0, 270, size=batch)] if pruned_keys else None
+    if pruned_keys:
+        valid[20], valid[22], valid[26] = 1100, 890, 2000
     Q, K, V = _qkv(batch, T, d)
     m = (util.rng(5).standard_normal((L, L)) * 0.5).astype(np.float16) if mask else None
     want = orc.attention(Q, K, V, lens, d, H, mask=m, valid_lens=None if valid is None else [min(v, n) for v, n in zip(valid, lens)])
@@ -244,6 +250,7 @@ def test_attention_ragged_batch_longer_than_a_wave(et, orc, batch, mask, pruned_
                        max_seq_len=L + 100, mask=None if m is None else dev(m), mask_ld=L if mask else 0,
                        valid_lens=None if valid is None else dev(np.array(valid, dtype=np.int32)))
     torch.cuda.synchronize()
+    et.attention_check()
     util.assert_close(host(out), want, what=f"{batch} ragged sequences")
 
 

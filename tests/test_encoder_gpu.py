@@ -353,13 +353,18 @@ def test_run_batch_on_the_legacy_stream_and_on_a_side_stream_agree(et, orc):
 
 @pytest.mark.parametrize("qk_keep,v_keep", [(None, [1, 17, 64, 16]), ([15, 64, 1, 33], [64, 2, 48, 31])])
 @pytest.mark.parametrize("mask", [False, True])
-def test_prune_layers_with_heads_of_any_width(et, orc, qk_keep, v_keep, mask):
+@pytest.mark.parametrize("many", [False, True])
+def test_prune_layers_with_heads_of_any_width(et, orc, qk_keep, v_keep, mask, many):
     """Heads that keep one feature, all of them and counts around the multiples of 16 that the layer pads them to; Q/K and V keep
-    different ones. Tolerance as for the other layers with unit-scale weights: fp16 storage of O(1) values through five stages."""
+    different ones; few sequences, or more than fit on the GPU at once, which are taken longest first. Tolerance as for the other
+    layers with unit-scale weights: fp16 storage of O(1) values through five stages."""
     d, H, S = 256, 4, 130
     lin, ln = make_layer(orc, d, 1024, 0.5, seed=80, unit_scale=True)
     ol = orc_lin(lin)
     lens = [130, 1, 65]
+    if many:
+        lens += [int(n) for n in util.rng(84).integers(0, 131, size=180)]
+        assert -(-sum(lens) // 128) * H > 2 * torch.cuda.get_device_properties(0).multi_processor_count
     T = sum(lens)
     X = util.activations(81, (T, d))
     M = util.activations(82, (S, S)) if mask else None

@@ -99,13 +99,14 @@ __global__ void __launch_bounds__(256, (CH <= 4 ? 3 : 1)) skip_layernorm_vec(hal
     }
 }
 
-// Rows of exactly CH * 256 elements (768, 1024): the next row is requested before this one's reductions, by as many blocks as an SM holds
+// Rows of exactly CH * 256 elements: the next row is requested before this one's reductions, by as many blocks as an SM holds
 // without spills (at 1024 elements a third one spilled 144 bytes: 17.8 us instead of 12.3 for 16384 rows); sizes known at compile time
-// leave the registers for it. What bounds it is memory, or L2 where the operands come from the linear before. Against the kernel above, with
-// operands in L2: 8192 x 768 6.3 -> 5.3 us, 17771 x 768 11.8 -> 9.2, 4096 x 1024 6.3 -> 3.9, 16384 x 1024 17.5 -> 12.3; from memory:
-// 17771 x 768 15.3 -> 14.4, 131072 x 1024 131 -> 123 (6.5 TB/s).
-constexpr int row_blocks(int ch) { return ch <= 3 ? 3 : 2; }   // per SM
-template <int CH>
+// leave the registers for it. What bounds it is memory (6.2 to 6.7 TB/s from 60000 rows on), or L2 where the operands come from the
+// linear before. Against the kernel above, with operands in L2: 8192 x 256 3.5 -> 3.0 us, x 512 5.5 -> 4.3, x 768 7.1 -> 5.6, x 1024
+// 9.2 -> 6.9, x 1280 16.9 -> 8.3, x 2048 22.2 -> 11.6; from memory: 17771 x 768 15.4 -> 14.2, x 1024 21.9 -> 18.3, x 2048 50 -> 35,
+// 131072 x 768 95.5 -> 96, x 1024 132 -> 124, x 2048 304 -> 240. Without a residual 17771 x 768 13.1 -> 10.4, x 2048 45.7 -> 25.5.
+constexpr int row_blocks(int ch) { return ch <= 1 ? 6 : ch <= 2 ? 4 : ch <= 3 ? 3 : ch <= 6 ? 2 : 1; }   // per SM
+template <int CH, bool kSkip>
 __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half* __restrict__ in_out, const half* __restrict__ skip,
                                                                        const half* __restrict__ gamma, const half* __restrict__ beta, int num) {
     pdl_launch_dependents();
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
             xv[i] = xr[32 * i];
-            sv[i] = __ldcs(sr + 32 * i);
+            if constexpr (kSkip) sv[i] = __ldcs(sr + 32 * i);
         }
     };
     if (warp < num) load();
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
             const half2* sh = reinterpret_cast<const half2*>(&sv[i]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float2 a = __half22float2(xh[j]), s = __half22float2(sh[j]);
+                const float2 a = __half22float2(xh[j]), s = kSkip ? __half22float2(sh[j]) : make_float2(0.f, 0.f);
                 v[i][2 * j] = a.x + s.x;
                 v[i][2 * j + 1] = a.y + s.y;
                 sum += v[i][2 * j] + v[i][2 * j + 1];
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
     }
 }
 
-// Any even size, any alignment of 4 bytes: one warp per row, three passes over the row.
+// Any size and alignment, by single elements: one warp per row, three passes over the row (17771 x 769: 33.7 us).
 __global__ void __launch_bounds__(256) skip_layernorm_generic(half* __restrict__ in_out,
                                                               const half* __restrict__ skip,
                                                               const half* __restrict__ gamma,
@@ -203,7 +204,8 @@ __global__ void __launch_bounds__(256) skip_layernorm_generic(half* __restrict__
     }
 }
 
-// The same for even sizes on 4-byte boundaries, two elements per access (17771 x 770: 34 us with 2-byte accesses).
+// The same for even sizes on 4-byte boundaries, two elements per access. What bounds it is the number of accesses: 17771 x 770 32.6 us by
+// single elements, 18.0 here; 131072 x 770 321 -> 160; 4096 x 2050 53 -> 24; 2048 x 770 12.7 -> 7.9.
 __global__ void __launch_bounds__(256) skip_layernorm_pairs(half* __restrict__ in_out, const half* __restrict__ skip, const half* __restrict__ gamma,
                                                             const half* __restrict__ beta, int num, int size) {
     pdl_launch_dependents();
@@ -271,19 +273,26 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
     int blocks = (warps_needed + 7) / 8;
     const bool vec = size % 8 == 0 && size <= 2048 && aligned16(x) && (!s || aligned16(s)) &&
                      aligned16(g) && aligned16(b);
-    // (skip_layernorm_rows aside:) blocks per SM, by what is resident there. Of the kernel for 257 to 1024 elements three blocks of eight warps are (registers): a
-    // multiple of three, two waves, or eight where a warp would have more than six rows, as shorter shares even out the SMs'
-    // shares of the bandwidth. Eight blocks per SM, 2.7 waves, before: 17771 x 768 12.2 -> 11.5 us, 32768 x 768 20.8 -> 19.2,
-    // 131072 x 1024 139 -> 132 (6.1 TB/s). Narrower rows and the kernel for any size leave room for eight blocks: with six, 17771 x
-    // 770 took 47 us instead of 33, and with 24, 60000 x 128 13.9 instead of 13.2 (but 131072 x 770 334 instead of 387). Wider
-    // rows: 24 cost 60000 x 2048 151 us instead of 142 with eight.
+    const bool pairs = size % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(g) |
+                                          reinterpret_cast<uintptr_t>(b)) & 3) == 0;
+    // (skip_layernorm_rows aside:) blocks per SM, by what is resident there. Of skip_layernorm_vec for 257 to 1024 elements three blocks
+    // of eight warps are (registers): a multiple of three, two waves, or eight where a warp would have more than six rows, as shorter
+    // shares even out the SMs' shares of the bandwidth (60000 x 1000: 64.2 us with 24, 68.8 with six). Narrower rows leave room for eight
+    // blocks: 131072 x 200 31.6 us with them, 33.1 with 24. Wider rows: 24 cost 60000 x 2000 158 us instead of 149 with eight. Pairs: six
+    // are resident, and four waves of them do better than one and a third (17771 x 770 18.0 us, 19.6 with eight; 131072 x 770 160 and
+    // 196). Single elements: eight are resident (17771 x 770 32.6 us, 45.7 with six, 35.6 with 24; 131072 x 770 361 with eight, 321 with 24).
     const bool long_share = num / 12 > sm_count() * 3 * 8;
-    const int per_sm = !vec ? (long_share ? 24 : 8) : size <= 256 ? 8 : size <= 1024 ? (long_share ? 24 : 6) : (long_share ? 8 : 6);
+    const int per_sm = !vec ? (pairs || long_share ? 24 : 8) : size <= 256 ? 8 : size <= 1024 ? (long_share ? 24 : 6) : (long_share ? 8 : 6);
     blocks = std::min(blocks, sm_count() * per_sm);
-    if (vec && s && (size == 768 || size == 1024)) {
-        const dim3 grid(std::min((warps_needed + 7) / 8, sm_count() * row_blocks(size / 256)));
-        if (size == 768) launch_pdl(skip_layernorm_rows<3>, grid, dim3(256), 0, st, x, s, g, b, num);
-        else launch_pdl(skip_layernorm_rows<4>, grid, dim3(256), 0, st, x, s, g, b, num);
+    if (vec && size % 256 == 0) {   // every lane's chunks are whole
+        using RowsFn = void (*)(half*, const half*, const half*, const half*, int);
+        static const RowsFn rows[8][2] = {{skip_layernorm_rows<1, false>, skip_layernorm_rows<1, true>}, {skip_layernorm_rows<2, false>, skip_layernorm_rows<2, true>},
+                                          {skip_layernorm_rows<3, false>, skip_layernorm_rows<3, true>}, {skip_layernorm_rows<4, false>, skip_layernorm_rows<4, true>},
+                                          {skip_layernorm_rows<5, false>, skip_layernorm_rows<5, true>}, {skip_layernorm_rows<6, false>, skip_layernorm_rows<6, true>},
+                                          {skip_layernorm_rows<7, false>, skip_layernorm_rows<7, true>}, {skip_layernorm_rows<8, false>, skip_layernorm_rows<8, true>}};
+        const int ch = size / 256;
+        const dim3 grid(std::min((warps_needed + 7) / 8, sm_count() * row_blocks(ch)));
+        launch_pdl(rows[ch - 1][s != nullptr], grid, dim3(256), 0, st, x, s, g, b, num);
     } else if (vec) {
         const int ch = (size / 8 + 31) / 32;
         switch (ch) {
@@ -295,7 +304,7 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
             case 6: launch_pdl(skip_layernorm_vec<6>, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size); break;
             default: launch_pdl(skip_layernorm_vec<8>, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size); break;
         }
-    } else if (size % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
+    } else if (pairs) {
         launch_pdl(skip_layernorm_pairs, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size);
     } else {
         launch_pdl(skip_layernorm_generic, dim3(blocks), dim3(256), 0, st, x, s, g, b, num, size);

@@ -593,7 +593,7 @@ def native_configs(torch, et, stream, pk):
     g = torch.ones(dm, dtype=torch.float16, device="cuda"); be = torch.zeros(dm, dtype=torch.float16, device="cuda")
     ln_ms = time_loop(torch, lambda: et.skip_layernorm(a, b, g, be, stream=stream), 20, 3, stream)
     gbs = 6.0 * dm * rows / (ln_ms * 1e-3) / 1e9
-    out["roofline_layernorm"] = {"kernel": "skip_layernorm_vec", "bound": "hbm", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
+    out["roofline_layernorm"] = {"kernel": "skip_layernorm_rows", "bound": "hbm", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
                                  "frac": gbs / pk["hbm_gbs"], "rows": rows, "size": dm, "bytes_per_row": 6 * dm}
     del a, b
     nmat, L = 16 * 64, 512

@@ -30,8 +30,10 @@
 // An additive mask is added to the scores as score + 8 x mask, one mixed-precision multiply-add per element (8 is 1 / scale). It comes
 // by TMA where the rows allow it, otherwise two warps copy granules; with an SM per item two blocks' masks are held. Before, the
 // softmax warps copied it and spent 3400 of 7700 clocks of a block on it: 1 x 384 tokens 14.1 -> 9.1 us, 1 x 701 (16 heads, rows
-// anywhere) 25.7 -> 20.5, 1 x 600 with compact V 28.9 -> 20.8, 64 x 384 116 -> 112, 64 x 383 121 -> 117.
-// Measured (12 heads): 64 ragged sequences of 32..512 tokens 49 us, 64 x 512 84, 256 x 128 in a ragged call 46 (64 before the sort).
+// anywhere) 25.7 -> 20.5, 1 x 600 with compact V 28.9 -> 20.8, 64 x 384 116 -> 112, 64 x 383 121 -> 117. Both ways and both numbers
+// of places are branches of one kernel, which spills 120 to 128 bytes for it (12 to 24 before).
+// Measured (12 heads), operands in L2: 64 ragged sequences of 32..512 tokens 49 us, 64 x 512 84, 256 x 128 in a ragged call 46 (64
+// before the sort); with operands from memory the ragged ones take 54.
 // Column-pruned operands come in two forms. kScatterV (the operator): V is compact, a head's columns start anywhere, results go
 // to their original columns with zeros between. kCompact (the encoder layers, which lay their weights out for it): every head's
 // columns of Q, K and V start at a multiple of 16 and are padded to one with zeros, so that Q K^T takes width / 16 steps, P V
@@ -102,8 +104,8 @@ template <bool kMask, int kForm>
 struct Cfg {
     static constexpr bool kPruneV = kForm == kScatterV;
     // The operator with compact V replaced a kernel that takes every exponential on the special-function unit, relative to the
-    // row's true maximum (the largest P is then exactly 1); it keeps that, as its results would be further from exact ones
-    // otherwise (up to 1.12 times with a mask and 1000 tokens). The other forms replaced packed fp16 exponentials, three times as far off.
+    // row's true maximum (the largest P is then 1, but for the fp32 rounding of that maximum); it keeps that, as its results would be
+    // further from exact ones otherwise (up to 1.12 times with a mask and 1000 tokens). The other forms replaced packed fp16 exponentials, three times as far off.
     static constexpr int kPolyPairs = kPruneV ? 0 : et::kPolyPairs;
     static constexpr float kRescaleStep = kPruneV ? 0.f : et::kRescaleStep;
     static constexpr int kQS = (kMask || kPruneV) ? 1 : 2;
@@ -198,7 +200,7 @@ __device__ __forceinline__ bool clc_query(const uint4* answer, int& x) {
 // Sorts a ragged batch by key blocks, the longest first (whole warp; sequences of one class keep their order): what is left when CTAs
 // run out of items are then short ones, and an item is found without reading memory. In the caller's order, with two rounds of loads per
 // item, the CTAs of 64 sequences of 32..512 tokens, 12 heads, finished between 43 and 52.5 us, and 256 x 128 tokens waited for items:
-// 51.7 -> 49.4 and 64 -> 46 us. It takes ~1 us before the first item, so only batches that outlast one wave of CTAs are sorted (16 x 128
+// 51.7 -> 49.4 and 64 -> 46 us with operands in L2 (55.7 -> 53.9 from memory). It takes ~1 us before the first item, so only batches that outlast one wave of CTAs are sorted (16 x 128
 // tokens would take 7.7 us instead of 6.1).
 __device__ __forceinline__ void sort_sequences(const TcParams& p, SeqTable* t, int lane) {
     if (lane <= kLenClasses) t->class_at[lane] = 0;

@@ -579,7 +579,8 @@ static double dense_cost(int tokens, int N, int K, int bn, int split) {
     const int tiles = std::max(1, (tokens + kBM - 1) / kBM) * tiles_n;
     const double panel = std::max({2.0 * bn, (kAPanel + bn * 128.0) / 58.0, 200.0});
     const int waves = (tiles * split + split_capacity(split) - 1) / split_capacity(split);
-    const double full = tiles * split > 132 ? 1500.0 : tiles * split > 100 ? 300.0 : 0.0;   // clusters on nearly all SMs: the last ones start late
+    // clusters on nearly all SMs: the last ones start late
+    const double full = tiles * split > sm_count() - 16 ? 1500.0 : tiles * split > sm_count() - 48 ? 300.0 : 0.0;
     return 5500.0 + full + waves * (3500.0 + ((panels + split - 1) / split) * panel + bn * 45.0);
 }
 

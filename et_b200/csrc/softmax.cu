@@ -23,7 +23,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 // group has many). Bound by HBM for rows above ~256
 // elements, by instruction issue below (~60 per granule: two fp32 operations per instruction, 32-bit index arithmetic).
 // Measured with a mask: 1024 matrices of 512 x 512 229 -> 173 us (6.2 TB/s; 64-bit modulo and scalar fp32 before), 128 of
-// 500 x 500 101 us (three passes, 2-byte accesses) -> 30 us.
+// 500 x 500 101 us (three passes, 2-byte accesses) -> 32 us.
 template <int G>
 __device__ __forceinline__ float group_max(float v) {
     if constexpr (G == 32) {
@@ -307,7 +307,7 @@ struct RowWalk {
 // fetched, shifted and put in place once for all matrices of its class, and added by mixed-precision additions. What bounds it is the
 // memory system at that size (aligned rows of 504 elements take 25.6 us, 128 matrices) and D times the registers; the kernel above, with
 // the next row requested when one is done, is the faster one where a group has few rows or a mask row few matrices.
-// 128 x 500 x 500 with a mask 33.6 -> 30.6 us, without 33.3 -> 27.8; 1024 x 500 x 500 with one 246 -> 212; 512 x 77 x 77 10.3 -> 8.7.
+// 128 x 500 x 500 with a mask 32.1 -> 29.5 us (from memory), without 33.3 -> 27.8; 1024 x 500 x 500 with one 246 -> 212; 512 x 77 x 77 10.3 -> 8.7.
 template <int G, int CH, int D, bool kMask>
 __global__ void __launch_bounds__(256, kManyBlocks) softmax_many_kernel(half* __restrict__ scores, const half* __restrict__ mask, int nmat, int L,
                                                                             int valid, unsigned rows) {

@@ -330,14 +330,17 @@ def test_dense_weights_run_alike_whatever_count_they_were_made_for(et, orc, K, N
         w.check()
 
 
-@pytest.mark.parametrize("T,K,N,gelu", [(1, 3072, 16, False), (64, 4096, 48, True), (130, 1024, 784, False), (257, 3072, 1040, True), (400, 2048, 272, False),
-                                        (128, 768, 768, True), (700, 3072, 768, False)])
-def test_dense_shares_meet_at_every_width(et, orc, T, K, N, gelu):
+@pytest.mark.parametrize("T,K,N,gelu,columns", [(1, 3072, 16, False, 4), (64, 4096, 48, True, 4), (130, 1024, 784, False, 16), (257, 3072, 1040, True, 24),
+                                                (400, 2048, 272, False, 12), (128, 768, 768, True, 8), (700, 3072, 768, False, 32),
+                                                (855, 3072, 784, True, 48), (916, 4096, 1024, False, 64)])
+def test_dense_shares_meet_at_every_width(et, orc, T, K, N, gelu, columns):
     """The K range in shares over a cluster: widths of 4 to 64 columns per CTA, outputs that begin between two sectors, and results
     that are not finite (found per column group and computed again)."""
-    rp, ro, data, bias = util.make_tile_linear(orc, K, N, 0.5, T + N, bernoulli=True, bias_std=0.1)
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, 0.5 if columns < 48 else 0.1, T + N, bernoulli=True, bias_std=0.1)
     X = util.activations(T, (T, K))
     w = et.TileWeight(K, N, T, data, rp, ro, bias, is_gelu=gelu)
+    info = w.info()
+    assert info["stage_bytes"] == 0 and info["stages"] > 1 and 16 * info["nb"] // info["stages"] == columns, info
     x = dev(X)
     buf = torch.full((T * N + 24,), 7.0, dtype=torch.float16, device="cuda")
     y = buf[8:8 + T * N].view(T, N)

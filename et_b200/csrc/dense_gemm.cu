@@ -52,6 +52,7 @@ constexpr int kMaxBN = 256;
 
 struct DenseParams {
     const half* bias;
+    bool bias_given;        // the caller's, not the weight's own: the preceding kernel may still be writing it
     half* Y;
     int T, N, K, k_panels, tiles_n, tiles, bn, stages, panels;   // panels: per stage; the last stage of a K range may hold fewer
     int* err;
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
         uint8_t* const buf = epi + (size_t)w * kUnitBytes;
         const int units = bn / kUnitCols;
         bool ok = true;
-        pdl_wait();   // the bias may be the caller's and the preceding kernel's result
+        if (p.bias_given) pdl_wait();
         for (int tl = 0; tl < my_tiles; ++tl) {
             const int tile = pair + tl * G;
             const int m0 = (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM + q * 32, n0 = (tile % p.tiles_n) * bn;
@@ -608,7 +609,7 @@ int dense_map_weight(DenseWeight* w) {
     return ET_OK;
 }
 
-int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int gelu, int* err, cudaStream_t st) {
+int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* X, const half* bias, bool bias_given, int T, int gelu, int* err, cudaStream_t st) {
     const int N = w.N, K = w.K;
     const int box = (int)(std::find(kBoxRows, kBoxRows + 6, plan.split > 1 ? plan.bn : plan.bn / 2) - kBoxRows);
     if (box == 6) return fail(ET_ERR_INVALID, "dense linear: no such tile width");
@@ -634,7 +635,7 @@ int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* 
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "dense linear: shared memory opt-in");
     DenseParams p;
-    p.bias = bias; p.Y = Y; p.T = T; p.N = N; p.K = K; p.bn = plan.bn;
+    p.bias = bias; p.bias_given = bias_given; p.Y = Y; p.T = T; p.N = N; p.K = K; p.bn = plan.bn;
     p.X = X; p.W = w.W; p.kept = w.kept;
     p.k_panels = (K + kBK - 1) / kBK;
     p.tiles_n = (N + plan.bn - 1) / plan.bn;

@@ -23,6 +23,7 @@ struct DenseWeight {
     CUtensorMap maps[6];   // one per number of weight rows that a CTA may copy at once
 };
 int dense_map_weight(DenseWeight* w);   // fills in the maps
-int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* X, const half* bias, int T, int gelu, int* err, cudaStream_t st);
+// bias_given: the bias is the caller's and may be the result of the kernel before.
+int dense_run(const DenseWeight& w, const DensePlan& plan, half* Y, const half* X, const half* bias, bool bias_given, int T, int gelu, int* err, cudaStream_t st);
 
 }  // namespace et

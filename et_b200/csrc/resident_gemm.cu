@@ -57,6 +57,7 @@ struct ResidentParams {
     const uint2* dir;         // [group][part]: {offset, size} in 16-byte units
     const uint8_t* stream;
     const half* bias;
+    bool bias_given;          // the caller's, not the weight's own: the preceding kernel may still be writing it
     const uint8_t* empty;     // per group, a bit per block-row without tiles; null when there is none
     int T, N, K, groups, parts, ranges, items, slabs;
     int nx, nw, block_bytes;   // nw: weight slots per set
@@ -303,7 +304,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
         uint8_t* const buf = epi + (size_t)e * kUnitBytes;
         bool ok = true;
         uint32_t gs = 0;
-        pdl_wait();   // the bias may be the caller's and the preceding kernel's result
+        // (the weight's own bias is read without waiting: 4808 x 768 -> 2304 at 90 % 12.68 us, 12.83 with the wait)
+        if (p.bias_given) pdl_wait();
         for (int item = blockIdx.x; item < p.items && ok; item += G) {
             const int r = item % p.ranges;
             const int g0 = r * p.groups / p.ranges, g1 = (r + 1) * p.groups / p.ranges;
@@ -487,7 +489,7 @@ void resident_free(ResidentWeight* w) {
 
 size_t resident_bytes(const ResidentWeight* w) { return w->bytes; }
 
-int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bias, int T, int gelu, int* err, cudaStream_t st) {
+int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bias, bool bias_given, int T, int gelu, int* err, cudaStream_t st) {
     CUtensorMap tm, tmy;
     if (!make_tmap_panels_f16(&tm, X, (uint64_t)T, (uint64_t)w->K, (uint64_t)w->K, kSlab, 2) ||
         !make_tmap_2d_f16(&tmy, Y, (uint64_t)T, (uint64_t)w->N, (uint64_t)w->N, 32, 32, 64))
@@ -504,7 +506,7 @@ int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bi
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "resident linear: shared memory opt-in");
     ResidentParams p;
-    p.dir = w->d_dir; p.stream = w->d_stream; p.bias = bias; p.empty = w->d_empty;
+    p.dir = w->d_dir; p.stream = w->d_stream; p.bias = bias; p.bias_given = bias_given; p.empty = w->d_empty;
     p.T = T; p.N = w->N; p.K = w->K; p.groups = w->groups; p.parts = w->parts;
     p.slabs = (T + kSlab - 1) / kSlab;
     launch_clocks(p.slabs, w->groups, w->K, w->group_clocks, &p.ranges);

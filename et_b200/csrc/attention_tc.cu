@@ -29,8 +29,8 @@
 // longest first (sort_sequences).
 // An additive mask is added to the scores as score + 8 x mask, one mixed-precision multiply-add per element (8 is 1 / scale). It comes
 // by TMA where the rows allow it, otherwise two warps copy granules; with an SM per item two blocks' masks are held. Before, the
-// softmax warps copied it and spent 3400 of 7700 clocks of a block on it: 1 x 384 tokens 14.1 -> 9.1 us, 1 x 701 (16 heads, rows
-// anywhere) 25.7 -> 20.5, 1 x 600 with compact V 28.9 -> 20.8, 64 x 384 116 -> 112, 64 x 383 121 -> 117. Both ways and both numbers
+// softmax warps copied it and spent 3400 of 7700 clocks of a block on it: 1 x 384 tokens 14.0 -> 9.4 us, 1 x 701 (16 heads, rows
+// anywhere) 26.7 -> 21.5, 1 x 600 with compact V 28.9 -> 20.8, 64 x 384 116 -> 79 (111 in a ragged call), 64 x 383 120 -> 114. Both ways and both numbers
 // of places are branches of one kernel, which spills 120 to 128 bytes for it (12 to 24 before).
 // Measured (12 heads), operands in L2: 64 ragged sequences of 32..512 tokens 49 us, 64 x 512 84, 256 x 128 in a ragged call 46 (64
 // before the sort); with operands from memory the ragged ones take 54.

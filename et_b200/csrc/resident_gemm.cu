@@ -19,7 +19,8 @@
 // run apart: while one accumulator is handed over and drained, the other set issues. One elected lane issues a block's UMMAs in one go;
 // each takes a warp ~120 clocks here (~20 in a kernel that does nothing else; 110 without the converting warps' stores).
 // As single predicated instructions, with the block's header known to one lane at a time, they took ~145: 17771 x 768 -> 2304 at 75 % 32.8 -> 31.9 us,
-// -> 3072 + GELU 44.7 -> 44.0, 8192 x 768 -> 2304 at 50 % 26.0 -> 25.3. A CTA takes (slab, range of features) items; the number of ranges is
+// -> 3072 + GELU 44.7 -> 44.0, 8192 x 768 -> 2304 at 50 % 26.0 -> 25.3. Those that read from shared memory in the same region:
+// 65536 x 1024 -> 3072 at 90 % 161.9 -> 157.4. A CTA takes (slab, range of features) items; the number of ranges is
 // chosen at the launch so that the last wave is full.
 // Every mbarrier wait is bounded; a role that gives up records a code and all threads meet at the common exit.
 #include <algorithm>
@@ -260,8 +261,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
                         accumulate = 1;
                     };
                     if (ready == chunks) {
-                        // the tiles whose activations are in tensor memory, by one lane in one go
-                        if (leader && nts > 0) {
+                        // by one lane in one go: the tiles whose activations are in tensor memory, then those that read them from shared memory
+                        if (leader && nall > 0) {
                             auto ts = [&](int i, uint32_t k, uint32_t acc) { umma_f16_ts(d, tmem + k * 8u, bd + (uint64_t)(i * 32), idesc, acc); };
                             uint32_t acc = accumulate;
                             int i = 0;
@@ -279,11 +280,17 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
                                 ts(i, k4 & 0xffu, acc);
                                 if (i + 1 < nts) ts(i + 1, (k4 >> 8) & 0xffu, 1u);
                                 if (i + 2 < nts) ts(i + 2, (k4 >> 16) & 0xffu, 1u);
+                                acc = 1;
+                            }
+#pragma unroll 1
+                            for (i = nts; i < nall; ++i) {
+                                const uint32_t t = list[i] - kTmemSlices;
+                                umma_f16(d, t_desc0 + (uint64_t)(((t >> 2) * kPanelBytes + (t & 3) * 32) >> 4), bd + (uint64_t)(i * 32), idesc, acc);
+                                acc = 1;
                             }
                         }
                         __syncwarp();
-                        if (nts > 0) accumulate = 1;
-                        for (int i = nts; i < nall; ++i) issue_one(i);
+                        if (nall > 0) accumulate = 1;
                     } else {
                         int i = 0;
                         for (const int c1 = (part + 1) * chunks / p.parts; ready < c1; ++ready) {

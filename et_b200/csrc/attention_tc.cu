@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 for (int c = 0; c < 4; ++c) {
                     uint32_t r[16];
                     tmem_ld16(o_addr + c * 16, r);
-                    tmem_ld_wait();
+                    tmem_ld_wait(r);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const int k = c * 16 + i - it.v_off;
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     if (kForm == kCompact && 16 * c >= it.v_n) break;   // the same for the whole CTA
                     uint32_t r[16];
                     tmem_ld16(o_addr + c * 16, r);
-                    tmem_ld_wait();
+                    tmem_ld_wait(r);
                     if (in) {
                         uint32_t ow[8];
 #pragma unroll
@@ -818,7 +818,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     float v[2][32];
                     tmem_ld32(s_addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(v[0]));
                     tmem_ld32(s_addr + c * 32 + 32, reinterpret_cast<uint32_t(&)[32]>(v[1]));
-                    tmem_ld_wait();
+                    tmem_ld_wait(v[0], v[1]);
                     if constexpr (kMask) {
                         // scale x score + mask = scale x (score + mask x 8): eight is 1 / scale, and the product with it exact
                         auto add_mask = [&](float& score, uint32_t two, bool high) {
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                     for (int c = 0; c < 4; ++c) {
                         uint32_t o[16];
                         tmem_ld16(o_addr + c * 16, o);
-                        tmem_ld_wait();
+                        tmem_ld_wait(o);
 #pragma unroll
                         for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
                         tmem_st16(o_addr + c * 16, o);
@@ -931,22 +931,23 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) attention_tc_kernel(cons
                 {
                     float v[32], w[32];
                     tmem_ld32(s_addr, reinterpret_cast<uint32_t(&)[32]>(v));
+                    tmem_ld_wait(v);
+                    int c = 0;
 #pragma unroll 1
-                    for (int c = 0; c < chunks; c += 2) {
-                        tmem_ld_wait();
+                    for (;; c += 2) {
                         tmem_ld32(s_addr + c * 32 + 32, reinterpret_cast<uint32_t(&)[32]>(w));
                         chunk(v, c);
-                        tmem_ld_wait();
-                        if (c + 2 < chunks) {
-                            tmem_ld32(s_addr + c * 32 + 64, reinterpret_cast<uint32_t(&)[32]>(v));
-                        } else {   // the next block's scores may be written
-                            tc_fence_before();
-                            __syncwarp();
-                            if (elect_one()) mbar_arrive(&sh->s_free);
-                            __syncwarp();
-                        }
+                        tmem_ld_wait(w);
+                        if (c + 2 == chunks) break;
+                        tmem_ld32(s_addr + c * 32 + 64, reinterpret_cast<uint32_t(&)[32]>(v));
                         chunk(w, c + 1);
+                        tmem_ld_wait(v);
                     }
+                    tc_fence_before();   // the next block's scores may be written
+                    __syncwarp();
+                    if (elect_one()) mbar_arrive(&sh->s_free);
+                    __syncwarp();
+                    chunk(w, c + 1);
                 }
                 tmem_st_wait();
                 tc_fence_before();

@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
             for (int u = h; u < units; u += kEpiWarps / 4) {
                 uint32_t acc[32];
                 tmem_ld32(tmem + a * bn + lane_base + u * kUnitCols, acc);
-                tmem_ld_wait();
+                tmem_ld_wait(acc);
                 if (u + kEpiWarps / 4 >= units) accumulator_read();   // this warp's share: it may be overwritten
                 uint4 ov[4];
                 epi_convert<kGelu>(acc, sh->bias[a] + u * kUnitCols, true, ov);
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     for (int c = h * 16; c < bn; c += 32) {
         uint32_t r[16];
         tmem_ld16(acc + c, r);
-        tmem_ld_wait();
+        tmem_ld_wait(r);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int dst = (c + 4 * i) / own_cols, g = (c + 4 * i - dst * own_cols) / 4;
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     for (int c = h * 16; c + 16 <= own_cols; c += 32) {
         uint32_t own[16], out[8];
         tmem_ld16(acc + rank * own_cols + c, own);
-        tmem_ld_wait();
+        tmem_ld_wait(own);
 #pragma unroll
         for (int i = 0; i < 4; ++i) finish(own + 4 * i, c + 4 * i, out + 2 * i);
         if (wide && c + 16 <= left) {   // a whole sector
@@ -533,11 +533,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     }
     for (int c = own_cols / 16 * 16 + h * 4; c < own_cols; c += 8) {
         uint32_t own[4], out[2];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(own[0]), "=r"(own[1]), "=r"(own[2]), "=r"(own[3])
-                     : "r"(acc + rank * own_cols + c)
-                     : "memory");
-        tmem_ld_wait();
+        tmem_ld4(acc + rank * own_cols + c, own);
+        tmem_ld_wait(own);
         finish(own, c, out);
         if (c < left) {
             *reinterpret_cast<uint2*>(y + c) = make_uint2(out[0], out[1]);

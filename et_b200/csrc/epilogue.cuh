@@ -26,9 +26,11 @@ __device__ __forceinline__ half2 gelu_tanh_h2(half2 x) {
 __device__ __forceinline__ void epi_load(uint32_t taddr, bool two, uint32_t (&acc)[32]) {
     if (two) {
         tmem_ld32(taddr, acc);
+        tmem_ld_wait(acc);
     } else {
         uint32_t lo[16];
         tmem_ld16(taddr, lo);
+        tmem_ld_wait(lo);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             acc[i] = lo[i];

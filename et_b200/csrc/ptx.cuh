@@ -178,8 +178,28 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() {
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Waits for the thread's loads from tensor memory. Until then their registers hold nothing yet, which the compiler does not know:
+// it could compute with them, or move them to other registers, ahead of the wait. So the arrays that have been loaded are named
+// here, and to the compiler they get their values behind the wait. (As operands of the wait itself they could be moved ahead of it.)
+// Between a load and its wait there is straight code only: where paths meet, registers are moved too.
+__device__ __forceinline__ void tmem_arrived(uint32_t& r) { asm volatile("" : "+r"(r)); }
+__device__ __forceinline__ void tmem_arrived(float& r) { asm volatile("" : "+f"(r)); }
+template <typename T, int N>
+__device__ __forceinline__ void tmem_arrived(T (&r)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) tmem_arrived(r[i]);
+}
+template <typename... Arrays>
+__device__ __forceinline__ void tmem_ld_wait(Arrays&... loaded) {
+    static_assert(sizeof...(loaded) > 0, "what has been loaded");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    (tmem_arrived(loaded), ...);
 }
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

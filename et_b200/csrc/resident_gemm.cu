@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
                 if (item + G >= p.items && g + 2 >= g1) pdl_launch_dependents();   // the next kernel's set-up overlaps the last stores
                 uint32_t acc[32];
                 tmem_ld32(src, acc);
-                tmem_ld_wait();
+                tmem_ld_wait(acc);
                 tc_fence_before();
                 __syncwarp();
                 if (elect_one()) mbar_arrive(&sh->acc_empty[set]);

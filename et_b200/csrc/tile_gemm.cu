@@ -595,8 +595,6 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 }
                 for (int u = h; u < units && ok; u += kEpiPerQuarter) {
                     const bool two = u * 2 + 1 < p.nb;
-                    uint32_t acc[32];
-                    epi_load(tmem + lane_base + u * 32, two, acc);
                     uint32_t rcur[16];
                     if constexpr (kMode >= 2) {
 #pragma unroll
@@ -604,7 +602,8 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                         if (u + kEpiPerQuarter < units)
                             resid_load(rnext, p.fz.resid, p.N, col0 + (u + kEpiPerQuarter) * kUnitCols, row, row_ok);
                     }
-                    tmem_ld_wait();
+                    uint32_t acc[32];
+                    epi_load(tmem + lane_base + u * 32, two, acc);
                     if (more) {   // clear what was just read, for the next tile
                         tmem_st16_zero(tmem + lane_base + u * 32);
                         if (two) tmem_st16_zero(tmem + lane_base + u * 32 + 16);

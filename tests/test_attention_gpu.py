@@ -306,6 +306,34 @@ def test_attention_keys_that_are_not_numbers_reach_every_query(et, orc, mask, pr
     assert not lost, lost
 
 
+@pytest.mark.parametrize("layout,H", [("padded", 2), ("packed", 1), ("packed", 5)])
+def test_attention_keys_beyond_the_end_of_every_remainder(et, orc, layout, H):
+    """Valid keys up to every place of a block, and keys that are large or not finite right behind them in memory: the padding's,
+    or the next sequence's (with five heads in more items than places, longest first). They count for nothing."""
+    d = 64 * H
+    poison = np.array([np.nan, np.inf, -np.inf, 60000.0, -60000.0], dtype=np.float16)
+    if layout == "padded":
+        S, valid = 256, list(range(1, 257))
+        T = S * len(valid)
+        behind = np.concatenate([np.arange(b * S + v, (b + 1) * S) for b, v in enumerate(valid)])
+        lens, kw = [S] * len(valid), dict(uniform_len=S, valid_lens=dev(np.array(valid, dtype=np.int32)))
+    else:
+        valid = lens = [n for i in range(1, 129) for n in (i, 1)]   # every other sequence is a token whose key is not finite
+        T = sum(lens)
+        starts = np.concatenate([[0], np.cumsum(lens)])
+        behind = starts[1:-1:2]
+        kw = dict(cu_seqlens=dev(starts.astype(np.int32)), max_seq_len=128)
+    Q, K, V = _qkv(T, T, d)
+    want = orc.attention(Q, K, V, lens, d, H, valid_lens=valid)
+    K[behind] = poison[(np.arange(len(behind))[:, None] + np.arange(d)[None, :]) % len(poison)]
+    out = torch.full((T, d), float("nan"), dtype=torch.float16, device="cuda")
+    et.attention_batch(out, dev(Q), dev(K), dev(V), d, H, batch=len(lens), **kw)
+    torch.cuda.synchronize()
+    et.attention_check()
+    rows = np.arange(T) if layout == "padded" else np.setdiff1d(np.arange(T), np.concatenate([behind, starts[-2:-1]]))
+    util.assert_close(host(out)[rows], want[rows], what=f"{layout}, every remainder")
+
+
 @pytest.mark.parametrize("L", [40, 128, 200])
 def test_attention_many_items_per_cta_repeat_exactly(et, orc, L):
     """Items of one or two key blocks taken over one after the other, so that the next item's first block is often, but not

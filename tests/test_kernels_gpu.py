@@ -320,6 +320,22 @@ def test_long_dense_launches_have_no_columns_to_fill_up(et, orc, N, tokens):
     assert info["nb"] * 16 * info["n_chunks"] == N
 
 
+@pytest.mark.parametrize("T,N", [(24000, 576), (23933, 592)])
+def test_long_dense_launches_against_the_oracle(et, orc, T, N):
+    """Three tiles of 192 columns, and four of which the last is nearly empty: first and last tokens, those on both sides of a
+    CTA's and of a pair's last one, and bits that do not depend on the launch."""
+    rp, ro, data, bias = util.make_tile_linear(orc, 768, N, 0.0, N, True, 0.05)
+    w = et.TileWeight(768, N, T, data, rp, ro, bias)
+    X = util.activations(T, (T, 768))
+    ys = [w.run(torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda"), dev(X)) for _ in range(2)]
+    torch.cuda.synchronize()
+    w.check()
+    assert torch.equal(ys[0], ys[1]) and torch.isfinite(ys[0]).all()
+    for first in (0, 120, 12150, T - 140):
+        rows = slice(first, first + 140)
+        util.assert_close(host(ys[0][rows]), orc.tile_linear(X[rows], rp, ro, data, bias, N), what=f"tokens from {first}")
+
+
 @pytest.mark.parametrize("K,N", [(3072, 768), (4096, 1040)])
 def test_dense_weights_run_alike_whatever_count_they_were_made_for(et, orc, K, N):
     """How a dense weight is cut into tiles and shares of the K range is chosen for the tokens of the call: the same bits from

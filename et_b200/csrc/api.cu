@@ -73,6 +73,16 @@ extern "C" int et_set_attention_scores_fp32(int on) {
 }
 extern "C" int et_attention_scores_fp32(void) { return et::attention_tc_scores_fp32(); }
 
+// Not part of the public header: the blocks that a weight is packed in, for a test of their layout that needs no GPU.
+extern "C" size_t et_debug_tile_blocks(int in_feat, int out_feat, int ntile, const void* data, const int* row_ptr, const int* row_offset, int block_rows,
+                                       uint32_t* dir, uint8_t* stream, size_t room) {
+    et::TileWeight* w = nullptr;
+    if (et::tile_weight_pack(&w, in_feat, out_feat, 128, ntile, static_cast<const half*>(data), row_ptr, row_offset, nullptr, block_rows, true)) return 0;
+    const size_t bytes = et::tile_weight_blocks(w, dir, stream, room);
+    et::tile_weight_free(w);
+    return bytes;
+}
+
 // Not part of the public header: used by profiling builds of the library only.
 extern "C" int et_debug_set_gemm_profile_buffer(void* dev_buf) {
     et::tile_gemm_set_profile_buffer(static_cast<long long*>(dev_buf));

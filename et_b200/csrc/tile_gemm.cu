@@ -72,8 +72,8 @@ constexpr int kUnitCols = 32;          // columns per epilogue store
 constexpr int kUnitBytes = 32 * kUnitCols * 2;   // one warp's staging buffer: 32 rows x 32 columns
 constexpr int kPanelBytes = kSlab * kPanel * 2;   // 16 KB
 constexpr int kXStageBytes = kSlab * kKC * 2;     // 32 KB
-// A weight block: a header {per issuing warp: first tile, count; 16-byte units of all lists; per issuing warp: unit at which its list
-// starts}, the lists (columns of A in its slot, and of D << 16, of each tile), the tiles.
+// A weight block: a header {per issuing warp: first tile, count; 16-byte units of all lists; per issuing warp: unit of the block at which
+// its list starts}, the lists (columns of A in its slot, and of D << 16, of each tile), the tiles.
 constexpr int kHeaderBytes = 64;
 constexpr int kListAt = 4 * kIssuers + 4;
 constexpr int kSmemMax = 232448;    // 227 KB: the per-CTA opt-in limit of sm_100
@@ -504,7 +504,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                         const uint8_t* const blk = wring + sh->w_at[ws];
                         const uint32_t hw = reinterpret_cast<const uint32_t*>(blk)[w];
                         const int ne = hw >> 16;
-                        const uint4* const list = reinterpret_cast<const uint4*>(blk + kHeaderBytes) + reinterpret_cast<const uint16_t*>(blk + kListAt)[w];
+                        const uint4* const list = reinterpret_cast<const uint4*>(blk) + reinterpret_cast<const uint16_t*>(blk + kListAt)[w];
                         const uint32_t units = reinterpret_cast<const uint32_t*>(blk)[8];
                         const uint32_t tile16 = ((smem_u32(blk) + kHeaderBytes) >> 4) + units + (hw & 0xffffu) * 32u;
                         const uint32_t abuf = tmem + a_col0 + a * kSlotCols;
@@ -512,7 +512,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                             umma_f16_ts(tmem + (e >> 16), abuf + (e & 0xffffu), b_desc0 | (uint64_t)((tile16 + i * 32) & 0x3fff), idesc, 1u);
                         };
                         // Short lists, which are most of those of up to 16 block-rows, without the loop (8192 x 4096 -> 1024 at 80 %
-                        // 37.8 -> 37.0 us). An empty one may be followed by anything: its four entries are read, not used.
+                        // 37.8 -> 37.0 us). Of an empty one four entries are read too, and not used: it lies in the header, which has landed with the block.
                         if (ne <= 4) {
                             if (elect_one()) {
                                 const uint4 e = *list;
@@ -739,9 +739,8 @@ static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double densi
     return best_nb > 0 ? best_nb : std::min(8, std::max(n_block_rows, 1));
 }
 
-// The tile form on the device: issue lists and tiles as the kernel reads them.
-static int build_tile_form(TileWeight* w) {
-    if (w->d_stream) return ET_OK;
+// The blocks of the tile form as the kernel reads them, back to back, and where each of them lies.
+static int pack_tile_blocks(TileWeight* w, std::vector<uint2>& dir, std::vector<uint8_t>& stream) {
     const int NBR = w->N / 16;
     w->n_chunks = (NBR + w->nb - 1) / w->nb;
     w->k_chunks = (w->K + kKC - 1) / kKC;
@@ -758,8 +757,7 @@ static int build_tile_form(TileWeight* w) {
             buckets[((size_t)c * w->k_chunks + kc) * kIssuers + (lb % kIssuers)].push_back({i, sl, lb});
         }
     }
-    std::vector<uint2> dir(nblocks);
-    std::vector<uint8_t> stream;
+    dir.resize(nblocks);
     stream.reserve(nblocks * (kHeaderBytes + 16 * kIssuers) + (size_t)w->ntile * 516);   // (grown block by block, 1.7 MB took up to 2 ms)
     size_t max_block = 0;
     for (size_t b = 0; b < nblocks; ++b) {
@@ -780,7 +778,7 @@ static int build_tile_form(TileWeight* w) {
             std::stable_sort(v.begin(), v.end(), [](const Ent& a, const Ent& c) { return a.slice < c.slice; });
             if (e > 0xffff || v.size() > 0xffff) return fail(ET_ERR_UNSUPPORTED, "tile weight: block too large");
             hdr[wv] = e | ((uint32_t)v.size() << 16);
-            list_at[wv] = (uint16_t)at;
+            list_at[wv] = v.empty() ? 0 : (uint16_t)(kHeaderBytes / 16 + at);   // an empty list: the header itself
             for (size_t i = 0; i < v.size(); ++i) {
                 const Ent& t = v[i];
                 list[at * 4 + i] = (uint32_t)t.slice * 8u | ((uint32_t)t.lb * 16u << 16);
@@ -797,10 +795,20 @@ static int build_tile_form(TileWeight* w) {
         dir[b] = make_uint2((uint32_t)(off / 16), (uint32_t)(bytes / 16));
         max_block = std::max(max_block, bytes);
     }
-    for (int c = 0; c < w->n_chunks && c < kDirInParams; ++c) w->h_first.push_back(dir[(size_t)c * w->k_chunks]);
     w->stage_b_bytes = (int)((max_block + 1023) / 1024 * 1024);
+    return ET_OK;
+}
+
+// The tile form on the device.
+static int build_tile_form(TileWeight* w) {
+    if (w->d_stream) return ET_OK;
+    std::vector<uint2> dir;
+    std::vector<uint8_t> stream;
+    const int rc = pack_tile_blocks(w, dir, stream);
+    if (rc) return rc;
+    for (int c = 0; c < w->n_chunks && c < kDirInParams; ++c) w->h_first.push_back(dir[(size_t)c * w->k_chunks]);
     {
-        const RingShape rs = ring_shape(w->nb, w->stage_b_bytes, (double)stream.size() / nblocks);
+        const RingShape rs = ring_shape(w->nb, w->stage_b_bytes, (double)stream.size() / dir.size());
         w->nx = rs.nx; w->w_ring = rs.w_ring; w->w_room = rs.w_room; w->a_slots = rs.a_slots;
     }
     if (w->nx < 2 || w->a_slots < 1) return fail(ET_ERR_UNSUPPORTED, "tile weight: weight block exceeds shared memory");
@@ -972,6 +980,15 @@ void tile_weight_free(TileWeight* w) {
     cudaFree(w->d_dir); cudaFree(w->d_stream); cudaFree(w->d_small); cudaFree(w->d_colc); cudaFree(w->d_cold); cudaFree(w->d_dense);
     resident_free(w->resident);
     delete w;
+}
+
+size_t tile_weight_blocks(TileWeight* w, uint32_t* dir_out, uint8_t* stream_out, size_t room) {
+    std::vector<uint2> dir;
+    std::vector<uint8_t> stream;
+    if (pack_tile_blocks(w, dir, stream) || stream.size() > room) return 0;
+    std::memcpy(dir_out, dir.data(), dir.size() * sizeof(uint2));
+    std::memcpy(stream_out, stream.data(), stream.size());
+    return stream.size();
 }
 
 static long long* g_prof = nullptr;

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <cstddef>
+#include <cstdint>
 
 namespace et {
 
@@ -57,6 +59,9 @@ void tile_weight_info(const TileWeight* w, int* info6);
 int tile_spmm_raw(half* Y, const half* X, const int* row_ptr, const int* row_offset, const half* data,
                   int M, int N, int K, const half* bias, int gelu, cudaStream_t st);
 void tile_spmm_cache_clear();
+// The packed blocks of the tile form and their directory ({offset, size} in units of 16 bytes, by chunk of block-rows and chunk of K)
+// on the host; returns the bytes, 0 if they exceed `room`. `w` may be a part.
+size_t tile_weight_blocks(TileWeight* w, uint32_t* dir, uint8_t* stream, size_t room);
 // Profiling builds (-DET_GEMM_PROFILE): device buffer of >= 1024 clock64 stamps written by CTA (0,0).
 void tile_gemm_set_profile_buffer(long long* dev_buf);
 

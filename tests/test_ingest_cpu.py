@@ -1,5 +1,7 @@
 """Magnitude-based ingestion of dense weights into the two pruned formats, and the length-bucketing scheduler:
 host logic, checked against numpy restatements (no GPU)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -107,3 +109,40 @@ def test_bucket_argument_checks():
         scheduler.bucket_by_length([-1], 16)
     with pytest.raises(ValueError):
         scheduler.bucket_ceiling(5, 0)
+
+
+@pytest.mark.parametrize("K,N,block_rows,sparsity", [(768, 3072, 24, 0.9), (4096, 1024, 16, 0.8), (400, 48, 24, 0.5), (256, 640, 4, 0.97), (128, 16, 24, 1.0)])
+def test_tile_blocks_hold_their_lists_and_every_tile(K, N, block_rows, sparsity):
+    """The blocks of the tile form, read the way the kernel reads them: a warp takes its list four entries at a time, the first
+    four even of an empty list, and all of that lies in the block (what follows it in shared memory may be on its way there)."""
+    rp, ro = et.gen_sparse_tile_mat(N, K, sparsity, 7, True)
+    ntile = len(ro)
+    data = np.random.default_rng(8).integers(0, 65536, (ntile, 256)).astype(np.uint16)
+    chunks, kc = -(-N // 16 // min(block_rows, N // 16)), -(-K // 128)
+    dir_, stream = np.zeros((chunks, kc, 2), np.uint32), np.zeros(1 << 24, np.uint8)
+    f = et.lib().et_debug_tile_blocks
+    f.restype = ctypes.c_size_t
+    p = lambda a: ctypes.c_void_p(a.ctypes.data)
+    size = f(K, N, ntile, p(data), p(rp), p(ro), block_rows, p(dir_), p(stream), ctypes.c_size_t(stream.size))
+    assert size and (dir_[..., 0] + dir_[..., 1]).max() * 16 == size
+    found = {}
+    for c in range(chunks):
+        for k in range(kc):
+            at, units = (int(x) for x in dir_[c, k])
+            block = stream[at * 16:(at + units) * 16]
+            head, list_at = block[:36].view(np.uint32), block[36:52].view(np.uint16)
+            for w in range(8):
+                first, count = int(head[w]) & 0xffff, int(head[w]) >> 16
+                for i in range(0, max(count, 1), 4):
+                    assert (int(list_at[w]) + i // 4 + 1) * 16 <= len(block), (c, k, w)
+                entries = block[16 * int(list_at[w]):][:4 * count].view(np.uint32)
+                for i, e in enumerate(entries):
+                    a, d = int(e) & 0xffff, int(e) >> 16
+                    assert a % 8 == 0 and d % 16 == 0 and d // 16 % 8 == w
+                    tile = block[64 + 16 * int(head[8]) + 512 * (first + i):][:512]
+                    row, col = c * min(block_rows, N // 16) + d // 16, k * 128 + a // 8 * 16
+                    found.setdefault((row, col), []).append(tile.view(np.uint16).reshape(2, 2, 8, 8).transpose(0, 2, 1, 3).reshape(256))
+    assert sum(len(v) for v in found.values()) == ntile
+    for r in range(N // 16):
+        for i in range(rp[r], rp[r + 1]):
+            assert np.array_equal(found[r, int(ro[i])][0], data[i])

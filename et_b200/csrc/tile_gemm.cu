@@ -704,6 +704,25 @@ static RingShape ring_shape(int nb, int largest, double mean) {
     }
     return best;
 }
+// Bytes of a block whose lists have these numbers of entries.
+static size_t block_bytes(const int (&entries)[kIssuers]) {
+    size_t bytes = kHeaderBytes;
+    for (int n : entries) bytes += (size_t)(n + 3) / 4 * 16 + (size_t)n * 512;   // a list's entries fill whole units of four
+    return bytes;
+}
+// The fullest block with `nb` block-rows to a CTA.
+static size_t largest_block(const std::vector<int>& tiles, int n_block_rows, int k_chunks, int nb) {
+    size_t largest = 0;
+    for (int r0 = 0; r0 < n_block_rows; r0 += nb)
+        for (int kc = 0; kc < k_chunks; ++kc) {
+            int entries[kIssuers] = {};
+            for (int r = r0; r < std::min(r0 + nb, n_block_rows); ++r) entries[(r - r0) % kIssuers] += tiles[(size_t)r * k_chunks + kc];
+            largest = std::max(largest, block_bytes(entries));
+        }
+    return largest;
+}
+static int ring_room(size_t largest) { return (int)((largest + 1023) / 1024 * 1024); }
+static bool fits(size_t largest, int nb) { return largest < kSmemMax && ring_shape(nb, ring_room(largest), (double)largest).nx >= 2; }
 // Block-rows per CTA from a model of the persistent kernel: a chunk takes the ring period, or its UMMAs (~10
 // clocks each with eight issuing warps), or its share of L2 bandwidth (~64 bytes per clock per SM), whichever
 // is longest; a tile ends with an epilogue of ~350 clocks per 32 columns and warp.
@@ -714,7 +733,9 @@ static int g_goal = 0;
 constexpr int kThroughputTilesPerCta = 2;
 void tile_gemm_set_goal(int goal) { g_goal = goal == 1 ? 1 : 0; }
 
-static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double density, double* cost_out) {
+// `tiles`: of each block-row and chunk of K. The model knows only their mean; what a weight's fullest block takes decides whether the
+// rings fit at all (rows of a compact V among sparse ones of Q and K: 24 block-rows of every tile are 99 KB).
+static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double density, const std::vector<int>& tiles, double* cost_out) {
     const int slabs = std::max(1, (size_hint + kSlab - 1) / kSlab);
     const int sms = std::max(1, sm_count());
     double best = 0;
@@ -730,13 +751,13 @@ static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double densi
                                           tiles_per_chunk + 3.0 * std::sqrt(nbe * kSlices * density * (1.0 - density)));
         const int stage_b = (int)((kHeaderBytes + tiles_max * 528.0 + 1023) / 1024) * 1024;
         const RingShape rs = ring_shape(nbe, stage_b, kHeaderBytes + tiles_per_chunk * 528.0);
-        if (rs.nx < 2 || rs.a_slots < 1) continue;
-        const long tiles = (long)slabs * ((n_block_rows + nbe - 1) / nbe);
-        const double per_cta = (double)((tiles + sms - 1) / sms);
+        if (rs.nx < 2 || rs.a_slots < 1 || !fits(largest_block(tiles, n_block_rows, k_chunks, nbe), nbe)) continue;
+        const long ctas = (long)slabs * ((n_block_rows + nbe - 1) / nbe);
+        const double per_cta = (double)((ctas + sms - 1) / sms);
         const double t_chunk = std::max({rs.period, 10.0 * tiles_per_chunk,
                                          (kXStageBytes + tiles_per_chunk * 528.0) / 64.0});
         const double t_tile = k_chunks * t_chunk + 350.0 * ((nbe + 3) / 4) + 800.0;
-        const double cost = g_goal == 1 ? (double)tiles * t_tile : per_cta * t_tile + 3000.0;
+        const double cost = g_goal == 1 ? (double)ctas * t_tile : per_cta * t_tile + 3000.0;
         if (best_nb == 0 || cost < best * 0.999) { best = cost; best_nb = nbe; }
     }
     *cost_out = best_nb > 0 ? best : 1e30;
@@ -765,12 +786,13 @@ static int pack_tile_blocks(TileWeight* w, std::vector<uint2>& dir, std::vector<
     stream.reserve(nblocks * (kHeaderBytes + 16 * kIssuers) + (size_t)w->ntile * 516);   // (grown block by block, 1.7 MB took up to 2 ms)
     size_t max_block = 0;
     for (size_t b = 0; b < nblocks; ++b) {
-        uint32_t n_entries = 0;
-        for (int wv = 0; wv < kIssuers; ++wv) n_entries += (uint32_t)buckets[b * kIssuers + wv].size();
+        int entries[kIssuers];
         uint32_t units = 0;   // of lists: four entries to 16 bytes, each warp's starts with a unit of its own
-        for (int wv = 0; wv < kIssuers; ++wv) units += ((uint32_t)buckets[b * kIssuers + wv].size() + 3) / 4;
-        const size_t bytes = kHeaderBytes + (size_t)units * 16 + (size_t)n_entries * 512;
-        const size_t off = stream.size();
+        for (int wv = 0; wv < kIssuers; ++wv) {
+            entries[wv] = (int)buckets[b * kIssuers + wv].size();
+            units += (uint32_t)(entries[wv] + 3) / 4;
+        }
+        const size_t bytes = block_bytes(entries), off = stream.size();
         stream.resize(off + bytes, 0);
         uint32_t* hdr = reinterpret_cast<uint32_t*>(stream.data() + off);
         uint16_t* list_at = reinterpret_cast<uint16_t*>(stream.data() + off + kListAt);
@@ -799,7 +821,7 @@ static int pack_tile_blocks(TileWeight* w, std::vector<uint2>& dir, std::vector<
         dir[b] = make_uint2((uint32_t)(off / 16), (uint32_t)(bytes / 16));
         max_block = std::max(max_block, bytes);
     }
-    w->stage_b_bytes = (int)((max_block + 1023) / 1024 * 1024);
+    w->stage_b_bytes = ring_room(max_block);
     return ET_OK;
 }
 
@@ -877,7 +899,11 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     w->tiles_per_cta = g_goal == 1 ? kThroughputTilesPerCta : 1;
     const double density = (double)ntile / std::max(1.0, (double)NBR * (K / 16));
     double tile_cost = 0;
-    w->nb = choose_nb(NBR, (K + kKC - 1) / kKC, size_hint, density, &tile_cost);
+    const int k_chunks = (K + kKC - 1) / kKC;
+    std::vector<int> tiles((size_t)NBR * k_chunks, 0);
+    for (int r = 0; r < NBR; ++r)
+        for (int i = row_ptr[r]; i < row_ptr[r + 1]; ++i) ++tiles[(size_t)r * k_chunks + row_offset[i] / kKC];
+    w->nb = choose_nb(NBR, k_chunks, size_hint, density, tiles, &tile_cost);
     if (nb_override > 0) {
         const int nbo = std::min(nb_override, kMaxNB);
         w->nb = NBR <= nbo ? NBR : std::max(4, nbo / 4 * 4);

@@ -484,6 +484,28 @@ def test_tile_linear_lists_of_every_length(et, orc, T, gelu):
     util.assert_close(host(Y), orc.tile_linear(X, rp, ro, data, bias, N, gelu=gelu), what="lists of every length")
 
 
+@pytest.mark.parametrize("goal", ["latency", "throughput"])
+@pytest.mark.parametrize("T,K,sparse,full,sparsity", [(1665, 1024, 2048, 544, 0.75), (300, 1024, 2048, 544, 0.9), (1665, 4096, 512, 384, 0.8), (200, 2048, 16, 368, 0.5)])
+def test_tile_linear_of_sparse_and_full_block_rows(et, orc, T, K, sparse, full, sparsity, goal):
+    """Block-rows of every tile behind sparse ones, as where a compact V follows Q and K: the fullest block decides how many
+    block-rows a CTA takes, not the mean."""
+    rp, ro = orc.gen_sparse_tile_mat(sparse, K, sparsity, 3, True)
+    rp = np.concatenate([rp, rp[-1] + np.arange(1, full // 16 + 1) * (K // 16)]).astype(np.int32)
+    ro = np.concatenate([ro, np.tile(np.arange(0, K, 16), full // 16)]).astype(np.int32)
+    N = sparse + full
+    data, bias, X = util.weights(5, (len(ro), 256)), util.weights(6, (N,), 0.05), util.activations(7, (T, K))
+    et.set_tuning_goal(goal)
+    try:
+        w = et.TileWeight(K, N, T, data, rp, ro, bias)
+    finally:
+        et.set_tuning_goal("latency")
+    Y = w.run(torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda"), dev(X))
+    torch.cuda.synchronize()
+    w.check()
+    rows = slice(max(0, T - 140), T)
+    util.assert_close(host(Y)[rows], orc.tile_linear(X[rows], rp, ro, data, bias, N), what=f"{sparse} sparse and {full} full outputs {w.info()}")
+
+
 def test_tile_linear_pruned_tiles_do_not_contribute(et, orc):
     """Mask exactness: output equals the dense product with the pruned tiles zeroed, and does not
     change when garbage is placed where the pruned tiles would be."""

@@ -76,6 +76,7 @@ constexpr int kXStageBytes = kSlab * kKC * 2;     // 32 KB
 // its list starts}, the lists (columns of A in its slot, and of D << 16, of each tile), the tiles.
 constexpr int kHeaderBytes = 64;
 constexpr int kListAt = 4 * kIssuers + 4;
+constexpr double kTileBytes = 512 + 4;   // a tile and its entry
 constexpr int kSmemMax = 232448;    // 227 KB: the per-CTA opt-in limit of sm_100
 constexpr int kMaxKChunks = 256;    // in_feat up to 32768
 
@@ -725,7 +726,8 @@ static int ring_room(size_t largest) { return (int)((largest + 1023) / 1024 * 10
 static bool fits(size_t largest, int nb) { return largest < kSmemMax && ring_shape(nb, ring_room(largest), (double)largest).nx >= 2; }
 // Block-rows per CTA from a model of the persistent kernel: a chunk takes the ring period, or its UMMAs (~10
 // clocks each with eight issuing warps), or its share of L2 bandwidth (~64 bytes per clock per SM), whichever
-// is longest; a tile ends with an epilogue of ~350 clocks per 32 columns and warp.
+// is longest; a tile ends with an epilogue of ~350 clocks per 32 columns and warp. Against 5576 launches (96 to 131072 tokens, the eight shapes
+// of BERT-base and BERT-large layers, 25 to 90 % of the tiles pruned, 4 to 24 block-rows) the rms error of 1.3 times this is 10 %.
 // What the pack optimises: 0 = the duration of one launch on an otherwise idle GPU (tiles spread over as many SMs
 // as possible), 1 = SM time per launch (fewer, larger tiles: the right choice when several independent batches
 // are in flight on separate streams and keep all SMs busy anyway).
@@ -745,17 +747,16 @@ static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double densi
         const int nbe = n_block_rows <= nb ? std::max(n_block_rows, 1) : nb;
         if (nbe > kMaxNB) continue;
         const double tiles_per_chunk = nbe * kSlices * density;
-        // the largest block of a Bernoulli pattern: mean + 3 standard deviations (a tile and its entry count as 528 bytes, with which
-        // the model was fitted: 516 would take 24 instead of 16 block-rows for 32768 x 1024 -> 1024 at 80 %, 43.6 instead of 42.4 us)
+        // the largest block of a Bernoulli pattern: mean + 3 standard deviations
         const double tiles_max = std::min((double)nbe * kSlices,
                                           tiles_per_chunk + 3.0 * std::sqrt(nbe * kSlices * density * (1.0 - density)));
-        const int stage_b = (int)((kHeaderBytes + tiles_max * 528.0 + 1023) / 1024) * 1024;
-        const RingShape rs = ring_shape(nbe, stage_b, kHeaderBytes + tiles_per_chunk * 528.0);
+        const int stage_b = (int)((kHeaderBytes + tiles_max * kTileBytes + 1023) / 1024) * 1024;
+        const RingShape rs = ring_shape(nbe, stage_b, kHeaderBytes + tiles_per_chunk * kTileBytes);
         if (rs.nx < 2 || rs.a_slots < 1 || !fits(largest_block(tiles, n_block_rows, k_chunks, nbe), nbe)) continue;
         const long ctas = (long)slabs * ((n_block_rows + nbe - 1) / nbe);
         const double per_cta = (double)((ctas + sms - 1) / sms);
         const double t_chunk = std::max({rs.period, 10.0 * tiles_per_chunk,
-                                         (kXStageBytes + tiles_per_chunk * 528.0) / 64.0});
+                                         (kXStageBytes + tiles_per_chunk * kTileBytes) / 64.0});
         const double t_tile = k_chunks * t_chunk + 350.0 * ((nbe + 3) / 4) + 800.0;
         const double cost = g_goal == 1 ? (double)ctas * t_tile : per_cta * t_tile + 3000.0;
         if (best_nb == 0 || cost < best * 0.999) { best = cost; best_nb = nbe; }
@@ -918,10 +919,11 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
         return ET_OK;
     }
     w->dense = dense_plan(size_hint, N, K);
-    // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's, which
-    // was made to compare its own shapes only, is 1.3 times too short). At 75 % sparsity and 32768 tokens, in us, tile / resident /
-    // dense: 768 -> 2304 74 / 63 / 83, 3072 -> 768 75 / - / 107, 1024 -> 3072 109 / 167 / 132; without zeros 160 / - / 96.
-    // (1.08: where the first two come this close, the resident kernel was the faster one in seven of ten measured launches.)
+    // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
+    // 1.3 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 73 / 62 / 83, 3072 -> 768 77 / - / 106, 1024 ->
+    // 3072 111 / 152 / 129; at 50 % 1024 -> 4096 215 / 332 / 186. Both constants were measured over 984 linears (96 to 131072 tokens,
+    // eight shapes, six sparsities): the form taken is 0.60 % slower than the fastest in the mean; with 1.25 and 1.35 instead of 1.3 1.02 and
+    // 0.74 %, with 1.00, 1.04 and 1.12 instead of 1.08 (what the resident kernel's model overestimates) 0.69, 0.64 and 0.61 %.
     tile_cost = 1.3 * tile_cost + 1000.0;
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens

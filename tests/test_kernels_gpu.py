@@ -312,6 +312,16 @@ def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
+@pytest.mark.parametrize("T,K,N,sparsity,form", [(300, 1024, 1024, 0.24, "tile"), (400, 1024, 1024, 0.24, "tile"),
+                                                 (32768, 768, 2304, 0.75, "resident"), (131072, 1024, 4096, 0.9, "resident"),
+                                                 (17771, 3072, 768, 0.75, "tile"), (32768, 4096, 1024, 0.75, "tile"), (128, 3072, 768, 0.75, "dense")])
+def test_the_form_that_was_measured_as_the_fastest_is_taken(et, orc, T, K, N, sparsity, form):
+    """Where another form takes at least 5 % longer."""
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, K + N, False, 0.05)
+    info = et.TileWeight(K, N, T, data, rp, ro, bias).info()
+    assert form == ("tile" if info["stage_bytes"] else "dense" if info["stages"] else "resident"), info
+
+
 @pytest.mark.parametrize("N,tokens", [(384, 65536), (576, 24000), (576, 65536)])
 def test_long_dense_launches_have_no_columns_to_fill_up(et, orc, N, tokens):
     """A launch at the power limit takes the tile width that divides its columns."""

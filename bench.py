@@ -808,7 +808,7 @@ def main():
     for name, w, yb, xb, gelu in launches:
         ms_l = time_loop(torch, lambda: w.run(yb, xb, gelu=gelu, stream=comp), 10, 3, comp)
         fl = 2.0 * T * 256 * w.ntile
-        alg_bytes = 2.0 * T * w.in_feat + 528.0 * w.ntile + 2.0 * T * w.out_feat
+        alg_bytes = 2.0 * T * w.in_feat + 516.0 * w.ntile + 2.0 * T * w.out_feat
         per.append({"launch": name, "K": w.in_feat, "N": w.out_feat, "kept_tiles": w.ntile, "ms": ms_l, "tflops": fl / (ms_l * 1e-3) / 1e12,
                     "algorithmic_bytes": alg_bytes, "packing": w.info()})
         w.check()

@@ -18,17 +18,16 @@
 // What bounds it: the softmax warps, at two per scheduler. The special-function unit delivers 16 results per clock and SM
 // whatever the format (measured: ex2.f32 16.0, ex2.f16x2 8.0 pairs), so a 128 x 128 block costs it 1024 clocks, against 512
 // clocks of UMMAs and ~450 issue slots per warp; kPolyPairs of every 16 pairs of exponentials are evaluated on the FMA pipe
-// (Cody-Waite reduction and a cubic; 0, 2, 4, 6, 8 of 16 measured: 86, 81, 80, 81, 88 us at 64 x 512 tokens, 12 heads). Loads, maximum,
-// exponentials and stores alone, two warps to a scheduler, take 1240 clocks a block; with everything else it is ~1640.
+// (Cody-Waite reduction and a cubic). 64 x 512 tokens, 12 heads, with 0, 2, 4, 6, 8 pairs: 84.1, 81.2, 81.2, 84.0, 85.8 us, and 2.880, 2.884,
+// 2.889, 2.895, 2.900e-4 away from 64 bits: two, the more exact of the two that are equally fast. Loads, maximum, exponentials and stores
+// alone, two warps to a scheduler, take 1240 clocks a block; with everything else it is ~1640.
 // Two CTAs share an SM (256 TMEM columns and ~100 KB of shared memory each), so that one's loads, maxima and hand-overs run
 // under the other's exponentials.
-// Both passes are loops over few columns, not a row unrolled in registers: with a thread's 128 scores held there (216 registers, handed
-// over by the other warps) a block took as long or longer, with masks that spilled 120 bytes much longer; whatever unrolled more code
-// was slower. Before and after, 12 heads: 64 x 512 tokens 83.4 -> 83.0 us, 64 x 200 28.4 -> 26.2,
-// 64 x 128 11.4 -> 10.8, 64 ragged sequences 58.9 -> 55.5; with masks 1 x 384 9.6 -> 9.1, 1 x 701 (16 heads, rows anywhere)
-// 21.2 -> 17.3, 64 x 384 78.6 -> 70, 64 x 383 114 -> 98, ragged 115 -> 100. Same bits. Also tried: two threads per row and sixteen softmax warps 83.5 us
-// (64 x 512), half blocks of 64 keys 100 (and 1.035 times the error), the next block's scores fetched under the last exponentials 85.6,
-// exponentials ahead of the maximum 101.
+// Both passes are loops over few columns: 110 registers, where a row's 128 scores unrolled in registers took 216, handed over by the other
+// warps, and with a mask spilled 120 bytes (20 here). Held so 64 x 512 tokens took 83.4 us, 64 x 200 28.4 (26.2 here), 64 ragged sequences 58.9
+// (54.8), 1 x 384 with a mask 9.6 (9.1), 64 x 384 with one 78.6 (69.4), 1 x 701 with one (16 heads, rows anywhere) 21.2 (17.4). Slower as well
+// (64 x 512): two threads per row and sixteen softmax warps 83.5, the next block's scores fetched under the last exponentials 85.6, the second
+// pass unrolled 82.4, half blocks of 64 keys 100 (and 1.035 times the error), exponentials ahead of the maximum 101.
 // CTAs are persistent: the grid has one CTA per item, and a running CTA takes over the next one that has not started (cluster
 // launch control), so that ragged batches balance themselves and an item's loads and first Q K^T are under way while the
 // previous one is finished; its rows are written inside the next item's first block. Ragged batches that outlast a wave are taken
@@ -1083,7 +1082,7 @@ int attention_tc_launch(half* Z, const half* Q, const half* K, const half* V, in
     const long items = cu_seqlens ? (total_tokens + kBQ - 1) / kBQ : nblk;
     p.take_over = items * nhead > (long)kCtasPerSm * sm_count();
     p.mask_two = mask && items * nhead <= sm_count() && !cu_seqlens;
-    // (The form that scatters V is not sorted: the table takes registers that it does not have.)
+    // (The form that scatters V is never ragged: the operator takes one sequence.)
     const bool sorted = p.take_over && cu_seqlens && batch <= kMaxSorted;
     const auto run = compact      ? (sorted ? (mask ? launch<true, kCompact, true> : launch<false, kCompact, true>)
                                             : (mask ? launch<true, kCompact> : launch<false, kCompact>))

@@ -16,12 +16,11 @@
 // a list of K slices, one byte per tile, then the tiles in UMMA layout. Roles: warp 0 copies activations, warps 2-3 weight
 // blocks (a warp that has requested a copy goes on only after ~700 clocks), warp 1 moves activations to tensor memory, warps
 // 4-11 issue and warps 12-27 convert and store. Copies of weights, issuing and converting come in two sets, one per accumulator: four issuing warps (one block-row of 16 features each), eight converting ones. The sets
-// run apart: while one accumulator is handed over and drained, the other set issues. One elected lane issues a block's UMMAs in one go;
-// each takes a warp ~120 clocks here (~20 in a kernel that does nothing else; 110 without the converting warps' stores).
-// As single predicated instructions, with the block's header known to one lane at a time, they took ~145: 17771 x 768 -> 2304 at 75 % 32.8 -> 31.9 us,
-// -> 3072 + GELU 44.7 -> 44.0, 8192 x 768 -> 2304 at 50 % 26.0 -> 25.3. Those that read from shared memory in the same region:
-// 65536 x 1024 -> 3072 at 90 % 161.9 -> 157.4. A CTA takes (slab, range of features) items; the number of ranges is
-// chosen at the launch so that the last wave is full.
+// run apart: while one accumulator is handed over and drained, the other set issues. One elected lane issues a block's UMMAs in one go:
+// ~120 clocks each (110 without the converting warps' stores); eight warps that do nothing else get one through in 55 to 60, which is
+// the tensor pipe. As single predicated instructions they took ~145: 17771 x 768 -> 2304 at 75 % 32.8 us instead of 31.9, 8192 x 768 ->
+// 2304 at 50 % 26.0 instead of 25.3; with those that read from shared memory outside the region 65536 x 1024 -> 3072 at 90 % 161.9
+// instead of 157.4. A CTA takes (slab, range of features) items; the number of ranges is chosen at the launch so that the last wave is full.
 // Every mbarrier wait is bounded; a role that gives up records a code and all threads meet at the common exit.
 #include <algorithm>
 #include <cstring>

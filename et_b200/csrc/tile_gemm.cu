@@ -11,10 +11,9 @@
 //     longer pays the 4 KB shared-memory read of A, which otherwise bounds small-N UMMAs to ~20 % of peak.
 //   * Every kept tile is one UMMA  D[128 x 16] += A[128 x 16] . tile^T  (B operand = the tile in
 //     shared memory, canonical no-swizzle K-major layout). Eight warps issue concurrently, each owning a disjoint set of
-//     block-rows. One elected lane issues a chunk's UMMAs in one go from a list of 4-byte entries, four to a load, and commits
-//     them: ~18 clocks a UMMA for one warp, ~9 for eight (the tensor pipe), where an election and a 16-byte entry for each
-//     took 45 and 18. 32768 x 1024 -> 4096 + GELU at 80 % 162.6 -> 154.6 us, 4096 -> 1024 125.8 -> 118.2, 17771 x 3072 -> 768 at
-//     75 % 40.3 -> 38.9, 1100 x 768 -> 3072 + GELU at 50 % 9.3 -> 8.4.
+//     block-rows. A lane elected once issues a chunk's UMMAs in one go from a list of 4-byte entries, four to a load, and commits
+//     them: ~18 clocks a UMMA for one warp, ~9 for eight (the tensor pipe); with an election and a 16-byte entry for each 45 and
+//     18, and 32768 x 1024 -> 4096 + GELU at 80 % 162.9 instead of 153.4 us, 17771 x 3072 -> 768 at 75 % 39.4 instead of 37.3.
 //   * The weight is re-packed once, on the host, into a stream of blocks, one per (block-row chunk,
 //     128-wide K chunk): a per-warp issue list followed by the tiles already in UMMA layout. One
 //     cp.async.bulk brings a block into shared memory. The sparsity pattern is kept exactly.

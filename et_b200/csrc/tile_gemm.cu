@@ -751,14 +751,14 @@ static int choose_nb(int n_block_rows, int k_chunks, int size_hint, double densi
                                           tiles_per_chunk + 3.0 * std::sqrt(nbe * kSlices * density * (1.0 - density)));
         const int stage_b = (int)((kHeaderBytes + tiles_max * kTileBytes + 1023) / 1024) * 1024;
         const RingShape rs = ring_shape(nbe, stage_b, kHeaderBytes + tiles_per_chunk * kTileBytes);
-        if (rs.nx < 2 || rs.a_slots < 1 || !fits(largest_block(tiles, n_block_rows, k_chunks, nbe), nbe)) continue;
+        if (rs.nx < 2 || rs.a_slots < 1) continue;
         const long ctas = (long)slabs * ((n_block_rows + nbe - 1) / nbe);
         const double per_cta = (double)((ctas + sms - 1) / sms);
         const double t_chunk = std::max({rs.period, 10.0 * tiles_per_chunk,
                                          (kXStageBytes + tiles_per_chunk * kTileBytes) / 64.0});
         const double t_tile = k_chunks * t_chunk + 350.0 * ((nbe + 3) / 4) + 800.0;
         const double cost = g_goal == 1 ? (double)ctas * t_tile : per_cta * t_tile + 3000.0;
-        if (best_nb == 0 || cost < best * 0.999) { best = cost; best_nb = nbe; }
+        if ((best_nb == 0 || cost < best * 0.999) && fits(largest_block(tiles, n_block_rows, k_chunks, nbe), nbe)) { best = cost; best_nb = nbe; }
     }
     *cost_out = best_nb > 0 ? best : 1e30;
     return best_nb > 0 ? best_nb : std::min(8, std::max(n_block_rows, 1));

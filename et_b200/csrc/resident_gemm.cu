@@ -9,18 +9,19 @@
 // 80 % sparsity. Here A is copied once per slab and CTA: 768 inputs take 384 columns, and the other 128 hold two accumulators
 // of 64 features, so that one is converted and stored while the next is multiplied. Inputs from 768 to 1024 stay in shared
 // memory, as the A operand of UMMAs that read it there (~40 clocks a tile).
-// What bounds it: for half-empty weights the UMMAs; at 75 % sparsity and above the stores, ~30 bytes per clock and SM
-// (546 clocks per 128 x 64 tile), which is about what L2 takes from all SMs together.
+// What bounds it: with K = 768 the stores at 75 % sparsity and above (17771 x 768 -> 2304 at 75 % 26.9 us, of which 17 are the bytes at the copy
+// bandwidth; without its stores 23), with GELU the converting warps (38.5 us; a warp has 16 packed tanh to a unit, 256 clocks of the special-function
+// unit alone, ~870 with the three other warps of its scheduler), with K = 1024 the UMMAs that read shared memory (50 clocks a tile).
 //
-// The weight is re-packed once into blocks of 64 features (x a part of the K range, so that two blocks per accumulator fit): per issuing warp
+// The weight is re-packed once into blocks of 64 features, or of a part of such a group's tiles where a block would exceed its slot: per issuing warp
 // a list of K slices, one byte per tile, then the tiles in UMMA layout. Roles: warp 0 copies activations, warps 2-3 weight
 // blocks (a warp that has requested a copy goes on only after ~700 clocks), warp 1 moves activations to tensor memory, warps
-// 4-11 issue and warps 12-27 convert and store. Copies of weights, issuing and converting come in two sets, one per accumulator: four issuing warps (one block-row of 16 features each), eight converting ones. The sets
-// run apart: while one accumulator is handed over and drained, the other set issues. One elected lane issues a block's UMMAs in one go:
-// ~120 clocks each (110 without the converting warps' stores); eight warps that do nothing else get one through in 55 to 60, which is
-// the tensor pipe. As single predicated instructions they took ~145: 17771 x 768 -> 2304 at 75 % 32.8 us instead of 31.9, 8192 x 768 ->
-// 2304 at 50 % 26.0 instead of 25.3; with those that read from shared memory outside the region 65536 x 1024 -> 3072 at 90 % 161.9
-// instead of 157.4. A CTA takes (slab, range of features) items; the number of ranges is chosen at the launch so that the last wave is full.
+// 4-11 issue and warps 12-27 convert and store. Copies of weights, issuing and converting come in two sets, one per accumulator: four issuing warps (one block-row
+// of 16 features each), eight converting ones. The sets run apart: while one accumulator is handed over and drained, the other set issues. Each
+// half of an accumulator is handed over by itself, so that its two issuing and four converting warps do not wait for the slowest of the other half (17771 x 768 -> 2304
+// at 75 % 27.9 instead of 27.1 us). A CTA takes (slab, range of features) items; the number of ranges is chosen at the launch so that the last wave is full.
+// Tried and dropped: two issuing warps per set (29.2 instead of 27.9 us), four accumulators of 32 columns with an issuing warp each (35), a token that lets the sets
+// issue in turn (33), stores from registers or through shared memory instead of TMA stores (34), one TMA store per 128 x 64 tile by warps of their own (28.7).
 // Every mbarrier wait is bounded; a role that gives up records a code and all threads meet at the common exit.
 #include <algorithm>
 #include <cstring>
@@ -46,9 +47,11 @@ constexpr int kTmemChunks = kTmemSlices * 16 / kKC;
 constexpr int kGroupRows = 4;                     // block-rows per accumulator, one per issuing warp
 constexpr int kAccCols = kGroupRows * 16;
 constexpr uint32_t kAccAt = kTmemSlices * 8;
-constexpr int kListBytes = 64;                    // entries per issuing warp and block
+constexpr int kListBytes = 64;                    // entries per issuing warp and block: a byte for each K slice of kMaxK
 constexpr int kHeadBytes = 64 + kGroupRows * kListBytes;
 constexpr int kMaxRing = 4;
+constexpr int kSlots = 2;                         // weight slots per set
+constexpr uint32_t kLast = 0x8000u;               // in a block's header: the last block of its group
 constexpr int kSets = 2;                          // accumulators, each with its own issuing and converting warps and weight slots
 constexpr int kFirstIssuer = 4, kIssuers = kSets * kGroupRows, kFirstEpi = kFirstIssuer + kIssuers, kEpiWarps = 16;
 constexpr int kThreads = 32 * (kFirstEpi + kEpiWarps);
@@ -56,41 +59,27 @@ constexpr int kUnitBytes = 32 * 32 * 2;
 constexpr int kSmemMax = 232448;
 
 struct ResidentParams {
-    const uint2* dir;         // [group][part]: {offset, size} in 16-byte units
+    const uint2* dir;         // per group: {offset of its blocks, their number << 16 | size of each}, in 16-byte units
     const uint8_t* stream;
     const half* bias;
     bool bias_given;          // the caller's, not the weight's own: the preceding kernel may still be writing it
     const uint8_t* empty;     // per group, a bit per block-row without tiles; null when there is none
-    int T, N, K, groups, parts, ranges, items, slabs;
-    int nx, nw, block_bytes;   // nw: weight slots per set
+    int T, N, K, groups, ranges, items, slabs;
+    int nx, block_bytes;
     int* err;
 };
 
 struct ResidentShared {
     uint64_t x_full[kMaxRing], x_empty[kMaxRing];   // chunk slots: landed / copied on to tensor memory
-    uint64_t w_full[kSets][kMaxRing], w_empty[kSets][kMaxRing];   // weight blocks: landed / their UMMAs have completed (4 commits)
+    uint64_t w_full[kSets][kSlots], w_empty[kSets][kSlots];   // weight blocks: landed / their UMMAs have completed (4 commits)
     uint64_t a_ready[kMaxChunks];                   // per chunk, once per item: in place for the UMMAs
     uint64_t a_free, tail_free;                     // the item's UMMAs have completed: its activations in tensor memory, in shared memory may be overwritten
-    uint64_t acc_full[2], acc_empty[2];
+    uint64_t acc_full[kSets][2], acc_empty[kSets][2];   // each half of an accumulator (two block-rows) by itself
     uint32_t tmem_base;
     volatile int abort;
+    __align__(16) half bias[kEpiWarps][32];         // of the unit that a converting warp works on
 };
 
-// UMMAs of the lane that `leader` names, without a branch.
-__device__ __forceinline__ void umma_ts_if(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p, q;\nsetp.ne.u32 p, %4, 0;\nsetp.ne.u32 q, %5, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
-__device__ __forceinline__ void umma_ss_if(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p, q;\nsetp.ne.u32 p, %4, 0;\nsetp.ne.u32 q, %5, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
 __device__ __forceinline__ void cp_128x256b(uint32_t taddr, uint64_t sdesc) {
     asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
@@ -105,20 +94,20 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
     uint8_t* const tail = smem;                                                    // chunks beyond the tensor-memory part
     uint8_t* const xring = tail + (size_t)(chunks - tchunks) * kChunkBytes;
     uint8_t* const wring = xring + (size_t)p.nx * kChunkBytes;
-    uint8_t* const epi = wring + (size_t)kSets * p.nw * p.block_bytes;             // a unit per converting warp
+    uint8_t* const epi = wring + (size_t)kSets * kSlots * p.block_bytes;           // a unit per converting warp
     ResidentShared* const sh = reinterpret_cast<ResidentShared*>(epi + kEpiWarps * kUnitBytes);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = gridDim.x;
 
     if (tid == 0) {
-        for (int i = 0; i < kMaxRing; ++i) {
-            mbar_init(&sh->x_full[i], 1); mbar_init(&sh->x_empty[i], 1);
-            for (int k = 0; k < kSets; ++k) { mbar_init(&sh->w_full[k][i], 1); mbar_init(&sh->w_empty[k][i], kGroupRows); }
-        }
+        for (int i = 0; i < kMaxRing; ++i) { mbar_init(&sh->x_full[i], 1); mbar_init(&sh->x_empty[i], 1); }
         for (int i = 0; i < kMaxChunks; ++i) mbar_init(&sh->a_ready[i], 1);
         mbar_init(&sh->a_free, kIssuers);
         mbar_init(&sh->tail_free, kIssuers);
-        for (int i = 0; i < 2; ++i) { mbar_init(&sh->acc_full[i], kGroupRows); mbar_init(&sh->acc_empty[i], kEpiWarps / 2); }
+        for (int k = 0; k < kSets; ++k) {
+            for (int i = 0; i < kSlots; ++i) { mbar_init(&sh->w_full[k][i], 1); mbar_init(&sh->w_empty[k][i], kGroupRows); }
+            for (int i = 0; i < 2; ++i) { mbar_init(&sh->acc_full[k][i], kGroupRows / 2); mbar_init(&sh->acc_empty[k][i], 4); }
+        }
         sh->abort = 0;
         fence_mbar_init();
         prefetch_tmap(&tmX);
@@ -180,16 +169,18 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
             const int g0 = r * p.groups / p.ranges, g1 = (r + 1) * p.groups / p.ranges;
             for (int g = g0; g < g1 && ok; ++g, ++gs) {
                 if ((int)(gs & 1u) != set) continue;
-                for (int b = g * p.parts; b < (g + 1) * p.parts; ++b) {
-                    const uint2 d = __ldg(p.dir + b);
+                const uint2 d = __ldg(p.dir + g);
+                const uint32_t bytes = (d.y & 0xffffu) * 16u;
+                const uint8_t* src = p.stream + (size_t)d.x * 16u;
+                for (uint32_t left = d.y >> 16; left > 0; --left, src += bytes) {
                     ok = mbar_wait(&sh->w_empty[set][ws], ph);
                     if (!ok) break;
                     if (lane == 0) {
-                        mbar_expect_tx(&sh->w_full[set][ws], d.y * 16u);
-                        bulk_load(wring + (size_t)(set * p.nw + ws) * p.block_bytes, p.stream + (size_t)d.x * 16u, d.y * 16u, &sh->w_full[set][ws]);
+                        mbar_expect_tx(&sh->w_full[set][ws], bytes);
+                        bulk_load(wring + (size_t)(set * kSlots + ws) * p.block_bytes, src, bytes, &sh->w_full[set][ws]);
                     }
                     __syncwarp();
-                    if (++ws == p.nw) { ws = 0; ph ^= 1u; }
+                    if (++ws == kSlots) { ws = 0; ph ^= 1u; }
                 }
             }
         }
@@ -220,162 +211,193 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
         }
         if (!ok) give_up(43);
     } else if (warp >= kFirstIssuer && warp < kFirstEpi) {
-        // ---- UMMAs: every second group, block-row w of it
+        // ---- UMMAs: every second group, block-row w of it. One lane is the whole role. What it executes between two UMMAs is what a
+        // group waits for: shared memory by 32-bit addresses, pointers carried along, one loop per kind of block. (Generic pointers, addresses
+        // made of indexes and a branch per case cost ~280 clocks for every wait on a barrier that had completed, 65 now, and ~95 per
+        // UMMA of eight warps, 65 now, which is the tensor pipe: 17771 x 768 -> 2304 at 75 % 31.1 instead of 29.2 us.)
         const int w = (warp - kFirstIssuer) & 3, set = (warp - kFirstIssuer) >> 2;
-        const uint64_t b_desc0 = make_smem_desc(0, 128, 256, 0);   // no swizzle: 128 B between core matrices along K, 256 B along N
         const uint64_t t_desc0 = make_smem_desc(smem_u32(tail), 16, 1024, 2);
+        const uint64_t b_desc0 = make_smem_desc(0, 128, 256, 0);   // no swizzle: 128 B between core matrices along K, 256 B along N
+        const uint32_t b_hi = (uint32_t)(b_desc0 >> 32), b_lo = (uint32_t)b_desc0;
         constexpr uint32_t idesc = make_idesc_f16(128, 16);
         const uint32_t d = tmem + kAccAt + set * kAccCols + (uint32_t)w * 16;
-        const uint32_t leader = elect_one() ? 1u : 0u;
-        bool ok = true;
-        int ws = 0, n = 0;
-        uint32_t ph = 0, gs = 0;
-        for (int item = blockIdx.x; item < p.items && ok; item += G, ++n) {
-            const int r = item % p.ranges;
-            const int g0 = r * p.groups / p.ranges, g1 = (r + 1) * p.groups / p.ranges;
-            int ready = 0;   // chunks of the item known to be in place: the set's first group follows them one by one
-            for (int g = g0; g < g1 && ok; ++g, ++gs) {
-                if ((int)(gs & 1u) != set) continue;
-                ok = mbar_wait(&sh->acc_empty[set], ((gs >> 1) & 1u) ^ 1u);
-                if (!ok) break;
-                uint32_t accumulate = 0;   // the block-row's first UMMA overwrites
-                for (int part = 0; part < p.parts; ++part) {
-                    ok = mbar_wait(&sh->w_full[set][ws], ph);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint8_t* blk = wring + (size_t)(set * p.nw + ws) * p.block_bytes;
-                    // (a reduction over equal values: the compiler then knows it to be the same for the warp, and so the descriptors)
-                    const uint32_t hdr = __reduce_max_sync(0xffffffffu, reinterpret_cast<const uint32_t*>(blk)[w]);
-                    const int nts = (hdr >> 16) & 0xff, nall = hdr >> 24;
-                    const uint8_t* list = blk + 64 + w * kListBytes;
-                    const uint64_t bd = b_desc0 + ((smem_u32(blk) + kHeadBytes + (hdr & 0xffffu) * 512u) >> 4);
-                    auto issue_one = [&](int i) {
-                        const uint32_t k = list[i];
-                        if (k < (uint32_t)kTmemSlices) {
-                            umma_ts_if(leader, d, tmem + k * 8u, bd + (uint64_t)(i * 32), idesc, accumulate);
-                        } else {
-                            const uint32_t t = k - kTmemSlices;
-                            umma_ss_if(leader, d, t_desc0 + (uint64_t)(((t >> 2) * kPanelBytes + (t & 3) * 32) >> 4), bd + (uint64_t)(i * 32), idesc, accumulate);
-                        }
-                        accumulate = 1;
-                    };
-                    if (ready == chunks) {
-                        // by one lane in one go: the tiles whose activations are in tensor memory, then those that read them from shared memory
-                        if (leader && nall > 0) {
-                            auto ts = [&](int i, uint32_t k, uint32_t acc) { umma_f16_ts(d, tmem + k * 8u, bd + (uint64_t)(i * 32), idesc, acc); };
-                            uint32_t acc = accumulate;
-                            int i = 0;
-#pragma unroll 1
-                            for (; i + 4 <= nts; i += 4) {
-                                const uint32_t k4 = *reinterpret_cast<const uint32_t*>(list + i);
-                                ts(i, k4 & 0xffu, acc);
-                                ts(i + 1, (k4 >> 8) & 0xffu, 1u);
-                                ts(i + 2, (k4 >> 16) & 0xffu, 1u);
-                                ts(i + 3, k4 >> 24, 1u);
-                                acc = 1;
-                            }
-                            if (i < nts) {
-                                const uint32_t k4 = *reinterpret_cast<const uint32_t*>(list + i);
-                                ts(i, k4 & 0xffu, acc);
-                                if (i + 1 < nts) ts(i + 1, (k4 >> 8) & 0xffu, 1u);
-                                if (i + 2 < nts) ts(i + 2, (k4 >> 16) & 0xffu, 1u);
-                                acc = 1;
-                            }
-#pragma unroll 1
-                            for (i = nts; i < nall; ++i) {
-                                const uint32_t t = list[i] - kTmemSlices;
-                                umma_f16(d, t_desc0 + (uint64_t)(((t >> 2) * kPanelBytes + (t & 3) * 32) >> 4), bd + (uint64_t)(i * 32), idesc, acc);
-                                acc = 1;
-                            }
-                        }
-                        __syncwarp();
-                        if (nall > 0) accumulate = 1;
-                    } else {
-                        int i = 0;
-                        for (const int c1 = (part + 1) * chunks / p.parts; ready < c1; ++ready) {
-                            ok = mbar_wait(&sh->a_ready[ready], (uint32_t)n & 1u);
-                            if (!ok) break;
-                            tc_fence_after();
-                            for (; i < nall && list[i] < 8 * (ready + 1); ++i) issue_one(i);
-                        }
+        const uint32_t block_bytes = p.block_bytes, ring0 = smem_u32(wring) + set * kSlots * block_bytes, ring1 = ring0 + kSlots * block_bytes;
+        const uint32_t full0 = smem_u32(&sh->w_full[set][0]), to_empty = smem_u32(&sh->w_empty[set][0]) - full0;
+        const uint32_t acc_full = smem_u32(&sh->acc_full[set][w >> 1]), acc_empty = smem_u32(&sh->acc_empty[set][w >> 1]);
+        if (elect_one()) {
+            bool ok = true;
+            int n = 0;
+            uint32_t blk = ring0, full = full0, ph = 0, acc_ph = 1, gs = 0;
+            auto b_desc = [&](uint32_t at) { return (uint64_t)b_hi << 32 | at; };
+            auto tail_desc = [&](uint32_t k) {
+                const uint32_t t = k - kTmemSlices;
+                return t_desc0 + (uint64_t)(((t >> 2) * kPanelBytes + (t & 3) * 32) >> 4);
+            };
+            auto finish_block = [&](bool last) {
+                umma_commit_at(full + to_empty);
+                if (last) umma_commit_at(acc_full);
+                blk += block_bytes;
+                full += 8;
+                if (blk == ring1) { blk = ring0; full = full0; ph ^= 1u; }
+            };
+            for (int item = blockIdx.x; item < p.items && ok; item += G, ++n) {
+                const int r = item % p.ranges;
+                const int g0 = r * p.groups / p.ranges, g1 = (r + 1) * p.groups / p.ranges;
+                int left = (g1 - g0 + ((gs & 1) == (uint32_t)set)) >> 1;   // groups of this set
+                gs += g1 - g0;
+                int ready = 0;   // chunks of the item known to be in place
+                auto follow = [&](int chunk) {
+                    for (; ok && ready <= chunk; ++ready) {
+                        ok = mbar_wait(&sh->a_ready[ready], (uint32_t)n & 1u);
+                        tc_fence_after();
+                    }
+                };
+                if (left > 0) {   // the set's first group follows the chunks
+                    ok = mbar_wait_at(acc_empty, acc_ph);
+                    acc_ph ^= 1u;
+                    uint32_t accumulate = 0;   // the block-row's first UMMA overwrites
+                    for (bool last = false; ok && !last;) {
+                        ok = mbar_wait_at(full, ph);
                         if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t hdr = lds32(blk + w * 4), list = blk + 64 + w * kListBytes, bd = b_lo + ((blk + kHeadBytes + (hdr & (kLast - 1)) * 512u) >> 4);
+                        last = hdr & kLast;
+                        const uint32_t nall = hdr >> 24;
+                        for (uint32_t i = 0; i < nall; ++i) {
+                            const uint32_t k = lds8(list + i);
+                            follow(k >> 3);
+                            if (!ok) break;
+                            if (k < (uint32_t)kTmemSlices) umma_f16_ts(d, tmem + k * 8u, b_desc(bd + i * 32), idesc, accumulate);
+                            else umma_f16(d, tail_desc(k), b_desc(bd + i * 32), idesc, accumulate);
+                            accumulate = 1;
+                        }
+                        if (last) follow(chunks - 1);
+                        if (ok) finish_block(last);
                     }
-                    if (leader) {
-                        umma_commit(&sh->w_empty[set][ws]);
-                        if (part + 1 == p.parts) umma_commit(&sh->acc_full[set]);
-                    }
-                    __syncwarp();
-                    if (++ws == p.nw) { ws = 0; ph ^= 1u; }
+                    --left;
                 }
-            }
-            // (a set without a group in this item has still to see every chunk's phase)
-            for (; ready < chunks && ok; ++ready) ok = mbar_wait(&sh->a_ready[ready], (uint32_t)n & 1u);
-            if (leader) {
+                bool fresh = true;   // the block is the first of its group
+                uint32_t accumulate = 0;
+#pragma unroll 1
+                while (ok && left > 0) {
+                    if (!mbar_wait_at(full, ph)) { ok = false; break; }
+                    const uint32_t hdr = lds32(blk + w * 4);
+                    uint32_t list = blk + 64 + w * kListBytes;
+                    uint4 e = lds128(list);   // sixteen entries
+                    if (fresh) {
+                        if (!mbar_wait_at(acc_empty, acc_ph)) { ok = false; break; }
+                        acc_ph ^= 1u;
+                        accumulate = 0;
+                    }
+                    tc_fence_after();
+                    // the tiles whose activations are in tensor memory, then those that read them from shared memory
+                    int nts = (hdr >> 16) & 0xff, nss = (int)(hdr >> 24) - nts;
+                    uint32_t bd = b_lo + ((blk + kHeadBytes + (hdr & (kLast - 1)) * 512u) >> 4);
+                    auto ts = [&](uint32_t k, uint32_t off, uint32_t acc) { umma_f16_ts(d, tmem + k * 8u, b_desc(bd + off), idesc, acc); };
+#pragma unroll 1
+                    for (; nts >= 4; nts -= 4) {
+                        ts(e.x & 0xffu, 0, accumulate);
+                        ts((e.x >> 8) & 0xffu, 32, 1u);
+                        ts((e.x >> 16) & 0xffu, 64, 1u);
+                        ts(e.x >> 24, 96, 1u);
+                        accumulate = 1;
+                        bd += 128;
+                        list += 4;
+                        e.x = e.y; e.y = e.z; e.z = e.w;
+                        if (!(list & 15)) e = lds128(list);
+                    }
+                    if (nts > 0) {
+                        ts(e.x & 0xffu, 0, accumulate);
+                        if (nts > 1) ts((e.x >> 8) & 0xffu, 32, 1u);
+                        if (nts > 2) ts((e.x >> 16) & 0xffu, 64, 1u);
+                        accumulate = 1;
+                        bd += nts * 32;
+                        list += nts;
+                    }
+#pragma unroll 1
+                    for (; nss > 0; --nss) {
+                        umma_f16(d, tail_desc(lds8(list)), b_desc(bd), idesc, accumulate);
+                        accumulate = 1;
+                        bd += 32;
+                        ++list;
+                    }
+                    fresh = hdr & kLast;
+                    finish_block(fresh);
+                    if (fresh) --left;
+                }
+                // (a set without a group in this item has still to see every chunk's phase)
+                follow(chunks - 1);
                 if (tchunks < chunks) umma_commit(&sh->tail_free);
                 umma_commit(&sh->a_free);
             }
-            __syncwarp();
+            if (!ok) {
+                if (!sh->abort) atomicExch(p.err, 44);
+                sh->abort = 1;
+            }
         }
-        if (!ok) give_up(44);
+        __syncwarp();
     } else if (warp >= kFirstEpi) {
         // ---- convert and store: set s has accumulator s, its eight warps a quarter of the rows and half of the columns each
         const int e = warp - kFirstEpi, q = warp & 3, set = e >> 3, half_of = (e >> 2) & 1;
         const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + kAccAt + set * kAccCols + half_of * 32;
-        const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+        const uint32_t acc_full = smem_u32(&sh->acc_full[set][half_of]), acc_empty = smem_u32(&sh->acc_empty[set][half_of]);
+        const uint32_t bias_at = smem_u32(sh->bias[e]);
         uint8_t* const buf = epi + (size_t)e * kUnitBytes;
+        const uint32_t to = smem_u32(buf) + lane * 64, swizzle = (lane >> 1) & 3;   // row `lane`: four 16-byte chunks under the 64-byte swizzle
         bool ok = true;
-        uint32_t gs = 0;
+        uint32_t gs = 0, ph = 0;
         // (the weight's own bias is read without waiting: 4808 x 768 -> 2304 at 90 % 12.68 us, 12.83 with the wait)
         if (p.bias_given) pdl_wait();
         for (int item = blockIdx.x; item < p.items && ok; item += G) {
             const int r = item % p.ranges;
             const int g0 = r * p.groups / p.ranges, g1 = (r + 1) * p.groups / p.ranges;
             const int row = (item / p.ranges) * kSlab + q * 32;
-            for (int g = g0; g < g1; ++g, ++gs) {
-                if ((int)(gs & 1u) != set) continue;
-                const int col = g * kAccCols + half_of * 32;
-                const int cols = min(32, p.N - col);   // 32, 16, or nothing of this half exists
-                uint4 bv[4];
-                if (bias_vec) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        bv[c] = c * 8 < cols ? __ldg(reinterpret_cast<const uint4*>(p.bias + col) + c) : make_uint4(0u, 0u, 0u, 0u);
-                } else {
-                    half* b = reinterpret_cast<half*>(bv);
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) b[c] = c < cols ? __ldg(p.bias + col + c) : __float2half(0.f);
-                }
-                const uint32_t e2 = kEmpty ? (__ldg(p.empty + g) >> (2 * half_of)) & 3u : 0u;
-                ok = mbar_wait(&sh->acc_full[set], (gs >> 1) & 1u);
-                if (!ok) break;
+            const int g = g0 + (int)((gs & 1) != (uint32_t)set);
+            gs += g1 - g0;
+            int col = g * kAccCols + half_of * 32;   // columns from N on do not exist
+            // A lane has one column's bias, read a unit ahead; a unit passes them on through shared memory (as four wide loads by every lane
+            // 17771 x 768 -> 2304 at 75 % 27.1 instead of 26.8 us).
+            auto bias_of = [&](int c) { return c + lane < p.N ? __ldg(reinterpret_cast<const uint16_t*>(p.bias) + c + lane) : (uint16_t)0; };
+            uint16_t b = g < g1 ? bias_of(col) : (uint16_t)0;
+#pragma unroll 1
+            for (int left = (g1 - g + 1) >> 1; left > 0; --left) {
+                const uint32_t e2 = kEmpty ? (__ldg(p.empty + col / kAccCols) >> (2 * half_of)) & 3u : 0u;
+                sts16(bias_at + lane * 2, b);
+                if (!mbar_wait_at(acc_full, ph)) { ok = false; break; }
+                ph ^= 1u;
                 tc_fence_after();
-                if (item + G >= p.items && g + 2 >= g1) pdl_launch_dependents();   // the next kernel's set-up overlaps the last stores
+                if (left == 1 && item + G >= p.items) pdl_launch_dependents();   // the next kernel's set-up overlaps the last stores
                 uint32_t acc[32];
                 tmem_ld32(src, acc);
                 tmem_ld_wait(acc);
                 tc_fence_before();
                 __syncwarp();
-                if (elect_one()) mbar_arrive(&sh->acc_empty[set]);
-                __syncwarp();
+                if (elect_one()) mbar_arrive_at(acc_empty);
                 if (kEmpty && e2) {   // what the zero tile of a block-row without tiles left is the bias alone, whatever the activations are
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
                         if ((e2 >> (i >> 4)) & 1u) acc[i] = 0u;
                 }
-                uint4 ov[4];
+                uint4 bv[4], ov[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) bv[c] = lds128(bias_at + c * 16);
                 epi_convert_regs<kGelu>(acc, bv, ov);
-                if (lane == 0) tma_store_wait_read();   // the buffer's previous store has read it
+                if (left > 1) b = bias_of(col + kSets * kAccCols);
+                tma_store_wait_read();   // the buffer's previous store has read it
                 __syncwarp();
-                epi_write(buf, lane, ov);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) sts128(to + ((c ^ swizzle) << 4), ov[c]);
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
-                    if (cols > 0 && row < p.T) tma_store_2d(&tmY, buf, col, row);
+                if (col < p.N && row < p.T && elect_one()) {
+                    tma_store_2d(&tmY, buf, col, row);
                     tma_store_commit();
                 }
+                __syncwarp();
+                col += kSets * kAccCols;
             }
         }
-        if (lane == 0) tma_store_wait_read();
+        tma_store_wait_read();
         if (!ok) give_up(45);
     }
     __syncwarp();
@@ -388,7 +410,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
 }  // namespace
 
 struct ResidentWeight {
-    int K = 0, N = 0, groups = 0, parts = 1, block_bytes = 0, nx = 0, nw = 0;
+    int K = 0, N = 0, groups = 0, block_bytes = 0, nx = 0;
     double group_clocks = 0;   // modelled, per group of 64 features and slab
     uint2* d_dir = nullptr;
     uint8_t* d_stream = nullptr;
@@ -396,19 +418,19 @@ struct ResidentWeight {
     size_t bytes = 0;
 };
 
-// Clocks per group, fitted to launches of 128 to 32768 tokens (within 15 %): half of an accumulator's round (issuing, the last
-// UMMAs' completion, hand-over to the converting warps and back), which grows with the tiles; a tile whose activations are
-// read from shared memory counts for many.
+// Clocks per group, fitted to 342 launches of 128 to 65536 tokens (rms 7.5 %) together with the choice between the forms: half of an
+// accumulator's round (issuing, the last UMMAs' completion, hand-over to the converting warps and back), which grows with the tiles and is
+// never shorter than the converting warps' round; a tile whose activations are read from shared memory counts for four.
 static double group_clocks(int K, double density) {
     const double ts = kGroupRows * density * std::min(K / 16, kTmemSlices), ss = kGroupRows * density * std::max(0, K / 16 - kTmemSlices);
-    return std::max(1000.0, 700.0 + 12.5 * ts) + 90.0 * ss;
+    return std::max(1000.0, 350.0 + 13.0 * ts + 54.0 * ss);
 }
 static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges) {
     double best = 0;
-    const double start = ((K + kKC - 1) / kKC) * 540.0 + 2000.0;   // copying a slab into place, per item
+    const double start = ((K + kKC - 1) / kKC) * 370.0 + 4600.0;   // copying a slab into place, per item
     for (int r = 1; r <= groups; ++r) {
         const int waves = (slabs * r + sm_count() - 1) / sm_count();
-        const double c = 7500.0 + waves * (start + ((groups + r - 1) / r) * per_group);
+        const double c = 4300.0 + waves * (start + ((groups + r - 1) / r) * per_group);
         if (best == 0 || c < best * 0.999) { best = c; *ranges = r; }
     }
     return best;
@@ -428,61 +450,55 @@ int resident_pack(ResidentWeight** out, int K, int N, const half* data, const in
     w->K = K; w->N = N; w->groups = (NBR + kGroupRows - 1) / kGroupRows;
     w->group_clocks = group_clocks(K, (double)row_ptr[NBR] / std::max(1.0, (double)NBR * (K / 16)));
     const int avail = kSmemMax - 1024 - (int)sizeof(ResidentShared) - kEpiWarps * kUnitBytes - std::max(0, chunks - kTmemChunks) * kChunkBytes;
+    // Tiles of each group in the order of their K slices (a block-row without tiles gets one of zeros: its accumulator is then written like the others).
+    struct Ent { int slice, row, tile; };
+    std::vector<std::vector<Ent>> tiles(w->groups);
+    size_t most = 0;
+    for (int r = 0; r < NBR; ++r) {
+        auto& v = tiles[r / kGroupRows];
+        if (row_ptr[r + 1] - row_ptr[r] > kListBytes) { delete w; return fail(ET_ERR_UNSUPPORTED, "resident linear: a tile is listed twice"); }
+        for (int i = row_ptr[r]; i < row_ptr[r + 1]; ++i) v.push_back({row_offset[i] / 16, r % kGroupRows, i});
+        if (row_ptr[r] == row_ptr[r + 1]) v.push_back({0, r % kGroupRows, -1});
+        most = std::max(most, v.size());
+    }
+    for (auto& v : tiles) std::stable_sort(v.begin(), v.end(), [](const Ent& a, const Ent& b) { return a.slice < b.slice; });
+    // Slots for activations as long as every group fits in one block beside them; two at least, and then the groups that do not fit are cut into
+    // equal blocks. (Cut at the same K slices everywhere, into as many as the largest needs, 131072 x 1024 -> 1024 at 80 % took 150 instead of 141 us
+    // when a kilobyte was short.)
+    auto room = [&](int nx) { return (avail - nx * kChunkBytes) / (kSets * kSlots) / 128 * 128; };
+    w->nx = 2;
+    for (int nx : {4, 3})
+        if (w->nx == 2 && (long)room(nx) >= (long)(kHeadBytes + most * 512)) w->nx = nx;
+    const size_t cap = (size_t)(room(w->nx) - kHeadBytes) / 512;
     std::vector<uint2> dir;
     std::vector<uint8_t> stream;
-    // the fewest parts of the K range with which two blocks per set fit beside at least two slots for activations
-    for (int parts = 1; parts <= chunks; ++parts) {
-        dir.clear();
-        stream.clear();
-        size_t largest = 0;
-        for (int g = 0; g < w->groups; ++g)
-            for (int part = 0; part < parts; ++part) {
-                const int s0 = part * chunks / parts * 8, s1 = (part + 1) * chunks / parts * 8;   // K slices of this part
-                struct Ent { int slice, tile; };
-                std::vector<Ent> lists[kGroupRows];
-                size_t n = 0;
-                for (int lb = 0; lb < kGroupRows; ++lb) {
-                    const int r = g * kGroupRows + lb;
-                    if (r >= NBR) continue;
-                    for (int i = row_ptr[r]; i < row_ptr[r + 1]; ++i) {
-                        const int s = row_offset[i] / 16;
-                        if (s >= s0 && s < s1) lists[lb].push_back({s, i});
-                    }
-                    std::sort(lists[lb].begin(), lists[lb].end(), [](const Ent& a, const Ent& b) { return a.slice < b.slice; });
-                    // a block-row without tiles gets one of zeros: its accumulator is then written like the others
-                    if (part == 0 && row_ptr[r] == row_ptr[r + 1]) lists[lb].push_back({0, -1});
-                    if (lists[lb].size() > kListBytes) { delete w; return fail(ET_ERR_UNSUPPORTED, "resident linear: a tile is listed twice"); }
-                    n += lists[lb].size();
+    for (const auto& v : tiles) {
+        const size_t parts = (v.size() + cap - 1) / cap, bytes = kHeadBytes + (v.size() + parts - 1) / parts * 512, off = stream.size();
+        stream.resize(off + parts * bytes, 0);
+        for (size_t part = 0; part < parts; ++part) {
+            uint8_t* blk = stream.data() + off + part * bytes;
+            const size_t first = part * v.size() / parts, end = (part + 1) * v.size() / parts;
+            uint32_t at = 0;
+            for (int lb = 0; lb < kGroupRows; ++lb) {
+                const uint32_t start = at;
+                uint32_t nts = 0;
+                for (size_t i = first; i < end; ++i) {
+                    const Ent& t = v[i];
+                    if (t.row != lb) continue;
+                    nts += t.slice < kTmemSlices;
+                    blk[64 + lb * kListBytes + (at - start)] = (uint8_t)t.slice;
+                    uint8_t* dst = blk + kHeadBytes + (size_t)at++ * 512;
+                    if (t.tile < 0) continue;
+                    for (int r = 0; r < 16; ++r)
+                        for (int k = 0; k < 16; k += 8)
+                            std::memcpy(dst + (r / 8) * 256 + (k / 8) * 128 + (r % 8) * 16, data + (size_t)t.tile * 256 + r * 16 + k, 16);
                 }
-                const size_t bytes = kHeadBytes + n * 512, off = stream.size();
-                stream.resize(off + bytes, 0);
-                uint8_t* blk = stream.data() + off;
-                uint32_t start = 0;
-                for (int lb = 0; lb < kGroupRows; ++lb) {
-                    uint32_t nts = 0;
-                    for (size_t i = 0; i < lists[lb].size(); ++i) {
-                        const Ent& t = lists[lb][i];
-                        nts += t.slice < kTmemSlices;
-                        blk[64 + lb * kListBytes + i] = (uint8_t)t.slice;
-                        if (t.tile < 0) continue;
-                        uint8_t* dst = blk + kHeadBytes + (size_t)(start + i) * 512;
-                        for (int r = 0; r < 16; ++r)
-                            for (int k = 0; k < 16; k += 8)
-                                std::memcpy(dst + (r / 8) * 256 + (k / 8) * 128 + (r % 8) * 16, data + (size_t)t.tile * 256 + r * 16 + k, 16);
-                    }
-                    reinterpret_cast<uint32_t*>(blk)[lb] = start | (nts << 16) | ((uint32_t)lists[lb].size() << 24);
-                    start += (uint32_t)lists[lb].size();
-                }
-                dir.push_back(make_uint2((uint32_t)(off / 16), (uint32_t)(bytes / 16)));
-                largest = std::max(largest, bytes);
+                reinterpret_cast<uint32_t*>(blk)[lb] = start | (part + 1 == parts ? kLast : 0) | (nts << 16) | ((at - start) << 24);
             }
-        w->parts = parts;
-        w->block_bytes = (int)((largest + 127) / 128 * 128);
-        for (int nx : {4, 3, 2})
-            if (!w->nx && nx * kChunkBytes + kSets * 2 * w->block_bytes <= avail) { w->nx = nx; w->nw = 2; }
-        if (w->nx) break;
+        }
+        dir.push_back(make_uint2((uint32_t)(off / 16), (uint32_t)(parts << 16 | bytes / 16)));
+        w->block_bytes = std::max(w->block_bytes, (int)((bytes + 127) / 128 * 128));
     }
-    if (!w->nx) { delete w; return fail(ET_ERR_UNSUPPORTED, "resident linear: weight blocks exceed shared memory"); }
     w->bytes = stream.size();
     std::vector<uint8_t> empty(w->groups, 0);
     for (int r = 0; r < NBR; ++r)
@@ -528,13 +544,13 @@ int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bi
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "resident linear: shared memory opt-in");
     ResidentParams p;
     p.dir = w->d_dir; p.stream = w->d_stream; p.bias = bias; p.bias_given = bias_given; p.empty = w->d_empty;
-    p.T = T; p.N = w->N; p.K = w->K; p.groups = w->groups; p.parts = w->parts;
+    p.T = T; p.N = w->N; p.K = w->K; p.groups = w->groups;
     p.slabs = (T + kSlab - 1) / kSlab;
     launch_clocks(p.slabs, w->groups, w->K, w->group_clocks, &p.ranges);
     p.items = p.slabs * p.ranges;
-    p.nx = w->nx; p.nw = w->nw; p.block_bytes = w->block_bytes; p.err = err;
+    p.nx = w->nx; p.block_bytes = w->block_bytes; p.err = err;
     const int chunks = (w->K + kKC - 1) / kKC;
-    const size_t smem = (size_t)(std::max(0, chunks - kTmemChunks) + w->nx) * kChunkBytes + (size_t)kSets * w->nw * w->block_bytes + kEpiWarps * kUnitBytes + sizeof(ResidentShared) + 1024;
+    const size_t smem = (size_t)(std::max(0, chunks - kTmemChunks) + w->nx) * kChunkBytes + (size_t)kSets * kSlots * w->block_bytes + kEpiWarps * kUnitBytes + sizeof(ResidentShared) + 1024;
     return cuda_status(launch_pdl(kernels[gelu ? 1 : 0][w->d_empty ? 1 : 0], dim3((unsigned)std::min(p.items, sm_count())),
                                   dim3(kThreads), smem, st, tm, tmy, p),
                        "resident linear launch");

@@ -919,18 +919,19 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     }
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
-    // 1.3 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 73 / 62 / 83, 3072 -> 768 77 / - / 106, 1024 ->
-    // 3072 111 / 152 / 129; at 50 % 1024 -> 4096 215 / 332 / 186. Both constants were measured over 984 linears (96 to 131072 tokens,
-    // eight shapes, six sparsities): the form taken is 0.60 % slower than the fastest in the mean; with 1.25 and 1.35 instead of 1.3 1.02 and
-    // 0.74 %, with 1.00, 1.04 and 1.12 instead of 1.08 (what the resident kernel's model overestimates) 0.69, 0.64 and 0.61 %.
-    tile_cost = 1.3 * tile_cost + 1000.0;
+    // 1.31 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 68 / 49 / 84, 1024 -> 3072 107 / 107 / 130, 1024 ->
+    // 4096 163 / 144 / 173; at 50 % 1024 -> 4096 201 / 218 / 184. All constants were measured over 456 linears (128 to 65536 tokens,
+    // eight shapes, six sparsities): the form taken is 0.36 % slower than the fastest in the mean, 12 choices are more than 5 % off.
+    tile_cost = 1.31 * tile_cost + 900.0;
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
     const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
-    w->packed_dense = plain && w->dense.cost < std::min(tile_cost, resident);
+    // (The dense form gives way to the resident one, which sums in another order, only for 14 % that its model promises: that costs 0.08 % in the
+    // mean of those linears, all of it at 4096 x 768 -> 2304 at 50 %, 14.8 instead of 12.7 us.)
+    w->packed_dense = plain && w->dense.cost < tile_cost && 0.86 * w->dense.cost < resident;
     int rc = w->packed_dense ? build_dense_form(w)
-             : plain && resident < 1.08 * tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
+             : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);
     if (rc) { tile_weight_free(w); return rc; }
     // the bias in both types and the error word in one allocation and one copy

@@ -516,6 +516,28 @@ def test_tile_linear_of_sparse_and_full_block_rows(et, orc, T, K, sparse, full, 
     util.assert_close(host(Y)[rows], orc.tile_linear(X[rows], rp, ro, data, bias, N), what=f"{sparse} sparse and {full} full outputs {w.info()}")
 
 
+@pytest.mark.parametrize("T,K,full,gelu", [(129, 1024, (0, 1, 2, 3), False), (129, 1024, (5, 190), True), (20000, 768, (0, 1, 2, 3, 143), False), (257, 1008, (7, 64, 65), True)])
+def test_resident_linear_with_groups_in_several_blocks(et, orc, T, K, full, gelu):
+    """Groups of four block-rows whose tiles exceed a slot of the weight ring are cut into blocks, first and last groups among them, beside groups in one block
+    and block-rows without tiles; a block may hold none of a block-row, and its first tile may come in any of them."""
+    rows = 192 if K > 768 else 144
+    rng = np.random.default_rng(K + T)
+    kept = [np.arange(K // 16) if r in full else np.sort(rng.choice(K // 16, rng.integers(0, K // 96), replace=False)) for r in range(rows)]
+    kept[9] = np.array([K // 16 - 1])
+    kept[10] = np.array([], np.int64)
+    rp, ro = np.concatenate([[0], np.cumsum([len(k) for k in kept])]).astype(np.int32), (np.concatenate(kept) * 16).astype(np.int32)
+    N = 16 * rows
+    data, bias, X = util.weights(5, (len(ro), 256)), util.weights(6, (N,), 0.05), util.activations(7, (T, K))
+    w = et.TileWeight(K, N, 32768, data, rp, ro, bias, is_gelu=gelu)
+    info = w.info()
+    assert info["stage_bytes"] == info["stages"] == 0, info   # the resident form
+    Y = w.run(torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda"), dev(X))
+    torch.cuda.synchronize()
+    w.check()
+    part = slice(max(0, T - 140), T)
+    util.assert_close(host(Y)[part], orc.tile_linear(X[part], rp, ro, data, bias, N, gelu=gelu), what=f"{full} full block-rows")
+
+
 def test_tile_linear_pruned_tiles_do_not_contribute(et, orc):
     """Mask exactness: output equals the dense product with the pruned tiles zeroed, and does not
     change when garbage is placed where the pruned tiles would be."""

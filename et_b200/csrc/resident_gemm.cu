@@ -418,19 +418,19 @@ struct ResidentWeight {
     size_t bytes = 0;
 };
 
-// Clocks per group, fitted to 342 launches of 128 to 65536 tokens (rms 7.5 %) together with the choice between the forms: half of an
+// Clocks per group, fitted to 342 launches of 128 to 65536 tokens (rms 11 %) together with the choice between the forms: half of an
 // accumulator's round (issuing, the last UMMAs' completion, hand-over to the converting warps and back), which grows with the tiles and is
 // never shorter than the converting warps' round; a tile whose activations are read from shared memory counts for four.
 static double group_clocks(int K, double density) {
     const double ts = kGroupRows * density * std::min(K / 16, kTmemSlices), ss = kGroupRows * density * std::max(0, K / 16 - kTmemSlices);
-    return std::max(1000.0, 350.0 + 13.0 * ts + 54.0 * ss);
+    return std::max(760.0, 430.0 + 11.0 * ts + 60.0 * ss);
 }
 static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges) {
     double best = 0;
-    const double start = ((K + kKC - 1) / kKC) * 370.0 + 4600.0;   // copying a slab into place, per item
+    const double start = ((K + kKC - 1) / kKC) * 400.0 + 3600.0;   // copying a slab into place, per item
     for (int r = 1; r <= groups; ++r) {
         const int waves = (slabs * r + sm_count() - 1) / sm_count();
-        const double c = 4300.0 + waves * (start + ((groups + r - 1) / r) * per_group);
+        const double c = 5600.0 + waves * (start + ((groups + r - 1) / r) * per_group);
         if (best == 0 || c < best * 0.999) { best = c; *ranges = r; }
     }
     return best;

@@ -11,9 +11,12 @@
 //     longer pays the 4 KB shared-memory read of A, which otherwise bounds small-N UMMAs to ~20 % of peak.
 //   * Every kept tile is one UMMA  D[128 x 16] += A[128 x 16] . tile^T  (B operand = the tile in
 //     shared memory, canonical no-swizzle K-major layout). Eight warps issue concurrently, each owning a disjoint set of
-//     block-rows. A lane elected once issues a chunk's UMMAs in one go from a list of 4-byte entries, four to a load, and commits
-//     them: ~18 clocks a UMMA for one warp, ~9 for eight (the tensor pipe); with an election and a 16-byte entry for each 45 and
-//     18, and 32768 x 1024 -> 4096 + GELU at 80 % 162.9 instead of 153.4 us, 17771 x 3072 -> 768 at 75 % 39.4 instead of 37.3.
+//     block-rows. A lane elected once is the issuing role: it waits for a chunk, issues its UMMAs in one go from a list of 4-byte entries, four to a
+//     load, and commits them (~18 clocks a UMMA for one warp, ~9 for eight, which is the tensor pipe). Every step from a hand-over to the next counts: with
+//     generic pointers, a converged wait and a region per chunk 1100 x 768 -> 3072 + GELU at 50 % took 7.82 us (7.30 now), 2048 x 768 -> 768 at 75 % 5.90 (5.29);
+//     as UMMAs under an election each 32768 x 1024 -> 4096 + GELU at 80 % 162.9 instead of 153.4. (Lane 0 instead of an elected lane: 8.40 us.)
+//   * What bounds a chunk of 24 block-rows at 75 % (17771 x 3072 -> 768, 36.9 us): the copies from L2 alone take 32.3 us (58 bytes a clock and SM),
+//     UMMAs and tcgen05.cp without the activations' copies 33.6, any two of the three 33 to 35.5.
 //   * The weight is re-packed once, on the host, into a stream of blocks, one per (block-row chunk,
 //     128-wide K chunk): a per-warp issue list followed by the tiles already in UMMA layout. One
 //     cp.async.bulk brings a block into shared memory. The sparsity pattern is kept exactly.
@@ -402,19 +405,23 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 
         if (warp < kFirstIssuer) {
             // ---------------- movers: shared memory -> tensor memory copy of the A operand. The mover warps take
-            // chunks in turn; lane 1 polls, lane 0 issues and commits. The tensor-memory slot is free when the
+            // chunks in turn; all lanes wait, lane 0 issues and commits (as one lane's loop 1100 x 768 -> 3072 7.90 instead of 7.42 us, with an elected lane
+            // 7.83). Places in the rings are carried along: divisions by the rings' sizes, two to a chunk, cost 8192 x 4096 -> 1024 1.8 of 35.8 us. The tensor-memory slot is free when the
             // UMMAs of the chunk a_slots earlier have completed: a tcgen05.cp is guaranteed to run ahead of UMMAs issued
             // after it, but not behind those issued before it (going by their issue saved 2-3 % with two
             // slots, 4096 -> 1024 at 75 % sparsity and 32768 tokens 130.3 us against 133.3, and nothing with more). The one commit per
             // chunk tells the issuers that A is in place and the activation producer that the shared-memory slot may be overwritten.
             const int m = warp - kFirstMover;
-            int xs = m % NX, a = m % RA, fx = m, fw = m, ar = m;
+            const uint32_t full_x0 = smem_u32(&sh->full_x[0]), full_w0 = smem_u32(&sh->full_w[0]), ready0 = smem_u32(&sh->a_ready[0]), done0 = smem_u32(&sh->done[0]);
+            const uint64_t x_desc0 = make_smem_desc(smem_u32(xring), 16, 1024, 2);
+            static_assert((512 - kMaxNB * 16) / kSlotCols >= kMovers, "a mover's next slot is at most one round on");
+            int xs = m, a = m, fx = m, fw = m, ar = m;   // (two slots of either at least)
             uint32_t phx = 0, phw = 0, phd = 0;
             int ds = (m + RA) & 1;   // of the chunk RA before this one, from the first that has one
             for (int it = m; it < n_items; it += kMovers) {
-                bool got = mbar_wait(&sh->full_x[fx], phx);
+                bool got = mbar_wait_at(full_x0 + fx * 8, phx);
                 if (got && it >= RA) {
-                    got = mbar_wait(&sh->done[ds], phd);
+                    got = mbar_wait_at(done0 + ds * 8, phd);
                     ds += kMovers;
                     if (ds >= kMaxRing) { ds -= kMaxRing; phd ^= 1u; }
                 }
@@ -426,28 +433,28 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 }
                 tc_fence_after();
                 if (lane == 0) {
-                    const uint32_t xa = smem_u32(xring + (size_t)xs * kXStageBytes);
+                    const uint64_t xd = x_desc0 + (uint32_t)xs * (kXStageBytes >> 4);
                     const uint32_t ta = tmem + a_col0 + a * kSlotCols;
 #pragma unroll
-                    for (int sl = 0; sl < kSlices; ++sl)
-                        tc_cp_128x256b(ta + sl * 8,
-                                       make_smem_desc(xa + (sl >> 2) * kPanelBytes + (sl & 3) * 32, 16, 1024, 2));
+                    for (int sl = 0; sl < kSlices; ++sl) tc_cp_128x256b(ta + sl * 8, xd + (((sl >> 2) * kPanelBytes + (sl & 3) * 32) >> 4));
                 }
                 // The issuers take "A is in place" to mean "the chunk is in place": the commit waits for the weight block,
                 // whose copy started later (its slot is free only when UMMAs have completed); the tcgen05.cp run meanwhile.
-                got = mbar_wait(&sh->full_w[fw], phw);
+                got = mbar_wait_at(full_w0 + fw * 8, phw);
                 if (!got) {
                     if (lane == 0) atomicExch(p.err, 12);
                     sh->abort = 1;
                     break;
                 }
                 if (lane == 0) {
-                    umma_commit(&sh->a_ready[ar]);
+                    umma_commit_at(ready0 + ar * 8);
                     if (it < 64) ET_STAMP(300 + it);
                 }
                 __syncwarp();
-                xs = (xs + kMovers) % NX;
-                a = (a + kMovers) % RA;
+                xs += kMovers;
+                if (xs >= NX) xs -= NX;
+                a += kMovers;
+                if (a >= RA) a -= RA;
                 fx += kMovers;
                 if (fx >= FX) { fx -= FX; phx ^= 1u; }
                 fw += kMovers;
@@ -466,22 +473,23 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             const int h = w >> 2;     // which of the four warps of this row quarter
             const uint32_t lane_base = (uint32_t)(q * 32) << 16;
             // B tile descriptor: no swizzle, 128 B between core matrices along K, 256 B along N.
-            const uint64_t b_desc0 = make_smem_desc(0, 128, 256, 0);
+            const uint32_t b_lo = (uint32_t)make_smem_desc(0, 128, 256, 0), b_hi = (uint32_t)(make_smem_desc(0, 128, 256, 0) >> 32);
             constexpr uint32_t idesc = make_idesc_f16(128, 16);
             // this warp's output staging: 32 rows x 32 columns (64-byte rows, 64-byte swizzle)
             uint8_t* const buf = epi + (size_t)w * kUnitBytes;
-            // The lane that issues this warp's UMMAs and commits them, elected once (for every chunk anew: 128 x 768 -> 3072 at 75 % 5.57
-            // instead of 5.48 us, 32768 x 1024 -> 4096 at 80 % 155.0 instead of 153.4).
+            const uint32_t to = smem_u32(buf) + lane * 64, swizzle = (lane >> 1) & 3;
+            // The lane that waits for chunks, issues this warp's UMMAs and commits them, elected once.
             const bool leader = elect_one();
             bool ok = true;
-            int ws = 0, a = 0, ar = 0;
-            uint32_t pha = 0;
+            uint32_t ws = 0, a = a_col0 + tmem, pha = 0;   // of the lane that issues: ring position, tensor-memory slot, parity
+            const uint32_t wring_at = smem_u32(wring), ready0 = smem_u32(&sh->a_ready[0]), done0 = smem_u32(&sh->done[0]), w_at0 = smem_u32(&sh->w_at[0]);
             // (the weight's own bias is read without waiting: 8 x 18..109 tokens through a layer 42.4 us, 42.9 with the wait)
             if (p.bias_given) pdl_wait();
             for (int tl = 0; tl < my_tiles; ++tl) {
                 const int tile = (int)blockIdx.x + tl * G;
                 const int slab = tile / p.n_chunks, chunk = tile - slab * p.n_chunks;
                 half* const tbias = sh->bias[tl & 1];
+                const uint32_t tbias_at = smem_u32(tbias);
                 {
                     const int col0 = chunk * p.nb * 16;
                     for (int i = tid - 32 * kFirstIssuer; i < p.nb * 16; i += 32 * kEpiWarps)
@@ -493,65 +501,49 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 if (tl > 0 && sh->issuer_abort[(tl - 1) & 1]) break;
                 tc_fence_after();
                 if (issuer) {
-                    for (int kc = 0; kc < p.k_chunks && ok; ++kc) {
-                        // a_ready implies that the weight block has landed too: the movers waited for both copies.
-                        const bool got = mbar_wait(&sh->a_ready[ar], pha);
-                        if (!got) {
-                            if (lane == 0) atomicExch(p.err, 13);
-                            sh->abort = 1;
-                            sh->issuer_abort[tl & 1] = 1;
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint8_t* const blk = wring + sh->w_at[ws];
-                        const uint32_t hw = reinterpret_cast<const uint32_t*>(blk)[w];
-                        const int ne = hw >> 16;
-                        const uint4* const list = reinterpret_cast<const uint4*>(blk) + reinterpret_cast<const uint16_t*>(blk + kListAt)[w];
-                        const uint32_t units = reinterpret_cast<const uint32_t*>(blk)[8];
-                        const uint32_t tile16 = ((smem_u32(blk) + kHeaderBytes) >> 4) + units + (hw & 0xffffu) * 32u;
-                        const uint32_t abuf = tmem + a_col0 + a * kSlotCols;
-                        auto issue = [&](int i, uint32_t e) {
-                            umma_f16_ts(tmem + (e >> 16), abuf + (e & 0xffffu), b_desc0 | (uint64_t)((tile16 + i * 32) & 0x3fff), idesc, 1u);
-                        };
-                        // Short lists, which are most of those of up to 16 block-rows, without the loop (with it 8192 x 4096 -> 1024 at 80 %
-                        // takes 37.0 instead of 36.7 us, 32768 x 1024 -> 4096 155.2 instead of 153.4). The first entries are read ahead of
-                        // the branch; of an empty list they are not used, and are the header's, which has landed with the block.
-                        const uint4 e0 = *list;
-                        if (ne <= 4) {
-                            if (leader) {
-                                if (ne > 0) issue(0, e0.x);
-                                if (ne > 1) issue(1, e0.y);
-                                if (ne > 2) issue(2, e0.z);
-                                if (ne > 3) issue(3, e0.w);
-                                umma_commit(&sh->done[ws]);
-                            }
-                        } else if (leader) {
-                            int i = 0;
+                    if (leader) {
 #pragma unroll 1
-                            for (; i + 4 <= ne; i += 4) {
-                                const uint4 e = list[i >> 2];
-                                issue(i, e.x);
-                                issue(i + 1, e.y);
-                                issue(i + 2, e.z);
-                                issue(i + 3, e.w);
+                        for (int kc = p.k_chunks; kc > 0; --kc) {
+                            // a_ready implies that the weight block has landed too: the movers waited for both copies.
+                            if (!mbar_wait_at(ready0 + ws * 8, pha)) {
+                                atomicExch(p.err, 13);
+                                sh->abort = 1;
+                                sh->issuer_abort[tl & 1] = 1;
+                                ok = false;
+                                break;
                             }
-                            if (i < ne) {
-                                const uint4 e = list[i >> 2];
-                                issue(i, e.x);
-                                if (i + 1 < ne) issue(i + 1, e.y);
-                                if (i + 2 < ne) issue(i + 2, e.z);
+                            tc_fence_after();
+                            const uint32_t blk = wring_at + lds32(w_at0 + ws * 4);
+                            const uint32_t hw = lds32(blk + w * 4), units = lds32(blk + 4 * kIssuers), at = lds16(blk + kListAt + w * 2);
+                            int ne = hw >> 16;
+                            uint32_t list = blk + at * 16;
+                            uint4 e = lds128(list);   // the first entries; of an empty list they are not used, and are the header's
+                            uint32_t bd = b_lo + ((blk + kHeaderBytes) >> 4) + units + (hw & 0xffffu) * 32u;
+                            auto issue = [&](uint32_t e, uint32_t off) {
+                                umma_f16_ts(tmem + (e >> 16), a + (e & 0xffffu), (uint64_t)b_hi << 32 | (bd + off), idesc, 1u);
+                            };
+#pragma unroll 1
+                            for (; ne > 4; ne -= 4) {
+                                issue(e.x, 0);
+                                issue(e.y, 32);
+                                issue(e.z, 64);
+                                issue(e.w, 96);
+                                bd += 128;
+                                list += 16;
+                                e = lds128(list);
                             }
-                            umma_commit(&sh->done[ws]);
+                            if (ne > 0) issue(e.x, 0);
+                            if (ne > 1) issue(e.y, 32);
+                            if (ne > 2) issue(e.z, 64);
+                            if (ne > 3) issue(e.w, 96);
+                            umma_commit_at(done0 + ws * 8);
+                            if (++ws == kMaxRing) { ws = 0; pha ^= 1u; }
+                            a += kSlotCols;
+                            if (a == tmem + 512) a = tmem + a_col0;
                         }
-                        if (w == 0 && lane == 0 && tl * p.k_chunks + kc < 64) ET_STAMP(600 + tl * p.k_chunks + kc);
-                        __syncwarp();
-                        if (++ws == kMaxRing) ws = 0;
-                        if (++a == RA) a = 0;
-                        if (++ar == kMaxRing) { ar = 0; pha ^= 1u; }
+                        umma_commit(&sh->acc_done);
                     }
-                    if (leader) umma_commit(&sh->acc_done);
-                    __syncwarp();
+                    ok = __all_sync(0xffffffffu, ok);
                     named_barrier_arrive(5, 32 * kEpiWarps);   // wakes the helpers: the tile's last UMMAs are on their way
                 } else {
                     // asleep on a hardware barrier while the issuers run the main loop (polling warps would take issue
@@ -613,19 +605,25 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                         if (two) tmem_st16_zero(tmem + lane_base + u * 32 + 16);
                     }
                     uint4 ov[4];
-                    if constexpr (kMode == 0) epi_convert<kGelu>(acc, tbias + u * 32, two, ov);
+                    if constexpr (kMode == 0) {
+                        uint4 bv[4];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) bv[c] = lds128(tbias_at + u * 64 + c * 16);   // (beyond an odd last block-row: columns that are not stored)
+                        epi_convert_regs<kGelu>(acc, bv, ov);
+                    }
                     else epi_fused<kGelu, kMode>(acc, rcur, p.fz, p.N, col0 + u * kUnitCols, ra, rb, s1, s2, ov);
                     // the buffer's previous store must have finished reading it (lane 0 issued it)
-                    if (lane == 0) tma_store_wait_read();
+                    tma_store_wait_read();
                     __syncwarp();
-                    epi_write(buf, lane, ov);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) sts128(to + ((c ^ swizzle) << 4), ov[c]);
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) {
-                        if (col0 + u * kUnitCols < p.N) tma_store_2d(&tmY, buf, col0 + u * kUnitCols, row0);
+                    if (col0 + u * kUnitCols < p.N && elect_one()) {
+                        tma_store_2d(&tmY, buf, col0 + u * kUnitCols, row0);
                         tma_store_commit();
-                        if (w == 0 && tl < 16 && (u >> 2) < 14) ET_STAMP(1400 + tl * 16 + 1 + (u >> 2));
                     }
+                    __syncwarp();
                 }
                 if constexpr (kMode >= 2) {
                     // this warp's share of the row: its own slot, written whether or not the warp had a unit
@@ -638,7 +636,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 }
                 if (w == 0 && lane == 0 && tl < 16) ET_STAMP(1400 + tl * 16 + 15);
             }
-            if (lane == 0) tma_store_wait_read();   // shared memory may go once the stores have read it
+            tma_store_wait_read();   // shared memory may go once the stores have read it
         }
     }
     tc_fence_before();
@@ -919,17 +917,17 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     }
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
-    // 1.31 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 68 / 49 / 84, 1024 -> 3072 107 / 107 / 130, 1024 ->
-    // 4096 163 / 144 / 173; at 50 % 1024 -> 4096 201 / 218 / 184. All constants were measured over 456 linears (128 to 65536 tokens,
-    // eight shapes, six sparsities): the form taken is 0.36 % slower than the fastest in the mean, 12 choices are more than 5 % off.
-    tile_cost = 1.31 * tile_cost + 900.0;
+    // 1.22 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 84, 1024 -> 3072 96 / 107 / 130, 1024 ->
+    // 4096 148 / 144 / 173; at 50 % 1024 -> 4096 186 / 218 / 184. All constants were measured over 456 linears (128 to 65536 tokens,
+    // eight shapes, six sparsities): the form and block-rows taken are 0.23 % slower than the fastest in the mean, 8 choices are more than 5 % off.
+    tile_cost = 1.22 * tile_cost + 1400.0;
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
     const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
-    // (The dense form gives way to the resident one, which sums in another order, only for 14 % that its model promises: that costs 0.08 % in the
-    // mean of those linears, all of it at 4096 x 768 -> 2304 at 50 %, 14.8 instead of 12.7 us.)
-    w->packed_dense = plain && w->dense.cost < tile_cost && 0.86 * w->dense.cost < resident;
+    // (The dense form gives way to the resident one, which sums in another order, only for 20 % that its model promises: that costs 0.1 % in the
+    // mean of those linears, all of it at 4096 x 768 -> 2304 at 50 %, 14.6 instead of 12.6 us.)
+    w->packed_dense = plain && 0.97 * w->dense.cost < tile_cost && 0.8 * w->dense.cost < resident;
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);

@@ -258,39 +258,46 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
         const uint32_t idesc = make_idesc_f16(2 * kBM, bn);
         const uint64_t a0 = make_smem_desc(smem_u32(smem), 16, 1024, 2);
         const uint64_t b0 = make_smem_desc(smem_u32(smem) + p.panels * kAPanel, 16, 1024, 2);
-        bool ok = true;
-        int s = 0;
-        uint32_t ph = 0;
-        for (int tl = 0; tl < my_tiles && ok; ++tl) {
-            const int buf = tl & 1;
-            ok = mbar_wait(&sh->acc_empty[buf], ((uint32_t)(tl >> 1) & 1u) ^ 1u);
-            if (!ok) break;
-            tc_fence_after();
-            for (int kc = 0; kc < k_stages; ++kc) {
-                ok = mbar_wait(&sh->full[s], ph);
+        if (elect_one()) {   // one lane is the role
+            const uint32_t full0 = smem_u32(&sh->full[0]);
+            bool ok = true;
+            int s = 0;
+            uint32_t ph = 0;
+            uint64_t a = a0, b = b0;
+            const uint32_t step = (uint32_t)stage_bytes >> 4;   // descriptors count 16-byte units
+            for (int tl = 0; tl < my_tiles && ok; ++tl) {
+                const int buf = tl & 1;
+                ok = mbar_wait(&sh->acc_empty[buf], ((uint32_t)(tl >> 1) & 1u) ^ 1u);
                 if (!ok) break;
                 tc_fence_after();
-                if (elect_one()) {
-                    const uint64_t at = (uint64_t)(s * stage_bytes) >> 4;   // descriptors count 16-byte units
-                    const int np = min(p.panels, p.k_panels - kc * p.panels);
+                const uint32_t d = tmem + buf * bn;
+                uint32_t accumulate = 0;
+                for (int left = p.k_panels; left > 0; left -= p.panels) {
+                    if (!mbar_wait_at(full0 + s * 8, ph)) { ok = false; break; }
+                    tc_fence_after();
+                    const int np = min(p.panels, left);
                     for (int i = 0; i < np; ++i)
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks)
-                            umma_f16_pair(tmem + buf * bn, a0 + at + (i * kAPanel >> 4) + ks * 2, b0 + at + (i * b_panel >> 4) + ks * 2,
-                                          idesc, (kc > 0 || i > 0 || ks > 0) ? 1u : 0u);
+                        for (int ks = 0; ks < 4; ++ks) {
+                            umma_f16_pair(d, a + (i * kAPanel >> 4) + ks * 2, b + (i * b_panel >> 4) + ks * 2, idesc, accumulate);
+                            accumulate = 1;
+                        }
                     umma_commit_pair(&sh->empty[s]);
-                    if (kc + 1 == k_stages) umma_commit_pair(&sh->acc_full[buf]);
+                    a += step;
+                    b += step;
+                    if (++s == S) { s = 0; ph ^= 1u; a = a0; b = b0; }
                 }
-                __syncwarp();
-                if (++s == S) { s = 0; ph ^= 1u; }
+                if (ok) umma_commit_pair(&sh->acc_full[buf]);
             }
+            if (!ok) atomicExch(p.err, 32);
         }
-        if (!ok && lane == 0) atomicExch(p.err, 32);
+        __syncwarp();
     } else if (warp >= kFirstEpi) {
         // ---- convert and store this CTA's 128 tokens: two warps per 32 rows take the tile's 32-column units in turn
         const int w = warp - kFirstEpi, q = warp & 3, h = w >> 2;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         uint8_t* const buf = epi + (size_t)w * kUnitBytes;
+        const uint32_t to = smem_u32(buf) + lane * 64, swizzle = (lane >> 1) & 3;   // row `lane`: four 16-byte chunks under the 64-byte swizzle
         const int units = bn / kUnitCols;
         bool ok = true;
         if (p.bias_given) pdl_wait();
@@ -298,6 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
             const int tile = pair + tl * G;
             const int m0 = (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM + q * 32, n0 = (tile % p.tiles_n) * bn;
             const int a = tl & 1;
+            const uint32_t bias_at = smem_u32(sh->bias[a]);
             for (int i = tid - 32 * kFirstEpi; i < bn; i += 32 * kEpiWarps)
                 sh->bias[a][i] = n0 + i < p.N ? p.bias[n0 + i] : __float2half(0.f);
             epi_barrier();
@@ -318,24 +326,29 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
                 tmem_ld_wait(acc);
                 if (u + kEpiWarps / 4 >= units) accumulator_read();   // this warp's share: it may be overwritten
                 uint4 ov[4];
-                epi_convert<kGelu>(acc, sh->bias[a] + u * kUnitCols, true, ov);
-                if (lane == 0) tma_store_wait_read();   // the buffer's previous store has read it
+                uint4 bv[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) bv[c] = lds128(bias_at + u * kUnitCols * 2 + c * 16);
+                epi_convert_regs<kGelu>(acc, bv, ov);
+                tma_store_wait_read();   // the buffer's previous store has read it
                 __syncwarp();
-                epi_write(buf, lane, ov);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) sts128(to + ((c ^ swizzle) << 4), ov[c]);
                 if constexpr (kPruned) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) odd.note(ov[c]);
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
-                    if (n0 + u * kUnitCols < p.N && m0 < p.T) tma_store_2d(&tmY, buf, n0 + u * kUnitCols, m0);
+                if (n0 + u * kUnitCols < p.N && m0 < p.T && elect_one()) {
+                    tma_store_2d(&tmY, buf, n0 + u * kUnitCols, m0);
                     tma_store_commit();
                 }
+                __syncwarp();
             }
             if (h >= units) accumulator_read();
             if (kPruned && __any_sync(0xffffffffu, odd.any())) {
-                if (lane == 0) tma_store_wait();   // the results are in memory
+                tma_store_wait();   // the results are in memory
                 __syncwarp();
                 fence_proxy_async_global();
                 for (int u = h; u < units && odd.any() && m0 + lane < p.T; u += kEpiWarps / 4)
@@ -344,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
             }
         }
         if (!ok && lane == 0) atomicExch(p.err, 33);
-        if (lane == 0) tma_store_wait_read();
+        tma_store_wait_read();
     }
     __syncwarp();
     tc_fence_before();

@@ -917,10 +917,10 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     }
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
-    // 1.22 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 84, 1024 -> 3072 96 / 107 / 130, 1024 ->
-    // 4096 148 / 144 / 173; at 50 % 1024 -> 4096 186 / 218 / 184. All constants were measured over 456 linears (128 to 65536 tokens,
-    // eight shapes, six sparsities): the form and block-rows taken are 0.23 % slower than the fastest in the mean, 8 choices are more than 5 % off.
-    tile_cost = 1.22 * tile_cost + 1400.0;
+    // 1.2 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 82, 1024 -> 3072 96 / 90 / 128, 1024 ->
+    // 4096 148 / 118 / 171; at 50 % 1024 -> 4096 186 / 189 / 181. All constants were measured over 456 linears (128 to 65536 tokens,
+    // eight shapes, six sparsities): the form and block-rows taken are 0.28 % slower than the fastest in the mean, 12 choices are more than 5 % off.
+    tile_cost = 1.2 * tile_cost + 1450.0;
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).

@@ -516,10 +516,12 @@ def test_tile_linear_of_sparse_and_full_block_rows(et, orc, T, K, sparse, full, 
     util.assert_close(host(Y)[rows], orc.tile_linear(X[rows], rp, ro, data, bias, N), what=f"{sparse} sparse and {full} full outputs {w.info()}")
 
 
-@pytest.mark.parametrize("T,K,full,gelu", [(129, 1024, (0, 1, 2, 3), False), (129, 1024, (5, 190), True), (20000, 768, (0, 1, 2, 3, 143), False), (257, 1008, (7, 64, 65), True)])
+@pytest.mark.parametrize("T,K,full,gelu", [(129, 1024, (0, 1, 2, 3), False), (129, 1024, (5, 190), True), (20000, 768, (0, 1, 2, 3, 143), False), (257, 1008, (7, 64, 65), True),
+                                           (300, 832, (3, 100), False), (130, 848, (0, 191), True), (1, 784, (17,), False)])
 def test_resident_linear_with_groups_in_several_blocks(et, orc, T, K, full, gelu):
-    """Groups of four block-rows whose tiles exceed a slot of the weight ring are cut into blocks, first and last groups among them, beside groups in one block
-    and block-rows without tiles; a block may hold none of a block-row, and its first tile may come in any of them."""
+    """Groups of block-rows whose tiles exceed a slot of the weight ring are cut into blocks, first and last groups among them, beside groups in one block
+    and block-rows without tiles; a block may hold none of a block-row, and its first tile may come in any of them. Inputs that tensor memory just holds, and one
+    slice more."""
     rows = 192 if K > 768 else 144
     rng = np.random.default_rng(K + T)
     kept = [np.arange(K // 16) if r in full else np.sort(rng.choice(K // 16, rng.integers(0, K // 96), replace=False)) for r in range(rows)]

@@ -212,6 +212,18 @@ def test_softmax_many_rows_of_any_alignment(et, orc, nmat, L, offset, use_mask, 
     assert (buf[:offset] == 7).all() and (buf[offset + nmat * L * L:] == 7).all()
 
 
+@pytest.mark.parametrize("nmat,L,use_mask", [(90, 231, True), (85, 233, True), (85, 233, False), (80, 255, True), (75, 255, False), (70, 257, False), (50, 463, True),
+                                             (50, 465, True), (50, 465, False), (49, 511, True)])
+def test_softmax_rows_in_flight_by_length(et, orc, nmat, L, use_mask):
+    """Lengths around which another number of rows is in flight, with enough matrices for it, three tokens masked at the end."""
+    S, mask = util.activations(L, (nmat, L, L)), util.activations(L + 1, (L, L))
+    Sd = dev(S)
+    et.softmax_mask(Sd, dev(mask) if use_mask else None, L - 3)
+    torch.cuda.synchronize()
+    some = [0, 1, 7, nmat // 2, nmat - 1]
+    util.assert_close(host(Sd)[some], orc.softmax_mask(S[some], mask if use_mask else None, L - 3), what=f"softmax {nmat}x{L}")
+
+
 @pytest.mark.parametrize("L", [1, 7, 241, 242, 243, 499, 1017, 1019, 2034, 2035])
 @pytest.mark.parametrize("offset", [0, 3])
 def test_softmax_mask_rows_of_any_alignment(et, orc, L, offset):

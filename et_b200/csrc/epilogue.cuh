@@ -1,4 +1,4 @@
-// What the linears do with an accumulator: bias, tanh-GELU, fp16, a swizzled unit of 32 rows x 32 columns for one TMA store.
+// What the linears do with an accumulator: bias, tanh-GELU, fp16.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -22,7 +22,8 @@ __device__ __forceinline__ half2 gelu_tanh_h2(half2 x) {
     return __hfma2(hx, *reinterpret_cast<const half2*>(&t), hx);
 }
 
-// One 32-column unit of an epilogue, in three steps.
+// One 32-column unit of an epilogue: its accumulators, then its results. The caller writes them under the 64-byte swizzle
+// (16-byte chunk ^= (row / 2) % 4).
 __device__ __forceinline__ void epi_load(uint32_t taddr, bool two, uint32_t (&acc)[32]) {
     if (two) {
         tmem_ld32(taddr, acc);
@@ -57,21 +58,6 @@ __device__ __forceinline__ void epi_convert_regs(const uint32_t (&acc)[32], cons
             oh[i] = __floats2half2_rn(lo, hi);
         }
     }
-}
-template <bool kGelu>
-__device__ __forceinline__ void epi_convert(const uint32_t (&acc)[32], const half* bias, bool two, uint4 (&ov)[4]) {
-    uint4 bv[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        bv[c] = (two || c < 2) ? reinterpret_cast<const uint4*>(bias)[c] : make_uint4(0u, 0u, 0u, 0u);
-    epi_convert_regs<kGelu>(acc, bv, ov);
-}
-// Row `lane` of a 32 x 32 unit: four 16-byte chunks under the 64-byte swizzle (chunk ^= (row / 2) % 4).
-__device__ __forceinline__ void epi_write(uint8_t* buf, int lane, const uint4 (&ov)[4]) {
-    uint8_t* prow = buf + lane * 64;
-    const int x = (lane >> 1) & 3;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(prow + ((c ^ x) << 4)) = ov[c];
 }
 
 }  // namespace et

@@ -8,7 +8,7 @@ namespace et {
 
 struct ResidentWeight;
 
-// Modelled clocks of a launch; 1e30 where the form does not exist (in_feat above 1024, or a block-row too dense for its lists).
+// Modelled clocks of a launch; 1e30 where the form does not exist (in_feat above 1024).
 double resident_cost(int tokens, int N, int K, double density);
 // Packs a validated weight (tile-BSR arrays as in tile_weight_pack; no tile twice in a block-row).
 int resident_pack(ResidentWeight** out, int K, int N, const half* data, const int* row_ptr, const int* row_offset);

@@ -723,8 +723,8 @@ static int ring_room(size_t largest) { return (int)((largest + 1023) / 1024 * 10
 static bool fits(size_t largest, int nb) { return largest < kSmemMax && ring_shape(nb, ring_room(largest), (double)largest).nx >= 2; }
 // Block-rows per CTA from a model of the persistent kernel: a chunk takes the ring period, or its UMMAs (~10
 // clocks each with eight issuing warps), or its share of L2 bandwidth (~64 bytes per clock per SM), whichever
-// is longest; a tile ends with an epilogue of ~350 clocks per 32 columns and warp. Against 5576 launches (96 to 131072 tokens, the eight shapes
-// of BERT-base and BERT-large layers, 25 to 90 % of the tiles pruned, 4 to 24 block-rows) the rms error of 1.3 times this is 10 %.
+// is longest; a tile ends with an epilogue of ~350 clocks per 32 columns and warp. What it chooses among 4 to 24 block-rows is measured
+// together with the choice of the form (tile_weight_pack).
 // What the pack optimises: 0 = the duration of one launch on an otherwise idle GPU (tiles spread over as many SMs
 // as possible), 1 = SM time per launch (fewer, larger tiles: the right choice when several independent batches
 // are in flight on separate streams and keep all SMs busy anyway).

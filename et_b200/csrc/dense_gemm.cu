@@ -70,6 +70,7 @@ inline int ring_stages(int n) { return n >= 8 ? 8 : n == 7 ? 6 : n == 5 ? 4 : n;
 struct DenseShared {
     uint64_t full[kMaxStages], empty[kMaxStages];
     uint64_t acc_full[2], acc_empty[2];
+    uint64_t received;   // split K: the other CTAs' parts of this CTA's columns
     uint32_t tmem_base;
     __align__(16) half bias[2][kMaxBN];
 };
@@ -213,11 +214,21 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
 
+    // Of the first tile's first stages the weight's panels are requested before the wait for the preceding kernel, the activations behind it by
+    // the epilogue's warps, which have nothing to do yet (one warp for both, behind its wait for an empty stage: 128 x 768 -> 2304 6.85
+    // instead of 6.3 us, 1100 x 3072 -> 768 12.2 instead of 11.4, 32768 x 768 -> 2304 the same).
+    const int ahead = min(S, k_stages);
+    auto load_x = [&](int s, int kc, int tile) {
+        const int np = min(p.panels, p.k_panels - kc * p.panels);
+        const uint32_t bar = in_cta(&sh->full[s], 0);
+        for (int i = 0; i < np; ++i)
+            tma_load_2d_pair(smem + (size_t)s * stage_bytes + i * kAPanel, &tmX, (kc * p.panels + i) * kBK,
+                             (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM, bar);
+    };
     if (warp < kCopyWarps) {
         // ---- copies, stages in turn; both CTAs' report to the first one's barriers
         bool ok = true;
         const int cw = copy_warps(S);
-        const int ahead = min(S, k_stages);   // weight panels of the first tile's first stages, requested before the wait
         auto load_w = [&](int s, int kc, int tile) {
             const int np = min(p.panels, p.k_panels - kc * p.panels);
             const uint32_t bar = in_cta(&sh->full[s], 0);
@@ -236,17 +247,12 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
             while (kc >= k_stages) { kc -= k_stages; ++tl; }
             if (s >= S) { s -= S; ph ^= 1u; }
             const int tile = pair + tl * G;
-            ok = mbar_wait(&sh->empty[s], ph);
-            if (!ok) break;
-            if (lane == 0) {
-                if (c >= ahead) load_w(s, kc, tile);
-                const int np = min(p.panels, p.k_panels - kc * p.panels);
-                const uint32_t bar = in_cta(&sh->full[s], 0);
-                for (int i = 0; i < np; ++i)
-                    tma_load_2d_pair(smem + (size_t)s * stage_bytes + i * kAPanel, &tmX, (kc * p.panels + i) * kBK,
-                                     (tile / p.tiles_n) * (2 * kBM) + (int)rank * kBM, bar);
+            if (c >= ahead) {
+                ok = c < S || mbar_wait(&sh->empty[s], ph);
+                if (!ok) break;
+                if (lane == 0) { load_w(s, kc, tile); load_x(s, kc, tile); }
+                __syncwarp();
             }
-            __syncwarp();
             kc += cw;
             s += cw;
         }
@@ -295,6 +301,12 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
     } else if (warp >= kFirstEpi) {
         // ---- convert and store this CTA's 128 tokens: two warps per 32 rows take the tile's 32-column units in turn
         const int w = warp - kFirstEpi, q = warp & 3, h = w >> 2;
+        static_assert(kEpiWarps >= kMaxStages, "a warp for the activations of each first stage");
+        if (w < ahead) {
+            pdl_wait();
+            if (lane == 0) load_x(w, w, pair);
+            __syncwarp();
+        }
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         uint8_t* const buf = epi + (size_t)w * kUnitBytes;
         const uint32_t to = smem_u32(buf) + lane * 64, swizzle = (lane >> 1) & 3;   // row `lane`: four 16-byte chunks under the 64-byte swizzle
@@ -370,13 +382,33 @@ __global__ void __launch_bounds__(kThreads, 1) dense_kernel(const __grid_constan
 // ------------------------------------------------------------------------------------------ K split over a cluster
 constexpr int kSplitThreads = 256;
 
-// Four words to the address `addr` of CTA `rank` of the cluster.
-__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t rank, const uint32_t* v) {
-    asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, %1;\nst.shared::cluster.v4.b32 [a], {%2,%3,%4,%5};\n}" ::"r"(addr), "r"(rank),
+// Four words to the address `addr` of CTA `rank` of the cluster, which count towards the bytes that its barrier at `bar` waits for.
+__device__ __forceinline__ void st_async_cluster(uint32_t addr, uint32_t bar, uint32_t rank, const uint32_t* v) {
+    asm volatile("{\n.reg .b32 a, b;\nmapa.shared::cluster.u32 a, %0, %2;\nmapa.shared::cluster.u32 b, %1, %2;\n"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [a], {%3,%4,%5,%6}, [b];\n}" ::"r"(addr), "r"(bar), "r"(rank),
                  "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
                  : "memory");
 }
+// A bounded wait like mbar_wait, for what other CTAs of the cluster have written.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < kMbarSpinLimit; ++i) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
 
+// Bound by a chain of latencies: of the ~7500 clocks from launch to launch of 128 x 768 -> 768 (3.9 us), ~2700 lie between the end of the
+// kernel before and the return of griddepcontrol.wait, 1300-1400 between the request of the activations and the first UMMA, 1200 to the
+// last panel's UMMAs, 700 are the sends of accumulators, 600 their way, 1000 the sums and stores. So nothing waits that need not: the first stages' weight is requested
+// before the other warps know the barriers, the activations by warps of their own without a look at empty stages, and each CTA
+// waits for the bytes of its own columns instead of a barrier of the cluster behind all sends (1450 clocks). Before: 4.2 us, 3072 -> 768 6.3 (5.6 now),
+// 4096 -> 1024 7.3 (6.3), 256 x 1024 -> 1024 6.3 (5.5).
 template <bool kGelu, bool kPruned>
 __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __grid_constant__ CUtensorMap tmX,
                                                                        const __grid_constant__ CUtensorMap tmW,
@@ -396,60 +428,70 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     const int m0 = (tile / p.tiles_n) * kBM, n0 = (tile % p.tiles_n) * bn;
     const int kp0 = rank * p.k_panels / split, kp1 = (rank + 1) * p.k_panels / split;   // this CTA's panels
     const int kn = (kp1 - kp0 + p.panels - 1) / p.panels;                               // in stages
-    if (tid == 0) {
-        for (int i = 0; i < S; ++i) { mbar_init(&sh->full[i], 1); mbar_init(&sh->empty[i], 1); }
-        mbar_init(&sh->acc_full[0], 1);
-        fence_mbar_init();
-    }
-    if (warp == kCopyWarps) {
-        tmem_alloc(&sh->tmem_base, tmem_cols(bn));
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this CTA runs: its memory may be written to
-    tc_fence_after();
-    const uint32_t tmem = sh->tmem_base;
-    // the weight's first panels, before anything that depends on the preceding kernel
+    const int cw = copy_warps(S), first = min(S, kn);
+    auto expect = [&](int s, int kc) { mbar_expect_tx(&sh->full[s], min(p.panels, kp1 - kp0 - kc * p.panels) * (kAPanel + b_panel)); };
     auto load_w = [&](int s, int kc) {
         const int k0 = kp0 + kc * p.panels, np = min(p.panels, kp1 - k0);
-        mbar_expect_tx(&sh->full[s], np * (kAPanel + b_panel));
         for (int i = 0; i < np; ++i)
             tma_load_2d(smem + (size_t)s * stage_bytes + p.panels * kAPanel + i * b_panel, &tmW, (k0 + i) * kBK, n0, &sh->full[s]);
     };
-    const int cw = copy_warps(S);
-    if (warp < cw && lane == 0)
-        for (int i = warp; i < min(S, kn); i += cw) load_w(i, i);
-    __syncwarp();
+    auto load_x = [&](int s, int kc) {
+        const int k0 = kp0 + kc * p.panels, np = min(p.panels, kp1 - k0);
+        for (int i = 0; i < np; ++i) tma_load_2d(smem + (size_t)s * stage_bytes + i * kAPanel, &tmX, (k0 + i) * kBK, m0, &sh->full[s]);
+    };
+    // The first stages: the weight's panels, which do not depend on the preceding kernel, by the warp that makes the barriers, as soon as
+    // they exist; the activations by three others, which wait for the preceding kernel meanwhile.
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int i = 0; i < S; ++i) { mbar_init(&sh->full[i], 1); mbar_init(&sh->empty[i], 1); }
+            mbar_init(&sh->acc_full[0], 1);
+            mbar_init(&sh->received, 1);
+            fence_mbar_init();
+            for (int i = 0; i < first; ++i) expect(i, i);
+            mbar_expect_tx(&sh->received, (uint32_t)((split - 1) * own_cols * kBM * 4));
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 2, %0;" ::"n"(kSplitThreads) : "memory");
+        if (lane == 0)
+            for (int i = 0; i < first; ++i) load_w(i, i);
+        __syncwarp();
+        asm volatile("bar.sync 3, 64;" ::: "memory");   // tensor memory has been allocated
+    } else {
+        if (warp == kCopyWarps) {
+            tmem_alloc(&sh->tmem_base, tmem_cols(bn));
+            tmem_relinquish();
+        }
+        tc_fence_before();
+        asm volatile("bar.sync 2, %0;" ::"n"(kSplitThreads) : "memory");
+        if (warp == kCopyWarps) asm volatile("bar.arrive 3, 64;" ::: "memory");
+    }
+    tc_fence_after();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this CTA runs: its memory may be written to
     pdl_wait();
     bool ok = true;
     if (warp < cw) {
         int s = warp;
-        uint32_t ph = 1;
-        for (int i = warp; i < kn; i += cw) {
-            if (s >= S) { s -= S; ph ^= 1u; }
+        uint32_t ph = 0;
+        for (int i = warp + S; i < kn; i += cw) {
             ok = mbar_wait(&sh->empty[s], ph);
             if (!ok) break;
-            if (lane == 0) {
-                if (i >= S) load_w(s, i);
-                const int k0 = kp0 + i * p.panels, np = min(p.panels, kp1 - k0);
-                for (int j = 0; j < np; ++j)
-                    tma_load_2d(smem + (size_t)s * stage_bytes + j * kAPanel, &tmX, (k0 + j) * kBK, m0, &sh->full[s]);
-            }
+            if (lane == 0) { expect(s, i); load_w(s, i); load_x(s, i); }
             __syncwarp();
             s += cw;
+            if (s >= S) { s -= S; ph ^= 1u; }
         }
     } else if (warp == kCopyWarps) {
+        const uint32_t tmem = lds32(smem_u32(&sh->tmem_base)), full = smem_u32(&sh->full[0]), empty = smem_u32(&sh->empty[0]);
         const uint32_t idesc = make_idesc_f16(kBM, bn);
         const uint64_t a0 = make_smem_desc(smem_u32(smem), 16, 1024, 2);
         const uint64_t b0 = make_smem_desc(smem_u32(smem) + p.panels * kAPanel, 16, 1024, 2);
-        int s = 0;
-        uint32_t ph = 0;
-        for (int i = 0; i < kn; ++i) {
-            ok = mbar_wait(&sh->full[s], ph);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t ph = 0;
+            for (int i = 0; i < kn; ++i) {
+                ok = mbar_wait_at(full + s * 8, ph);
+                if (!ok) break;
+                tc_fence_after();
                 const uint64_t at = (uint64_t)(s * stage_bytes) >> 4;   // descriptors count 16-byte units
                 const int np = min(p.panels, kp1 - kp0 - i * p.panels);
                 for (int j = 0; j < np; ++j)
@@ -457,14 +499,18 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
                     for (int ks = 0; ks < 4; ++ks)
                         umma_f16(tmem, a0 + at + (j * kAPanel >> 4) + ks * 2, b0 + at + (j * b_panel >> 4) + ks * 2, idesc,
                                  (i > 0 || j > 0 || ks > 0) ? 1u : 0u);
-                umma_commit(&sh->empty[s]);
-                if (i + 1 == kn) umma_commit(&sh->acc_full[0]);
+                umma_commit_at(empty + s * 8);
+                if (i + 1 == kn) umma_commit_at(smem_u32(&sh->acc_full[0]));
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
-            __syncwarp();
-            if (++s == S) { s = 0; ph ^= 1u; }
         }
-    } else {
-        // the bias, which may be the caller's and the preceding kernel's result (read after the second cluster barrier)
+        __syncwarp();
+    }
+    if (warp > kCopyWarps) {
+        if (lane == 0)
+            for (int i = warp - kCopyWarps - 1; i < first; i += kSplitThreads / 32 - kCopyWarps - 1) load_x(i, i);
+        __syncwarp();
+        // the bias, which may be the caller's and the preceding kernel's result (read behind the barrier below)
         for (int i = tid - 32 * (kCopyWarps + 1); i < own_cols; i += kSplitThreads - 32 * (kCopyWarps + 1)) {
             const int n = n0 + rank * own_cols + i;
             sh->bias[0][i] = n < p.N ? p.bias[n] : __float2half(0.f);
@@ -479,6 +525,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
     }
     __syncwarp();
     tc_fence_after();
+    const uint32_t tmem = sh->tmem_base;
     pdl_launch_dependents();
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA of the cluster runs
     const int q = warp & 3, h = warp >> 2;   // two warps per 32 rows
@@ -495,10 +542,14 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
             const int dst = (c + 4 * i) / own_cols, g = (c + 4 * i - dst * own_cols) / 4;
             if (dst == rank) continue;   // the same for the whole CTA
             const int from = rank < dst ? rank : rank - 1;
-            st_cluster(smem_u32(recv + ((size_t)from * (own_cols / 4) + g) * kBM + row), dst, r + 4 * i);
+            st_async_cluster(smem_u32(recv + ((size_t)from * (own_cols / 4) + g) * kBM + row), smem_u32(&sh->received), dst, r + 4 * i);
         }
     }
-    cluster_sync();   // what was sent has arrived (nobody touches another CTA's memory from here on)
+    __syncthreads();                                                        // the bias lies in shared memory
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this warp has sent everything
+    const bool got = mbar_wait_cluster(smem_u32(&sh->received), 0);
+    if (!got && lane == 0) atomicExch(p.err, 35);
+    __syncwarp();
     auto finish = [&](const uint32_t* own, int c, uint32_t* out) {   // four of the own columns, from c on
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         for (int k = 0; k < split; ++k) {   // in the order of the shares
@@ -557,6 +608,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) dense_split_kernel(const __g
         }
         __syncwarp();
     }
+    // Normally all have sent when this CTA has received. One that gave up stays until nothing is on its way to it.
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (!got) mbar_wait_cluster(smem_u32(&sh->received), 0);
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -573,27 +628,31 @@ static int panels_for(int bn, int split) { return split > 1 || bn <= 128 ? 2 : 1
 static int split_capacity(int split) { return split == 8 ? 14 * 8 : split == 4 ? 33 * 4 : sm_count() / split * split; }
 
 // Cost in clocks of a launch over `tokens` with tile width bn and the K range split over `split` CTAs: waves of tiles, each
-// K panel taking its UMMAs (2 bn clocks) or its copies (an SM gets ~58 bytes per clock from L2 when all ask), plus what comes
-// before the first UMMA and after the last one. Fitted to launches of 64 to 32768 tokens (within 20 %).
+// K panel taking its UMMAs (2 bn clocks) or its copies (an SM gets 55-67 bytes per clock from L2 when all ask), plus what comes
+// before the first UMMA and after the last one, and what the columns exchanged within a cluster take. Fitted to launches of 64 to 4096 tokens
+// and ten shapes in every width and split: the plan taken is 0.3 % slower than the fastest in the mean, 8 % at most. (64 x 768 -> 2304 5.8 us in 36 tiles split in two, 7.4 in 9
+// pairs; 384 x 768 -> 1152 5.6 in 36 pairs' tiles of 64, 6.5 in 72 of 32.)
 static double dense_cost(int tokens, int N, int K, int bn, int split) {
     const int tiles_n = (N + bn - 1) / bn;
     const int panels = (K + kBK - 1) / kBK;
     if (split == 1) {
-        const int pairs = sm_count() / 2;
-        const int waves = ((tokens + 2 * kBM - 1) / (2 * kBM) * tiles_n + pairs - 1) / pairs;
-        const double panel = std::max({2.0 * bn, (kAPanel + bn * 64.0) / 58.0, 400.0 / panels_for(bn, 1)});
+        const int pairs = sm_count() / 2, tiles = (tokens + 2 * kBM - 1) / (2 * kBM) * tiles_n;
+        const int waves = (tiles + pairs - 1) / pairs;
+        // Where the next launch finds SMs free it starts under this one: 512 x 768 -> 1152 takes 5.6 us on 72 SMs and 6.6 on 144.
+        const double full = 2 * tiles > sm_count() - 16 ? 2400.0 : 2 * tiles > sm_count() / 2 ? 1950.0 : 0.0;
+        const double panel = std::max({2.0 * bn, (kAPanel + bn * 64.0) / 67.0, 475.0 / panels_for(bn, 1)});
         const double tile = std::max(panels * panel, bn * 9.0);   // the main loop, or the stores of the tile before
         // a long launch of dense UMMAs runs at the power limit: 1.4e15 operations per second on the whole GPU, those for the columns
         // that fill up the last tile included (65536 x 768 -> 384 in tiles of 256 columns 45.4 us, of 192 41.7; 24000 -> 576 25.2 and 23.5)
         const double power = 2.0 * tokens * tiles_n * bn * (double)K / 1.4e15 * 1.9e9;
-        return 9500.0 + std::max(waves * tile + bn * 9.0, power);
+        return 5800.0 + std::max(full + waves * tile + bn * 15.0, power);
     }
     const int tiles = std::max(1, (tokens + kBM - 1) / kBM) * tiles_n;
-    const double panel = std::max({2.0 * bn, (kAPanel + bn * 128.0) / 58.0, 200.0});
+    const double panel = std::max({2.0 * bn, (kAPanel + bn * 128.0) / 55.0, 360.0});
     const int waves = (tiles * split + split_capacity(split) - 1) / split_capacity(split);
     // clusters on nearly all SMs: the last ones start late
-    const double full = tiles * split > sm_count() - 16 ? 1500.0 : tiles * split > sm_count() - 48 ? 300.0 : 0.0;
-    return 5500.0 + full + waves * (3500.0 + ((panels + split - 1) / split) * panel + bn * 45.0);
+    const double full = tiles * split > sm_count() - 16 ? 1250.0 : tiles * split > sm_count() - 48 ? 650.0 : 0.0;
+    return 6000.0 + full + waves * (((panels + split - 1) / split) * panel + bn * 48.0 * (split - 1) / split);
 }
 
 DensePlan dense_plan(int tokens, int N, int K) {

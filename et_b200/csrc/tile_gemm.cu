@@ -917,17 +917,21 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     }
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
-    // 1.2 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 82, 1024 -> 3072 96 / 90 / 128, 1024 ->
+    // 1.28 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 82, 1024 -> 3072 96 / 90 / 128, 1024 ->
     // 4096 148 / 118 / 171; at 50 % 1024 -> 4096 186 / 189 / 181. All constants were measured over 456 linears (128 to 65536 tokens,
-    // eight shapes, six sparsities): the form and block-rows taken are 0.28 % slower than the fastest in the mean, 12 choices are more than 5 % off.
-    tile_cost = 1.2 * tile_cost + 1450.0;
+    // eight shapes, six sparsities): the form and block-rows taken are 0.24 % slower than the fastest in the mean, 10 choices are more than 5 % off.
+    tile_cost = 1.28 * tile_cost + 50.0;
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
     const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
-    // (The dense form gives way to the resident one, which sums in another order, only for 20 % that its model promises: that costs 0.1 % in the
-    // mean of those linears, all of it at 4096 x 768 -> 2304 at 50 %, 14.6 instead of 12.6 us.)
-    w->packed_dense = plain && 0.97 * w->dense.cost < tile_cost && 0.8 * w->dense.cost < resident;
+    // (The dense form, which may sum in another order, is taken over the tile form only where its model promises 5 % and 1300 clocks: 300 x 1024 ->
+    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5. A long launch of a weight with every tile needs no such
+    // margin, its epilogue does not look for results to be computed again: 4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024 14.6 and 11.7. The dense
+    // form gives way to the resident one for 15 %: 4096 x 768 -> 2304 at 50 % stays dense, 14.7 against 12.9 us, the largest loss of the rules.)
+    const bool every_tile = ntile == (long)NBR * (K / 16);
+    const double dense_cost = every_tile && w->dense.cost > 16000.0 ? w->dense.cost : 1.05 * w->dense.cost + 1300.0;
+    w->packed_dense = plain && dense_cost < tile_cost && 0.85 * w->dense.cost < resident;
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);

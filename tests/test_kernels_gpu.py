@@ -324,6 +324,29 @@ def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
+@pytest.mark.parametrize("T,K,N,sparsity,gelu", [
+    (1, 768, 768, 0.0, False),        # K in four shares of three panels, the last stage of one panel
+    (128, 768, 2304, 0.0, False),     # two shares
+    (130, 4096, 1024, 0.0, True),     # a second tile of two tokens
+    (128, 4096, 1040, 0.5, False),    # columns beyond N, zeros among the tiles
+    (256, 8192, 768, 0.0, False),     # more stages than the ring holds: stages filled again by the copying warps
+    (96, 1040, 400, 0.0, True),       # a partial last panel, shares of unequal length
+    (200, 528, 336, 0.25, False),
+])
+def test_dense_linear_split_over_a_cluster(et, orc, T, K, N, sparsity, gelu):
+    """The K range split over a cluster: first stages and later ones, sums from all shares, repeated calls with other activations in
+    between give the same bits."""
+    got, want, w = _run_tile(et, orc, T, K, N, sparsity, seed=T + K + N, gelu=gelu, size=T)
+    util.assert_close(got, want, what=f"split dense linear T={T} K={K} N={N}")
+    xs = [dev(util.activations(7 + i, (T, K))) for i in range(2)]
+    ys = [torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(6)]
+    for i, y in enumerate(ys):
+        w.run(y, xs[i % 2])
+    torch.cuda.synchronize()
+    w.check()
+    assert all(torch.equal(ys[i % 2], y) for i, y in enumerate(ys))
+
+
 @pytest.mark.parametrize("T,K,N,sparsity,form", [(300, 1024, 1024, 0.24, "tile"), (400, 1024, 1024, 0.24, "tile"),
                                                  (32768, 768, 2304, 0.75, "resident"), (131072, 1024, 4096, 0.9, "resident"),
                                                  (17771, 3072, 768, 0.75, "tile"), (32768, 4096, 1024, 0.75, "tile"), (128, 3072, 768, 0.75, "dense")])

@@ -510,12 +510,13 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
         // Rows in flight per group against blocks per SM. A row of two granules a lane leaves registers for a fourth block when only one is in flight, which
         // is the faster way without a mask (300 x 300 x 300 31.5 -> 30.6 us, 370 39.3 -> 37.6, 500 60.8 -> 56.5), and with one where rows fill their granules and a
         // group has few of them (128 x 500 x 500 30.2 -> 28.5, 300 60.3 -> 58.8; but 512 98.5 -> 100.4, 128 x 411 x 411 23.1 -> 23.8, 300 x 300 x 300 33.5 -> 36.4). Rows of nearly
-        // one granule a lane: two in flight and four blocks (512 x 250 x 250 without a mask 34.8 -> 33.1, with one 36.7 -> 36.0; 512 x 203 x 203 with one 29.2 -> 29.6).
+        // one granule a lane: two in flight and four blocks where a group has many (512 x 242 x 242 without a mask 33.1 -> 31.9, 239 17.5 -> 16.9, with one 400 28.9 -> 28.0;
+        // but 128 10.6 -> 10.9, with a mask 239 18.0 -> 18.3 and 128 11.6 -> 12.1; 512 x 203 x 203 with one 29.2 -> 29.6).
+        const bool many = seq_len > 232 && (long)nmat * seq_len > (kMask ? 17L : 9L) * sm_count() * 4 * 8;
         const bool deep = kMask && (seq_len < 464 || (long)nmat * seq_len > 42L * sm_count() * 4 * 8);
         if (seq_len <= 64 ? run_many(softmax_many_kernel<8, 1, 3, kMask, 3>, 8, 3)
             : seq_len <= 128 ? run_many(softmax_many_kernel<16, 1, 3, kMask, 3>, 16, 3)
-            : seq_len <= 232 ? run_many(softmax_many_kernel<32, 1, 3, kMask, 3>, 32, 3)
-            : seq_len <= 256 ? run_many(softmax_many_kernel<32, 1, 2, kMask, 4>, 32, 4)
+            : seq_len <= 256 ? (many ? run_many(softmax_many_kernel<32, 1, 2, kMask, 4>, 32, 4) : run_many(softmax_many_kernel<32, 1, 3, kMask, 3>, 32, 3))
             : seq_len <= 512 ? (deep ? run_many(softmax_many_kernel<32, 2, 2, true, 3>, 32, 3) : run_many(softmax_many_kernel<32, 2, 1, kMask, 4>, 32, 4)) : false)
             return;
         if (seq_len <= 64) run(softmax_mask_kernel<8, 1, R, kMask>, 8, R);

@@ -105,9 +105,11 @@ __global__ void __launch_bounds__(256, (CH <= 4 ? 3 : 1)) skip_layernorm_vec(hal
 // linear before. Against the kernel above, with operands in L2: 8192 x 256 3.5 -> 3.0 us, x 512 5.5 -> 4.3, x 768 7.1 -> 5.6, x 1024
 // 9.2 -> 6.9, x 1280 16.9 -> 8.3, x 2048 22.2 -> 11.6; from memory: 17771 x 768 15.4 -> 14.2, x 1024 21.9 -> 18.3, x 2048 50 -> 35,
 // 131072 x 768 95.5 -> 96, x 1024 132 -> 124, x 2048 304 -> 240. Without a residual 17771 x 768 13.1 -> 10.4, x 2048 45.7 -> 25.5.
+// kOne, for few rows, which a chain of latencies bounds: a warp has one row and requests gamma and beta with it, not behind its reductions, and
+// small blocks spread the rows over the SMs.
 constexpr int row_blocks(int ch) { return ch <= 1 ? 6 : ch <= 2 ? 4 : ch <= 3 ? 3 : ch <= 6 ? 2 : 1; }   // per SM
-template <int CH, bool kSkip>
-__global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half* __restrict__ in_out, const half* __restrict__ skip,
+template <int CH, bool kSkip, bool kOne>
+__global__ void __launch_bounds__(256, kOne ? 1 : row_blocks(CH)) skip_layernorm_rows(half* __restrict__ in_out, const half* __restrict__ skip,
                                                                        const half* __restrict__ gamma, const half* __restrict__ beta, int num) {
     pdl_launch_dependents();
     pdl_wait();
@@ -126,7 +128,17 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
             if constexpr (kSkip) sv[i] = __ldcs(sr + 32 * i);
         }
     };
-    if (warp < num) load();
+    uint4 gv[CH], bv[CH];   // kOne
+    if (warp < num) {
+        load();
+        if constexpr (kOne) {
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                gv[i] = __ldg(reinterpret_cast<const uint4*>(gamma) + lane + 32 * i);
+                bv[i] = __ldg(reinterpret_cast<const uint4*>(beta) + lane + 32 * i);
+            }
+        }
+    }
     for (int row = warp; row < num; row += nwarp) {
         uint4* const out = xr;
         float v[CH][8];
@@ -143,9 +155,11 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
                 sum += v[i][2 * j] + v[i][2 * j + 1];
             }
         }
-        xr += step;
-        sr += step;
-        if (row + nwarp < num) load();
+        if constexpr (!kOne) {
+            xr += step;
+            sr += step;
+            if (row + nwarp < num) load();
+        }
         sum = warp_sum(sum);
         float sq = 0.f;
 #pragma unroll
@@ -155,8 +169,14 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
         const float rstd = inv_std(warp_sum(sq), 1.0f / kSize);
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
-            const uint4 g = __ldg(reinterpret_cast<const uint4*>(gamma) + lane + 32 * i);
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(beta) + lane + 32 * i);
+            uint4 g, b;
+            if constexpr (kOne) {
+                g = gv[i];
+                b = bv[i];
+            } else {
+                g = __ldg(reinterpret_cast<const uint4*>(gamma) + lane + 32 * i);
+                b = __ldg(reinterpret_cast<const uint4*>(beta) + lane + 32 * i);
+            }
             const half2* gh = reinterpret_cast<const half2*>(&g);
             const half2* bh = reinterpret_cast<const half2*>(&b);
             uint4 o;
@@ -169,6 +189,7 @@ __global__ void __launch_bounds__(256, row_blocks(CH)) skip_layernorm_rows(half*
             }
             out[32 * i] = o;
         }
+        if constexpr (kOne) break;
     }
 }
 
@@ -286,13 +307,26 @@ int et::layernorm_launch(half* x, const half* s, const half* g, const half* b, i
     blocks = std::min(blocks, sm_count() * per_sm);
     if (vec && size % 256 == 0) {   // every lane's chunks are whole
         using RowsFn = void (*)(half*, const half*, const half*, const half*, int);
-        static const RowsFn rows[8][2] = {{skip_layernorm_rows<1, false>, skip_layernorm_rows<1, true>}, {skip_layernorm_rows<2, false>, skip_layernorm_rows<2, true>},
-                                          {skip_layernorm_rows<3, false>, skip_layernorm_rows<3, true>}, {skip_layernorm_rows<4, false>, skip_layernorm_rows<4, true>},
-                                          {skip_layernorm_rows<5, false>, skip_layernorm_rows<5, true>}, {skip_layernorm_rows<6, false>, skip_layernorm_rows<6, true>},
-                                          {skip_layernorm_rows<7, false>, skip_layernorm_rows<7, true>}, {skip_layernorm_rows<8, false>, skip_layernorm_rows<8, true>}};
+        static const RowsFn rows[8][2] = {{skip_layernorm_rows<1, false, false>, skip_layernorm_rows<1, true, false>}, {skip_layernorm_rows<2, false, false>, skip_layernorm_rows<2, true, false>},
+                                          {skip_layernorm_rows<3, false, false>, skip_layernorm_rows<3, true, false>}, {skip_layernorm_rows<4, false, false>, skip_layernorm_rows<4, true, false>},
+                                          {skip_layernorm_rows<5, false, false>, skip_layernorm_rows<5, true, false>}, {skip_layernorm_rows<6, false, false>, skip_layernorm_rows<6, true, false>},
+                                          {skip_layernorm_rows<7, false, false>, skip_layernorm_rows<7, true, false>}, {skip_layernorm_rows<8, false, false>, skip_layernorm_rows<8, true, false>}};
+        static const RowsFn one[8][2] = {{skip_layernorm_rows<1, false, true>, skip_layernorm_rows<1, true, true>}, {skip_layernorm_rows<2, false, true>, skip_layernorm_rows<2, true, true>},
+                                         {skip_layernorm_rows<3, false, true>, skip_layernorm_rows<3, true, true>}, {skip_layernorm_rows<4, false, true>, skip_layernorm_rows<4, true, true>},
+                                         {skip_layernorm_rows<5, false, true>, skip_layernorm_rows<5, true, true>}, {skip_layernorm_rows<6, false, true>, skip_layernorm_rows<6, true, true>},
+                                         {skip_layernorm_rows<7, false, true>, skip_layernorm_rows<7, true, true>}, {skip_layernorm_rows<8, false, true>, skip_layernorm_rows<8, true, true>}};
         const int ch = size / 256;
-        const dim3 grid(std::min((warps_needed + 7) / 8, sm_count() * row_blocks(ch)));
-        launch_pdl(rows[ch - 1][s != nullptr], grid, dim3(256), 0, st, x, s, g, b, num);
+        // One row a warp in blocks of two warps where all have a place at once and an SM gets up to seven rows of 768; of rows of up to 768 elements
+        // up to 14, in blocks of one (128 x 768 2.22 -> 1.70 us, 1024 x 768 2.73 -> 2.22, 2048 x 768 2.92 -> 2.56, 300 x 1024 2.30 -> 1.81, 256 x 2048
+        // 2.90 -> 2.30; but 1024 x 1024 2.69 and 2.67, 1500 x 1024 2.84 and 2.97).
+        const long sms = sm_count(), elements = (long)num * size;
+        const int one_warps = elements <= 5400 * sms ? 2 : size <= 768 && num <= 14 * sms ? 1 : 0;
+        if (one_warps) {
+            launch_pdl(one[ch - 1][s != nullptr], dim3((num + one_warps - 1) / one_warps), dim3(32 * one_warps), 0, st, x, s, g, b, num);
+        } else {
+            const dim3 grid(std::min((warps_needed + 7) / 8, sm_count() * row_blocks(ch)));
+            launch_pdl(rows[ch - 1][s != nullptr], grid, dim3(256), 0, st, x, s, g, b, num);
+        }
     } else if (vec) {
         const int ch = (size / 8 + 31) / 32;
         switch (ch) {

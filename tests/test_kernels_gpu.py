@@ -104,6 +104,19 @@ def test_skip_layernorm_rounds_alike_in_every_kernel(et, num, size):
     assert torch.equal(x, want), f"{int((x != want).sum())} results differ"
 
 
+@pytest.mark.parametrize("num,size", [(1, 256), (3121, 256), (3122, 256), (3, 512), (2072, 512), (2073, 512), (1040, 768), (1041, 768), (2072, 768), (2073, 768), (780, 1024),
+                                      (781, 1024), (5, 1280), (520, 1536), (445, 1792), (390, 2048), (391, 2048)])
+def test_skip_layernorm_of_few_rows_rounds_alike(et, num, size):
+    """One row to a warp, in blocks of one and two warps, and the first sizes that are not: the bits of the other kernels."""
+    gen = torch.Generator("cuda").manual_seed(num + size)
+    x, s = (torch.randn((num, size), generator=gen, device="cuda").half() for _ in range(2))
+    g, b = (torch.randn((size,), generator=gen, device="cuda").half() for _ in range(2))
+    want = _layernorm_in_fp32(x, s, g, b)
+    et.skip_layernorm(x, s, g, b)
+    torch.cuda.synchronize()
+    assert torch.equal(x, want), f"{int((x != want).sum())} results differ"
+
+
 @pytest.mark.parametrize("num,size,offset", [(3, 1, 0), (5, 33, 0), (4, 769, 0), (2, 2049, 0), (5, 200, 1), (3, 768, 3), (2, 1538, 1), (7, 2, 0), (9, 770, 2)])
 def test_skip_layernorm_rows_anywhere(et, orc, num, size, offset):
     """Odd widths, and bases on 2-byte and 4-byte boundaries: single elements and pairs."""

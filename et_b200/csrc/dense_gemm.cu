@@ -14,14 +14,15 @@
 // so that a tile is stored while the next one is multiplied. 16384 x 4096 x 1024: tensor pipe 90 % busy.
 //
 // dense_split_kernel, few tiles (small batches): the K range is split over a thread-block cluster. Each CTA accumulates its
-// share and finishes 1/cluster of the tile's columns: it sends the other CTAs the fp32 parts of theirs (stores to distributed shared
-// memory), and after a cluster barrier adds what it was sent to its own, in rank order (no atomics: results do not depend on timing).
-// Until then each left its whole part in its own memory and loaded rows of the others': 128 x 3072 -> 768 8.5 -> 6.6 us, 4096 -> 1024
-// 10.6 -> 7.7, 256 x 3072 -> 768 12.0 -> 8.1. 128 tokens, 768 (1024) inputs and outputs, which were faster in the tile kernel, 6.4 -> 4.4
-// (8.2 -> 4.6).
+// share and finishes 1/cluster of the tile's columns: it sends the other CTAs the fp32 parts of theirs (asynchronous stores to
+// distributed shared memory that count towards a barrier of the receiver), and when its own bytes have arrived adds them to its part, in rank order
+// (no atomics: results do not depend on timing). With parts left in place and rows of the others' loaded 128 x 3072 -> 768 took 8.5 us (5.7 now),
+// 4096 -> 1024 10.6 (6.3), 256 x 3072 -> 768 12.0 (7.0); with stores and a barrier of the cluster 6.3, 7.3 and 7.8. 128 x 768 -> 768 in the tile
+// kernel 5.1 us, here 3.9.
 // (A K share per pair of CTAs with tiles of 256 tokens: 1024 x 3072 -> 768 12.4 against 12.1 us, 2048 16.8 against 13.9.)
 //
-// The weight does not depend on the preceding kernel: its first copies are requested before griddepcontrol.wait.
+// The weight does not depend on the preceding kernel: its first copies are requested before griddepcontrol.wait. In both kernels the activations of the
+// first stages are requested by warps that have nothing else to do yet, right behind that wait.
 // Every mbarrier wait is bounded; a role that gives up records a code, and all threads reach the common exit (and the
 // cluster barriers) whatever happened.
 #include <algorithm>

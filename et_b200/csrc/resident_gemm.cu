@@ -570,6 +570,8 @@ void resident_free(ResidentWeight* w) {
 }
 
 size_t resident_bytes(const ResidentWeight* w) { return w->bytes; }
+int resident_block_rows() { return kRows; }
+int resident_groups(const ResidentWeight* w) { return w->groups; }
 
 template <typename F>
 static int run(const ResidentWeight* w, half* Y, const half* X, const half* bias, bool bias_given, int T, int gelu, int* err, cudaStream_t st) {

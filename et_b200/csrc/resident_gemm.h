@@ -14,6 +14,9 @@ double resident_cost(int tokens, int N, int K, double density);
 int resident_pack(ResidentWeight** out, int K, int N, const half* data, const int* row_ptr, const int* row_offset);
 void resident_free(ResidentWeight* w);
 size_t resident_bytes(const ResidentWeight* w);
+// Block-rows per group of features, and groups.
+int resident_block_rows();
+int resident_groups(const ResidentWeight* w);
 // bias_given: the bias is the caller's and may be the result of the kernel before.
 int resident_run(const ResidentWeight* w, half* Y, const half* X, const half* bias, bool bias_given, int T, int gelu, int* err, cudaStream_t st);
 

@@ -1155,7 +1155,7 @@ int tile_weight_error(const TileWeight* w, int* code) {
 
 void tile_weight_info(const TileWeight* w, int* info) {
     if (w->resident) {
-        const int v[6] = {4, (w->N + 63) / 64, (w->K + kKC - 1) / kKC, 0, 0, (int)std::min<size_t>(resident_bytes(w->resident), 0x7fffffff)};
+        const int v[6] = {resident_block_rows(), resident_groups(w->resident), (w->K + kKC - 1) / kKC, 0, 0, (int)std::min<size_t>(resident_bytes(w->resident), 0x7fffffff)};
         std::copy(v, v + 6, info);
         return;
     }

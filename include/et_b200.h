@@ -73,7 +73,8 @@ int et_set_attention_scores_fp32(int on);
 int et_attention_scores_fp32(void);
 /* info[6] = {block_rows_per_cta, n_chunks, k_chunks, stages, stage_bytes, packed_bytes}. The form the weight was packed in
  * for the expected token count: tile (stage_bytes > 0), dense (stage_bytes 0, stages = CTAs that share a tile's K range), or
- * activations resident in tensor memory (stages and stage_bytes 0). */
+ * activations resident in tensor memory (stages and stage_bytes 0; the chunks are groups of features, every CTA takes a
+ * range of them). */
 int et_tile_weight_info(const et_tile_weight* w, int* info);
 /* Same contraction from DEVICE-resident tile arrays, K = in_feat explicit. The packed form of a
  * weight is built on its first use (device-to-host copy, synchronous: not inside a stream capture) and cached

@@ -370,6 +370,18 @@ def test_the_form_that_was_measured_as_the_fastest_is_taken(et, orc, T, K, N, sp
     assert form == ("tile" if info["stage_bytes"] else "dense" if info["stages"] else "resident"), info
 
 
+@pytest.mark.parametrize("K,N,sparsity,size,form,rows", [(768, 2304, 0.75, 32768, "resident", 2), (768, 3088, 0.75, 32768, "resident", 2), (1024, 1024, 0.9, 32768, "resident", 2),
+                                                         (3072, 768, 0.75, 17792, "tile", None), (3072, 784, 0.0, 512, "dense", None)])
+def test_weight_info_tells_how_the_features_are_cut(et, orc, K, N, sparsity, size, form, rows):
+    """Block-rows per chunk times chunks cover the features, without a chunk too many, in every form; a group of the resident form is two block-rows
+    (an odd number of block-rows leaves the last group with one)."""
+    rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, K + N, True, 0.05)
+    info = et.TileWeight(K, N, size, data, rp, ro, bias).info()
+    assert form == ("tile" if info["stage_bytes"] else "dense" if info["stages"] else "resident"), info
+    assert rows in (None, info["nb"])
+    assert info["n_chunks"] == -(-N // (16 * info["nb"])) and info["k_chunks"] == -(-K // 128), info
+
+
 @pytest.mark.parametrize("N,tokens", [(384, 65536), (576, 24000), (576, 65536)])
 def test_long_dense_launches_have_no_columns_to_fill_up(et, orc, N, tokens):
     """A launch at the power limit takes the tile width that divides its columns."""

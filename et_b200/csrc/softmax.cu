@@ -268,7 +268,6 @@ __global__ void __launch_bounds__(256) softmax_mask_kernel(half* __restrict__ sc
     }
 }
 
-
 // The order in which the rows of any alignment are taken: a row index of the matrices c, c + 8, c + 16, ... (whose rows have the same
 // alignment whatever the length, so the mask row stays in registers), the next row index, the next c.
 struct RowWalk {
@@ -306,11 +305,11 @@ struct RowWalk {
 // fetched, shifted and put in place once for all matrices of its class, and added by mixed-precision additions. What bounds it is the
 // memory system at that size (aligned rows of 504 elements take 25.6 us, 128 matrices) and D times the registers; the kernel above, with
 // the next row requested when one is done, is the faster one where a group has few rows or a mask row few matrices.
-// 128 x 500 x 500 with a mask 32.1 -> 28.5 us (from memory), without 33.3 -> 26.4; 1024 x 500 x 500 with one 246 -> 207; 512 x 77 x 77 10.3 -> 8.7.
+// 128 x 500 x 500 with a mask 32.1 -> 29.3 us, without 33.3 -> 26.4; 1024 x 500 x 500 with one 246 -> 212; 512 x 77 x 77 10.3 -> 8.7.
 // (As blocks of rows that a warp of its own copies in and out in bulk: 32.8 us and slower at every length.)
 template <int G, int CH, int D, bool kMask, int kPerSm>
 __global__ void __launch_bounds__(256, kPerSm) softmax_many_kernel(half* __restrict__ scores, const half* __restrict__ mask, int nmat, int L,
-                                                                            int valid, unsigned rows) {
+                                                                   int valid, unsigned rows) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & (G - 1);
@@ -491,8 +490,9 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
             launch_pdl(kernel, dim3((unsigned)blocks), dim3(256), 0, st, s + (size_t)at * seq_len * seq_len, m, nrow, seq_len, valid_len);
         }
     };
-    // Five rows a group, and for a mask six matrices of a class (30 x 509 x 509, four rows: 10.4 us here, 10.7 there; 500 x 45 x 45,
-    // two rows: 3.1 and 4.0; 16 x 1001 x 1001, two matrices: 18.8 and 24.4).
+    // Five rows to each group that three blocks an SM have (whatever the grid), and for a mask six matrices of a class (softmax_mask_kernel and this one, us:
+    // 30 x 509 x 509, four rows, 10.4 and 10.7; 500 x 45 x 45, two rows, 3.1 and 4.0; 16 x 1001 x 1001, two matrices, 18.8 and 24.4. Without a mask around the line, in
+    // L2 / from memory: 36 x 500 x 500 7.0 / 10.6 and 8.3 / 10.2, 48 x 465 x 465 12.0 / 14.6 and 10.5 / 11.7, 64 x 300 x 300 11.4 / 12.7 and 9.5 / 9.5.)
     auto run_many = [&](auto kernel, int group, int per_sm) {
         if ((long)nmat * seq_len < 5L * sm_count() * 3 * (256 / group) || (m && nmat < 48)) return false;
         const int most = std::max(8, per_launch / 8 * 8);   // a launch begins with a matrix of the first one's alignment
@@ -507,17 +507,16 @@ extern "C" int et_softmax_mask(void* scores, const void* mask, int nmat, int seq
     auto pick = [&](auto masked) {
         constexpr bool kMask = decltype(masked)::value;
         constexpr int R = kMask ? 1 : 2;
-        // Rows in flight per group against blocks per SM. A row of two granules a lane leaves registers for a fourth block when only one is in flight, which
-        // is the faster way without a mask (300 x 300 x 300 31.5 -> 30.6 us, 370 39.3 -> 37.6, 500 60.8 -> 56.5), and with one where rows fill their granules and a
-        // group has few of them (128 x 500 x 500 30.2 -> 28.5, 300 60.3 -> 58.8; but 512 98.5 -> 100.4, 128 x 411 x 411 23.1 -> 23.8, 300 x 300 x 300 33.5 -> 36.4). Rows of nearly
-        // one granule a lane: two in flight and four blocks where a group has many (512 x 242 x 242 without a mask 33.1 -> 31.9, 239 17.5 -> 16.9, with one 400 28.9 -> 28.0;
-        // but 128 10.6 -> 10.9, with a mask 239 18.0 -> 18.3 and 128 11.6 -> 12.1; 512 x 203 x 203 with one 29.2 -> 29.6).
-        const bool many = seq_len > 232 && (long)nmat * seq_len > (kMask ? 17L : 9L) * sm_count() * 4 * 8;
-        const bool deep = kMask && (seq_len < 464 || (long)nmat * seq_len > 42L * sm_count() * 4 * 8);
+        // Rows in flight per group against blocks per SM. A row of two granules a lane without a mask leaves registers for a fourth block when only one is in
+        // flight, which is the faster way whether the rows were just written, lie in L2 or come from memory (us, three rows and three blocks -> one and four: 300 x 300 x 300
+        // 31.5 -> 30.6, 370 39.3 -> 37.6, 500 60.8 -> 56.5; just written 512 x 465 x 465 83.1 -> 75.6; from memory 200 x 500 x 500 50.0 -> 41.6), but long rows want ten to a
+        // group (64 x 478 x 478 from memory 14.4 -> 15.3, 48 x 500 x 500 12.4 -> 12.9; 128 x 478 x 478 26.5 -> 25.3). With a mask, and up to 256 elements, it is not: its rows pass again
+        // and again 128 x 500 x 500 takes 29.3 -> 28.7 us, for the first time 39.0 -> 41.0, just written 24.2 -> 24.9; 512 x 233 x 233 just written 30.9 -> 32.8, without a mask 28.7 -> 29.1.
+        const bool four = !kMask && (seq_len < 430 || (long)nmat * seq_len >= 10L * sm_count() * 4 * 8);
         if (seq_len <= 64 ? run_many(softmax_many_kernel<8, 1, 3, kMask, 3>, 8, 3)
             : seq_len <= 128 ? run_many(softmax_many_kernel<16, 1, 3, kMask, 3>, 16, 3)
-            : seq_len <= 256 ? (many ? run_many(softmax_many_kernel<32, 1, 2, kMask, 4>, 32, 4) : run_many(softmax_many_kernel<32, 1, 3, kMask, 3>, 32, 3))
-            : seq_len <= 512 ? (deep ? run_many(softmax_many_kernel<32, 2, 2, true, 3>, 32, 3) : run_many(softmax_many_kernel<32, 2, 1, kMask, 4>, 32, 4)) : false)
+            : seq_len <= 256 ? run_many(softmax_many_kernel<32, 1, 3, kMask, 3>, 32, 3)
+            : seq_len <= 512 ? (four ? run_many(softmax_many_kernel<32, 2, 1, false, 4>, 32, 4) : run_many(softmax_many_kernel<32, 2, kMask ? 2 : 3, kMask, 3>, 32, 3)) : false)
             return;
         if (seq_len <= 64) run(softmax_mask_kernel<8, 1, R, kMask>, 8, R);
         else if (seq_len <= 128) run(softmax_mask_kernel<16, 1, R, kMask>, 16, R);

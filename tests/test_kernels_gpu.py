@@ -226,7 +226,8 @@ def test_softmax_many_rows_of_any_alignment(et, orc, nmat, L, offset, use_mask, 
 
 
 @pytest.mark.parametrize("nmat,L,use_mask", [(90, 231, True), (85, 233, True), (85, 233, False), (80, 255, True), (75, 255, False), (70, 257, False), (50, 463, True),
-                                             (50, 465, True), (50, 465, False), (49, 511, True), (190, 233, False), (330, 255, True)])
+                                             (50, 465, True), (50, 465, False), (49, 511, True), (190, 233, False), (330, 255, True), (109, 429, False),
+                                             (109, 431, False), (110, 431, False), (93, 510, False)])
 def test_softmax_rows_in_flight_by_length(et, orc, nmat, L, use_mask):
     """Lengths around which another number of rows is in flight, with enough matrices for it, three tokens masked at the end."""
     S, mask = util.activations(L, (nmat, L, L)), util.activations(L + 1, (L, L))

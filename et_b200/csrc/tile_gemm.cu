@@ -926,13 +926,16 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
     const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
     // (The dense form, which may sum in another order, is taken over the tile form only where its model promises 5 % and 1300 clocks: 300 x 1024 ->
-    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5. A long launch of a weight with every tile needs no such
-    // margin, its epilogue does not look for results to be computed again: 4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024 14.6 and 11.7. The dense
+    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5. Long launches need no such margin: those of a weight with every
+    // tile, whose epilogue does not look for results to be computed again (4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024 14.6 and 11.7), and
+    // beyond 60000 clocks all, where the tile kernel comes to the power limit, which its model does not know (32768 x 1024 -> 4096 at 40 % 229 and 188 us, 65536
+    // x 4096 -> 1024 414 and 354; with the line at 50000 or none the forms taken of 2106 linears are 0.53 and 0.57 % slower than the fastest, 0.51 here). The dense
     // and the resident form are taken as their models say. When the resident form had to promise 15 %, 24 of 1190 linears (0 to 80 % pruned, 64 to 65536
     // tokens, in_feat 768 and 1024) stayed dense that are 1 to 28 % faster resident: 8192 x 768 -> 3072 at 40 % 35.5 and 27.8 us, 8192 x 768 -> 1152 at
     // 50 % 15.8 and 13.0.)
     const bool every_tile = ntile == (long)NBR * (K / 16);
-    const double dense_cost = every_tile && w->dense.cost > 16000.0 ? w->dense.cost : 1.05 * w->dense.cost + 1300.0;
+    const bool as_it_says = w->dense.cost > (every_tile ? 16000.0 : 60000.0);
+    const double dense_cost = as_it_says ? w->dense.cost : 1.05 * w->dense.cost + 1300.0;
     w->packed_dense = plain && dense_cost < tile_cost && w->dense.cost < resident;
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)

@@ -454,9 +454,9 @@ static double group_clocks(int K, double density) {
     const double ts = kRows * density * std::min(K / 16, F::kSlices), ss = kRows * density * std::max(0, K / 16 - F::kSlices);
     return narrow ? std::max(420.0, 274.0 + 10.5 * ts) : std::max(530.0, 164.0 + 10.0 * ts + 64.0 * ss);
 }
-static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges) {
+static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges, double more = 0.0) {
     double best = 0;
-    const double start = ((K + 127) / 128) * 350.0 + 4400.0;   // copying a slab into place, per item
+    const double start = ((K + 127) / 128) * 350.0 + 4400.0 + more;   // copying a slab into place, per item
     for (int r = 1; r <= groups; ++r) {
         const int waves = (slabs * r + sm_count() - 1) / sm_count();
         const double c = 5200.0 + waves * (start + ((groups + r - 1) / r) * per_group);
@@ -470,9 +470,14 @@ static bool is_wide(int K) { return K / 16 > Narrow::kSlices; }
 double resident_cost(int tokens, int N, int K, double density) {
     if (K > kMaxK) return 1e30;
     int r = 1;
-    const int slabs = std::max(1, (tokens + kSlab - 1) / kSlab);
-    return is_wide(K) ? launch_clocks(slabs, (N / 16 + kRows - 1) / kRows, K, group_clocks<Wide>(K, density), &r)
-                      : launch_clocks(slabs, (N / 16 + kRows - 1) / kRows, K, group_clocks<Narrow>(K, density), &r);
+    const int slabs = std::max(1, (tokens + kSlab - 1) / kSlab), groups = (N / 16 + kRows - 1) / kRows;
+    const bool in_l2 = 2.0 * tokens * (K + N) <= 95e6;   // a launch's operands, beside the next one's
+    // Slabs that come from memory take longer with the ring of single panels, which covers L2's latency (65536 x 1024 -> 512 at 75 / 90 % resident 53 / 45 us, tile
+    // 43 / 38; two panels to a chunk fit as well without it: 65536 x 768 -> 1152 at 40 % 91, dense 100). Launches of many slabs from L2 are overestimated
+    // by 3 to 20 %, more than the other forms' by their models (12000 x 1024 -> 1536 at 95 % 15.7, tile 18.9; 4096 x 768 -> 3072 at 40 % 17.1, dense 20.5).
+    const double clocks = is_wide(K) ? launch_clocks(slabs, groups, K, group_clocks<Wide>(K, density), &r, in_l2 ? 0.0 : 2.0 * K)
+                                     : launch_clocks(slabs, groups, K, group_clocks<Narrow>(K, density), &r);
+    return in_l2 && tokens >= 2048 ? 0.96 * clocks : clocks;
 }
 
 template <typename F>

@@ -918,25 +918,25 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
     // 1.28 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 82, 1024 -> 3072 96 / 90 / 128, 1024 ->
-    // 4096 148 / 118 / 171; at 50 % 1024 -> 4096 186 / 189 / 181. All constants were measured over 456 linears (128 to 65536 tokens,
-    // eight shapes, six sparsities): the form and block-rows taken are 0.24 % slower than the fastest in the mean, 10 choices are more than 5 % off.
+    // 4096 148 / 118 / 171; at 50 % 1024 -> 4096 186 / 189 / 181. Over 2106 linears (1 to 65536 tokens, thirteen shapes, 0 to 95 %
+    // pruned) the form taken is 0.38 % slower than the fastest of the three in the mean, 47 are more than 5 % off, 14 more than 10 % (eleven of
+    // them one token); the constants of the tile and resident models were fitted together with the number of block-rows over 456 (128 to 65536 tokens).
     tile_cost = 1.28 * tile_cost + 50.0;
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
     const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
-    // (The dense form, which may sum in another order, is taken over the tile form only where its model promises 5 % and 1300 clocks: 300 x 1024 ->
-    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5. Long launches need no such margin: those of a weight with every
-    // tile, whose epilogue does not look for results to be computed again (4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024 14.6 and 11.7), and
-    // beyond 60000 clocks all, where the tile kernel comes to the power limit, which its model does not know (32768 x 1024 -> 4096 at 40 % 229 and 188 us, 65536
-    // x 4096 -> 1024 414 and 354; with the line at 50000 or none the forms taken of 2106 linears are 0.53 and 0.57 % slower than the fastest, 0.51 here). The dense
-    // and the resident form are taken as their models say. When the resident form had to promise 15 %, 24 of 1190 linears (0 to 80 % pruned, 64 to 65536
-    // tokens, in_feat 768 and 1024) stayed dense that are 1 to 28 % faster resident: 8192 x 768 -> 3072 at 40 % 35.5 and 27.8 us, 8192 x 768 -> 1152 at
-    // 50 % 15.8 and 13.0.)
+    // (The dense form, which may sum in another order, is taken over the tile form only where its model promises 5 % and, of short launches, 1300 clocks: 300 x 1024 ->
+    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5; but 4096 x 1024 -> 4096 at 40 % 30.7 and 27.9. Long launches need no such
+    // margin: those of a weight with every tile, whose epilogue does not look for results to be computed again (4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024
+    // 14.6 and 11.7), and beyond 60000 clocks all, where the tile kernel comes to the power limit, which its model does not know (32768 x 1024 -> 4096 at 40 %
+    // 229 and 188 us, 65536 x 4096 -> 1024 414 and 354). The dense and the resident form are taken as their models say. When the resident form had to promise 15 %, 24
+    // of 1190 linears (0 to 80 % pruned, 64 to 65536 tokens, in_feat 768 and 1024) stayed dense that are 1 to 28 % faster resident: 8192 x 768 -> 3072 at 40 %
+    // 35.5 and 27.8 us, 8192 x 768 -> 1152 at 50 % 15.8 and 13.0.)
     const bool every_tile = ntile == (long)NBR * (K / 16);
-    const bool as_it_says = w->dense.cost > (every_tile ? 16000.0 : 60000.0);
-    const double dense_cost = as_it_says ? w->dense.cost : 1.05 * w->dense.cost + 1300.0;
-    w->packed_dense = plain && dense_cost < tile_cost && w->dense.cost < resident;
+    const double dense = w->dense.cost;
+    const double dense_cost = dense > (every_tile ? 16000.0 : 60000.0) ? dense : 1.05 * dense + (dense > 30000.0 ? 0.0 : 1300.0);
+    w->packed_dense = plain && dense_cost < tile_cost && dense < resident;
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);

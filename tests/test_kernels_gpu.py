@@ -367,7 +367,8 @@ def test_dense_linear_split_over_a_cluster(et, orc, T, K, N, sparsity, gelu):
                                                  (8192, 768, 3072, 0.4, "resident"), (8192, 768, 1152, 0.5, "resident"), (17771, 768, 1152, 0.4, "resident"),
                                                  (4096, 768, 2304, 0.25, "dense"), (32768, 1024, 4096, 0.4, "dense"), (65536, 4096, 1024, 0.4, "dense"),
                                                  (65536, 1536, 1536, 0.4, "dense"), (65536, 1024, 512, 0.8, "tile"), (65536, 1024, 512, 0.9, "tile"),
-                                                 (65536, 1024, 1536, 0.9, "resident"), (12000, 1024, 1536, 0.95, "resident"), (4096, 768, 3072, 0.4, "resident")])
+                                                 (65536, 1024, 1536, 0.9, "resident"), (12000, 1024, 1536, 0.95, "resident"), (4096, 768, 3072, 0.4, "resident"),
+                                                 (4096, 1024, 4096, 0.4, "dense")])
 def test_the_form_that_was_measured_as_the_fastest_is_taken(et, orc, T, K, N, sparsity, form):
     """Where another form takes at least 5 % longer."""
     rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, K + N, False, 0.05)

@@ -457,12 +457,15 @@ static double group_clocks(int K, double density) {
 static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges, double more = 0.0) {
     double best = 0;
     const double start = ((K + 127) / 128) * 350.0 + 4400.0 + more;   // copying a slab into place, per item
-    for (int r = 1; r <= groups; ++r) {
-        const int waves = (slabs * r + sm_count() - 1) / sm_count();
-        const double c = 5200.0 + waves * (start + ((groups + r - 1) / r) * per_group);
+    const int sms = sm_count();
+    // Of the numbers of ranges with as many groups in the largest only the first can be the best (this runs at every launch: 128 groups all tried 0.61 us, 0.22 now).
+    for (int r = 1;;) {
+        const int most = (groups + r - 1) / r, waves = (slabs * r + sms - 1) / sms;
+        const double c = 5200.0 + waves * (start + most * per_group);
         if (best == 0 || c < best * 0.999) { best = c; *ranges = r; }
+        if (most == 1) return best;
+        r = (groups + most - 2) / (most - 1);
     }
-    return best;
 }
 
 static bool is_wide(int K) { return K / 16 > Narrow::kSlices; }

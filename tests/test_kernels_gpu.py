@@ -338,19 +338,22 @@ def test_tile_linear_forms(et, orc, T, K, N, sparsity, gelu, size, form):
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
-@pytest.mark.parametrize("T,K,N,sparsity,gelu", [
-    (1, 768, 768, 0.0, False),        # K in four shares of three panels, the last stage of one panel
-    (128, 768, 2304, 0.0, False),     # two shares
-    (130, 4096, 1024, 0.0, True),     # a second tile of two tokens
-    (128, 4096, 1040, 0.5, False),    # columns beyond N, zeros among the tiles
-    (256, 8192, 768, 0.0, False),     # more stages than the ring holds: stages filled again by the copying warps
-    (96, 1040, 400, 0.0, True),       # a partial last panel, shares of unequal length
-    (200, 528, 336, 0.25, False),
+@pytest.mark.parametrize("T,K,N,sparsity,gelu,shares,columns", [
+    (1, 768, 768, 0.0, False, 4, 8),         # three panels to a share, the last stage of one panel
+    (128, 768, 1152, 0.0, False, 2, 16),
+    (130, 4096, 1024, 0.0, True, 4, 16),     # a second tile of two tokens
+    (128, 4096, 1040, 0.5, False, 4, 8),     # columns beyond N, zeros among the tiles
+    (256, 8192, 768, 0.0, False, 8, 16),     # more stages than the ring holds: stages filled again by the copying warps
+    (96, 1040, 400, 0.0, True, 4, 8),        # a partial last panel, shares of unequal length
+    (64, 1552, 2304, 0.25, False, 4, 24),    # pruned, a partial last panel, 24 columns to a CTA
+    (700, 2064, 784, 0.25, True, 2, 48),
 ])
-def test_dense_linear_split_over_a_cluster(et, orc, T, K, N, sparsity, gelu):
+def test_dense_linear_split_over_a_cluster(et, orc, T, K, N, sparsity, gelu, shares, columns):
     """The K range split over a cluster: first stages and later ones, sums from all shares, repeated calls with other activations in
     between give the same bits."""
     got, want, w = _run_tile(et, orc, T, K, N, sparsity, seed=T + K + N, gelu=gelu, size=T)
+    info = w.info()
+    assert info["stage_bytes"] == 0 and info["stages"] == shares and 16 * info["nb"] == shares * columns, info
     util.assert_close(got, want, what=f"split dense linear T={T} K={K} N={N}")
     xs = [dev(util.activations(7 + i, (T, K))) for i in range(2)]
     ys = [torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(6)]
@@ -583,11 +586,12 @@ def test_tile_linear_of_sparse_and_full_block_rows(et, orc, T, K, sparse, full, 
 
 
 @pytest.mark.parametrize("T,K,full,gelu", [(129, 1024, (0, 1, 2, 3), False), (129, 1024, (5, 190), True), (20000, 768, (0, 1, 2, 3, 143), False), (257, 1008, (7, 64, 65), True),
-                                           (300, 832, (3, 100), False), (130, 848, (0, 191), True), (1, 784, (17,), False)])
+                                           (300, 832, (3, 100), False), (130, 848, (0, 191), True), (1, 784, (17,), False),
+                                           (20000, 1024, (0, 5, 100, 190, 191), True)])
 def test_resident_linear_with_groups_in_several_blocks(et, orc, T, K, full, gelu):
     """Groups of block-rows whose tiles exceed a slot of the weight ring are cut into blocks, first and last groups among them, beside groups in one block
     and block-rows without tiles; a block may hold none of a block-row, and its first tile may come in any of them. Inputs that tensor memory just holds, and one
-    slice more."""
+    slice more. 20000 tokens are three or four items to a CTA: rings, parities and the turn of the sets go on from one to the next."""
     rows = 192 if K > 768 else 144
     rng = np.random.default_rng(K + T)
     kept = [np.arange(K // 16) if r in full else np.sort(rng.choice(K // 16, rng.integers(0, K // 96), replace=False)) for r in range(rows)]
@@ -599,11 +603,14 @@ def test_resident_linear_with_groups_in_several_blocks(et, orc, T, K, full, gelu
     w = et.TileWeight(K, N, 32768, data, rp, ro, bias, is_gelu=gelu)
     info = w.info()
     assert info["stage_bytes"] == info["stages"] == 0, info   # the resident form
-    Y = w.run(torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda"), dev(X))
+    Y, again = (w.run(torch.full((T, N), float("nan"), dtype=torch.float16, device="cuda"), dev(X)) for _ in range(2))
     torch.cuda.synchronize()
     w.check()
-    part = slice(max(0, T - 140), T)
-    util.assert_close(host(Y)[part], orc.tile_linear(X[part], rp, ro, data, bias, N, gelu=gelu), what=f"{full} full block-rows")
+    assert torch.isfinite(Y).all() and torch.equal(Y, again)
+    # the first tokens, those on both sides of a third and two thirds of the slabs (where CTAs pass on to their next item), the last
+    for first in {0, max(0, T - 140), *([128 * 49 - 70, 128 * 99 - 70] if T > 15000 else [])}:
+        part = slice(first, first + 140)
+        util.assert_close(host(Y[part]), orc.tile_linear(X[part], rp, ro, data, bias, N, gelu=gelu), what=f"{full} full block-rows, tokens from {first}")
 
 
 def test_tile_linear_pruned_tiles_do_not_contribute(et, orc):

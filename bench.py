@@ -41,11 +41,17 @@ METRIC = "encoder sequences/sec (24-layer tile-pruned BERT-large, 256 x 512 toke
 LARGE = dict(d=1024, H=16, ff=4096, S=512, B=256, layers=24, sparsity=0.8)
 BASE = dict(d=768, H=12, ff=3072)
 LOG2E = 1.4426950408889634
-# DRAM traffic of the dominant kernel from its ncu capture (profiles/): bytes per launch divided by the
-# algorithmic bytes of that launch (activations once, packed weight once, output once). Used to scale the
-# algorithmic bytes of the bench's launches; None where no capture exists.
-NCU_TRAFFIC_RATIO = {"tile_gemm_kernel": 1.0, "source": "profiles/tile_gemm_kernel_T16384_K1024_N4096_s80.md: 35.3 MB read "
-                     "= activations + packed weight; writes = the output"}
+# DRAM bytes read per launch over the algorithmic ones (activations and packed weight once), from ncu captures of each linear kernel at 16384 tokens,
+# 80 % of the tiles pruned (1024 -> 4096: 35.3 MB of 35.2; 4096 -> 1024: 136.4 of 135.9). Used to scale the algorithmic bytes of the bench's
+# launches; None where no capture exists.
+NCU_TRAFFIC_RATIO = {"resident_kernel": 1.0, "tile_gemm_kernel": 1.0}
+
+
+def linear_kernel(info):
+    """The kernel that a packed weight runs in, from what et_tile_weight_info tells of it."""
+    if info["stage_bytes"]:
+        return "tile_gemm_kernel"
+    return "resident_kernel" if info["stages"] == 0 else "dense_kernel" if info["stages"] == 1 else "dense_split_kernel"
 
 
 def peaks():
@@ -793,7 +799,7 @@ def main():
                   "overlap on three streams over two buffer sets; wall clock, maximum over ranks"}
     del hx, ho, xin
 
-    # ---- roofline of the dominant kernel: the four tile-GEMM launches of one layer at the shard's token count,
+    # ---- roofline of the dominant kernels: the four linears of one layer at the shard's token count,
     # each timed alone with CUDA events on its stream (operands far larger than L2)
     qkv_rp = np.concatenate([lin0["q"][0], lin0["k"][0][1:] + lin0["q"][0][-1],
                              lin0["v"][0][1:] + lin0["q"][0][-1] + lin0["k"][0][-1]]).astype(np.int32)
@@ -804,25 +810,28 @@ def main():
     ybuf = torch.zeros((T, c["ff"]), dtype=torch.float16, device="cuda")
     launches = [("fused Q|K|V", wq, ybuf, x, False), ("output projection", wo, ybuf, x, False),
                 ("FFN1 + GELU", w1, ybuf, x, True), ("FFN2", w2, outs[0], hbuf, False)]
-    per, tot_ms, tot_fl, tot_bytes = [], 0.0, 0.0, 0.0
+    per, tot_ms, tot_fl, traffic, parts = [], 0.0, 0.0, 0.0, {}
     for name, w, yb, xb, gelu in launches:
         ms_l = time_loop(torch, lambda: w.run(yb, xb, gelu=gelu, stream=comp), 10, 3, comp)
         fl = 2.0 * T * 256 * w.ntile
         alg_bytes = 2.0 * T * w.in_feat + 516.0 * w.ntile + 2.0 * T * w.out_feat
-        per.append({"launch": name, "K": w.in_feat, "N": w.out_feat, "kept_tiles": w.ntile, "ms": ms_l, "tflops": fl / (ms_l * 1e-3) / 1e12,
+        kernel = linear_kernel(w.info())
+        per.append({"launch": name, "kernel": kernel, "K": w.in_feat, "N": w.out_feat, "kept_tiles": w.ntile, "ms": ms_l, "tflops": fl / (ms_l * 1e-3) / 1e12,
                     "algorithmic_bytes": alg_bytes, "packing": w.info()})
         w.check()
-        tot_ms += ms_l; tot_fl += fl; tot_bytes += alg_bytes
+        tot_ms += ms_l; tot_fl += fl
+        parts.setdefault(kernel, []).append(name)
+        ratio = NCU_TRAFFIC_RATIO.get(kernel)
+        traffic = None if traffic is None or ratio is None else traffic + ratio * alg_bytes
     achieved = tot_fl / (tot_ms * 1e-3) / 1e12
-    ratio = NCU_TRAFFIC_RATIO.get("tile_gemm_kernel")
-    roofline = {"kernel": "tile_gemm_kernel (the 4 launches of a layer: fused Q|K|V, output, FFN1+GELU, FFN2)", "bound": "tensor",
+    roofline = {"kernel": "; ".join(f"{k} ({', '.join(v)})" for k, v in parts.items()) + ": the 4 linears of a layer", "bound": "tensor",
                 "achieved": achieved, "peak": pk["tflops"], "unit": "TFLOP/s", "frac": achieved / pk["tflops"],
                 "peak_source": pk["source"] + " (bf16 burst; each launch is timed alone)",
                 "frac_of_sustained_peak": achieved / pk["tflops_sustained"] if pk.get("tflops_sustained") else None,
                 "flops_per_launch_set": tot_fl, "ms_per_launch_set": tot_ms, "launches": per, "tokens": T,
-                "traffic": None if ratio is None else ratio * tot_bytes,
-                "traffic_note": "DRAM bytes per launch set: algorithmic bytes of these launches times the measured/algorithmic ratio "
-                                "of the ncu capture of the same kernel on a smaller case (" + NCU_TRAFFIC_RATIO["source"] + ")",
+                "traffic": traffic,
+                "traffic_note": "DRAM bytes per launch set: algorithmic bytes of each launch times the measured/algorithmic ratio of bytes read "
+                                "in an ncu capture of its kernel on a smaller case (16384 tokens, 80 % pruned: 1.00 for both kernels)",
                 "dense_equivalent_tflops": achieved / max(1e-9, 1.0 - c["sparsity"]),
                 "note": "algorithmic FLOPs count kept tiles only (2 * tokens * 256 * kept tiles)"}
     # the attention kernel alone at the same shape (tensor bound)
@@ -855,8 +864,8 @@ def main():
               "launches_per_step": (f"{5 * c['layers'] + 1}: per layer fused Q|K|V tile GEMM, attention, output tile GEMM (+ residual, row sums), "
                                     "FFN1 tile GEMM (normalises its input, GELU), FFN2 tile GEMM (+ LayerNorm of the residual, row sums); one "
                                     "LayerNorm at the end; all replayed as one CUDA graph") if fused else
-                                   (f"{7 * c['layers']}: per layer fused Q|K|V tile GEMM, attention, output tile GEMM, LayerNorm, FFN1 tile "
-                                    "GEMM (GELU), FFN2 tile GEMM, LayerNorm; all layers replayed as one CUDA graph"),
+                                   (f"{7 * c['layers']}: per layer fused Q|K|V linear, attention, output linear, LayerNorm, FFN1 linear "
+                                    "(GELU), FFN2 linear, LayerNorm; all layers replayed as one CUDA graph"),
               "layernorm_folded_into_linears": fused,
               "roofline": roofline, "roofline_attention": roofline_attention,
               "model_tflops": layer_fl * c["layers"] * world / (ms * 1e-3) / 1e12, "gather_check": gather_check,

@@ -1,5 +1,6 @@
 """The benchmark's contract on a machine without a GPU: the reference arm falls back to the CPU oracle and still
 prints one JSON line with the agreed keys; the native arm refuses to run (no CPU fallback in the product)."""
+import importlib.util
 import json
 import os
 import subprocess
@@ -37,3 +38,11 @@ def test_native_arm_has_no_cpu_fallback():
                        capture_output=True, text=True, timeout=600, cwd=ROOT)
     assert r.returncode != 0
     assert "no CPU fallback" in (r.stderr + r.stdout)
+
+
+@pytest.mark.parametrize("stages,stage_bytes,kernel", [(3, 26624, "tile_gemm_kernel"), (0, 0, "resident_kernel"), (1, 0, "dense_kernel"), (4, 0, "dense_split_kernel")])
+def test_roofline_names_the_kernel_that_a_weight_runs_in(stages, stage_bytes, kernel):
+    spec = importlib.util.spec_from_file_location("bench", os.path.join(ROOT, "bench.py"))
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    assert bench.linear_kernel({"stages": stages, "stage_bytes": stage_bytes}) == kernel

@@ -930,13 +930,15 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5; but 4096 x 1024 -> 4096 at 40 % 30.7 and 27.9. Long launches need no such
     // margin: those of a weight with every tile, whose epilogue does not look for results to be computed again (4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024
     // 14.6 and 11.7), and beyond 60000 clocks all, where the tile kernel comes to the power limit, which its model does not know (32768 x 1024 -> 4096 at 40 %
-    // 229 and 188 us, 65536 x 4096 -> 1024 414 and 354). The dense and the resident form are taken as their models say. When the resident form had to promise 15 %, 24
-    // of 1190 linears (0 to 80 % pruned, 64 to 65536 tokens, in_feat 768 and 1024) stayed dense that are 1 to 28 % faster resident: 8192 x 768 -> 3072 at 40 %
-    // 35.5 and 27.8 us, 8192 x 768 -> 1152 at 50 % 15.8 and 13.0.)
+    // 229 and 188 us, 65536 x 4096 -> 1024 414 and 354). To the resident form it gives way for 10 %: of slabs that come from memory the resident model says too
+    // little (resident over dense, by the models and measured: 32768 x 768 -> 3072 at 25 % 1.00 and 1.16, 65536 x 768 -> 2304 0.97 and 1.13, 65536 x 768 -> 3072 0.93 and
+    // 1.12; at 40 % 32768 x 768 -> 3072 0.87 and 0.92); of slabs in L2 it says too much (8192 x 768 -> 3072 at 40 % 0.89 and 0.83, but 4096 x 768 -> 2304 at 50 %
+    // 0.97 and 0.86): there the line could lie higher, but these weights have always been dense and stay so. With 15 % 8192 x 768 -> 3072 at 40 %
+    // took 32.0 us (26.7 resident), 8192 x 768 -> 1152 at 50 % 15.0 (12.2).)
     const bool every_tile = ntile == (long)NBR * (K / 16);
     const double dense = w->dense.cost;
     const double dense_cost = dense > (every_tile ? 16000.0 : 60000.0) ? dense : 1.05 * dense + (dense > 30000.0 ? 0.0 : 1300.0);
-    w->packed_dense = plain && dense_cost < tile_cost && dense < resident;
+    w->packed_dense = plain && dense_cost < tile_cost && 0.9 * dense < resident;
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);

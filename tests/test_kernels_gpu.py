@@ -370,8 +370,8 @@ def test_dense_linear_split_over_a_cluster(et, orc, T, K, N, sparsity, gelu, sha
                                                  (8192, 768, 3072, 0.4, "resident"), (8192, 768, 1152, 0.5, "resident"), (17771, 768, 1152, 0.4, "resident"),
                                                  (4096, 768, 2304, 0.25, "dense"), (32768, 1024, 4096, 0.4, "dense"), (65536, 4096, 1024, 0.4, "dense"),
                                                  (65536, 1536, 1536, 0.4, "dense"), (65536, 1024, 512, 0.8, "tile"), (65536, 1024, 512, 0.9, "tile"),
-                                                 (65536, 1024, 1536, 0.9, "resident"), (12000, 1024, 1536, 0.95, "resident"), (4096, 768, 3072, 0.4, "resident"),
-                                                 (4096, 1024, 4096, 0.4, "dense")])
+                                                 (65536, 1024, 1536, 0.9, "resident"), (12000, 1024, 1536, 0.95, "resident"), (32768, 768, 3072, 0.25, "dense"),
+                                                 (4096, 1024, 4096, 0.4, "dense"), (65536, 768, 2304, 0.25, "dense"), (65536, 768, 3072, 0.25, "dense"), (32768, 768, 3072, 0.4, "resident")])
 def test_the_form_that_was_measured_as_the_fastest_is_taken(et, orc, T, K, N, sparsity, form):
     """Where another form takes at least 5 % longer."""
     rp, ro, data, bias = util.make_tile_linear(orc, K, N, sparsity, K + N, False, 0.05)
@@ -465,8 +465,8 @@ def test_dense_shares_meet_at_every_width(et, orc, T, K, N, gelu, columns):
 @pytest.mark.parametrize("T,K,N,sparsity,gelu,size,form", [
     (200, 3072, 768, 0.75, False, 128, "dense"),         # K split over a cluster
     (200, 3072, 784, 0.75, True, 128, "dense"),
-    (700, 768, 2304, 0.25, False, 4096, "dense"),        # pairs of CTAs (14.7 us for 4096 tokens, resident 16.0, tile 16.7)
-    (700, 768, 2320, 0.25, True, 4096, "dense"),
+    (700, 768, 2304, 0.5, False, 4096, "dense"),         # pairs of CTAs
+    (700, 768, 2320, 0.5, True, 4096, "dense"),
     (300, 768, 2304, 0.98, False, 32768, "resident"),    # block-rows without tiles among them
     (300, 1024, 1040, 0.9, True, 32768, "resident"),
     (300, 3072, 768, 0.9, False, 17792, "tile"),

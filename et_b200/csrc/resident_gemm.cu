@@ -2,7 +2,7 @@
 // slab of 128 tokens stays in tensor memory, whole, while the weight streams past it.
 // Replaces, for those sizes, kernels/linear.cu:54-167 of the reference.
 //
-// Why: with A in tensor memory a kept tile is one UMMA 128x16x16 of ~9 clocks (four issuing warps), but bringing A there is
+// Why: with A in tensor memory a kept tile is one UMMA 128x16x16 of ~9 clocks (eight issuing warps, or six), but bringing A there is
 // dear: tcgen05.cp moves 64 bytes per clock and takes turns with the UMMAs on the tensor pipe (measured: 2048 UMMAs and 256
 // copies of 4 KB take the sum of their times). The tile kernel (tile_gemm.cu) keeps 384 accumulator columns and streams A
 // through the other 128 once per 384 output features: 512 clocks of copying per 128 x 128 chunk against ~350 of UMMAs at
@@ -82,7 +82,7 @@ struct ResidentParams {
 template <typename F>
 struct ResidentShared {
     uint64_t x_full[kMaxRing], x_empty[kMaxRing];   // chunk slots: landed / copied on to tensor memory
-    uint64_t w_full[F::kSets][kSlots], w_empty[F::kSets][kSlots];   // weight blocks: landed / their UMMAs have completed (4 commits)
+    uint64_t w_full[F::kSets][kSlots], w_empty[F::kSets][kSlots];   // weight blocks: landed / their UMMAs have completed (a commit of each issuing warp)
     uint64_t a_ready[F::kMaxChunks];                   // per chunk, once per item: in place for the UMMAs
     uint64_t a_free, tail_free;                     // the item's UMMAs have completed: its activations in tensor memory, in shared memory may be overwritten
     uint64_t acc_full[F::kSets], acc_empty[F::kSets];
@@ -208,15 +208,14 @@ __global__ void __launch_bounds__(F::kThreads, 1) resident_kernel(const __grid_c
         const int slices = min(p.K / 16, F::kSlices);
         bool ok = true;
         if (elect_one()) {
-        int xs = 0, n = 0;
-        uint32_t ph = 0;
-        for (int item = blockIdx.x; item < p.items && ok; item += G, ++n) {
-            if (n > 0) ok = mbar_wait(&sh->a_free, (uint32_t)(n - 1) & 1u);
-            for (int c = 0; c < tchunks && ok; ++c) {
-                ok = mbar_wait_at(full0 + xs * 8, ph);
-                if (!ok) break;
-                tc_fence_after();
-                {
+            int xs = 0, n = 0;
+            uint32_t ph = 0;
+            for (int item = blockIdx.x; item < p.items && ok; item += G, ++n) {
+                if (n > 0) ok = mbar_wait(&sh->a_free, (uint32_t)(n - 1) & 1u);
+                for (int c = 0; c < tchunks && ok; ++c) {
+                    ok = mbar_wait_at(full0 + xs * 8, ph);
+                    if (!ok) break;
+                    tc_fence_after();
                     const uint64_t xd = x_desc0 + (uint32_t)xs * (kChunkBytes >> 4);
                     const uint32_t ta = tmem + c * F::kChunkSlices * 8;
                     if (slices - c * F::kChunkSlices >= F::kChunkSlices) {
@@ -227,11 +226,13 @@ __global__ void __launch_bounds__(F::kThreads, 1) resident_kernel(const __grid_c
                     }
                     umma_commit_at(ready0 + c * 8);
                     umma_commit_at(empty0 + xs * 8);
+                    if (++xs == p.nx) { xs = 0; ph ^= 1u; }
                 }
-                if (++xs == p.nx) { xs = 0; ph ^= 1u; }
             }
-        }
-        if (!ok) { if (!sh->abort) atomicExch(p.err, 43); sh->abort = 1; }
+            if (!ok) {
+                if (!sh->abort) atomicExch(p.err, 43);
+                sh->abort = 1;
+            }
         }
         __syncwarp();
     } else if (warp >= F::kFirstIssuer && warp < F::kFirstEpi) {
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(F::kThreads, 1) resident_kernel(const __grid_c
 struct ResidentWeight {
     int K = 0, N = 0, groups = 0, block_bytes = 0, nx = 0;
     bool wide = false;
-    double group_clocks = 0;   // modelled, per group of 64 features and slab
+    double group_clocks = 0;   // modelled, per group of features and slab
     uint2* d_dir = nullptr;
     uint8_t* d_stream = nullptr;
     const uint8_t* d_empty = nullptr;   // behind the stream

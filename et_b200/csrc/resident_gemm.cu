@@ -455,9 +455,9 @@ static double group_clocks(int K, double density) {
     const double ts = kRows * density * std::min(K / 16, F::kSlices), ss = kRows * density * std::max(0, K / 16 - F::kSlices);
     return narrow ? std::max(420.0, 274.0 + 10.5 * ts) : std::max(530.0, 164.0 + 10.0 * ts + 64.0 * ss);
 }
-static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges, double more = 0.0) {
+static double launch_clocks(int slabs, int groups, int K, double per_group, int* ranges) {
     double best = 0;
-    const double start = ((K + 127) / 128) * 350.0 + 4400.0 + more;   // copying a slab into place, per item
+    const double start = ((K + 127) / 128) * 350.0 + 4400.0;   // copying a slab into place, per item
     const int sms = sm_count();
     // Of the numbers of ranges with as many groups in the largest only the first can be the best (this runs at every launch: 128 groups all tried 0.61 us, 0.22 now).
     for (int r = 1;;) {
@@ -475,13 +475,13 @@ double resident_cost(int tokens, int N, int K, double density) {
     if (K > kMaxK) return 1e30;
     int r = 1;
     const int slabs = std::max(1, (tokens + kSlab - 1) / kSlab), groups = (N / 16 + kRows - 1) / kRows;
-    const bool in_l2 = 2.0 * tokens * (K + N) <= 95e6;   // a launch's operands, beside the next one's
-    // Slabs that come from memory take longer with the ring of single panels, which covers L2's latency (65536 x 1024 -> 512 at 75 / 90 % resident 53 / 45 us, tile
-    // 43 / 38; two panels to a chunk fit as well without it: 65536 x 768 -> 1152 at 40 % 91, dense 100). Launches of many slabs from L2 are overestimated
-    // by 3 to 20 %, more than the other forms' by their models (12000 x 1024 -> 1536 at 95 % 15.7, tile 18.9; 4096 x 768 -> 3072 at 40 % 17.1, dense 20.5).
-    const double clocks = is_wide(K) ? launch_clocks(slabs, groups, K, group_clocks<Wide>(K, density), &r, in_l2 ? 0.0 : 2.0 * K)
-                                     : launch_clocks(slabs, groups, K, group_clocks<Narrow>(K, density), &r);
-    return in_l2 && tokens >= 2048 ? 0.96 * clocks : clocks;
+    const bool wide = is_wide(K);
+    double clocks = launch_clocks(slabs, groups, K, wide ? group_clocks<Wide>(K, density) : group_clocks<Narrow>(K, density), &r);
+    // Measured / modelled from L2 and from memory (means over in_feat 768 and 1024): 0.94 and 1.20. With a quarter of the tiles or less 0.85 from L2 (and 0.95 in the tile form). A slab from memory takes
+    // longer with the ring of single panels, which covers L2's latency (65536 x 1024 -> 512 at 90 % 47 us, tile 40; 65536 x 1024 -> 1024 62 and 70).
+    const double far = beyond_l2(tokens, K, N);
+    if (tokens >= 2048 && density <= 0.3) clocks *= 0.93 + 0.07 * far;
+    return wide ? (1.0 + 0.12 * far) * clocks + (slabs + sm_count() - 1) / sm_count() * 3000.0 * far : (1.0 + 0.1 * far) * clocks;
 }
 
 template <typename F>

@@ -8,6 +8,14 @@ namespace et {
 
 struct ResidentWeight;
 
+// How far a launch's activations and results exceed what L2 holds of them beside the next launch's: 0 up to 60 MB, 1 from 140 MB. In between
+// the tile and resident forms go from 0.93 to 1.2 times what their models say (the power limit comes to long launches as well), the dense form from 1.01 to 1.03. (Of short K
+// ranges the dense form's model knows as little: 47112 x 512 -> 1024 52 us, 38 by the model.)
+inline double beyond_l2(double tokens, int K, int N) {
+    if (K < 640) return 0.0;
+    const double mb = 2e-6 * tokens * (K + N);
+    return mb <= 60.0 ? 0.0 : mb >= 140.0 ? 1.0 : (mb - 60.0) / 80.0;
+}
 // Modelled clocks of a launch; 1e30 where the form does not exist (in_feat above 1024).
 double resident_cost(int tokens, int N, int K, double density);
 // Packs a validated weight (tile-BSR arrays as in tile_weight_pack; no tile twice in a block-row).

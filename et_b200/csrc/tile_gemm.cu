@@ -918,28 +918,25 @@ int tile_weight_pack(TileWeight** out, int K, int N, int size_hint, long ntile, 
     }
     w->dense = dense_plan(size_hint, N, K);
     // The form whose model promises the shortest launch. The models are fitted to measured launches (the tile kernel's counts in units of
-    // 1.28 clocks). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 82, 1024 -> 3072 96 / 90 / 128, 1024 ->
-    // 4096 148 / 118 / 171; at 50 % 1024 -> 4096 186 / 189 / 181. Over 2106 linears (1 to 65536 tokens, thirteen shapes, 0 to 95 %
-    // pruned) the form taken is 0.38 % slower than the fastest of the three in the mean, 47 are more than 5 % off, 14 more than 10 % (eleven of
-    // them one token); the constants of the tile and resident models were fitted together with the number of block-rows over 456 (128 to 65536 tokens).
-    tile_cost = 1.28 * tile_cost + 50.0;
+    // 1.28 clocks, 15 % more from memory). At 75 % sparsity and 32768 tokens, in us, tile / resident / dense: 768 -> 2304 64 / 49 / 82, 1024 -> 3072 96 / 90 / 128, 1024 ->
+    // 4096 148 / 118 / 171; at 40 % 1024 -> 4096 276 / 295 / 185. Over 3472 linears (64 to 65536 tokens, twenty shapes, 0 to 90 % pruned, the forms
+    // measured in turn) the form taken is 0.78 % slower than the fastest in the mean, 91 are more than 10 % off (without the difference between L2 and memory
+    // 1.29 % and 166); the constants of the tile and resident models were fitted together with the number of block-rows over 456 linears.
+    tile_cost = (1.28 * tile_cost + 50.0) * (1.0 + 0.15 * beyond_l2(size_hint, K, N));
     const double resident = resident_cost(size_hint, N, K, density);
     // Packed for SM time, the tile form stays: its few large tiles leave SMs to other batches (six in flight, 16 x 128 tokens
     // at 75 %: 29 us a batch; with the forms of the shortest launch 45).
     const bool plain = nb_override <= 0 && g_goal == 0 && !repeats_a_tile(row_ptr, row_offset, NBR);
-    // (The dense form, which may sum in another order, is taken over the tile form only where its model promises 5 % and, of short launches, 1300 clocks: 300 x 1024 ->
-    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5; but 4096 x 1024 -> 4096 at 40 % 30.7 and 27.9. Long launches need no such
-    // margin: those of a weight with every tile, whose epilogue does not look for results to be computed again (4096 x 768 -> 768 8.9 and 9.2, 4096 x 1024 -> 1024
-    // 14.6 and 11.7), and beyond 60000 clocks all, where the tile kernel comes to the power limit, which its model does not know (32768 x 1024 -> 4096 at 40 %
-    // 229 and 188 us, 65536 x 4096 -> 1024 414 and 354). To the resident form it gives way for 10 %: of slabs that come from memory the resident model says too
-    // little (resident over dense, by the models and measured: 32768 x 768 -> 3072 at 25 % 1.00 and 1.16, 65536 x 768 -> 2304 0.97 and 1.13, 65536 x 768 -> 3072 0.93 and
-    // 1.12; at 40 % 32768 x 768 -> 3072 0.87 and 0.92); of slabs in L2 it says too much (8192 x 768 -> 3072 at 40 % 0.89 and 0.83, but 4096 x 768 -> 2304 at 50 %
-    // 0.97 and 0.86): there the line could lie higher, but these weights have always been dense and stay so. With 15 % 8192 x 768 -> 3072 at 40 %
-    // took 32.0 us (26.7 resident), 8192 x 768 -> 1152 at 50 % 15.0 (12.2).)
+    // (The dense form, which may sum in another order, is taken over the tile form only where its model promises 5 % and 1300 clocks: 300 x 1024 ->
+    // 1024 at 75 % tile 5.6, dense 5.9 us, 1100 x 768 -> 768 with every tile 5.5 and 6.5. (Without the 1300 beyond 30000 clocks 6502 x 4096 -> 1024 at 75 % went from 32 to
+    // 44 us.) A long launch of a weight with every tile needs no such margin, its epilogue does not look for results to be computed again: 4096 x 768 -> 768 8.9 and
+    // 9.2, 4096 x 1024 -> 1024 14.6 and 11.7. Dense and resident are taken as their models say, except that short dense launches give way for 6 %: those from
+    // 0.94 to 1 are 0 to 18 % faster resident (4096 x 768 -> 2320 at 50 % 15.3 and 12.7 us), but have been dense all along and stay so. 15 % at every length cost
+    // 17771 x 768 -> 1152 at 40 % 6 of 27 us, 6502 x 768 -> 2304 at 65 % 6 of 22.)
     const bool every_tile = ntile == (long)NBR * (K / 16);
     const double dense = w->dense.cost;
-    const double dense_cost = dense > (every_tile ? 16000.0 : 60000.0) ? dense : 1.05 * dense + (dense > 30000.0 ? 0.0 : 1300.0);
-    w->packed_dense = plain && dense_cost < tile_cost && 0.9 * dense < resident;
+    const double dense_cost = every_tile && dense > 16000.0 ? dense : 1.05 * dense + 1300.0;
+    w->packed_dense = plain && dense_cost < tile_cost && (dense < 30000.0 ? 0.94 : 1.0) * dense < resident;
     int rc = w->packed_dense ? build_dense_form(w)
              : plain && resident < tile_cost ? resident_pack(&w->resident, K, N, w->h_data.data(), row_ptr, row_offset)
                                              : build_tile_form(w);

@@ -397,8 +397,9 @@ def test_the_form_that_was_measured_as_the_fastest_is_taken(et, orc, T, K, N, sp
 @pytest.mark.parametrize("T,K,N,sparsity,form", [
     (8192, 768, 3072, 0.4, "resident"), (8192, 768, 1152, 0.5, "resident"), (17771, 768, 1152, 0.4, "resident"), (4096, 768, 2304, 0.25, "dense"),
     (32768, 768, 3072, 0.25, "dense"), (65536, 768, 2304, 0.25, "dense"), (65536, 768, 3072, 0.25, "dense"), (32768, 768, 3072, 0.4, "resident"),
-    (32768, 1024, 4096, 0.4, "dense"), (65536, 4096, 1024, 0.4, "dense"), (65536, 1536, 1536, 0.4, "dense"), (4096, 1024, 4096, 0.4, "dense"),
-    (65536, 1024, 512, 0.8, "tile"), (65536, 1024, 512, 0.9, "tile"), (65536, 1024, 1536, 0.9, "resident"), (12000, 1024, 1536, 0.95, "resident"),
+    (32768, 1024, 4096, 0.4, "dense"), (65536, 4096, 1024, 0.4, "dense"), (65536, 1536, 1536, 0.4, "dense"), (6502, 4096, 1024, 0.75, "tile"),
+    (65536, 1024, 512, 0.9, "tile"), (65536, 1024, 1024, 0.9, "resident"), (32768, 1024, 3072, 0.75, "resident"), (2299, 768, 768, 0.0, "tile"),
+    (9195, 768, 192, 0.0, "tile"), (12000, 1024, 1536, 0.95, "resident"), (12000, 768, 1536, 0.9, "resident"),
 ])
 def test_the_form_is_the_fastest_where_the_models_had_gone_wrong(et, orc, T, K, N, sparsity, form):
     """Where another form takes at least 5 % longer: long dense launches, which come to the power limit in the tile form, slabs that come from memory, many
